@@ -38,6 +38,7 @@
 #include "../../include/avbd.h"
 #include "dmath.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace avbd {
 
@@ -179,6 +180,42 @@ __device__ __forceinline__ void ld16(uint32_t taddr, float (&v)[16]) {
 }
 }  // namespace tc
 
+// eight consecutive floats, 16-byte loads where the address allows them
+__device__ __forceinline__ void load8(const float* p, bool vec, float (&v)[8]) {
+    if (vec) {
+        const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[e] = p[e];
+    }
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+    return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+}
+// position of the k-th bias (b1 | b2 | b3 | b4) in the parameter block
+__device__ __forceinline__ uint32_t bias_at(uint32_t k) {
+    using namespace mlp;
+    return k < 128u ? OB1 + k : (k < 256u ? OB2 + k - 128u : (k < 384u ? OB3 + k - 256u : OB4 + k - 384u));
+}
+// fp32 weights -> the BF16 weight image at the head of shared memory, eight
+// columns of a row at a time
+__device__ __forceinline__ void stage_weights(const float* prm, bool vec, unsigned char* sm, uint32_t t,
+                                              uint32_t threads) {
+    using namespace mlp;
+    for (uint32_t g = t; g < NHALF / 8; g += threads) {
+        uint32_t src, base, cols, sbo, j = 8 * g;
+        if (j < HW2) { src = OW1; base = tc::W1; cols = DIN; sbo = tc::SBO_K32; }
+        else if (j < HW3) { j -= HW2; src = OW2; base = tc::W2; cols = HID; sbo = tc::SBO_K128; }
+        else if (j < HW4) { j -= HW3; src = OW3; base = tc::W3; cols = HID; sbo = tc::SBO_K128; }
+        else { j -= HW4; src = OW4; base = tc::W4; cols = HID; sbo = tc::SBO_K128; }
+        float v[8];
+        load8(prm + src + j, vec, v);
+        *reinterpret_cast<uint4*>(sm + base + tc::off(j / cols, j % cols, sbo)) = pack8(v);
+    }
+}
+
 __global__ void __launch_bounds__(128) k_mlp_infer_tc(const bf16* __restrict__ W, const float* __restrict__ prm,
                                                       const float* __restrict__ norm, const float* __restrict__ X,
                                                       uint32_t n, float* __restrict__ Y, uint32_t* status,
@@ -310,256 +347,427 @@ __global__ void __launch_bounds__(128) k_mlp_infer_tc(const bf16* __restrict__ W
 }
 
 // ---------------------------------------------------------------------------
-// Training GEMM on the tensor cores: C[M][N] (fp32) = op(A) op(B), BF16
-// operands, FP32 accumulation in TMEM.  A is [M][K] (lda = K) or, with TA,
-// stored [K][M]; B is [N][K] or, with TB, stored [K][N].  A CTA of four warps
-// owns a 128-row x BN-column tile (BN = N rounded up to 16, at most 128;
-// rows past M are zero): K runs in chunks of 64 through two shared-memory
-// stages in the UMMA canonical K-major layout (row-group stride 1024 B),
-// staged by all threads (transposing on the fly) while the previous chunk's
-// four M = 128, K = 16 tcgen05.mma instructions run; each stage is reused
-// only after the tcgen05.commit of its MMAs has arrived on its mbarrier.
-// Every wait is bounded (one second); a timeout sets *status and the CTA
-// frees its TMEM and stops.  Split-K writes one partial per z-slice
-// (reduced in a fixed order by k_split_sum).
+// Training step on the tensor cores, two launches.
+//
+// k_train_tile: a CTA of eight warps takes 128-row tiles of the batch (tile
+// blockIdx.x, + gridDim.x, ...) through the whole forward and backward pass
+// without leaving the SM.  The BF16 weights, the tile's inputs and the three
+// hidden activations stay in shared memory in the canonical K-major layout
+// [row][column]; the same image serves both roles an operand has:
+//   forward      Z_l  = H_{l-1} W_l^T    A, B K-major
+//   input grads  G_l  = dH_{l+1} W_{l+1} A K-major, B = W MN-major (N = in)
+//   weight grads dW_l = dH_l^T H_{l-1}   A, B MN-major (K = the tile's rows)
+// (MN-major core matrices are the same 8 x 16-byte blocks: the stride over
+// 8-row groups becomes the K stride.)  dW_4 is formed transposed, H_3^T dY,
+// because M is 128.  The four weight gradients accumulate in their own TMEM
+// columns over all tiles of the CTA; layer outputs and input gradients share
+// 128 columns.  The weight-gradient MMAs are issued after the commit that the
+// next epilogue waits for, so they run beside it; dH_3 goes to a spare tile
+// and dH_2, dH_1 to the tiles of H_3 and H_2, whose last readers an earlier
+// commit has covered.  Two threads share a row (64 columns each).
+//
+// Bias gradients are fp32 column sums of the unrounded dH: a warp folds its
+// 32 rows by a shuffle exchange (lane j ends with column j), the warps of a
+// column half are added in order at the end.
+//
+// k_train_reduce adds the CTAs' partial gradients in CTA order, and either
+// stores the gradient or applies Adam.
+//
+// What bounds it: at the trainer's 8,192 rows a tile is a chain of eight
+// dependent products with their epilogues (2.7 GFLOP in all), so latency, not
+// the tensor pipe; one row tile per CTA keeps 64 SMs busy with one pass over
+// the batch: 28.7 us a step at 8,192 rows, launches included (1,005 us as ~35
+// launches with the activations in global memory and one thread per bias
+// column, whose four serial sums over the rows were most of it).
 // ---------------------------------------------------------------------------
-namespace tg {
-constexpr uint32_t BK = 64, SBO = (BK / 8) * 128;          // chunk of K; row-group stride (1024 B)
-constexpr uint32_t STAGE = 128 * BK * 2;                    // one operand tile (16 KiB)
-constexpr uint32_t A0 = 0, B0 = A0 + 2 * STAGE, BAR = B0 + 2 * STAGE, TSLOT = BAR + 16, SMEM = TSLOT + 16;
-constexpr uint32_t TMEM_COLS = 128;
-}  // namespace tg
+namespace tt {
+constexpr uint32_t THREADS = 256;
+constexpr uint32_t SBO128 = 2048, SBO32 = 512, SBO16 = 256;   // row-group strides of 128-, 32-, 16-column images
+constexpr uint32_t X = tc::WBYTES, H1 = X + 128 * 32 * 2, H2 = H1 + 128 * 128 * 2, H3 = H2 + 128 * 128 * 2,
+                   SP = H3 + 128 * 128 * 2, DY = SP + 128 * 128 * 2, BIAS = DY + 128 * 16 * 2,
+                   NORM = BIAS + (3 * 128 + 16) * 4, RED = NORM + 96 * 4, BAR = RED + 8 * 64 * 4, TSLOT = BAR + 8,
+                   SMEM = TSLOT + 8;
+static_assert(SMEM <= 227 * 1024, "shared memory of a training CTA");
+// TMEM columns: D (layer outputs, input gradients) | dW3 | dW2 | dW1 | dW4^T
+constexpr uint32_t TD = 0, TW3 = 128, TW2 = 256, TW1 = 384, TW4 = 416, TMEM_COLS = 512;
+// a CTA's partial gradient (floats): dW3, dW2, dW1 as [in][out], dW4 as
+// [out][in], the biases, the loss; the lane of every TMEM row is contiguous
+constexpr uint32_t P3 = 0, P2 = P3 + 128 * 128, P1 = P2 + 128 * 128, P4 = P1 + 32 * 128, PB1 = P4 + 16 * 128,
+                   PB2 = PB1 + 128, PB3 = PB2 + 128, PB4 = PB3 + 128, PL = PB4 + 16, PART = PL + 16;
 
-// one 8-element K group of row r of an operand tile: 16 bytes in the
-// canonical layout; T: the operand is stored transposed ([K][rows], ld = rows)
-template <bool T>
-__device__ __forceinline__ uint4 stage_group(const bf16* __restrict__ X, uint32_t rows, uint32_t K, uint32_t row,
-                                             uint32_t k, uint32_t kEnd) {
-    uint32_t w[4];
-    if (!T && row < rows && k + 8 <= kEnd && (K & 7u) == 0u)
-        return *reinterpret_cast<const uint4*>(X + (size_t)row * K + k);
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const uint32_t k0 = k + 2 * e, k1 = k0 + 1;
-        bf16 lo = __float2bfloat16(0.0f), hi = __float2bfloat16(0.0f);
-        if (row < rows && k0 < kEnd) lo = T ? X[(size_t)k0 * rows + row] : X[(size_t)row * K + k0];
-        if (row < rows && k1 < kEnd) hi = T ? X[(size_t)k1 * rows + row] : X[(size_t)row * K + k1];
-        w[e] = (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
-    }
-    return make_uint4(w[0], w[1], w[2], w[3]);
+// K-major descriptor (second 8-column K chunk 128 B on) and MN-major one of
+// the same image: 8-column groups 128 B apart, 8-row (K) groups `sbo` apart
+__device__ __forceinline__ uint64_t kmajor(uint32_t saddr, uint32_t sbo) { return tc::desc(saddr, sbo); }
+__device__ __forceinline__ uint64_t mnmajor(uint32_t saddr, uint32_t sbo) {
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(sbo >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) |
+           (1ull << 46);
 }
+constexpr uint32_t MN_A = 1u << 15, MN_B = 1u << 16;          // instruction descriptor: operand is MN-major
 
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, const bf16* __restrict__ B,
-                                                 float* __restrict__ C, uint32_t M, uint32_t N, uint32_t K,
-                                                 uint32_t kPerSplit, uint32_t bn, uint32_t* status) {
-    extern __shared__ __align__(1024) unsigned char sm[];
-    const uint32_t t = threadIdx.x, warp = t >> 5;
+// v[c] of 32 lanes -> lane j returns the sum of v[j] over the warp
+__device__ __forceinline__ float column_sums(float (&v)[32], uint32_t lane) {
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        const bool up = (lane & (uint32_t)o) != 0u;
+#pragma unroll
+        for (int j = 0; j < o; j++) {
+            const float give = up ? v[j] : v[j + o], keep = up ? v[j + o] : v[j];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return v[0];
+}
+}  // namespace tt
+
+__global__ void __launch_bounds__(tt::THREADS, 1)
+k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, const float* __restrict__ Xg,
+             const float* __restrict__ Tg, uint32_t n, float* __restrict__ part, uint32_t* status) {
+    using namespace mlp;
+    extern __shared__ __align__(128) unsigned char sm[];
+    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31u;
+    const uint32_t row = t & 127u, half = t >> 7;             // tile row and column half of this thread
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
-    const uint32_t m0 = blockIdx.y * 128u, n0 = blockIdx.x * bn;
-    const uint32_t kBeg = blockIdx.z * kPerSplit, kEnd = min(K, kBeg + kPerSplit);
+    const uint32_t bar = sbase + tt::BAR;
+    float* sbias = reinterpret_cast<float*>(sm + tt::BIAS);
+    float* snorm = reinterpret_cast<float*>(sm + tt::NORM);
     if (t == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbase + tg::BAR) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbase + tg::BAR + 8) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + tg::TSLOT),
-                     "r"(tg::TMEM_COLS)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + tt::TSLOT),
+                     "r"(tt::TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // the weights as BF16 images, biases and normalisation block
+    const bool vecX = (reinterpret_cast<uintptr_t>(Xg) & 15u) == 0u;
+    stage_weights(prm, (reinterpret_cast<uintptr_t>(prm) & 15u) == 0u, sm, t, tt::THREADS);
+    for (uint32_t i = t; i < 3 * HID + DOUT; i += tt::THREADS) sbias[i] = prm[bias_at(i)];
+    if (t < 96) snorm[t] = norm[t];
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + tg::TSLOT);
-    const uint32_t id = tc::idesc(128, bn);
-    const uint32_t chunks = kEnd > kBeg ? (kEnd - kBeg + tg::BK - 1) / tg::BK : 0u;
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + tt::TSLOT);
+    const uint32_t lane_addr = tmem + (((warp & 3u) * 32u) << 16);  // this warp's 32 TMEM lanes
+    uint32_t phase = 0;
     bool ok = true;
-    for (uint32_t c = 0; c < chunks && ok; c++) {
-        const uint32_t buf = c & 1u, bar = sbase + tg::BAR + 8u * buf;
-        if (c >= 2) {
-            // the MMAs that last read this stage have completed (block-uniform)
-            ok = __syncthreads_and(tc::wait(bar, ((c >> 1) - 1u) & 1u) ? 1 : 0) != 0;
-            if (!ok) break;
-        }
-        const uint32_t k0 = kBeg + c * tg::BK;
-        unsigned char* sa = sm + tg::A0 + buf * tg::STAGE;
-        unsigned char* sb = sm + tg::B0 + buf * tg::STAGE;
-        // thread t stages row t of the A tile and (t < bn) row t of the B tile
-#pragma unroll 2
-        for (uint32_t kg = 0; kg < tg::BK / 8; kg++) {
-            *reinterpret_cast<uint4*>(sa + tc::off(t, kg * 8, tg::SBO)) =
-                stage_group<TA>(A, M, K, m0 + t, k0 + kg * 8, kEnd);
-            if (t < bn)
-                *reinterpret_cast<uint4*>(sb + tc::off(t, kg * 8, tg::SBO)) =
-                    stage_group<TB>(B, N, K, n0 + t, k0 + kg * 8, kEnd);
-        }
-        tc::fence_proxy();               // generic-proxy writes, read by the tensor core
+    // block-uniform outcome of the bounded wait for the last commit
+    auto wait_mma = [&]() {
+        ok = __syncthreads_and(tc::wait(bar, phase) ? 1 : 0) != 0;
+        phase ^= 1u;
+        tc::fence_after();
+        return ok;
+    };
+    // shared-memory writes and TMEM reads of every thread are done
+    auto publish = [&]() {
+        tc::fence_proxy();
         tc::fence_before();
         __syncthreads();
         tc::fence_after();
+    };
+    // bias + ReLU + BF16 of this thread's 64 columns of D into the image at `dst`
+    auto activate = [&](const float* bias, uint32_t dst) {
+#pragma unroll
+        for (uint32_t c = 0; c < 2; c++) {
+            const uint32_t c0 = half * 64u + c * 32u;
+            float v[32];
+            tc::ld32(lane_addr + tt::TD + c0, v);
+#pragma unroll
+            for (uint32_t kg = 0; kg < 4; kg++) {
+                float w[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) w[e] = fmaxf(v[kg * 8 + e] + bias[c0 + kg * 8 + e], 0.0f);
+                *reinterpret_cast<uint4*>(sm + dst + tc::off(row, c0 + kg * 8, tt::SBO128)) = pack8(w);
+            }
+        }
+    };
+    float bsum[3][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
+    // dH = G where the activation at `act` is positive: BF16 into `dst`, fp32 column sums into bsum
+    auto relu_back = [&](uint32_t act, uint32_t dst, float (&bs)[2]) {
+#pragma unroll
+        for (uint32_t c = 0; c < 2; c++) {
+            const uint32_t c0 = half * 64u + c * 32u;
+            float v[32];
+            tc::ld32(lane_addr + tt::TD + c0, v);
+#pragma unroll
+            for (uint32_t kg = 0; kg < 4; kg++) {
+                const uint4 a = *reinterpret_cast<const uint4*>(sm + act + tc::off(row, c0 + kg * 8, tt::SBO128));
+                const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+                float w[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const float h = __uint_as_float((e & 1) ? (aw[e >> 1] & 0xFFFF0000u) : (aw[e >> 1] << 16));
+                    w[e] = h > 0.0f ? v[kg * 8 + e] : 0.0f;
+                    v[kg * 8 + e] = w[e];
+                }
+                *reinterpret_cast<uint4*>(sm + dst + tc::off(row, c0 + kg * 8, tt::SBO128)) = pack8(w);
+            }
+            bs[c] += tt::column_sums(v, lane);
+        }
+    };
+    float b4sum[USED_OUT] = {}, lossSum = 0.0f;               // per row (half 0), folded over the rows at the end
+    const uint32_t tiles = (n + 127u) / 128u;
+    uint32_t accum = 0;                                       // the weight gradients hold earlier tiles
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint32_t r = tile * 128u + row;
+        const bool in = r < n;
+        // normalised inputs, 16 columns a thread
+#pragma unroll
+        for (uint32_t kg = 0; kg < 2; kg++) {
+            const uint32_t c = half * 16u + kg * 8u;
+            float v[8] = {};
+            if (in) {
+                load8(Xg + (size_t)r * DIN + c, vecX, v);
+#pragma unroll
+                for (int e = 0; e < 8; e++) v[e] = (v[e] - snorm[NX_MEAN + c + e]) * snorm[NX_INV + c + e];
+            }
+            *reinterpret_cast<uint4*>(sm + tt::X + tc::off(row, c, tt::SBO32)) = pack8(v);
+        }
+        publish();
+        // forward
         if (t == 0) {
-            const uint32_t steps = min(tg::BK, kEnd - k0 + 15u) / 16u;
-            const uint32_t a = sbase + tg::A0 + buf * tg::STAGE, b = sbase + tg::B0 + buf * tg::STAGE;
-            for (uint32_t s = 0; s < steps; s++)
-                tc::mma(tmem, tc::desc(a + 256u * s, tg::SBO), tc::desc(b + 256u * s, tg::SBO), id,
-                        (c > 0 || s > 0) ? 1u : 0u);
+            for (uint32_t s = 0; s < DIN / 16; s++)
+                tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::X + 256u * s, tt::SBO32),
+                        tt::kmajor(sbase + tc::W1 + 256u * s, tc::SBO_K32), tc::idesc(128, 128), s > 0);
             tc::commit(bar);
         }
-    }
-    if (ok && chunks) {
-        // the last commit covers every MMA issued before it
-        const uint32_t last = chunks - 1u;
-        ok = __syncthreads_and(tc::wait(sbase + tg::BAR + 8u * (last & 1u), (last >> 1) & 1u) ? 1 : 0) != 0;
-        tc::fence_after();
-    }
-    if (ok) {
-        const uint32_t r = m0 + t;
-        const uint32_t lane_addr = tmem + ((warp * 32u) << 16);
-        float* Cz = C + (size_t)blockIdx.z * M * N;
-        for (uint32_t c0 = 0; c0 < bn; c0 += 16) {
-            float v[16];
-            if (chunks) {
-                tc::ld16(lane_addr + c0, v);
-            } else {
+        if (!wait_mma()) break;
+        activate(sbias, tt::H1);
+        publish();
+        if (t == 0) {
+            for (uint32_t s = 0; s < HID / 16; s++)
+                tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::H1 + 256u * s, tt::SBO128),
+                        tt::kmajor(sbase + tc::W2 + 256u * s, tc::SBO_K128), tc::idesc(128, 128), s > 0);
+            tc::commit(bar);
+        }
+        if (!wait_mma()) break;
+        activate(sbias + 128, tt::H2);
+        publish();
+        if (t == 0) {
+            for (uint32_t s = 0; s < HID / 16; s++)
+                tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::H2 + 256u * s, tt::SBO128),
+                        tt::kmajor(sbase + tc::W3 + 256u * s, tc::SBO_K128), tc::idesc(128, 128), s > 0);
+            tc::commit(bar);
+        }
+        if (!wait_mma()) break;
+        activate(sbias + 256, tt::H3);
+        publish();
+        if (t == 0) {
+            for (uint32_t s = 0; s < HID / 16; s++)
+                tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::H3 + 256u * s, tt::SBO128),
+                        tt::kmajor(sbase + tc::W4 + 256u * s, tc::SBO_K128), tc::idesc(128, 16), s > 0);
+            tc::commit(bar);
+        }
+        if (!wait_mma()) break;
+        // output layer, squared error and its gradient 2 (y - t) / n on the used columns
+        if (half == 0) {
+            float v[16], g[16] = {};
+            tc::ld16(lane_addr + tt::TD, v);
+            if (in) {
 #pragma unroll
-                for (int j = 0; j < 16; j++) v[j] = 0.0f;
+                for (int c = 0; c < USED_OUT; c++) {
+                    const float y = v[c] + sbias[384 + c];
+                    const float tn = (Tg[(size_t)r * USED_OUT + c] - snorm[NY_MEAN + c]) / snorm[NY_STD + c];
+                    const float e = y - tn;
+                    lossSum += e * e;
+                    g[c] = 2.0f * e / (float)n;
+                    b4sum[c] += g[c];
+                }
             }
-            if (r < M) {
+            const float lo[8] = {g[0], g[1], g[2], g[3], g[4], g[5], g[6], g[7]}, hi[8] = {};
+            *reinterpret_cast<uint4*>(sm + tt::DY + tc::off(row, 0, tt::SBO16)) = pack8(lo);
+            *reinterpret_cast<uint4*>(sm + tt::DY + tc::off(row, 8, tt::SBO16)) = pack8(hi);
+        }
+        publish();
+        // backward: the input gradient is committed, then the layer's weight gradient follows it
+        if (t == 0) {
+            tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::DY, tt::SBO16), tt::mnmajor(sbase + tc::W4, tc::SBO_K128),
+                    tc::idesc(128, 128) | tt::MN_B, 0u);
+            tc::commit(bar);
+            for (uint32_t s = 0; s < 8; s++)
+                tc::mma(tmem + tt::TW4, tt::mnmajor(sbase + tt::H3 + 2u * tt::SBO128 * s, tt::SBO128),
+                        tt::mnmajor(sbase + tt::DY + 2u * tt::SBO16 * s, tt::SBO16),
+                        tc::idesc(128, 16) | tt::MN_A | tt::MN_B, accum | (s > 0));
+        }
+        if (!wait_mma()) break;
+        relu_back(tt::H3, tt::SP, bsum[2]);
+        publish();
+        if (t == 0) {
+            for (uint32_t s = 0; s < HID / 16; s++)
+                tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::SP + 256u * s, tt::SBO128),
+                        tt::mnmajor(sbase + tc::W3 + 2u * tc::SBO_K128 * s, tc::SBO_K128),
+                        tc::idesc(128, 128) | tt::MN_B, s > 0);
+            tc::commit(bar);
+            for (uint32_t s = 0; s < 8; s++)
+                tc::mma(tmem + tt::TW3, tt::mnmajor(sbase + tt::SP + 2u * tt::SBO128 * s, tt::SBO128),
+                        tt::mnmajor(sbase + tt::H2 + 2u * tt::SBO128 * s, tt::SBO128),
+                        tc::idesc(128, 128) | tt::MN_A | tt::MN_B, accum | (s > 0));
+        }
+        if (!wait_mma()) break;                               // dW4's products are complete as well
+        relu_back(tt::H2, tt::H3, bsum[1]);
+        publish();
+        if (t == 0) {
+            for (uint32_t s = 0; s < HID / 16; s++)
+                tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::H3 + 256u * s, tt::SBO128),
+                        tt::mnmajor(sbase + tc::W2 + 2u * tc::SBO_K128 * s, tc::SBO_K128),
+                        tc::idesc(128, 128) | tt::MN_B, s > 0);
+            tc::commit(bar);
+            for (uint32_t s = 0; s < 8; s++)
+                tc::mma(tmem + tt::TW2, tt::mnmajor(sbase + tt::H3 + 2u * tt::SBO128 * s, tt::SBO128),
+                        tt::mnmajor(sbase + tt::H1 + 2u * tt::SBO128 * s, tt::SBO128),
+                        tc::idesc(128, 128) | tt::MN_A | tt::MN_B, accum | (s > 0));
+        }
+        if (!wait_mma()) break;                               // dW3's products are complete as well
+        relu_back(tt::H1, tt::H2, bsum[0]);
+        publish();
+        if (t == 0) {
+            for (uint32_t s = 0; s < 8; s++)
+                tc::mma(tmem + tt::TW1, tt::mnmajor(sbase + tt::H2 + 2u * tt::SBO128 * s, tt::SBO128),
+                        tt::mnmajor(sbase + tt::X + 2u * tt::SBO32 * s, tt::SBO32),
+                        tc::idesc(128, 32) | tt::MN_A | tt::MN_B, accum | (s > 0));
+            tc::commit(bar);
+        }
+        if (!wait_mma()) break;                               // every product of the tile
+        accum = 1u;
+    }
+    pdl_trigger();
+    float* out = part + (size_t)blockIdx.x * tt::PART;
+    if (ok) {
+        // weight gradients: lane = output row (input row for dW4), contiguous over the warp
+        float v[32];
+        const uint32_t lr = (warp & 3u) * 32u + lane;
+        for (uint32_t c0 = half * 64u; c0 < half * 64u + 64u; c0 += 32u) {
+            tc::ld32(lane_addr + tt::TW3 + c0, v);
 #pragma unroll
-                for (uint32_t j = 0; j < 16; j++)
-                    if (n0 + c0 + j < N) Cz[(size_t)r * N + n0 + c0 + j] = v[j];
+            for (int j = 0; j < 32; j++) out[tt::P3 + (c0 + j) * 128u + lr] = v[j];
+            tc::ld32(lane_addr + tt::TW2 + c0, v);
+#pragma unroll
+            for (int j = 0; j < 32; j++) out[tt::P2 + (c0 + j) * 128u + lr] = v[j];
+        }
+        if (half == 0) {
+            tc::ld32(lane_addr + tt::TW1, v);
+#pragma unroll
+            for (int j = 0; j < 32; j++) out[tt::P1 + j * 128u + lr] = v[j];
+        } else {
+            float w[16];
+            tc::ld16(lane_addr + tt::TW4, w);
+#pragma unroll
+            for (int j = 0; j < 16; j++) out[tt::P4 + j * 128u + lr] = w[j];
+        }
+        // biases: the four warps of a column half, in order
+        float* red = reinterpret_cast<float*>(sm + tt::RED);   // [8 warps][64]
+        for (int l = 0; l < 3; l++) {
+            __syncthreads();
+            red[warp * 64u + lane] = bsum[l][0];
+            red[warp * 64u + 32u + lane] = bsum[l][1];
+            __syncthreads();
+            if (t < 128) {
+                const uint32_t w0 = (t >> 6) * 4u, c = t & 63u;
+                const uint32_t at = l == 0 ? tt::PB1 : (l == 1 ? tt::PB2 : tt::PB3);
+                out[at + t] = ((red[w0 * 64u + c] + red[(w0 + 1u) * 64u + c]) + red[(w0 + 2u) * 64u + c]) +
+                              red[(w0 + 3u) * 64u + c];
             }
         }
-    } else if (t == 0) {
-        atomicCAS(status, 0u, (uint32_t)AVBD_FAIL_WAIT_TIMEOUT);
-    }
-    if (!ok) {
-        // let MMAs still in flight finish (bounded) before the TMEM is freed
-        for (uint32_t b = 0; b < 2; b++) tc::wait(sbase + tg::BAR + 8u * b, 0u);
+        __syncthreads();
+        if (half == 0) {
+#pragma unroll
+            for (int k = 0; k <= USED_OUT; k++) {
+                float s = k < USED_OUT ? b4sum[k < USED_OUT ? k : 0] : lossSum;
+#pragma unroll
+                for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) red[warp * 8u + k] = s;
+            }
+        }
+        __syncthreads();
+        if (t < 16) {
+            float s = 0.0f;
+            if (t < USED_OUT) s = ((red[t] + red[8 + t]) + red[16 + t]) + red[24 + t];
+            out[tt::PB4 + t] = s;
+        }
+        if (t == 32) out[tt::PL] = ((red[USED_OUT] + red[8 + USED_OUT]) + red[16 + USED_OUT]) + red[24 + USED_OUT];
+    } else {
+        // products still in flight, the weight gradients' included (bounded waits)
+        if (t == 0) {
+            atomicCAS(status, 0u, (uint32_t)AVBD_FAIL_WAIT_TIMEOUT);
+            tc::commit(bar);
+        }
+        if (tc::wait(bar, phase ^ 1u)) tc::wait(bar, phase);
     }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tg::TMEM_COLS)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tt::TMEM_COLS)
                      : "memory");
 }
 
-__global__ void k_split_sum(const float* part, uint32_t splits, uint32_t count, float* out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    float s = 0.0f;
-    for (uint32_t z = 0; z < splits; z++) s += part[(size_t)z * count + i];
-    out[i] = s;
-}
+struct AdamArgs { float *prm, *m, *v; uint32_t step; float lr, b1, b2, eps; };
 
-// H = bf16(relu(Z + b)) for Z [rows][cols]
-__global__ void k_bias_relu(const float* Z, const float* b, uint32_t rows, uint32_t cols, bf16* H) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * cols) return;
-    H[i] = __float2bfloat16(fmaxf(Z[i] + b[i % cols], 0.0f));
-}
-
-// normalised inputs as BF16 [rows][16]
-__global__ void k_norm_input(const float* X, const float* norm, uint32_t rows, bf16* Xb) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * mlp::DIN) return;
-    const uint32_t c = i % mlp::DIN;
-    Xb[i] = __float2bfloat16((X[i] - norm[mlp::NX_MEAN + c]) * norm[mlp::NX_INV + c]);
-}
-
-// Output layer and loss: Y = Z + b4; dY = 2 (Y - Tn) / rows on the used
-// columns (Tn: targets normalised by ymean, ystd), 0 elsewhere; loss sums.
-__global__ void k_loss_grad(const float* Z, const float* b4, const float* T, const float* norm, uint32_t rows,
-                            float* dY, bf16* dYb, float* lossPart) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.0f;
-    if (i < rows * mlp::DOUT) {
-        const uint32_t r = i / mlp::DOUT, c = i % mlp::DOUT;
-        float g = 0.0f;
-        if (c < (uint32_t)mlp::USED_OUT) {
-            const float y = Z[i] + b4[c];
-            const float t = (T[r * mlp::USED_OUT + c] - norm[mlp::NY_MEAN + c]) / norm[mlp::NY_STD + c];
-            const float e = y - t;
-            l = e * e;
-            g = 2.0f * e / (float)rows;
-        }
-        dY[i] = g;
-        dYb[i] = __float2bfloat16(g);
+// Adds `parts` partial gradients in CTA order and stores the gradient (ADAM =
+// false) or applies Adam to the fp32 parameters.  Blocks of 256 elements: for
+// the matrices held as [in][out], eight inputs x 32 outputs, read along the
+// outputs and, after an exchange in shared memory, written along the inputs
+// (whole 32-byte sectors both ways).
+template <bool ADAM>
+__global__ void __launch_bounds__(256) k_train_reduce(const float* __restrict__ part, uint32_t parts, uint32_t n,
+                                                      float* __restrict__ grad, AdamArgs a, float* loss) {
+    using namespace mlp;
+    __shared__ float ex[8][33];
+    constexpr uint32_t B3 = 64, B2 = B3 + 64, B1 = B2 + 16, B4 = B1 + 8;   // blocks of dW3, dW2, dW1, dW4
+    const uint32_t t = threadIdx.x, b = blockIdx.x;
+    uint32_t src, dst = 0xFFFFFFFFu;
+    const bool turn = b < B1;
+    if (turn) {
+        const uint32_t q = b < B3 ? b : (b < B2 ? b - B3 : b - B2);
+        const uint32_t cols = b < B2 ? 128u : 32u, i0 = (q >> 2) * 8u, o0 = (q & 3u) * 32u;
+        src = (b < B3 ? tt::P3 : (b < B2 ? tt::P2 : tt::P1)) + (i0 + (t >> 5)) * 128u + o0 + (t & 31u);
+        dst = (b < B3 ? OW3 : (b < B2 ? OW2 : OW1)) + (o0 + (t >> 3)) * cols + i0 + (t & 7u);
+    } else if (b < B4) {
+        src = tt::P4 + (b - B1) * 256u + t;
+        dst = OW4 + (b - B1) * 256u + t;
+    } else {
+        const uint32_t i = (b - B4) * 256u + t;               // biases, then the loss
+        src = tt::PB1 + i;
+        if (i < 128) dst = OB1 + i;
+        else if (i < 256) dst = OB2 + i - 128u;
+        else if (i < 384) dst = OB3 + i - 256u;
+        else if (i < 400) dst = OB4 + i - 384u;
+        else if (i > 400) return;                             // i == 400: the loss
     }
-    // block sum of the squared errors (fixed order)
-    __shared__ float red[256];
-    red[threadIdx.x] = l;
-    __syncthreads();
-    for (uint32_t w = blockDim.x >> 1; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    pdl_wait();
+    float s = 0.0f;
+    uint32_t z = 0;
+    for (; z + 8 <= parts; z += 8) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = part[(size_t)(z + k) * tt::PART + src];
+#pragma unroll
+        for (int k = 0; k < 8; k++) s += v[k];
+    }
+    for (; z < parts; z++) s += part[(size_t)z * tt::PART + src];
+    if (turn) {
+        ex[t >> 5][t & 31u] = s;
         __syncthreads();
+        s = ex[t & 7u][t >> 3];
     }
-    if (threadIdx.x == 0) lossPart[blockIdx.x] = red[0];
+    if (dst == 0xFFFFFFFFu) {
+        if (loss) *loss = s * (1.0f / (float)n);              // mean over the batch
+        return;
+    }
+    if (ADAM) {
+        const float mi = a.b1 * a.m[dst] + (1.0f - a.b1) * s;
+        const float vi = a.b2 * a.v[dst] + (1.0f - a.b2) * s * s;
+        a.m[dst] = mi;
+        a.v[dst] = vi;
+        const float mh = mi / (1.0f - powf(a.b1, (float)a.step));
+        const float vh = vi / (1.0f - powf(a.b2, (float)a.step));
+        a.prm[dst] = a.prm[dst] - a.lr * mh / (sqrtf(vh) + a.eps);
+    } else if (grad) {
+        grad[dst] = s;
+    }
 }
-
-// dH = bf16(G * (H > 0)), G fp32 [rows][cols]; also keeps fp32 for bias sums
-__global__ void k_relu_back(const float* G, const bf16* H, uint32_t n, float* dH, bf16* dHb) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float v = __bfloat162float(H[i]) > 0.0f ? G[i] : 0.0f;
-    dH[i] = v;
-    dHb[i] = __float2bfloat16(v);
-}
-
-// column sums of G [rows][cols] in a fixed order (one thread per column)
-__global__ void k_col_sum(const float* G, uint32_t rows, uint32_t cols, float* out) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.0f;
-    for (uint32_t r = 0; r < rows; r++) s += G[(size_t)r * cols + c];
-    out[c] = s;
-}
-
-// fixed-order sum of n values, times `scale`
-__global__ void k_fixed_sum(const float* v, uint32_t n, float scale, float* out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    float s = 0.0f;
-    for (uint32_t i = 0; i < n; i++) s += v[i];
-    *out = s * scale;
-}
-
-// Adam on the fp32 parameters; refreshes the BF16 weight mirror.
-__global__ void k_adam(float* prm, const float* grad, float* m, float* v, uint32_t step, float lr, float b1,
-                       float b2, float eps, bf16* half) {
-    using namespace mlp;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NPARAM) return;
-    const float gi = grad[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float mh = mi / (1.0f - powf(b1, (float)step));
-    const float vh = vi / (1.0f - powf(b2, (float)step));
-    const float p = prm[i] - lr * mh / (sqrtf(vh) + eps);
-    prm[i] = p;
-    int h = -1;
-    if (i < OB1) h = (int)(HW1 + i);
-    else if (i >= OW2 && i < OB2) h = (int)(HW2 + i - OW2);
-    else if (i >= OW3 && i < OB3) h = (int)(HW3 + i - OW3);
-    else if (i >= OW4 && i < OB4) h = (int)(HW4 + i - OW4);
-    if (h >= 0) half[h] = __float2bfloat16(p);
-}
-
-__global__ void k_mirror(const float* prm, bf16* half) {
-    using namespace mlp;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NPARAM) return;
-    int h = -1;
-    if (i < OB1) h = (int)(HW1 + i);
-    else if (i >= OW2 && i < OB2) h = (int)(HW2 + i - OW2);
-    else if (i >= OW3 && i < OB3) h = (int)(HW3 + i - OW3);
-    else if (i >= OW4 && i < OB4) h = (int)(HW4 + i - OW4);
-    if (h >= 0) half[h] = __float2bfloat16(prm[i]);
-}
+constexpr uint32_t kTrainReduceBlocks = 64 + 64 + 16 + 8 + 2;
 
 // BF16 weight image of the inference kernel: W1..W4 in the UMMA canonical
 // K-major layout, byte for byte the kernel's shared-memory weight region.
@@ -579,113 +787,49 @@ __global__ void k_mirror_umma(const float* prm, unsigned char* img) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Host side of training (forward with saved activations, backward, Adam).
-// Workspace layout for a batch of B rows (all offsets 256-byte aligned).
+// Host side of training.  Workspace for a batch of B rows: the status word
+// (256 bytes), then one partial gradient per CTA of k_train_tile.
 // ---------------------------------------------------------------------------
 namespace {
-constexpr uint32_t kSplits = 32;
+inline uint32_t blocks(size_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t); }
+
+// one 128-row tile per CTA while the batch has no more tiles than the device
+// SMs (an SM holds one CTA: 220 KiB of shared memory, all of TMEM)
+uint32_t train_ctas(uint32_t B) { return std::min<uint32_t>((B >> 7) + ((B & 127u) ? 1u : 0u), 148u); }
+
 struct Work {
-    bf16 *Xb, *H1, *H2, *H3, *dYb, *dH3b, *dH2b, *dH1b, *half;
-    float *Z, *dY, *dH, *part, *grad, *lossPart;
     uint32_t* status;        // nonzero when a tensor-core wait gave up
+    float* part;
 };
-size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 size_t work_layout(uint32_t B, char* base, Work* w) {
-    using namespace mlp;
-    size_t off = 0;
-    auto take = [&](size_t bytes) { char* p = base ? base + off : nullptr; off += align256(bytes); return p; };
-    const size_t Bp = (size_t)B;
-    char* p;
-    p = take(Bp * DIN * 2); if (w) w->Xb = (bf16*)p;
-    p = take(Bp * HID * 2); if (w) w->H1 = (bf16*)p;
-    p = take(Bp * HID * 2); if (w) w->H2 = (bf16*)p;
-    p = take(Bp * HID * 2); if (w) w->H3 = (bf16*)p;
-    p = take(Bp * DOUT * 2); if (w) w->dYb = (bf16*)p;
-    p = take(Bp * HID * 2); if (w) w->dH3b = (bf16*)p;
-    p = take(Bp * HID * 2); if (w) w->dH2b = (bf16*)p;
-    p = take(Bp * HID * 2); if (w) w->dH1b = (bf16*)p;
-    p = take((size_t)NHALF * 2); if (w) w->half = (bf16*)p;
-    p = take(Bp * HID * 4); if (w) w->Z = (float*)p;
-    p = take(Bp * DOUT * 4); if (w) w->dY = (float*)p;
-    p = take(Bp * HID * 4); if (w) w->dH = (float*)p;
-    p = take((size_t)kSplits * HID * HID * 4); if (w) w->part = (float*)p;
-    p = take((size_t)NPARAM * 4); if (w) w->grad = (float*)p;
-    p = take(((Bp * DOUT + 255) / 256) * 4 + 4); if (w) w->lossPart = (float*)p;
-    p = take(4); if (w) w->status = (uint32_t*)p;
-    return off;
+    if (w) {
+        w->status = reinterpret_cast<uint32_t*>(base);
+        w->part = reinterpret_cast<float*>(base + 256);
+    }
+    return 256 + sizeof(float) * (size_t)tt::PART * train_ctas(B);
 }
 
-// 64 KiB of dynamic shared memory for the two stages (set once per device)
-template <bool TA, bool TB>
-void gemm_attributes() {
+// 220 KiB of dynamic shared memory (set once per device)
+void train_attributes() {
     static std::atomic<uint64_t> done{0};
     int dev = 0;
     cudaGetDevice(&dev);
     const uint64_t bit = 1ull << (dev & 63);
     if (done.load() & bit) return;
-    cudaFuncSetAttribute(k_gemm_tc<TA, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tg::SMEM);
+    cudaFuncSetAttribute(k_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tt::SMEM);
     done.fetch_or(bit);
 }
 
-template <bool TA, bool TB>
-void launch_gemm_tc(dim3 grid, const bf16* A, const bf16* B, float* dst, uint32_t M, uint32_t N, uint32_t K,
-                    uint32_t kPer, uint32_t bn, uint32_t* status, cudaStream_t st) {
-    gemm_attributes<TA, TB>();
-    k_gemm_tc<TA, TB><<<grid, 128, tg::SMEM, st>>>(A, B, dst, M, N, K, kPer, bn, status);
-}
-
-void gemm(const bf16* A, bool ta, const bf16* B, bool tb, float* C, uint32_t M, uint32_t N, uint32_t K,
-          uint32_t splits, float* part, uint32_t* status, cudaStream_t st) {
-    const uint32_t kPer = ((K + splits - 1) / splits + 63) / 64 * 64;
-    splits = (K + kPer - 1) / kPer;
-    // 64-column tiles: two column blocks for the 128-wide layers (more CTAs
-    // for the batch-row GEMMs, which have only 64 row blocks at batch 8,192)
-    const uint32_t bn = std::min<uint32_t>(64u, (N + 15u) / 16u * 16u);
-    dim3 grid((N + bn - 1) / bn, (M + 127) / 128, splits);
-    float* dst = splits > 1 ? part : C;
-    if (!ta && !tb) launch_gemm_tc<false, false>(grid, A, B, dst, M, N, K, kPer, bn, status, st);
-    else if (!ta && tb) launch_gemm_tc<false, true>(grid, A, B, dst, M, N, K, kPer, bn, status, st);
-    else if (ta && !tb) launch_gemm_tc<true, false>(grid, A, B, dst, M, N, K, kPer, bn, status, st);
-    else launch_gemm_tc<true, true>(grid, A, B, dst, M, N, K, kPer, bn, status, st);
-    if (splits > 1) k_split_sum<<<(M * N + 255) / 256, 256, 0, st>>>(part, splits, M * N, C);
-}
-
-inline uint32_t blocks(size_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t); }
-
-// Forward with saved activations, loss and full gradient into w.grad.
-void forward_backward(const float* prm, const float* norm, const float* X, const float* T, uint32_t B, Work& w,
-                      cudaStream_t st) {
-    using namespace mlp;
-    k_mirror<<<blocks(NPARAM, 256), 256, 0, st>>>(prm, w.half);
-    k_norm_input<<<blocks((size_t)B * DIN, 256), 256, 0, st>>>(X, norm, B, w.Xb);
-    // forward: Z = Hprev W^T (W stored [out][in] = [N][K])
-    gemm(w.Xb, false, w.half + HW1, false, w.Z, B, HID, DIN, 1, w.part, w.status, st);
-    k_bias_relu<<<blocks((size_t)B * HID, 256), 256, 0, st>>>(w.Z, prm + OB1, B, HID, w.H1);
-    gemm(w.H1, false, w.half + HW2, false, w.Z, B, HID, HID, 1, w.part, w.status, st);
-    k_bias_relu<<<blocks((size_t)B * HID, 256), 256, 0, st>>>(w.Z, prm + OB2, B, HID, w.H2);
-    gemm(w.H2, false, w.half + HW3, false, w.Z, B, HID, HID, 1, w.part, w.status, st);
-    k_bias_relu<<<blocks((size_t)B * HID, 256), 256, 0, st>>>(w.Z, prm + OB3, B, HID, w.H3);
-    gemm(w.H3, false, w.half + HW4, false, w.Z, B, DOUT, HID, 1, w.part, w.status, st);
-    const uint32_t lb = blocks((size_t)B * DOUT, 256);
-    k_loss_grad<<<lb, 256, 0, st>>>(w.Z, prm + OB4, T, norm, B, w.dY, w.dYb, w.lossPart);
-    k_fixed_sum<<<1, 32, 0, st>>>(w.lossPart, lb, 1.0f / (float)B, w.lossPart + lb);   // mean over the batch
-    // backward.  dW = dH^T Hprev: A = dH stored [B][out] = [K][M] (TA),
-    // B-operand = Hprev stored [B][in] = [K][N] (TB).  dHprev = dH W:
-    // A = dH [B][out] = [M][K], B-operand W stored [out][in] = [K][N] (TB).
-    gemm(w.dYb, true, w.H3, true, w.grad + OW4, DOUT, HID, B, kSplits, w.part, w.status, st);
-    k_col_sum<<<1, DOUT, 0, st>>>(w.dY, B, DOUT, w.grad + OB4);
-    gemm(w.dYb, false, w.half + HW4, true, w.Z, B, HID, DOUT, 1, w.part, w.status, st);
-    k_relu_back<<<blocks((size_t)B * HID, 256), 256, 0, st>>>(w.Z, w.H3, B * HID, w.dH, w.dH3b);
-    k_col_sum<<<1, HID, 0, st>>>(w.dH, B, HID, w.grad + OB3);
-    gemm(w.dH3b, true, w.H2, true, w.grad + OW3, HID, HID, B, kSplits, w.part, w.status, st);
-    gemm(w.dH3b, false, w.half + HW3, true, w.Z, B, HID, HID, 1, w.part, w.status, st);
-    k_relu_back<<<blocks((size_t)B * HID, 256), 256, 0, st>>>(w.Z, w.H2, B * HID, w.dH, w.dH2b);
-    k_col_sum<<<1, HID, 0, st>>>(w.dH, B, HID, w.grad + OB2);
-    gemm(w.dH2b, true, w.H1, true, w.grad + OW2, HID, HID, B, kSplits, w.part, w.status, st);
-    gemm(w.dH2b, false, w.half + HW2, true, w.Z, B, HID, HID, 1, w.part, w.status, st);
-    k_relu_back<<<blocks((size_t)B * HID, 256), 256, 0, st>>>(w.Z, w.H1, B * HID, w.dH, w.dH1b);
-    k_col_sum<<<1, HID, 0, st>>>(w.dH, B, HID, w.grad + OB1);
-    gemm(w.dH1b, true, w.Xb, true, w.grad + OW1, HID, DIN, B, kSplits, w.part, w.status, st);
+// Forward, loss and partial gradients; then their sum into `grad` (a == null)
+// or Adam on the parameters.
+void forward_backward(const float* prm, const float* norm, const float* X, const float* T, uint32_t B, const Work& w,
+                      float* grad, const AdamArgs* a, float* loss, cudaStream_t st) {
+    train_attributes();
+    const uint32_t ctas = train_ctas(B);
+    k_train_tile<<<ctas, tt::THREADS, tt::SMEM, st>>>(prm, norm, X, T, B, w.part, w.status);
+    if (a) launch_pdl(k_train_reduce<true>, kTrainReduceBlocks, 256, st, (const float*)w.part, ctas, B, (float*)nullptr, *a, loss);
+    else if (grad || loss)
+        launch_pdl(k_train_reduce<false>, kTrainReduceBlocks, 256, st, (const float*)w.part, ctas, B, grad, AdamArgs{}, loss);
 }
 }  // namespace
 
@@ -974,26 +1118,23 @@ static int workspace_status(const Work& w, cudaStream_t st) {
 }
 
 static int gradients(const float* params, const float* norm, const float* features, const float* targets,
-                     uint32_t batch, void* workspace, float* grad_out, float* loss_out, cudaStream_t st,
-                     bool check) {
+                     uint32_t batch, void* workspace, float* grad_out, const AdamArgs* adam, float* loss_out,
+                     cudaStream_t st) {
     if (!params || !norm || !features || !targets || !workspace || batch == 0) return AVBD_ERR_INVALID_ARGUMENT;
     Work w{};
     work_layout(batch, static_cast<char*>(workspace), &w);
-    if (check) cudaMemsetAsync(w.status, 0, sizeof(uint32_t), st);
-    forward_backward(params, norm, features, targets, batch, w, st);
-    const uint32_t lb = blocks((size_t)batch * mlp::DOUT, 256);
-    if (grad_out) cudaMemcpyAsync(grad_out, w.grad, sizeof(float) * mlp::NPARAM, cudaMemcpyDeviceToDevice, st);
-    if (loss_out) cudaMemcpyAsync(loss_out, w.lossPart + lb, sizeof(float), cudaMemcpyDeviceToDevice, st);
+    if (!adam) cudaMemsetAsync(w.status, 0, sizeof(uint32_t), st);
+    forward_backward(params, norm, features, targets, batch, w, grad_out, adam, loss_out, st);
     if (cudaGetLastError() != cudaSuccess) return AVBD_ERR_RUNTIME_FAILURE;
-    // a tensor-core wait that gave up fails the call (the GEMM kernels latch
-    // it in the workspace's status word)
-    return check ? workspace_status(w, st) : AVBD_OK;
+    // a tensor-core wait that gave up fails the call (the kernel latches it
+    // in the workspace's status word); the training step stays asynchronous
+    return adam ? AVBD_OK : workspace_status(w, st);
 }
 
 int avbd_mlp_gradients(const float* params, const float* norm, const float* features, const float* targets,
                        uint32_t batch, void* workspace, float* grad_out, float* loss_out, void* stream) {
-    return gradients(params, norm, features, targets, batch, workspace, grad_out, loss_out,
-                     static_cast<cudaStream_t>(stream), true);
+    return gradients(params, norm, features, targets, batch, workspace, grad_out, nullptr, loss_out,
+                     static_cast<cudaStream_t>(stream));
 }
 
 int avbd_mlp_workspace_status(const void* workspace, uint32_t batch, void* stream) {
@@ -1008,16 +1149,13 @@ int avbd_mlp_train_step(float* params, const float* norm, const float* features,
                         float* loss_out, void* stream) {
     if (!params || !adam_m || !adam_v || step == 0) return AVBD_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    Work w{};
-    if (workspace && batch) {
+    if (workspace && batch && step == 1) {
+        Work w{};
         work_layout(batch, static_cast<char*>(workspace), &w);
-        if (step == 1) cudaMemsetAsync(w.status, 0, sizeof(uint32_t), st);   // sticky from here on
+        cudaMemsetAsync(w.status, 0, sizeof(uint32_t), st);   // sticky from here on
     }
-    int rc = gradients(params, norm, features, targets, batch, workspace, nullptr, loss_out, st, false);
-    if (rc != AVBD_OK) return rc;
-    k_adam<<<blocks(mlp::NPARAM, 256), 256, 0, st>>>(params, w.grad, adam_m, adam_v, step, lr, 0.9f, 0.999f, 1e-8f,
-                                                     w.half);
-    return cudaGetLastError() == cudaSuccess ? AVBD_OK : AVBD_ERR_RUNTIME_FAILURE;
+    const AdamArgs adam{params, adam_m, adam_v, step, lr, 0.9f, 0.999f, 1e-8f};
+    return gradients(params, norm, features, targets, batch, workspace, nullptr, &adam, loss_out, st);
 }
 
 static int mlp_infer(const float* params, const float* norm, const float* features, uint32_t n, float* out,

@@ -1,0 +1,62 @@
+"""The training kernels at the edges of their tiles: one row, one short of a
+128-row tile, one past it, and more tiles than a pass over the device's SMs
+holds; and inputs whose addresses allow no 16-byte loads."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from avbd_b200 import learned
+from avbd_b200.solver import load_library
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(B):
+    rng = np.random.default_rng(B)
+    p = learned.init_params(seed=B)
+    p[learned.HID * learned.DIN:learned.HID * learned.DIN + learned.HID] = rng.normal(0, 0.1, learned.HID)
+    norm = np.ones(learned.NNORM, np.float32)
+    norm[:learned.DIN] = rng.normal(0, 0.1, learned.DIN)
+    norm[learned.YM:learned.YM + learned.USED] = rng.normal(0, 0.1, learned.USED)
+    X = rng.normal(size=(B, learned.DIN)).astype(np.float32)
+    T = rng.normal(size=(B, learned.USED)).astype(np.float32)
+    return p, norm, X, T
+
+
+# 5e-3: the bar of the oracle comparison at ordinary batches (a different fp32
+# accumulation order moves single BF16 roundings of the activations)
+@pytest.mark.parametrize("B", [1, 127, 128, 129, 148 * 128 + 37])
+def test_gradients_at_tile_edges(cuda_lib, oracle_lib, B):
+    from oracle import mlp_oracle as M
+    p, norm, X, T = _case(B)
+    loss, g = learned.gradients(p, norm, X, T)
+    want_loss, want = M.forward_backward(p, norm, X, T, rounded=True)
+    assert abs(loss - want_loss) <= 1e-4 * max(1.0, abs(want_loss))
+    for a, b in ((M.OW1, M.OB1), (M.OB1, M.OW2), (M.OW2, M.OB2), (M.OB2, M.OW3), (M.OW3, M.OB3), (M.OB3, M.OW4),
+                 (M.OW4, M.OB4), (M.OB4, M.NPARAM)):
+        assert np.linalg.norm(g[a:b] - want[a:b]) <= 5e-3 * max(np.linalg.norm(want[a:b]), 1e-12)
+
+
+def test_gradients_of_unaligned_inputs(cuda_lib):
+    """Parameters, features and targets four bytes off a 16-byte boundary give
+    the aligned call's gradients bit for bit."""
+    import torch
+    lib = load_library()
+    p, norm, X, T = _case(200)
+    want_loss, want = learned.gradients(p, norm, X, T)
+
+    def shifted(a):
+        t = torch.zeros(a.size + 1, dtype=torch.float32, device="cuda")
+        t[1:] = torch.from_numpy(a.ravel()).cuda()
+        return t[1:]
+
+    args = [shifted(a) for a in (p, norm, X, T)]
+    grad = torch.zeros(learned.NPARAM, device="cuda")
+    loss = torch.zeros(1, device="cuda")
+    ws = torch.empty(lib.avbd_mlp_workspace_bytes(200), dtype=torch.uint8, device="cuda")
+    rc = lib.avbd_mlp_gradients(*(a.data_ptr() for a in args), 200, ws.data_ptr(), grad.data_ptr(), loss.data_ptr(),
+                                C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    assert float(loss.item()) == want_loss
+    assert np.array_equal(grad.cpu().numpy(), want)
