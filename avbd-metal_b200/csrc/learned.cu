@@ -64,40 +64,60 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 
 // ---------------------------------------------------------------------------
-// Fused inference on the Blackwell tensor cores (tcgen05): one CTA of four
-// warps per 128-row tile, persistent over the batch.  The weights live in
-// global memory as an image of their shared-memory form — the UMMA canonical
-// K-major layout without swizzle (8-row x 16-byte core matrices: element
-// (r, k) of an operand with row-group stride `sbo` at (r / 8) sbo + (k / 8)
-// 128 + (r % 8) 16 + (k % 8) 2 bytes) — and each CTA stages them once with
-// bulk asynchronous copies completing on an mbarrier; a layer is 2 (K = 32) or 8 (K = 128) tcgen05.mma instructions of
-// M = 128, K = 16, issued by one thread, accumulating in TMEM (128 lanes =
-// the tile's rows, N fp32 columns); each warp reads its 32 rows back with
-// tcgen05.ld, adds the bias, applies ReLU, rounds to BF16 and writes the next
-// layer's A operand in place.  Completion of every layer's MMAs is signalled
-// by tcgen05.commit on an mbarrier; every wait on it is bounded and a
-// timeout sets *status (the CTA then frees its TMEM and stops).
+// Fused inference on the Blackwell tensor cores (tcgen05): one CTA per SM
+// whose two groups of eight warps each walk 128-row tiles of their own, so
+// that one group's MMAs run beside the other's epilogues; the weights are
+// shared.  Shared-memory operands are in the UMMA canonical K-major layout
+// without swizzle (8-row x 16-byte core matrices: element (r, k) of an operand
+// with row-group stride `sbo` at (r / 8) sbo + (k / 8) 128 + (r % 8) 16 +
+// (k % 8) 2 bytes); the hidden activations never leave tensor memory.  A layer
+// is 2 (K = 32) or 8 (K = 128) tcgen05.mma instructions of M = 128, K = 16,
+// issued by one thread, accumulating in TMEM (128 lanes = the tile's rows).
+// Two threads share a row: each reads 64 of its fp32 columns with tcgen05.ld,
+// adds the bias (two fp32 additions an instruction), applies ReLU, rounds to
+// BF16 and writes them back with tcgen05.st as the A operand of the next layer
+// (two columns a 32-bit TMEM cell).  A warp reads feature rows whole (four
+// 128-byte rows a load) one tile ahead, and the next tile's first layer is
+// issued together with this tile's last, into columns of their own.
+// Completion is signalled by tcgen05.commit on the group's mbarriers; every
+// wait on them is bounded and a timeout sets *status (the CTA then frees its
+// TMEM and stops).  Tiles go to group tile / gridDim of a CTA, so that up to
+// 148 tiles spread over all SMs before any SM takes a second one.
+//
+// What bounds it: the chain of a layer, about 2,200 cycles of which the eight
+// MMAs (512 cycles of arithmetic, shared with the other group's) take 1,300
+// from their issue to the waiting threads and the epilogue 800; the call over
+// 1,048,576 rows takes 122 us of which about 30 are the launch, the status
+// read-back and the wait for it (236 us with one tile in flight per CTA and
+// two CTAs per SM; 150 us with four groups of 128 threads and the activations
+// in shared memory; 159 us before the issuing lane was elected, see elect_one).
 // ---------------------------------------------------------------------------
 namespace tc {
 constexpr uint32_t ROWS = 128;
 constexpr uint32_t SBO_K128 = 2048, SBO_K32 = 512;      // row-group strides (K = 128, K = 32)
-// shared memory: weight image | layer operand | biases b1 b2 b3 b4 (fp32) |
-// normalisation block (fp32) | MMA barrier | staging barrier | TMEM address
+// shared memory: weight image | input tiles | biases b1 b2 b3 b4 (fp32) |
+// normalisation block (fp32) | MMA barriers | staging barrier | TMEM address
+constexpr uint32_t GROUPS = 2, GROUP_THREADS = 256;         // tiles in flight of a CTA, threads of each
+// input tile: 16-byte chunks 160 B apart, so that the eight lanes writing two
+// rows' chunks touch all banks once
+constexpr uint32_t XLBO = 160, XSBO = 4 * XLBO, XBYTES = (ROWS / 8) * XSBO;
 constexpr uint32_t W1 = 0, W2 = W1 + 128 * 32 * 2, W3 = W2 + 128 * 128 * 2, W4 = W3 + 128 * 128 * 2,
-                   ACT = W4 + 16 * 128 * 2, BIAS = ACT + ROWS * 128 * 2, NORM = BIAS + (3 * 128 + 16) * 4,
-                   BAR = NORM + 96 * 4, WBAR = BAR + 8, TSLOT = WBAR + 8, SMEM = TSLOT + 8;
-constexpr uint32_t WBYTES = ACT - W1;                    // the weight image: 77,824 bytes
+                   XT = W4 + 16 * 128 * 2, BIAS = XT + GROUPS * XBYTES, NORM = BIAS + (3 * 128 + 16) * 4,
+                   BAR = NORM + 96 * 4, WBAR = BAR + 16 * GROUPS, TSLOT = WBAR + 8, SMEM = TSLOT + 8;
+// TMEM columns of a group: layer outputs | A operand (BF16 pairs) | last layer's output
+constexpr uint32_t TD = 0, TA = 128, TY = 192, TGROUP = 256;
+constexpr uint32_t WBYTES = XT - W1;                     // the weight image: 77,824 bytes
 constexpr uint32_t STAGED = WBYTES + (NORM - BIAS) + 96 * 4;   // every byte the staging barrier expects
-constexpr uint32_t TMEM_COLS = 128;
+constexpr uint32_t TMEM_COLS = TGROUP * GROUPS;
 constexpr uint64_t WAIT_NS = 1000000000ull;              // a wait gives up after one second
 
 __device__ __forceinline__ uint32_t off(uint32_t r, uint32_t k, uint32_t sbo) {
     return (r >> 3) * sbo + (k >> 3) * 128u + (r & 7u) * 16u + (k & 7u) * 2u;
 }
-// shared-memory matrix descriptor: start address, LBO = 128 B (the second
-// 8-element K chunk), SBO, descriptor version 1, no swizzle
-__device__ __forceinline__ uint64_t desc(uint32_t saddr, uint32_t sbo) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
+// shared-memory matrix descriptor: start address, LBO (the second 8-element K
+// chunk), SBO, descriptor version 1, no swizzle
+__device__ __forceinline__ uint64_t desc(uint32_t saddr, uint32_t sbo, uint32_t lbo = 128u) {
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
            (1ull << 46);
 }
 // instruction descriptor of kind::f16: F32 accumulator, BF16 A and B, both
@@ -122,11 +142,16 @@ __device__ __forceinline__ uint64_t now_ns() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-// bounded wait for the mbarrier phase `parity`; false on timeout
+// bounded wait for the mbarrier phase `parity`; false on timeout.  The global
+// timer is first read after 64 polls: reading it costs more than most waits.
 __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity) {
-    const uint64_t t0 = now_ns();
+    uint64_t t0 = 0;
     for (uint32_t i = 0;; i++) {
-        if ((i & 255u) == 255u && now_ns() - t0 > WAIT_NS) return false;
+        if ((i & 63u) == 63u) {
+            const uint64_t t = now_ns();
+            if (t0 == 0) t0 = t;
+            else if (t - t0 > WAIT_NS) return false;
+        }
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -149,6 +174,16 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 __device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// one lane of a converged warp; with warp-uniform operands (uniform()) the
+// MMA instructions that follow need no per-lane to uniform register moves
+// (eight MMAs took 1,150 cycles to issue from a lane that the compiler could
+// not know to be alone)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0u;
+}
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -216,32 +251,110 @@ __device__ __forceinline__ void stage_weights(const float* prm, bool vec, unsign
     }
 }
 
-__global__ void __launch_bounds__(128) k_mlp_infer_tc(const bf16* __restrict__ W, const float* __restrict__ prm,
-                                                      const float* __restrict__ norm, const float* __restrict__ X,
-                                                      uint32_t n, float* __restrict__ Y, uint32_t* status,
-                                                      bool issue = true) {
+namespace tc {
+// 64 consecutive fp32 columns of this thread's TMEM lane
+__device__ __forceinline__ void ld64(uint32_t taddr, float (&v)[64]) {
+    uint32_t r[64];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32,%33,%34,%35,%36,%37,%38,%39,"
+        "%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%64];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]),
+          "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]),
+          "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]),
+          "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
+          "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int j = 0; j < 64; j++) v[j] = __uint_as_float(r[j]);
+}
+// two fp32 additions in one instruction, each rounded as a scalar addition
+__device__ __forceinline__ void add2(float& x, float& y, float a, float b) {
+    asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\tadd.rn.f32x2 p, p, q;\n\t"
+        "mov.b64 {%0, %1}, p;\n\t}"
+        : "+f"(x), "+f"(y)
+        : "f"(a), "f"(b));
+}
+// bf16(max(x, 0)) of two values: rounded first (rounding keeps the order), a NaN gives 0 as fmaxf does
+__device__ __forceinline__ uint32_t relu_bf16(float lo, float hi) {
+    const __nv_bfloat162 v = __hmax2(__floats2bfloat162_rn(lo, hi), __float2bfloat162_rn(0.0f));
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+// barrier of one group (ids 1, 2); true when no thread passed `failed`
+__device__ __forceinline__ bool group_sync(uint32_t id, bool failed) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 0, 1, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(failed ? 1u : 0u), "r"(id), "n"(GROUP_THREADS)
+        : "memory");
+    return r != 0u;
+}
+// A from TMEM (BF16 pairs, lane = row), B from shared memory
+__device__ __forceinline__ void mma_ta(uint32_t tmem, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+        :
+        : "r"(tmem), "r"(a), "l"(b), "r"(id), "r"(acc));
+}
+// 32 consecutive 32-bit columns of this thread's TMEM lane
+__device__ __forceinline__ void st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n\t"
+        "tcgen05.wait::st.sync.aligned;" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+        "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+}  // namespace tc
+
+// IMAGE: W is the weight image and arrives by bulk copies; otherwise every CTA
+// converts the fp32 parameters itself (38,912 weights, about a microsecond,
+// against the launch of a kernel that would write the image first).
+template <bool IMAGE>
+__global__ void __launch_bounds__(tc::GROUPS * tc::GROUP_THREADS, 1)
+k_mlp_infer_tc(const bf16* __restrict__ W, const float* __restrict__ prm, const float* __restrict__ norm,
+               const float* __restrict__ X, uint32_t n, float* __restrict__ Y, uint32_t* status, bool issue) {
     using namespace mlp;
     extern __shared__ __align__(128) unsigned char sm[];
-    const uint32_t t = threadIdx.x, warp = t >> 5;
+    const uint32_t t = threadIdx.x, warp = tc::uniform(t >> 5), lane = t & 31u;
+    const uint32_t group = warp / (tc::GROUP_THREADS / 32), row = t & 127u;
+    const uint32_t half = (t >> 7) & 1u;                       // row and column half of this thread
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
-    const uint32_t bar = sbase + tc::BAR, wbar = sbase + tc::WBAR;
-    // the weight image (already in the canonical layout), the biases and the
-    // normalisation block: nine bulk copies on one barrier
+    const uint32_t bar = sbase + tc::BAR + 16u * group, bar4 = bar + 8u, wbar = sbase + tc::WBAR;
     if (t == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        for (uint32_t g = 0; g < 2 * tc::GROUPS; g++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbase + tc::BAR + 8u * g) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        tc::expect_tx(wbar, tc::STAGED);
-        const unsigned char* img = reinterpret_cast<const unsigned char*>(W);
-        tc::bulk_load(sbase + tc::W1, img + tc::W1, tc::W2 - tc::W1, wbar);
-        tc::bulk_load(sbase + tc::W2, img + tc::W2, tc::W3 - tc::W2, wbar);
-        tc::bulk_load(sbase + tc::W3, img + tc::W3, tc::W4 - tc::W3, wbar);
-        tc::bulk_load(sbase + tc::W4, img + tc::W4, tc::ACT - tc::W4, wbar);
-        tc::bulk_load(sbase + tc::BIAS, prm + OB1, 128 * 4, wbar);
-        tc::bulk_load(sbase + tc::BIAS + 512, prm + OB2, 128 * 4, wbar);
-        tc::bulk_load(sbase + tc::BIAS + 1024, prm + OB3, 128 * 4, wbar);
-        tc::bulk_load(sbase + tc::BIAS + 1536, prm + OB4, 16 * 4, wbar);
-        tc::bulk_load(sbase + tc::NORM, norm, 96 * 4, wbar);
+        if (IMAGE) {
+            // the weight image (already in the canonical layout), the biases
+            // and the normalisation block: nine bulk copies on one barrier
+            tc::expect_tx(wbar, tc::STAGED);
+            const unsigned char* img = reinterpret_cast<const unsigned char*>(W);
+            tc::bulk_load(sbase + tc::W1, img + tc::W1, tc::W2 - tc::W1, wbar);
+            tc::bulk_load(sbase + tc::W2, img + tc::W2, tc::W3 - tc::W2, wbar);
+            tc::bulk_load(sbase + tc::W3, img + tc::W3, tc::W4 - tc::W3, wbar);
+            tc::bulk_load(sbase + tc::W4, img + tc::W4, tc::XT - tc::W4, wbar);
+            tc::bulk_load(sbase + tc::BIAS, prm + OB1, 128 * 4, wbar);
+            tc::bulk_load(sbase + tc::BIAS + 512, prm + OB2, 128 * 4, wbar);
+            tc::bulk_load(sbase + tc::BIAS + 1024, prm + OB3, 128 * 4, wbar);
+            tc::bulk_load(sbase + tc::BIAS + 1536, prm + OB4, 16 * 4, wbar);
+            tc::bulk_load(sbase + tc::NORM, norm, 96 * 4, wbar);
+        }
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + tc::TSLOT),
@@ -249,100 +362,151 @@ __global__ void __launch_bounds__(128) k_mlp_infer_tc(const bf16* __restrict__ W
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (!IMAGE) {
+        stage_weights(prm, true, sm, t, tc::GROUPS * tc::GROUP_THREADS);
+        float* sb = reinterpret_cast<float*>(sm + tc::BIAS);
+        for (uint32_t i = t; i < 3 * HID + DOUT; i += tc::GROUPS * tc::GROUP_THREADS) sb[i] = prm[bias_at(i)];
+        if (t < 96) reinterpret_cast<float*>(sm + tc::NORM)[t] = norm[t];
+        tc::fence_proxy();
+    }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + tc::TSLOT);
-    const uint32_t lane_addr = tmem + ((warp * 32u) << 16);   // this warp's 32 TMEM lanes
-    const uint32_t row = t;                                    // tile row held by this thread
-    uint32_t phase = 0;
-    // the weights have landed (bounded wait; block-uniform outcome)
-    bool ok = __syncthreads_and(tc::wait(wbar, 0) ? 1 : 0) != 0;
-    if (!ok) tc::wait(wbar, 0);        // give copies still in flight one more bounded wait
+    const uint32_t tbase = tc::uniform(*reinterpret_cast<volatile uint32_t*>(sm + tc::TSLOT));
+    const uint32_t tmem = tbase + tc::TGROUP * group;
+    const uint32_t lane_addr = tmem + (((warp & 3u) * 32u) << 16);   // this warp's 32 TMEM lanes
+    unsigned char* xt = sm + tc::XT + tc::XBYTES * group;
+    const uint32_t sxt = sbase + tc::XT + tc::XBYTES * group;
+    bool ok = true;
+    if (IMAGE) {
+        // the weights have landed (bounded wait; block-uniform outcome)
+        ok = __syncthreads_and(tc::wait(wbar, 0) ? 1 : 0) != 0;
+        if (!ok) tc::wait(wbar, 0);    // give copies still in flight one more bounded wait
+    }
     const float* sbias = reinterpret_cast<const float*>(sm + tc::BIAS);
     const float* snorm = reinterpret_cast<const float*>(sm + tc::NORM);
-    const uint32_t tiles = (n + tc::ROWS - 1) / tc::ROWS;
-    for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const uint32_t r = tile * tc::ROWS + row;
-        // layer-1 operand: normalised features, BF16 (the row's 128 bytes as
-        // eight 16-byte loads, all in flight together)
-        float4 xr[DIN / 4];
+    const uint32_t tiles = n / tc::ROWS + (n % tc::ROWS ? 1u : 0u);
+    const uint32_t stride = tc::GROUPS * gridDim.x;
+    // A warp loads 16 feature rows four at a time, eight lanes a row: the
+    // lane's four columns (and their normalisation) are the same in each.
+    const uint32_t xr = (warp & 7u) * 16u + (lane >> 3), xc = (lane & 7u) * 4u;
+    const float4 xmean = *reinterpret_cast<const float4*>(snorm + NX_MEAN + xc);
+    const float4 xinv = *reinterpret_cast<const float4*>(snorm + NX_INV + xc);
+    float4 x[4];
+    auto fetch = [&](uint32_t tile) {
 #pragma unroll
-        for (uint32_t q = 0; q < DIN / 4; q++)
-            xr[q] = r < n ? reinterpret_cast<const float4*>(X + (size_t)r * DIN)[q] : make_float4(0, 0, 0, 0);
-#pragma unroll
-        for (uint32_t kg = 0; kg < DIN / 8; kg++) {
-            const float* xv = reinterpret_cast<const float*>(&xr[2 * kg]);
-            uint32_t w[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const uint32_t c = kg * 8 + 2 * e;
-                const float a = r < n ? (xv[2 * e] - snorm[NX_MEAN + c]) * snorm[NX_INV + c] : 0.0f;
-                const float b = r < n ? (xv[2 * e + 1] - snorm[NX_MEAN + c + 1]) * snorm[NX_INV + c + 1] : 0.0f;
-                w[e] = pack_bf16(a, b);
-            }
-            *reinterpret_cast<uint4*>(sm + tc::ACT + tc::off(row, kg * 8, tc::SBO_K128)) = make_uint4(w[0], w[1], w[2], w[3]);
+        for (uint32_t i = 0; i < 4; i++) {
+            const size_t r = (size_t)tile * tc::ROWS + xr + 4u * i;
+            x[i] = tile < tiles && r < n ? __ldg(reinterpret_cast<const float4*>(X + r * DIN + xc))
+                                         : make_float4(0, 0, 0, 0);
         }
-        for (int layer = 0; layer < 4 && ok; layer++) {
-            tc::fence_proxy();          // the operand writes above are read by the tensor core
-            tc::fence_before();
-            __syncthreads();
-            tc::fence_after();
-            if (t == 0 && issue) {       // issue = false only in the timeout test: nothing ever arrives
-                const uint32_t wbase = layer == 0 ? tc::W1 : (layer == 1 ? tc::W2 : (layer == 2 ? tc::W3 : tc::W4));
-                const uint32_t wsbo = layer == 0 ? tc::SBO_K32 : tc::SBO_K128;
-                const uint32_t steps = layer == 0 ? DIN / 16 : HID / 16;
-                const uint32_t id = tc::idesc(128, layer == 3 ? DOUT : HID);
-                for (uint32_t s = 0; s < steps; s++)
-                    tc::mma(tmem, tc::desc(sbase + tc::ACT + 256u * s, tc::SBO_K128),
-                            tc::desc(sbase + wbase + 256u * s, wsbo), id, s > 0 ? 1u : 0u);
-                tc::commit(bar);
-            }
-            // block-uniform outcome: every thread leaves the loop together
-            ok = __syncthreads_and(tc::wait(bar, phase) ? 1 : 0) != 0;
-            phase ^= 1u;
-            tc::fence_after();
-            if (!ok) break;
-            if (layer < 3) {
-                // bias, ReLU, BF16: the next layer's operand, written in place
-                const float* bias = sbias + 128 * layer;
-#pragma unroll 1
-                for (uint32_t c0 = 0; c0 < HID; c0 += 32) {
-                    float v[32];
-                    tc::ld32(lane_addr + c0, v);
+    };
+    // the fetched rows, normalised, as the BF16 operand of the first layer
+    auto stage = [&](uint32_t tile) {
 #pragma unroll
-                    for (uint32_t kg = 0; kg < 4; kg++) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const uint32_t j = kg * 8 + 2 * e;
-                            w[e] = pack_bf16(fmaxf(v[j] + bias[c0 + j], 0.0f), fmaxf(v[j + 1] + bias[c0 + j + 1], 0.0f));
-                        }
-                        *reinterpret_cast<uint4*>(sm + tc::ACT + tc::off(row, c0 + kg * 8, tc::SBO_K128)) =
-                            make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                }
-            } else {
-                float v[16];
-                tc::ld16(lane_addr, v);
-                if (r < n) {
-#pragma unroll
-                    for (uint32_t c = 0; c < (uint32_t)USED_OUT; c++) {
-                        const float y = v[c] + sbias[3 * 128 + c];
-                        Y[(size_t)r * USED_OUT + c] = y * snorm[NY_STD + c] + snorm[NY_MEAN + c];
-                    }
-                }
-            }
+        for (uint32_t i = 0; i < 4; i++) {
+            const uint32_t rr = xr + 4u * i;
+            const bool in = tile < tiles && (size_t)tile * tc::ROWS + rr < n;
+            const float4 v = x[i];
+            const uint2 w = make_uint2(pack_bf16((v.x - xmean.x) * xinv.x, (v.y - xmean.y) * xinv.y),
+                                       pack_bf16((v.z - xmean.z) * xinv.z, (v.w - xmean.w) * xinv.w));
+            *reinterpret_cast<uint2*>(xt + (rr >> 3) * tc::XSBO + (xc >> 3) * tc::XLBO + (rr & 7u) * 16u +
+                                      (xc & 7u) * 2u) = in ? w : make_uint2(0u, 0u);
         }
-        // every lane's TMEM reads are done before the next tile's MMAs
+    };
+    const bool issuer = warp % (tc::GROUP_THREADS / 32) == 0u && issue;   // a warp; issue = false only in the timeout test
+    auto first_layer = [&]() {
+        for (uint32_t s = 0; s < DIN / 16; s++)
+            tc::mma(tmem + tc::TD, tc::desc(sxt + 2u * tc::XLBO * s, tc::XSBO, tc::XLBO),
+                    tc::desc(sbase + tc::W1 + 256u * s, tc::SBO_K32), tc::idesc(128, HID), s > 0 ? 1u : 0u);
+        tc::commit(bar);
+    };
+    // every thread's TMEM and shared-memory writes and TMEM reads are done;
+    // false when a thread's wait gave up (the same answer for the group)
+    bool failed = false;
+    auto publish = [&]() {
+        tc::fence_proxy();
         tc::fence_before();
-        __syncthreads();
+        const bool all = tc::group_sync(1u + group, failed);
         tc::fence_after();
+        return all;
+    };
+    auto wait = [&](uint32_t b, uint32_t parity) {
+        if (!tc::wait(b, parity)) failed = true;
+        tc::fence_after();
+    };
+    uint32_t tile = blockIdx.x + group * gridDim.x, phase = 0, phase4 = 0;
+    if (tile < tiles && ok) {
+        fetch(tile);
+        stage(tile);
+        fetch(tile + stride);
+        ok = publish();
+        if (issuer && tc::elect_one()) first_layer();
+        for (; tile < tiles && ok; tile += stride) {
+#pragma unroll 1
+            for (int layer = 0; layer < 3 && ok; layer++) {
+                wait(bar, phase);
+                phase ^= 1u;
+                // bias, ReLU, BF16 of this thread's 64 columns: the next layer's operand
+                const float* bias = sbias + 128 * layer + 64u * half;
+                float v[64];
+                tc::ld64(lane_addr + tc::TD + 64u * half, v);
+                uint32_t a[32];
+#pragma unroll
+                for (uint32_t q = 0; q < 16; q++) {
+                    const float4 b = *reinterpret_cast<const float4*>(bias + 4 * q);
+                    float* u = v + 4 * q;
+                    tc::add2(u[0], u[1], b.x, b.y);
+                    tc::add2(u[2], u[3], b.z, b.w);
+                    a[2 * q] = tc::relu_bf16(u[0], u[1]);
+                    a[2 * q + 1] = tc::relu_bf16(u[2], u[3]);
+                }
+                tc::st32(lane_addr + tc::TA + 32u * half, a);
+                ok = publish();
+                if (!ok) break;
+                if (issuer && tc::elect_one()) {
+                    const uint32_t wbase = sbase + (layer == 0 ? tc::W2 : (layer == 1 ? tc::W3 : tc::W4));
+                    const uint32_t id = tc::idesc(128, layer == 2 ? DOUT : HID);
+                    for (uint32_t s = 0; s < HID / 16; s++)
+                        tc::mma_ta(tmem + (layer == 2 ? tc::TY : tc::TD), tmem + tc::TA + 8u * s,
+                                   tc::desc(wbase + 256u * s, tc::SBO_K128), id, s > 0 ? 1u : 0u);
+                    tc::commit(layer == 2 ? bar4 : bar);
+                    if (layer == 2 && tile + stride < tiles) first_layer();
+                }
+                if (layer == 0) {       // the first layer has read its operand: write the next tile's
+                    stage(tile + stride);
+                    if (tile + stride < tiles) fetch(tile + 2u * stride);
+                }
+            }
+            if (!ok) break;
+            wait(bar4, phase4);
+            phase4 ^= 1u;
+            float v[16];
+            tc::ld16(lane_addr + tc::TY, v);
+            const size_t r = (size_t)tile * tc::ROWS + row;
+            if (r < n && !failed) {
+#pragma unroll
+                for (uint32_t c = 0; c < (uint32_t)USED_OUT / 2; c++) {
+                    const uint32_t k = c + half * (USED_OUT / 2);
+                    const float y = (half ? v[c + USED_OUT / 2] : v[c]) + sbias[3 * 128 + k];
+                    Y[r * USED_OUT + k] = y * snorm[NY_STD + k] + snorm[NY_MEAN + k];
+                }
+            }
+        }
+        ok = publish();
     }
-    if (!ok && t == 0) atomicCAS(status, 0u, (uint32_t)AVBD_FAIL_WAIT_TIMEOUT);
+    if (!ok) {
+        if ((t & (tc::GROUP_THREADS - 1u)) == 0u) atomicCAS(status, 0u, (uint32_t)AVBD_FAIL_WAIT_TIMEOUT);
+        if (issue) {                    // products still in flight (bounded)
+            tc::wait(bar, phase ^ 1u);
+            tc::wait(bar4, phase4 ^ 1u);
+        }
+    }
+    tc::fence_before();
     __syncthreads();
+    tc::fence_after();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tc::TMEM_COLS)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(tc::TMEM_COLS)
                      : "memory");
 }
 
@@ -399,8 +563,7 @@ constexpr uint32_t P3 = 0, P2 = P3 + 128 * 128, P1 = P2 + 128 * 128, P4 = P1 + 3
 // the same image: 8-column groups 128 B apart, 8-row (K) groups `sbo` apart
 __device__ __forceinline__ uint64_t kmajor(uint32_t saddr, uint32_t sbo) { return tc::desc(saddr, sbo); }
 __device__ __forceinline__ uint64_t mnmajor(uint32_t saddr, uint32_t sbo) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(sbo >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) |
-           (1ull << 46);
+    return tc::desc(saddr, 128u, sbo);
 }
 constexpr uint32_t MN_A = 1u << 15, MN_B = 1u << 16;          // instruction descriptor: operand is MN-major
 
@@ -424,7 +587,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
              const float* __restrict__ Tg, uint32_t n, float* __restrict__ part, uint32_t* status) {
     using namespace mlp;
     extern __shared__ __align__(128) unsigned char sm[];
-    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31u;
+    const uint32_t t = threadIdx.x, warp = tc::uniform(t >> 5), lane = t & 31u;
     const uint32_t row = t & 127u, half = t >> 7;             // tile row and column half of this thread
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
     const uint32_t bar = sbase + tt::BAR;
@@ -448,7 +611,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + tt::TSLOT);
+    const uint32_t tmem = tc::uniform(*reinterpret_cast<volatile uint32_t*>(sm + tt::TSLOT));
     const uint32_t lane_addr = tmem + (((warp & 3u) * 32u) << 16);  // this warp's 32 TMEM lanes
     uint32_t phase = 0;
     bool ok = true;
@@ -526,7 +689,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
         }
         publish();
         // forward
-        if (t == 0) {
+        if (warp == 0 && tc::elect_one()) {
             for (uint32_t s = 0; s < DIN / 16; s++)
                 tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::X + 256u * s, tt::SBO32),
                         tt::kmajor(sbase + tc::W1 + 256u * s, tc::SBO_K32), tc::idesc(128, 128), s > 0);
@@ -535,7 +698,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
         if (!wait_mma()) break;
         activate(sbias, tt::H1);
         publish();
-        if (t == 0) {
+        if (warp == 0 && tc::elect_one()) {
             for (uint32_t s = 0; s < HID / 16; s++)
                 tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::H1 + 256u * s, tt::SBO128),
                         tt::kmajor(sbase + tc::W2 + 256u * s, tc::SBO_K128), tc::idesc(128, 128), s > 0);
@@ -544,7 +707,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
         if (!wait_mma()) break;
         activate(sbias + 128, tt::H2);
         publish();
-        if (t == 0) {
+        if (warp == 0 && tc::elect_one()) {
             for (uint32_t s = 0; s < HID / 16; s++)
                 tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::H2 + 256u * s, tt::SBO128),
                         tt::kmajor(sbase + tc::W3 + 256u * s, tc::SBO_K128), tc::idesc(128, 128), s > 0);
@@ -553,7 +716,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
         if (!wait_mma()) break;
         activate(sbias + 256, tt::H3);
         publish();
-        if (t == 0) {
+        if (warp == 0 && tc::elect_one()) {
             for (uint32_t s = 0; s < HID / 16; s++)
                 tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::H3 + 256u * s, tt::SBO128),
                         tt::kmajor(sbase + tc::W4 + 256u * s, tc::SBO_K128), tc::idesc(128, 16), s > 0);
@@ -581,7 +744,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
         }
         publish();
         // backward: the input gradient is committed, then the layer's weight gradient follows it
-        if (t == 0) {
+        if (warp == 0 && tc::elect_one()) {
             tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::DY, tt::SBO16), tt::mnmajor(sbase + tc::W4, tc::SBO_K128),
                     tc::idesc(128, 128) | tt::MN_B, 0u);
             tc::commit(bar);
@@ -593,7 +756,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
         if (!wait_mma()) break;
         relu_back(tt::H3, tt::SP, bsum[2]);
         publish();
-        if (t == 0) {
+        if (warp == 0 && tc::elect_one()) {
             for (uint32_t s = 0; s < HID / 16; s++)
                 tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::SP + 256u * s, tt::SBO128),
                         tt::mnmajor(sbase + tc::W3 + 2u * tc::SBO_K128 * s, tc::SBO_K128),
@@ -607,7 +770,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
         if (!wait_mma()) break;                               // dW4's products are complete as well
         relu_back(tt::H2, tt::H3, bsum[1]);
         publish();
-        if (t == 0) {
+        if (warp == 0 && tc::elect_one()) {
             for (uint32_t s = 0; s < HID / 16; s++)
                 tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::H3 + 256u * s, tt::SBO128),
                         tt::mnmajor(sbase + tc::W2 + 2u * tc::SBO_K128 * s, tc::SBO_K128),
@@ -621,7 +784,7 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
         if (!wait_mma()) break;                               // dW3's products are complete as well
         relu_back(tt::H1, tt::H2, bsum[0]);
         publish();
-        if (t == 0) {
+        if (warp == 0 && tc::elect_one()) {
             for (uint32_t s = 0; s < 8; s++)
                 tc::mma(tmem + tt::TW1, tt::mnmajor(sbase + tt::H2 + 2u * tt::SBO128 * s, tt::SBO128),
                         tt::mnmajor(sbase + tt::X + 2u * tt::SBO32 * s, tt::SBO32),
@@ -1063,27 +1226,30 @@ void launch_learn_target(const Params& P, const DevPtrs& d, const Sizes& z, cuda
 }
 void launch_copy_double(const double* src, double* dst, cudaStream_t st) { k_copy_double<<<1, 32, 0, st>>>(src, dst); }
 
-// weights, one activation tile, biases and normalisation: 110 KiB of shared
-// memory (set once per device)
+// weights, two input tiles, biases and normalisation: 98 KiB of shared memory
+// (set once per device)
 static void mlp_infer_attributes() {
     static std::atomic<uint64_t> done{0};
     int dev = 0;
     cudaGetDevice(&dev);
     const uint64_t bit = 1ull << (dev & 63);
     if (done.load() & bit) return;
-    cudaFuncSetAttribute(k_mlp_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM);
+    cudaFuncSetAttribute(k_mlp_infer_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM);
+    cudaFuncSetAttribute(k_mlp_infer_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM);
     done.fetch_or(bit);
 }
 
+// halfW: the weight image of launch_mlp_mirror, or null to convert `prm` in
+// the kernel (a call that would otherwise need the image written first)
 void launch_mlp_infer(const void* halfW, const float* prm, const float* norm, const float* X, uint32_t n, float* Y,
                       uint32_t* status, cudaStream_t st) {
     if (n == 0) return;
     mlp_infer_attributes();
-    // two CTAs per SM (110 KiB of shared memory and 128 TMEM columns each),
-    // every CTA walking 128-row tiles
-    const uint32_t tiles = (n + tc::ROWS - 1) / tc::ROWS;
-    const uint32_t blocks = std::min<uint32_t>(tiles, 2u * 148u);
-    k_mlp_infer_tc<<<blocks, 128, tc::SMEM, st>>>(static_cast<const bf16*>(halfW), prm, norm, X, n, Y, status);
+    const uint32_t tiles = n / tc::ROWS + (n % tc::ROWS ? 1u : 0u);
+    const uint32_t blocks = std::min<uint32_t>(tiles, 148u);
+    const bf16* W = static_cast<const bf16*>(halfW);
+    if (W) k_mlp_infer_tc<true><<<blocks, tc::GROUPS * tc::GROUP_THREADS, tc::SMEM, st>>>(W, prm, norm, X, n, Y, status, true);
+    else k_mlp_infer_tc<false><<<blocks, tc::GROUPS * tc::GROUP_THREADS, tc::SMEM, st>>>(W, prm, norm, X, n, Y, status, true);
 }
 
 void launch_mlp_mirror(const float* prm, void* halfW, cudaStream_t st) {
@@ -1167,17 +1333,14 @@ static int mlp_infer(const float* params, const float* norm, const float* featur
          reinterpret_cast<uintptr_t>(params) | reinterpret_cast<uintptr_t>(norm)) & 15u)
         return AVBD_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // the BF16 weight mirror, then the kernel's status word
-    uint32_t* status = reinterpret_cast<uint32_t*>(static_cast<char*>(workspace) +
-                                                   ((sizeof(bf16) * mlp::NHALF + 255) / 256) * 256);
+    uint32_t* status = static_cast<uint32_t*>(workspace);
     cudaMemsetAsync(status, 0, sizeof(uint32_t), st);
-    launch_mlp_mirror(params, workspace, st);
     if (issue) {
-        launch_mlp_infer(workspace, params, norm, features, n, out, status, st);
+        launch_mlp_infer(nullptr, params, norm, features, n, out, status, st);
     } else if (n) {
         mlp_infer_attributes();
-        k_mlp_infer_tc<<<1, 128, tc::SMEM, st>>>(static_cast<const bf16*>(workspace), params, norm, features, n, out,
-                                                 status, false);
+        k_mlp_infer_tc<false><<<1, tc::GROUPS * tc::GROUP_THREADS, tc::SMEM, st>>>(nullptr, params, norm, features, n, out, status,
+                                                                     false);
     }
     uint32_t h = 0;
     if (cudaMemcpyAsync(&h, status, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
