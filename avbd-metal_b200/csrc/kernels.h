@@ -215,6 +215,7 @@ void launch_soft_normals(const DevPtrs& d, uint32_t numTris, const uint32_t* sur
                          float clothScale, float4* out, cudaStream_t st);
 void launch_skin_deform(const float4* posLin, const SkinBinding* b, uint32_t n, float4* out, cudaStream_t st);
 // shapes: 6 float4 of scratch per environment
+constexpr uint32_t PUSHT_RECORD = 11;   // float4 of an environment's shapes: 24 floats, five pixel ranges
 void launch_pusht_obs(const float4* posLin, const float4* posAng, const PushTDev* envs, uint32_t numEnvs,
                       uint32_t res, float4* shapes, uint8_t* out, cudaStream_t st);
 // spinners and legacy rate motors, then the end-of-frame failure check

@@ -19,12 +19,12 @@ __device__ __forceinline__ void pdl_prologue() {
 
 
 template <typename... KArgs, typename... Args>
-static void launch_pdl(void (*kernel)(KArgs...), uint32_t blocks, uint32_t threads, cudaStream_t st,
-                       Args&&... args) {
+static void launch_pdl_smem(void (*kernel)(KArgs...), uint32_t blocks, uint32_t threads, size_t smem, cudaStream_t st,
+                            Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -32,6 +32,12 @@ static void launch_pdl(void (*kernel)(KArgs...), uint32_t blocks, uint32_t threa
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+static void launch_pdl(void (*kernel)(KArgs...), uint32_t blocks, uint32_t threads, cudaStream_t st,
+                       Args&&... args) {
+    launch_pdl_smem(kernel, blocks, threads, 0, st, std::forward<Args>(args)...);
 }
 
 }  // namespace avbd

@@ -4,10 +4,10 @@
 //
 // Follows Shaders/50_render.metal:7-212 and Shaders/60_robotics.metal:8-69.
 // All of them are one pass over independent records; the Push-T kernel is
-// the byte-heavy one (num_envs x res^2 x 3 bytes) and writes 12-byte pixel
-// quads per thread so that consecutive threads store consecutive words.
+// the byte-heavy one (num_envs x res^2 x 3 bytes).
 #include "dmath.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace avbd {
 
@@ -169,28 +169,44 @@ __device__ __forceinline__ void heading(float4 q, float& cs, float& sn) {
 
 // Push-T observations (60_robotics.metal:21-69) in two passes.
 // k_pusht_shapes: one thread per environment places its shapes (goal T from
-// the table, block T and pusher from the body poses) into 24 floats.
-// k_pusht_obs: blockIdx.y walks the environments; every thread reads its
-// environment's 24 floats (the same address across the block) and
-// classifies pixels.  The pixel-centre offsets (float)j / (res - 1) - 0.5
-// are a shared table (the same division as per pixel, done once per block).
-// A quad of pixels whose centre is farther from a shape's centre than the
-// shape's bounding radius plus two pixel widths cannot touch it, so that
-// shape's exact test is skipped (most quads are background).
-// QUADS (res a multiple of 4): each thread classifies four consecutive
-// pixels of a row into three 32-bit words, the block stages its 3 KB run in
-// shared memory and writes it out as 16-byte stores (the run starts on a
-// 16-byte boundary: 3 * res^2 and 3072 are multiples of 48).  Otherwise one
-// thread per pixel with byte stores.
+// the table, block T and pusher from the body poses) and bounds each of the
+// five (two bars, two stems, the disc) by a range of pixel columns and rows.
+// k_pusht_obs: a block takes tiles of whole pixel rows of one environment: it
+// fills the tile in shared memory with the background (whose three bytes are
+// equal), classifies the pixels of the five ranges only — each by all five
+// tests, so ranges may overlap in any order — and writes the tile out as
+// 16-byte stores.  The tile stands in shared memory at the destination's
+// offset in a 16-byte word, so every resolution takes the same path; the
+// bytes before and after the whole words go out singly.  The next tile's
+// shapes are fetched while the current one is drawn.
+//
+// A range covers the shape's extent plus two pixels and a rounding allowance
+// of the coordinates; a pixel outside it cannot pass the shape's test.  A
+// bound that is not finite (an empty window, a lost pose) covers everything.
+//
+// What bounds it: the 3 bytes a pixel of output and a call's two launches;
+// 4096 environments of 64 x 64 in 24.7 us a call (41.2 us when every quad of
+// pixels ran five bounding-circle tests).
 constexpr uint32_t kObsThreads = 256;
+constexpr uint32_t kObsTile = 16384;             // bytes of whole rows a block draws at once
+constexpr uint32_t kObsRecord = PUSHT_RECORD;    // float4 per environment: 24 floats, five ranges
 
-__device__ __forceinline__ bool near_(float x, float y, float cx, float cy, float r2) {
-    const float dx = x - cx, dy = y - cy;
-    return dx * dx + dy * dy <= r2;
+// pixel range [lo, hi] of world coordinates [c - e, c + e] on an axis whose
+// pixel j has coordinate origin + (j / denom - 0.5) * size; hi < lo if empty
+__device__ __forceinline__ void pixel_range(float c, float e, float origin, float size, float denom, int& lo,
+                                            int& hi) {
+    const float m = e + 2.0f * fabsf(size) / denom + 1.0e-6f * (fabsf(origin) + fabsf(c));
+    const float a = ((c - m - origin) / size + 0.5f) * denom, b = ((c + m - origin) / size + 0.5f) * denom;
+    if (!(fabsf(a) <= 3.0e38f) || !(fabsf(b) <= 3.0e38f)) { lo = 0; hi = (int)denom; return; }
+    lo = (int)floorf(clampf(fminf(a, b), -1.0f, denom + 1.0f));
+    hi = (int)ceilf(clampf(fmaxf(a, b), -1.0f, denom + 1.0f));
+    lo = lo < 0 ? 0 : lo;
+    hi = hi > (int)denom ? (int)denom : hi;
 }
 
 __global__ void k_pusht_shapes(const float4* posLin, const float4* posAng, const PushTDev* envs, uint32_t numEnvs,
                                uint32_t res, float4* shapes) {
+    pdl_trigger();
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= numEnvs) return;
     const PushTDev env = envs[e];
@@ -208,115 +224,109 @@ __global__ void k_pusht_shapes(const float4* posLin, const float4* posAng, const
     sh[14] = posLin[env.ids.x].x; sh[15] = posLin[env.ids.x].y;
     sh[16] = env.frame.x; sh[17] = env.frame.y;
     sh[18] = 2.0f * env.halfWin;
-    // squared cull radii: bar (0.5 x 0.125 half extents), stem (0.125 x
-    // 0.325), pusher disc (0.13), each plus two pixel widths
-    const float pw = fabsf(sh[18]) / (float)(res - 1u);
-    const float rb = 0.5154f + 2.0f * pw, rs = 0.3483f + 2.0f * pw, rt = 0.13f + 2.0f * pw;
-    sh[19] = rb * rb; sh[20] = rs * rs; sh[21] = rt * rt;
-    sh[22] = 0.0f; sh[23] = 0.0f;
-    for (int k = 0; k < 6; k++) shapes[6 * e + k] = make_float4(sh[4 * k], sh[4 * k + 1], sh[4 * k + 2], sh[4 * k + 3]);
+    sh[19] = sh[20] = sh[21] = sh[22] = sh[23] = 0.0f;
+    float4* out = shapes + kObsRecord * (size_t)e;
+    for (int k = 0; k < 6; k++) out[k] = make_float4(sh[4 * k], sh[4 * k + 1], sh[4 * k + 2], sh[4 * k + 3]);
+    // bar (half extents 0.5 x 0.125), stem (0.125 x 0.325) and pusher disc (0.13)
+    const float denom = (float)(res - 1u);
+    const float cx[5] = {sh[0], sh[2], sh[6], sh[10], sh[14]}, cy[5] = {sh[1], sh[3], sh[7], sh[11], sh[15]};
+    const float cc[4] = {gc, gc, sh[8], sh[12]}, ss[4] = {gs, gs, sh[9], sh[13]};
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        const float hx = k == 4 ? 0.13f : ((k & 1) ? 0.125f : 0.5f), hy = k == 4 ? 0.13f : ((k & 1) ? 0.325f : 0.125f);
+        const float c = k == 4 ? 1.0f : fabsf(cc[k < 4 ? k : 0]), s = k == 4 ? 0.0f : fabsf(ss[k < 4 ? k : 0]);
+        int x0, x1, y0, y1;
+        pixel_range(cx[k], c * hx + s * hy, sh[16], sh[18], denom, x0, x1);
+        pixel_range(cy[k], s * hx + c * hy, sh[17], sh[18], denom, y0, y1);
+        out[6 + k] = make_float4(__int_as_float(x0), __int_as_float(x1), __int_as_float(y0), __int_as_float(y1));
+    }
 }
 
-template <bool QUADS>
+// rows of a tile: whole rows, about kObsTile bytes
+__host__ __device__ __forceinline__ uint32_t obs_rows(uint32_t res) {
+    const uint32_t r = kObsTile / (3u * res);
+    return r == 0u ? 1u : (r < res ? r : res);
+}
+
 __global__ void __launch_bounds__(kObsThreads) k_pusht_obs(const float4* shapes, uint32_t numEnvs, uint32_t res,
                                                            uint8_t* out) {
-    extern __shared__ float offs[];  // res entries
-    __shared__ uint32_t words[3 * kObsThreads];
-    const uint32_t perRow = QUADS ? res / 4u : res;
-    const uint32_t perEnv = perRow * res;
-    const uint32_t blockFirst = blockIdx.x * kObsThreads;
-    const uint32_t valid = perEnv - blockFirst < kObsThreads ? perEnv - blockFirst : kObsThreads;
+    extern __shared__ __align__(16) uint8_t img[];   // the tile (from offset 0-15), then the pixel offsets
+    __shared__ float4 rec[2][kObsRecord];
+    const uint32_t t = threadIdx.x;
+    const uint32_t rows = obs_rows(res), perEnv = (res + rows - 1u) / rows;
+    float* offs = reinterpret_cast<float*>(img + ((rows * res * 3u + 31u) & ~15u));
     const float denom = (float)(res - 1u);
-    __shared__ float4 shs[2][6];     // QUADS: this and the next environment's shapes
-    for (uint32_t j = threadIdx.x; j < res; j += kObsThreads) offs[j] = (float)j / denom - 0.5f;
-    if (QUADS && threadIdx.x < 6u && blockIdx.y < numEnvs)
-        shs[0][threadIdx.x] = shapes[6 * (size_t)blockIdx.y + threadIdx.x];
-    __syncthreads();
-    // row and column of this thread's first pixel (quad index / row length)
-    const uint32_t i = blockFirst + threadIdx.x;
-    uint32_t py = i / perRow;
-    const uint32_t px0 = (QUADS ? 4u : 1u) * (i - py * perRow);
+    for (uint32_t j = t; j < res; j += kObsThreads) offs[j] = (float)j / denom - 0.5f;
+    pdl_wait();
+    const uint64_t tiles = (uint64_t)numEnvs * perEnv;
     uint32_t buf = 0;
-    for (uint32_t e = blockIdx.y; e < numEnvs; e += gridDim.y, buf ^= 1u) {
-        float4 s0, s1, s2, s3, s4, s5;
-        if (QUADS) {
-            // six threads fetch the next environment's shapes into the other
-            // buffer (last read an iteration ago, before that iteration's
-            // barriers); they are visible after this iteration's barriers
-            const uint32_t en = e + gridDim.y;
-            if (threadIdx.x < 6u && en < numEnvs) shs[buf ^ 1u][threadIdx.x] = shapes[6 * (size_t)en + threadIdx.x];
-            s0 = shs[buf][0]; s1 = shs[buf][1]; s2 = shs[buf][2]; s3 = shs[buf][3]; s4 = shs[buf][4]; s5 = shs[buf][5];
-        } else {
-            const float4* S = shapes + 6 * (size_t)e;
-            s0 = S[0]; s1 = S[1]; s2 = S[2]; s3 = S[3]; s4 = S[4]; s5 = S[5];
+    if (t < kObsRecord && blockIdx.x < tiles) rec[0][t] = shapes[kObsRecord * (size_t)(blockIdx.x / perEnv) + t];
+    // the palette entries as bytes
+    const uint32_t pal[4][3] = {
+        {to_byte(0.06f), to_byte(0.06f), to_byte(0.06f)},
+        {to_byte(0.10f), to_byte(0.55f), to_byte(0.12f)},
+        {to_byte(0.85f), to_byte(0.15f), to_byte(0.12f)},
+        {to_byte(0.2f), to_byte(0.4f), to_byte(0.95f)}};
+    const uint32_t bg = pal[0][0] * 0x01010101u;
+    for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1u) {
+        const uint32_t e = (uint32_t)(tile / perEnv), row0 = (uint32_t)(tile - (uint64_t)e * perEnv) * rows;
+        const uint32_t nr = row0 + rows <= res ? rows : res - row0, bytes = nr * res * 3u;
+        uint8_t* dst = out + ((size_t)e * res + row0) * res * 3u;
+        const uint32_t skew = (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 15u);
+        for (uint32_t v = t; v < (skew + bytes + 15u) / 16u; v += kObsThreads)
+            reinterpret_cast<uint4*>(img)[v] = make_uint4(bg, bg, bg, bg);
+        if (t < kObsRecord && tile + gridDim.x < tiles)
+            rec[buf ^ 1u][t] = shapes[kObsRecord * (size_t)((tile + gridDim.x) / perEnv) + t];
+        __syncthreads();
+        const float4 s0 = rec[buf][0], s1 = rec[buf][1], s2 = rec[buf][2], s3 = rec[buf][3], s4 = rec[buf][4];
+        // the pixels of the five ranges that lie in this tile's rows, one after another
+        uint32_t width[5], first[6];
+        int x0[5], y0[5];
+        first[0] = 0u;
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            const float4 r = rec[buf][6 + k];
+            x0[k] = __float_as_int(r.x);
+            const int x1 = __float_as_int(r.y), yb = (int)row0, ye = (int)(row0 + nr) - 1;
+            y0[k] = max(__float_as_int(r.z), yb);
+            const int y1 = min(__float_as_int(r.w), ye);
+            width[k] = x1 >= x0[k] ? (uint32_t)(x1 - x0[k] + 1) : 0u;
+            first[k + 1] = first[k] + (y1 >= y0[k] ? width[k] * (uint32_t)(y1 - y0[k] + 1) : 0u);
         }
-        uint32_t kinds = 0;  // 2 bits per pixel: 0 background, 1 goal, 2 block, 3 pusher
-        if (threadIdx.x < valid) {
-            constexpr int N = QUADS ? 4 : 1;
-            const float wy = s4.y + offs[py] * s4.z;
-            float wx[N];
+        for (uint32_t i = t; i < first[5]; i += kObsThreads) {
+            uint32_t w = width[0], f = first[0];
+            int bx = x0[0], by = y0[0];
 #pragma unroll
-            for (int k = 0; k < N; k++) wx[k] = s4.x + offs[px0 + k] * s4.z;
-            const float cx = 0.5f * (wx[0] + wx[N - 1]);
-            const bool gBar = near_(cx, wy, s0.x, s0.y, s4.w), gStem = near_(cx, wy, s0.z, s0.w, s5.x);
-            const bool bBar = near_(cx, wy, s1.z, s1.w, s4.w), bStem = near_(cx, wy, s2.z, s2.w, s5.x);
-            const bool tip = near_(cx, wy, s3.z, s3.w, s5.y);
-            if (gBar || gStem || bBar || bStem || tip) {
-#pragma unroll
-                for (int k = 0; k < N; k++) {
-                    uint32_t kind = 0;
-                    if ((gBar && in_box(wx[k], wy, s0.x, s0.y, s1.x, s1.y, 0.5f, 0.125f)) ||
-                        (gStem && in_box(wx[k], wy, s0.z, s0.w, s1.x, s1.y, 0.125f, 0.325f)))
-                        kind = 1;
-                    if (bBar && in_box(wx[k], wy, s1.z, s1.w, s2.x, s2.y, 0.5f, 0.125f)) kind = 2;
-                    if (bStem && in_box(wx[k], wy, s2.z, s2.w, s3.x, s3.y, 0.125f, 0.325f)) kind = 2;
-                    if (tip) {
-                        const float dx = wx[k] - s3.z, dy = wy - s3.w;
-                        if (sqrtf(dx * dx + dy * dy) < 0.13f) kind = 3;
-                    }
-                    kinds |= kind << (2 * k);
-                }
+            for (int k = 1; k < 5; k++)
+                if (i >= first[k]) { w = width[k]; f = first[k]; bx = x0[k]; by = y0[k]; }
+            const uint32_t q = (i - f) / w;
+            const uint32_t py = (uint32_t)by + q, px = (uint32_t)bx + (i - f - q * w);
+            const float wx = s4.x + offs[px] * s4.z, wy = s4.y + offs[py] * s4.z;
+            uint32_t kind = 0;
+            if (in_box(wx, wy, s0.x, s0.y, s1.x, s1.y, 0.5f, 0.125f) ||
+                in_box(wx, wy, s0.z, s0.w, s1.x, s1.y, 0.125f, 0.325f))
+                kind = 1;
+            if (in_box(wx, wy, s1.z, s1.w, s2.x, s2.y, 0.5f, 0.125f)) kind = 2;
+            if (in_box(wx, wy, s2.z, s2.w, s3.x, s3.y, 0.125f, 0.325f)) kind = 2;
+            const float dx = wx - s3.z, dy = wy - s3.w;
+            if (sqrtf(dx * dx + dy * dy) < 0.13f) kind = 3;
+            if (kind) {
+                uint8_t* o = img + skew + ((py - row0) * res + px) * 3u;
+                o[0] = (uint8_t)(kind == 1 ? pal[1][0] : (kind == 2 ? pal[2][0] : pal[3][0]));
+                o[1] = (uint8_t)(kind == 1 ? pal[1][1] : (kind == 2 ? pal[2][1] : pal[3][1]));
+                o[2] = (uint8_t)(kind == 1 ? pal[1][2] : (kind == 2 ? pal[2][2] : pal[3][2]));
             }
         }
-        // the four palette entries as bytes
-        const uint32_t pal[4][3] = {
-            {to_byte(0.06f), to_byte(0.06f), to_byte(0.06f)},
-            {to_byte(0.10f), to_byte(0.55f), to_byte(0.12f)},
-            {to_byte(0.85f), to_byte(0.15f), to_byte(0.12f)},
-            {to_byte(0.2f), to_byte(0.4f), to_byte(0.95f)}};
-        if (QUADS) {
-            uint32_t w0, w1, w2;
-            if (kinds == 0u) {  // four background pixels
-                const uint32_t g = pal[0][0];
-                w0 = w1 = w2 = g | (g << 8) | (g << 16) | (g << 24);
-            } else {
-                uint32_t b[12];
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const uint32_t kind = (kinds >> (2 * k)) & 3u;
-                    b[3 * k] = pal[kind][0]; b[3 * k + 1] = pal[kind][1]; b[3 * k + 2] = pal[kind][2];
-                }
-                w0 = b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24);
-                w1 = b[4] | (b[5] << 8) | (b[6] << 16) | (b[7] << 24);
-                w2 = b[8] | (b[9] << 8) | (b[10] << 16) | (b[11] << 24);
-            }
-            __syncthreads();  // the previous environment's words are out
-            words[3 * threadIdx.x] = w0;
-            words[3 * threadIdx.x + 1] = w1;
-            words[3 * threadIdx.x + 2] = w2;
-            __syncthreads();
-            // 3 * valid words from byte (e * res^2 + 4 * blockFirst) * 3
-            uint32_t* dst = reinterpret_cast<uint32_t*>(out + ((size_t)e * res * res + 4u * (size_t)blockFirst) * 3u);
-            const uint32_t nWords = 3u * valid, nVec = nWords / 4u;
-            for (uint32_t v = threadIdx.x; v < nVec; v += kObsThreads)
-                reinterpret_cast<uint4*>(dst)[v] =
-                    make_uint4(words[4 * v], words[4 * v + 1], words[4 * v + 2], words[4 * v + 3]);
-            for (uint32_t w = 4u * nVec + threadIdx.x; w < nWords; w += kObsThreads) dst[w] = words[w];
-        } else if (threadIdx.x < valid) {
-            const uint32_t kind = kinds & 3u;
-            uint8_t* o = out + ((size_t)e * res * res + i) * 3u;
-            o[0] = (uint8_t)pal[kind][0]; o[1] = (uint8_t)pal[kind][1]; o[2] = (uint8_t)pal[kind][2];
-        }
+        __syncthreads();
+        // whole 16-byte words, then the bytes at the two ends
+        const uint32_t head = skew ? min(16u - skew, bytes) : 0u, words = (bytes - head) / 16u;
+        const uint32_t tail = bytes - head - 16u * words;
+        const uint4* src = reinterpret_cast<const uint4*>(img + skew + head);
+        uint4* dv = reinterpret_cast<uint4*>(dst + head);
+        for (uint32_t v = t; v < words; v += kObsThreads) dv[v] = src[v];
+        if (t < head) dst[t] = img[skew + t];
+        else if (t >= 32u && t - 32u < tail) dst[head + 16u * words + t - 32u] = img[skew + head + 16u * words + t - 32u];
+        __syncthreads();
     }
 }
 
@@ -343,19 +353,14 @@ void launch_skin_deform(const float4* posLin, const SkinBinding* b, uint32_t n, 
 void launch_pusht_obs(const float4* posLin, const float4* posAng, const PushTDev* envs, uint32_t numEnvs,
                       uint32_t res, float4* shapes, uint8_t* out, cudaStream_t st) {
     if (!numEnvs) return;
-    k_pusht_shapes<<<blocks_for(numEnvs, 128), 128, 0, st>>>(posLin, posAng, envs, numEnvs, res, shapes);
-    const bool quads = res % 4u == 0u;
-    const uint32_t perEnv = quads ? res * res / 4u : res * res;
-    // about eight resident blocks per SM in all; each block walks several
-    // environments so that its offset table is built once for many
-    const uint32_t bx = blocks_for(perEnv, kObsThreads);
-    uint32_t by = (148u * 8u + bx - 1u) / bx;
-    by = by < numEnvs ? by : numEnvs;
-    by = by < 65535u ? (by ? by : 1u) : 65535u;
-    const dim3 grid(bx, by);
-    const size_t smem = sizeof(float) * res;  // res <= 4096: at most 16 KB
-    if (quads) k_pusht_obs<true><<<grid, kObsThreads, smem, st>>>(shapes, numEnvs, res, out);
-    else k_pusht_obs<false><<<grid, kObsThreads, smem, st>>>(shapes, numEnvs, res, out);
+    k_pusht_shapes<<<blocks_for(numEnvs, 64), 64, 0, st>>>(posLin, posAng, envs, numEnvs, res, shapes);
+    // one resident wave of blocks walks the tiles (about 17 KB of shared
+    // memory and 256 threads each: eight blocks an SM)
+    const uint32_t rows = obs_rows(res);
+    const uint64_t tiles = (uint64_t)numEnvs * ((res + rows - 1u) / rows);
+    const uint32_t grid = (uint32_t)(tiles < 148u * 8u ? tiles : 148u * 8u);
+    const size_t smem = ((rows * res * 3u + 31u) & ~15u) + sizeof(float) * res;   // at most 33 KB
+    launch_pdl_smem(k_pusht_obs, grid, kObsThreads, smem, st, (const float4*)shapes, numEnvs, res, out);
 }
 
 }  // namespace avbd

@@ -179,7 +179,7 @@ struct avbd_solver {
     // caller passes the same records
     std::vector<avbd_pusht_env> pushtHost;
     PushTDev* pushtDev = nullptr;
-    float4* pushtShapes = nullptr;  // 6 float4 per environment
+    float4* pushtShapes = nullptr;  // PUSHT_RECORD float4 per environment
     size_t pushtCap = 0;
 
     ~avbd_solver() {
@@ -1514,7 +1514,7 @@ int avbd_render_pusht_obs(avbd_solver* s, const avbd_pusht_env* envs, uint32_t n
             s->pushtShapes = nullptr;
             s->pushtCap = 0;
             if (cudaMalloc(&s->pushtDev, sizeof(PushTDev) * (size_t)num_envs) != cudaSuccess ||
-                cudaMalloc(&s->pushtShapes, 6 * sizeof(float4) * (size_t)num_envs) != cudaSuccess)
+                cudaMalloc(&s->pushtShapes, PUSHT_RECORD * sizeof(float4) * (size_t)num_envs) != cudaSuccess)
                 return AVBD_ERR_ALLOC_FAILED;
             s->pushtCap = num_envs;
         }
