@@ -152,6 +152,8 @@ struct Counters {
     uint32_t numSoftVT, numSoftEE;   // isotropic element contacts of this frame
     uint32_t ogcQueue;               // trackers that reseed from the grid this frame
     uint32_t adjLong;                // bodies whose contact segment is sorted by a block
+    uint32_t tailTickets[2];         // DevPtrs::tailTicket of the solve and of a predicted trial branch
+    uint32_t activeManifolds;        // manifolds with contacts (DevPtrs::activeManifolds)
 };
 
 }  // namespace avbd

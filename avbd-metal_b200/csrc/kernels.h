@@ -64,6 +64,8 @@ struct DevPtrs {
     uint32_t *dynCount, *dynStart, *dynCursor, *dynList;
     uint32_t* dynSplit;                   // manifold entries at the head of each sorted dyn segment
     uint32_t* adjLongQueue;               // bodies with long contact segments this frame
+    uint32_t* activeManifolds;            // manifolds with contacts, in no order
+    uint32_t* tailTicket;                 // blocks done with the last launched color (zero between launches)
     uint32_t* postTets;                   // tet entries at the head of each static post segment
     const TetGPU* tetInc;                 // tet records in postList order (null without tets)
     // coloring
@@ -183,14 +185,13 @@ void launch_dynamic_coloring(const Params& P, const DevPtrs& d, const Sizes& z, 
 constexpr uint32_t NO_HOST_START = 0xFFFFFFFFu;   // a color start the kernel reads on the device
 constexpr uint32_t AVBD_PRIMAL_STAGED = 1;
 void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t color,
-                         uint32_t count, uint32_t lanes, cudaStream_t st, cudaStream_t side = nullptr,
+                         uint32_t count, uint32_t lanes, bool last, cudaStream_t st, cudaStream_t side = nullptr,
                          cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
 // squared AL-gradient norm of every dynamic body (perBody[numDynamicBodies])
 // and their fixed-order sum (total)
 void launch_residual(const Params& P, const DevPtrs& d, const Sizes& z, float* perBody, double* total,
                      cudaStream_t st);
 // dynamic coloring: colors [first, 64) in one block, after the per-color launches
-void launch_primal_tail(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t first, cudaStream_t st);
 // every iteration of a small scene in one thread block
 void launch_solve_small(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t colorBound,
                         cudaStream_t st);

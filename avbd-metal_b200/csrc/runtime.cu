@@ -130,8 +130,8 @@ struct avbd_solver {
     uint64_t kernelsPerFrame = 0;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     bool graphsValid = false;
-    // Dynamic coloring: the frame graph launches this many colors one by one
-    // and a single-block tail kernel takes the rest.  It grows (and the graphs
+    // Dynamic coloring: the frame graph launches this many colors one by one;
+    // one block of the last launch takes the rest.  It grows (and the graphs
     // are re-captured) when a retired frame used more colors.
     uint32_t colorLaunchBound = 8;
     bool colorBoundFitted = false;
@@ -273,6 +273,8 @@ struct avbd_solver {
                                                                       offsetof(Counters, ogcSlots))
                                         : nullptr;
         f.ogcExceed = ogcSlots;
+        uint32_t* tickets = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(d.counters) + offsetof(Counters, tailTickets));
+        f.tailTicket = tickets;
         usedEvents = 0;
         uint32_t primalLaunch = 0;
         auto mark = [&](int stage) {
@@ -314,11 +316,10 @@ struct avbd_solver {
             for (uint32_t c = 0; c < colorBound; c++) {
                 const uint32_t count = z.dynamicColoring ? 0xFFFFFFFFu : H.colorCounts[c];
                 if (count == 0) continue;
-                launch_primal_color(P, g, z, c, count, H.colorLanes[c], sst);
+                launch_primal_color(P, g, z, c, count, H.colorLanes[c], c + 1 == colorBound, sst);
                 if (P.ogc)
                     launch_publish_color(P, g, c, count, z.dynamicColoring ? NO_HOST_START : H.colorStart[c], sst);
             }
-            if (z.dynamicColoring) launch_primal_tail(P, g, z, colorLaunchBound, sst);
         };
         const bool tuningFrame = primalEvents != nullptr;
         const bool learned = !tuningFrame && learnMode == AVBD_WARM_START_LEARNED && modelSet && z.numLearn;
@@ -345,6 +346,7 @@ struct avbd_solver {
             DevPtrs fb = f, fp = f;
             fb.posLin = f.learnSweptLin;
             fb.posAng = f.learnSweptAng;
+            fb.tailTicket = tickets + 1;       // the two branches' sweeps run side by side
             // the trial sweeps count OGC bound exceeders in slots 2 (plain) and 3 (predicted)
             if (ogcSlots) { fp.ogcExceed = ogcSlots + 2; fb.ogcExceed = ogcSlots + 3; }
             launch_mlp_infer(f.learnHalf, f.learnPrm, f.learnNorm, f.learnFeat, z.numLearn, f.learnPred,
@@ -395,8 +397,8 @@ struct avbd_solver {
                     if (count == 0) continue;
                     mark(AVBD_STAGE_PRIMAL);
                     if (primalEvents) cudaEventRecord(primalEvents[2 * primalLaunch], st);
-                    launch_primal_color(P, g, z, c, count, lanes ? lanes[c] : H.colorLanes[c], st, branchStream,
-                                        wideFork, wideJoin);
+                    launch_primal_color(P, g, z, c, count, lanes ? lanes[c] : H.colorLanes[c], c + 1 == colorBound, st,
+                                        branchStream, wideFork, wideJoin);
                     if (primalEvents) cudaEventRecord(primalEvents[2 * primalLaunch + 1], st);
                     primalLaunch++;
                     if (P.cloth) {
@@ -407,7 +409,6 @@ struct avbd_solver {
                                              st);
                     }
                 }
-                if (z.dynamicColoring && !(reuseTrial && it == 0)) launch_primal_tail(P, g, z, colorLaunchBound, st);
                 mark(AVBD_STAGE_DUAL);
                 launch_dual(P, f, z, st);
                 if (P.ogc && it + 1 < P.iterations) {
@@ -596,7 +597,7 @@ struct avbd_solver {
             d.tetInc = ti;
         }
 #endif
-        ok = ok && alloc(d.adjLongQueue, nb, "adjLongQueue");
+        ok = ok && alloc(d.adjLongQueue, nb, "adjLongQueue") && alloc(d.activeManifolds, H.maxPairs, "activeManifolds");
         ok = ok && alloc(d.dynList, 2 * (size_t)H.maxPairs + ((P.cloth || P.ogc) ? 4 * (size_t)P.maxSoft : 0), "dynList");
         // coloring
         ok = ok && upload(d.colorsA, H.colors, "colorsA", true) && upload(d.colorsB, H.colors, "colorsB");
@@ -765,9 +766,10 @@ struct avbd_solver {
         if (!check(cudaMemcpy(hostLatch, d.failureLatch, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost), "latch readback"))
             return AVBD_ERR_RUNTIME_FAILURE;
         if (z.dynamicColoring && hostLatch[3] > 0) {
-            // first retirement: fit the bound to the palette seen so far
-            // (two colors of headroom); later frames only grow it
-            const uint32_t want = std::min<uint32_t>(MAX_COLORS, hostLatch[3] + 2);
+            // first retirement: fit the bound to the palette seen so far;
+            // later frames only grow it (a frame that needs more colors
+            // solves them in its last color's launch)
+            const uint32_t want = std::min<uint32_t>(MAX_COLORS, hostLatch[3]);
             if (want > colorLaunchBound || (!colorBoundFitted && want < colorLaunchBound)) {
                 colorLaunchBound = want;
                 graphsValid = false;
@@ -892,7 +894,7 @@ struct avbd_solver {
         const DynShape sh = kDynShapes[dynTuneStage];
         z.dynBlocks = 148u * sh.blocksPerSM;
         z.dynThreads = sh.threads;
-        const size_t need = 2 * (size_t)P.iterations * (colorLaunchBound + 1);
+        const size_t need = 2 * (size_t)P.iterations * colorLaunchBound;
         while (tuneEvents.size() < need) {
             cudaEvent_t e;
             if (!check(cudaEventCreate(&e), "event create")) return AVBD_ERR_RUNTIME_FAILURE;

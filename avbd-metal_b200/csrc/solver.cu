@@ -14,6 +14,8 @@
 // tets) is built once at upload; only contact entries are rebuilt per frame.
 #include <utility>
 
+#include <atomic>
+
 #include "dmath.cuh"
 #include "kernels.h"
 #include "pdl.cuh"
@@ -178,6 +180,9 @@ __global__ void k_adj_dyn(const Params P, const DevPtrs d) {
             const u4 h = d.manifolds[i].header;
             if (h.z == 0) continue;
             const uint32_t e = (FK_MANIFOLD << ADJ_KIND_SHIFT) | i;
+            // the dual visits only manifolds with contacts, in any order
+            // (their updates are independent)
+            if (!SCATTER) d.activeManifolds[atomicAdd(&d.counters->activeManifolds, 1u)] = i;
             put(h.x, e);
             put(h.y, e);
         } else {
@@ -370,10 +375,9 @@ __device__ __forceinline__ void scan_neighbors(const DevPtrs& d, uint32_t b, uin
 
 __device__ __forceinline__ uint32_t ctz32(uint32_t x) { return (uint32_t)(__ffs((int)x) - 1); }
 
-__global__ void k_color_iterate(const Params P, const DevPtrs d, const uint32_t* src, uint32_t* dst, uint32_t pass) {
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= P.numBodies) return;
-    if (pass > 0 && d.counters->changed[pass - 1] == 0u) return;
+// One body of a Jacobi coloring pass.
+__device__ __forceinline__ void color_step(const DevPtrs& d, uint32_t gid, const uint32_t* src, uint32_t* dst,
+                                           uint32_t pass) {
     if (d.posLin[gid].w <= 0.0f) { dst[gid] = 0; return; }
     const uint32_t my = src[gid];
     uint32_t mLo = 0, mHi = 0, aLo = 0, aHi = 0;
@@ -395,9 +399,7 @@ __global__ void k_color_iterate(const Params P, const DevPtrs d, const uint32_t*
 }
 
 // Serial greedy completion when the bounded parallel phase has not settled.
-__global__ void k_color_repair(const Params P, const DevPtrs d, uint32_t* colors, uint32_t finalPass) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    if (d.counters->changed[finalPass] == 0u) return;
+__device__ void color_repair(const Params& P, const DevPtrs& d, uint32_t* colors) {
     for (uint32_t self = 0; self < P.numBodies; self++) {
         if (d.posLin[self].w <= 0.0f) { colors[self] = 0; continue; }
         uint32_t mLo = 0, mHi = 0, aLo = 0, aHi = 0;
@@ -409,9 +411,8 @@ __global__ void k_color_repair(const Params P, const DevPtrs d, uint32_t* colors
     }
 }
 
-__global__ void k_color_validate_count(const Params P, const DevPtrs d, const uint32_t* colors) {
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= P.numBodies || d.posLin[gid].w <= 0.0f) return;
+__device__ __forceinline__ void color_count(const DevPtrs& d, uint32_t gid, const uint32_t* colors) {
+    if (d.posLin[gid].w <= 0.0f) return;
     uint32_t mLo = 0, mHi = 0, aLo = 0, aHi = 0;
     bool conflict = false;
     scan_neighbors(d, gid, colors[gid], colors, mLo, mHi, aLo, aHi, conflict);
@@ -419,8 +420,7 @@ __global__ void k_color_validate_count(const Params P, const DevPtrs d, const ui
     d.bodySlot[gid] = atomicAdd(&d.counters->colorCount[colors[gid]], 1u);
 }
 
-__global__ void k_color_scan(const DevPtrs d) {
-    if (threadIdx.x != 0) return;
+__device__ void color_scan(const DevPtrs& d) {
     uint32_t run = 0, used = 0;
     for (int c = 0; c < MAX_COLORS; c++) {
         d.counters->colorStart[c] = run;
@@ -433,22 +433,103 @@ __global__ void k_color_scan(const DevPtrs d) {
     d.counters->usedColors = used;
 }
 
-__global__ void k_color_scatter(const Params P, const DevPtrs d, const uint32_t* colors) {
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= P.numBodies || d.posLin[gid].w <= 0.0f) return;
+__device__ __forceinline__ void color_place(const DevPtrs& d, uint32_t gid, const uint32_t* colors) {
+    if (d.posLin[gid].w <= 0.0f) return;
     d.colorList[d.counters->colorStart[colors[gid]] + d.bodySlot[gid]] = gid;
 }
 
+constexpr int kColorPasses = 20;
+
+// The whole coloring in one launch of a cluster (one CTA for small scenes):
+// passes between barriers until one changes nothing, usually the first or
+// second because a frame starts from the last frame's colors, then count, scan
+// and place.  As 24 launches, most of which found nothing to do, it took 28 us
+// of a 250 us frame of 20 bodies and 54 us at 28,673 bodies (4,096 worlds).
+// Above 65,536 bodies the passes use the whole device, a launch each.
+template <bool CLUSTER>
+__global__ void __launch_bounds__(1024) k_color(const Params P, const DevPtrs d) {
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    const volatile uint32_t* changed = d.counters->changed;
+    auto barrier = [&]() {
+        if (CLUSTER) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+    };
+    for (int pass = 0; pass < kColorPasses; pass++) {
+        if (pass > 0 && changed[pass - 1] == 0u) break;          // the same in every thread
+        const uint32_t* src = (pass & 1) ? d.colorsB : d.colorsA;
+        uint32_t* dst = (pass & 1) ? d.colorsA : d.colorsB;
+        for (uint32_t gid = first; gid < P.numBodies; gid += step) color_step(d, gid, src, dst, (uint32_t)pass);
+        barrier();
+    }
+    if (changed[kColorPasses - 1] != 0u) {
+        if (first == 0) color_repair(P, d, d.colorsA);
+        barrier();
+    }
+    for (uint32_t gid = first; gid < P.numBodies; gid += step) color_count(d, gid, d.colorsA);
+    barrier();
+    if (first == 0) color_scan(d);
+    barrier();
+    for (uint32_t gid = first; gid < P.numBodies; gid += step) color_place(d, gid, d.colorsA);
+}
+
+__global__ void k_color_iterate(const Params P, const DevPtrs d, const uint32_t* src, uint32_t* dst, uint32_t pass) {
+    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid >= P.numBodies) return;
+    if (pass > 0 && d.counters->changed[pass - 1] == 0u) return;
+    color_step(d, gid, src, dst, pass);
+}
+__global__ void k_color_repair(const Params P, const DevPtrs d, uint32_t* colors, uint32_t finalPass) {
+    if (threadIdx.x == 0 && d.counters->changed[finalPass] != 0u) color_repair(P, d, colors);
+}
+__global__ void k_color_validate_count(const Params P, const DevPtrs d, const uint32_t* colors) {
+    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid < P.numBodies) color_count(d, gid, colors);
+}
+__global__ void k_color_scan(const DevPtrs d) {
+    if (threadIdx.x == 0) color_scan(d);
+}
+__global__ void k_color_scatter(const Params P, const DevPtrs d, const uint32_t* colors) {
+    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid < P.numBodies) color_place(d, gid, colors);
+}
+
+// one launch of a grid that is one cluster
+template <typename... KArgs, typename... Args>
+static void launch_cluster(void (*kernel)(KArgs...), uint32_t ctas, uint32_t threads, size_t smem, cudaStream_t st,
+                           Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 void launch_dynamic_coloring(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
+    if (P.numBodies <= 1024u) { launch_cluster(k_color<false>, 1, 1024, 0, st, P, d); return; }
+    if (P.numBodies <= 65536u) {
+        launch_cluster(k_color<true>, P.numBodies <= 4096u ? 4 : 8, 1024, 0, st, P, d);
+        return;
+    }
     const int T = 128;
     const uint32_t blocks = (P.numBodies + T - 1) / T;
-    const int passes = 20;
-    for (int pass = 0; pass < passes; pass++) {
+    for (int pass = 0; pass < kColorPasses; pass++) {
         const uint32_t* src = (pass & 1) ? d.colorsB : d.colorsA;
         uint32_t* dst = (pass & 1) ? d.colorsA : d.colorsB;
         k_color_iterate<<<blocks, T, 0, st>>>(P, d, src, dst, (uint32_t)pass);
     }
-    k_color_repair<<<1, 1, 0, st>>>(P, d, d.colorsA, passes - 1);
+    k_color_repair<<<1, 32, 0, st>>>(P, d, d.colorsA, kColorPasses - 1);
     k_color_validate_count<<<blocks, T, 0, st>>>(P, d, d.colorsA);
     k_color_scan<<<1, 32, 0, st>>>(d);
     k_color_scatter<<<blocks, T, 0, st>>>(P, d, d.colorsA);
@@ -652,14 +733,41 @@ __device__ __forceinline__ float3 contact_force(const ContactGPU& c, float3 nrm,
 // What one contact point (or one rigid element-contact slot) adds to a
 // body's 6x6 system: each accumulator component takes exactly one add per
 // point, so a point's increment can be formed anywhere and added later in
-// the original order with the same result.
+// the original order with the same result.  The solve reads the lower
+// triangles of the two diagonal blocks only, so a stored increment keeps 27
+// of the 33 floats.
 struct PointInc { M3 lhsLin, lhsAng, lhsCross; float3 rhsLin, rhsAng; };
+constexpr int kIncWords = 27;
 __device__ __forceinline__ void add_inc(Accum& acc, const PointInc& x) {
     acc.lhsLin = m3_add(acc.lhsLin, x.lhsLin);
     acc.lhsAng = m3_add(acc.lhsAng, x.lhsAng);
     acc.lhsCross = m3_add(acc.lhsCross, x.lhsCross);
     acc.rhsLin += x.rhsLin;
     acc.rhsAng += x.rhsAng;
+}
+// the component-th float of a stored increment is `stride` floats after the one before
+__device__ __forceinline__ void store_inc(float* at, int stride, const PointInc& x) {
+    const float w[kIncWords] = {x.lhsLin.r0.x, x.lhsLin.r1.x, x.lhsLin.r1.y, x.lhsLin.r2.x, x.lhsLin.r2.y,
+                                x.lhsLin.r2.z, x.lhsAng.r0.x, x.lhsAng.r1.x, x.lhsAng.r1.y, x.lhsAng.r2.x,
+                                x.lhsAng.r2.y, x.lhsAng.r2.z, x.lhsCross.r0.x, x.lhsCross.r0.y, x.lhsCross.r0.z,
+                                x.lhsCross.r1.x, x.lhsCross.r1.y, x.lhsCross.r1.z, x.lhsCross.r2.x, x.lhsCross.r2.y,
+                                x.lhsCross.r2.z, x.rhsLin.x, x.rhsLin.y, x.rhsLin.z, x.rhsAng.x, x.rhsAng.y, x.rhsAng.z};
+#pragma unroll
+    for (int c = 0; c < kIncWords; c++) at[c * stride] = w[c];
+}
+__device__ __forceinline__ void add_stored_inc(Accum& acc, const float* at, int stride) {
+    float w[kIncWords];
+#pragma unroll
+    for (int c = 0; c < kIncWords; c++) w[c] = at[c * stride];
+    acc.lhsLin.r0.x += w[0]; acc.lhsLin.r1.x += w[1]; acc.lhsLin.r1.y += w[2];
+    acc.lhsLin.r2.x += w[3]; acc.lhsLin.r2.y += w[4]; acc.lhsLin.r2.z += w[5];
+    acc.lhsAng.r0.x += w[6]; acc.lhsAng.r1.x += w[7]; acc.lhsAng.r1.y += w[8];
+    acc.lhsAng.r2.x += w[9]; acc.lhsAng.r2.y += w[10]; acc.lhsAng.r2.z += w[11];
+    acc.lhsCross.r0 += mk3(w[12], w[13], w[14]);
+    acc.lhsCross.r1 += mk3(w[15], w[16], w[17]);
+    acc.lhsCross.r2 += mk3(w[18], w[19], w[20]);
+    acc.rhsLin += mk3(w[21], w[22], w[23]);
+    acc.rhsAng += mk3(w[24], w[25], w[26]);
 }
 // Jacobian-weighted increment of a contact frame with world lever rW.
 __device__ __forceinline__ PointInc point_inc(const M3& jLin, float3 rW, const M3& K, float3 F) {
@@ -852,11 +960,12 @@ __device__ void stamp_soft(const Params& P, const DevPtrs& d, const SoftContactG
     }
 }
 
+template <bool MANIFOLDS = true>
 __device__ __forceinline__ void stamp_entry(const Params& P, const DevPtrs& d, uint32_t entry, uint32_t body,
                                             Accum& acc) {
     const uint32_t kind = entry >> ADJ_KIND_SHIFT, idx = entry & ADJ_INDEX_MASK;
     if (kind == FK_TET) stamp_tet(d, d.tets[idx], body, acc);
-    else if (kind == FK_MANIFOLD) stamp_manifold(P, d, d.manifolds[idx], body, acc);
+    else if (MANIFOLDS && kind == FK_MANIFOLD) stamp_manifold(P, d, d.manifolds[idx], body, acc);
     else if (kind == FK_JOINT) stamp_joint(P, d, d.joints[idx], body, acc);
     else if (kind == FK_SPRING) stamp_spring(P, d, d.springs[idx], body, acc);
     else if (kind == FK_SOFT) stamp_soft(P, d, d.soft[idx], body, acc);
@@ -868,6 +977,14 @@ __device__ __forceinline__ float3 shfl3(unsigned mask, float3 v, int o) {
     return mk3(__shfl_xor_sync(mask, v.x, o, 8), __shfl_xor_sync(mask, v.y, o, 8), __shfl_xor_sync(mask, v.z, o, 8));
 }
 __device__ __forceinline__ void add_shfl3(unsigned mask, float3& v, int o) { v = v + shfl3(mask, v, o); }
+// the lower triangle of a diagonal block: all that the solves read (what no
+// lane sends is not computed either)
+__device__ __forceinline__ void add_shfl_lower(unsigned mask, M3& m, int o) {
+    m.r0.x += __shfl_xor_sync(mask, m.r0.x, o, 8);
+    m.r1.x += __shfl_xor_sync(mask, m.r1.x, o, 8);
+    m.r1.y += __shfl_xor_sync(mask, m.r1.y, o, 8);
+    add_shfl3(mask, m.r2, o);
+}
 
 // Isotropic-OGC conservative-bound truncation (ogcTruncate,
 // 40_solver.metal:1361-1382): the displacement since the bound's anchor stays
@@ -903,14 +1020,10 @@ __device__ __forceinline__ void body_commit(const Params& P, const DevPtrs& d, u
     const bool rigid = shp.w >= 0.0f;
 #pragma unroll
     for (int o = 4; o >= 1; o >>= 1) {
-        add_shfl3(mask, acc.lhsLin.r0, o);
-        add_shfl3(mask, acc.lhsLin.r1, o);
-        add_shfl3(mask, acc.lhsLin.r2, o);
+        add_shfl_lower(mask, acc.lhsLin, o);
         add_shfl3(mask, acc.rhsLin, o);
         if (rigid) {
-            add_shfl3(mask, acc.lhsAng.r0, o);
-            add_shfl3(mask, acc.lhsAng.r1, o);
-            add_shfl3(mask, acc.lhsAng.r2, o);
+            add_shfl_lower(mask, acc.lhsAng, o);
             add_shfl3(mask, acc.lhsCross.r0, o);
             add_shfl3(mask, acc.lhsCross.r1, o);
             add_shfl3(mask, acc.lhsCross.r2, o);
@@ -951,26 +1064,86 @@ __device__ __forceinline__ void body_commit(const Params& P, const DevPtrs& d, u
     if (rigid) d.posAng[body] = q_addw(d.posAng[body], dxAng);
 }
 
-// One body on an 8-lane group; lane 0 writes the result.
-__device__ void primal_body(const Params& P, const DevPtrs& d, uint32_t body, uint32_t lane, unsigned mask) {
+// One body on an 8-lane group; lane 0 writes the result.  Logical lane l adds
+// the entries l, l + 8, ... in order, as the reference's SIMD group does, but a
+// manifold's contact points are not evaluated by the lane that adds them: the
+// points of eight consecutive entries are dealt out to the group's lanes, eight
+// at a time, and their increments pass through shared memory (`slots`: this
+// group's column of `stride` columns).  A box resting on the ground has one
+// manifold of four points among its entries; one lane used to form the four
+// increments one after another while seven waited.
+__device__ __forceinline__ void primal_body(const Params& P, const DevPtrs& d, uint32_t body, uint32_t lane, unsigned mask,
+                            float* slots, int stride) {
     const float4 shp = d.shape[body];
     Accum acc{m3_zero(), m3_zero(), m3_zero(), s3(0), s3(0)};
     const AdjView v = adj_view(d, body);
     const uint32_t cnt = v.count();
-    for (uint32_t k = lane; k < cnt; k += 8) stamp_entry(P, d, v.at(k), body, acc);
+    for (uint32_t base = 0; base < cnt; base += 8) {
+        uint32_t entry = 0, np = 0;
+        if (base + lane < cnt) {
+            entry = v.at(base + lane);
+            if ((entry >> ADJ_KIND_SHIFT) == FK_MANIFOLD) np = d.manifolds[entry & ADJ_INDEX_MASK].header.z;
+            else stamp_entry<false>(P, d, entry, body, acc);
+        }
+        uint32_t end = np;                                   // points of this and the lower lanes' entries
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(mask, end, o, 8);
+            if ((int)lane >= o) end += y;
+        }
+        const uint32_t total = __shfl_sync(mask, end, 7, 8), begin = end - np;
+        for (uint32_t c0 = 0; c0 < total; c0 += 8) {
+            const uint32_t i = c0 + lane;
+            uint32_t owner = 0;                              // the lane whose entry holds point i
+#pragma unroll
+            for (int j = 0; j < 7; j++) owner += __shfl_sync(mask, end, j, 8) <= i ? 1u : 0u;
+            const uint32_t e = __shfl_sync(mask, entry, (int)owner, 8), first = __shfl_sync(mask, begin, (int)owner, 8);
+            if (i < total) {
+                const ManifoldGPU& m = d.manifolds[e & ADJ_INDEX_MASK];
+                store_inc(slots + lane, stride, manifold_point_inc(P, manifold_ctx(d, m, body), m.contacts[i - first]));
+            }
+            __syncwarp(mask);
+            const uint32_t last = min(end, c0 + 8);
+            for (uint32_t k = max(begin, c0); k < last; k++) add_stored_inc(acc, slots + (k - c0), stride);
+            __syncwarp(mask);
+        }
+    }
     body_commit(P, d, body, shp, lane, mask, acc);
 }
 
-__global__ void k_primal(const Params P, const DevPtrs d, uint32_t color, uint32_t count) {
+// Dynamic coloring: the frame graph launches colors [0, bound) one by one.
+// A frame that needs more colors than the graph was built for is rare; in the
+// launch of the last of them (`last`) the block that finishes last solves the
+// remaining colors, one after another with a block barrier between them.
+constexpr int kPrimalThreads = 128;         // most threads of a k_primal block
+__global__ void __launch_bounds__(kPrimalThreads, 4) k_primal(const Params P, const DevPtrs d, uint32_t color,
+                                                           uint32_t last) {
+    __shared__ float slots[kIncWords * kPrimalThreads];
     pdl_prologue();
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lane = tid & 7u, groups = (gridDim.x * blockDim.x) >> 3;
-    const uint32_t s = d.colorStart[color];
-    const uint32_t n = count != 0xFFFFFFFFu ? count : d.colorStart[color + 1] - s;
     const unsigned mask = 0xFFu << (threadIdx.x & 24u);
     // one 8-lane group per body, striding over the color (uniform across
     // the group)
-    for (uint32_t slot = tid >> 3; slot < n; slot += groups) primal_body(P, d, d.colorList[s + slot], lane, mask);
+    uint32_t slot = tid >> 3, step = groups;
+    __shared__ uint32_t finished;
+    for (uint32_t c = color;; c++) {
+        const uint32_t b = d.colorStart[c], e = d.colorStart[c + 1];
+        for (; b + slot < e; slot += step)
+            primal_body(P, d, d.colorList[b + slot], lane, mask, slots + (threadIdx.x & ~7u), kPrimalThreads);
+        if (!last || c + 1u >= d.colorStart[MAX_COLORS + 1]) return;       // [MAX_COLORS + 1]: used colors
+        __threadfence();
+        __syncthreads();
+        if (c == color) {
+            if (threadIdx.x == 0) finished = atomicAdd(d.tailTicket, 1u);
+            __syncthreads();
+            if (finished != gridDim.x - 1u) return;
+            if (threadIdx.x == 0) *d.tailTicket = 0u;
+            __threadfence();
+        }
+        slot = threadIdx.x >> 3;
+        step = blockDim.x >> 3;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -988,12 +1161,12 @@ __global__ void k_primal(const Params P, const DevPtrs d, uint32_t color, uint32
 // ---------------------------------------------------------------------------
 constexpr int kWideThreads = 128;
 constexpr int kWideEntries = 512;          // entries whose points may be staged
-constexpr int kWidePoints = 320;           // staged points (33 floats each)
+constexpr int kWidePoints = 320;           // staged points
 constexpr uint32_t kWideInline = 0xFFFFFFFFu;
 
 __global__ void __launch_bounds__(kWideThreads) k_primal_wide(const Params P, const DevPtrs d, uint32_t color,
                                                              uint32_t first, uint32_t start) {
-    __shared__ PointInc pts[kWidePoints];
+    __shared__ float pts[kIncWords * kWidePoints];
     __shared__ uint32_t entOff[kWideEntries];  // (first point << 8) | points, or kWideInline
     __shared__ uint32_t warpSums[kWideThreads / 32];
     pdl_trigger();
@@ -1048,10 +1221,10 @@ __global__ void __launch_bounds__(kWideThreads) k_primal_wide(const Params P, co
             if (kind == FK_MANIFOLD) {
                 const ManifoldGPU& m = d.manifolds[idx];
                 const ManifoldCtx x = manifold_ctx(d, m, body);
-                for (uint32_t i = 0; i < np; i++) pts[off + i] = manifold_point_inc(P, x, m.contacts[i]);
+                for (uint32_t i = 0; i < np; i++) store_inc(pts + off + i, kWidePoints, manifold_point_inc(P, x, m.contacts[i]));
             } else {
                 const SoftContactGPU& sc = d.soft[idx];
-                pts[off] = soft_rigid_inc(sc, soft_force(P, d, sc, body));
+                store_inc(pts + off, kWidePoints, soft_rigid_inc(sc, soft_force(P, d, sc, body)));
             }
         }
         base += total;
@@ -1063,7 +1236,7 @@ __global__ void __launch_bounds__(kWideThreads) k_primal_wide(const Params P, co
         const uint32_t eo = k < (uint32_t)kWideEntries ? entOff[k] : kWideInline;
         if (eo != kWideInline) {
             const uint32_t off = eo >> 8, np = eo & 0xFFu;
-            for (uint32_t i = 0; i < np; i++) add_inc(acc, pts[off + i]);
+            for (uint32_t i = 0; i < np; i++) add_stored_inc(acc, pts + off + i, kWidePoints);
         } else {
             stamp_entry(P, d, v.at(k), body, acc);
         }
@@ -1523,13 +1696,10 @@ __global__ void __launch_bounds__(128, GENERAL ? 4 : (CLOTH ? AVBD_LEAN_CLOTH_MI
     const unsigned mask = LANES == 32 ? 0xffffffffu
                                       : (((1u << LANES) - 1u) << ((threadIdx.x & 31u) & ~(uint32_t)(LANES - 1)));
     (void)GROUPS;
+    static_assert(RESID || !GENERAL, "a solve's rigid bodies run in k_primal_wide");
     if (GENERAL && shp.w >= 0.0f) {                          // rigid: the 8-lane path
         const unsigned mask8 = mask & (0xFFu << ((threadIdx.x & 31u) & ~(uint32_t)(LANES - 1)));
-        if (RESID) {
-            if (lane < 8) rigid_residual(P, d, body, lane, mask8, d.learnResidBodies + s + slot);
-        } else if (lane < 8) {
-            primal_body(P, d, body, lane, mask8);
-        }
+        if (lane < 8) rigid_residual(P, d, body, lane, mask8, d.learnResidBodies + s + slot);
         return;
     }
     // lane 0 needs these after the reduction; issue the loads now
@@ -1578,10 +1748,8 @@ __global__ void __launch_bounds__(128, GENERAL ? 4 : (CLOTH ? AVBD_LEAN_CLOTH_MI
     // xor butterfly over the 8 logical lanes (offsets 4, 2, 1)
 #pragma unroll
     for (int o = 4; o >= 1; o >>= 1) {
-        acc.lhs.r0 = acc.lhs.r0 + mk3(__shfl_xor_sync(mask, acc.lhs.r0.x, o, LANES), __shfl_xor_sync(mask, acc.lhs.r0.y, o, LANES), __shfl_xor_sync(mask, acc.lhs.r0.z, o, LANES));
-        acc.lhs.r1 = acc.lhs.r1 + mk3(__shfl_xor_sync(mask, acc.lhs.r1.x, o, LANES), __shfl_xor_sync(mask, acc.lhs.r1.y, o, LANES), __shfl_xor_sync(mask, acc.lhs.r1.z, o, LANES));
-        acc.lhs.r2 = acc.lhs.r2 + mk3(__shfl_xor_sync(mask, acc.lhs.r2.x, o, LANES), __shfl_xor_sync(mask, acc.lhs.r2.y, o, LANES), __shfl_xor_sync(mask, acc.lhs.r2.z, o, LANES));
-        acc.rhs = acc.rhs + mk3(__shfl_xor_sync(mask, acc.rhs.x, o, LANES), __shfl_xor_sync(mask, acc.rhs.y, o, LANES), __shfl_xor_sync(mask, acc.rhs.z, o, LANES));
+        add_shfl_lower(mask, acc.lhs, o);
+        add_shfl3(mask, acc.rhs, o);
     }
     if (lane != 0) return;
     if (RESID) {
@@ -1592,15 +1760,15 @@ __global__ void __launch_bounds__(128, GENERAL ? 4 : (CLOTH ? AVBD_LEAN_CLOTH_MI
     particle_commit(P, d, body, shp, pl, inert, acc);
 }
 
-template <bool GENERAL, bool CLOTH>
+template <bool CLOTH>
 static void launch_primal_group(const Params& P, const DevPtrs& d, uint32_t color, uint32_t count,
                                 uint32_t first, uint32_t start, uint32_t lanes, cudaStream_t st) {
     const int T = 128;
     const uint32_t blocks = (count * lanes + T - 1) / T;
-    if (lanes <= 8) launch_pdl(k_primal_group<8, GENERAL, CLOTH>, blocks, T, st, P, d, color, count, first, start);
+    if (lanes <= 8) launch_pdl(k_primal_group<8, false, CLOTH>, blocks, T, st, P, d, color, count, first, start);
     else if (lanes <= 16)
-        launch_pdl(k_primal_group<16, GENERAL, CLOTH>, blocks, T, st, P, d, color, count, first, start);
-    else launch_pdl(k_primal_group<32, GENERAL, CLOTH>, blocks, T, st, P, d, color, count, first, start);
+        launch_pdl(k_primal_group<16, false, CLOTH>, blocks, T, st, P, d, color, count, first, start);
+    else launch_pdl(k_primal_group<32, false, CLOTH>, blocks, T, st, P, d, color, count, first, start);
 }
 
 // ---------------------------------------------------------------------------
@@ -1614,7 +1782,6 @@ static void launch_primal_group(const Params& P, const DevPtrs& d, uint32_t colo
 // entry and moves every term through warp shuffles; here the evaluation
 // runs dense and the fold reads shared memory.  Entries past the block's
 // staging capacity are evaluated inline by the fold, in the same order.
-// Rigid bodies (GENERAL) take the 8-lane 6x6 path unchanged.
 // ---------------------------------------------------------------------------
 constexpr int kStagedThreads = 128;
 constexpr int kStagedGroups = kStagedThreads / 8;
@@ -1634,8 +1801,8 @@ __device__ __forceinline__ AdjView staged_view(const DevPtrs& d, const StagedBod
     return v;
 }
 
-template <bool GENERAL, bool CLOTH>
-__global__ void __launch_bounds__(kStagedThreads, GENERAL ? 4 : 5)
+template <bool CLOTH>
+__global__ void __launch_bounds__(kStagedThreads, 5)
 k_primal_staged(const Params P, const DevPtrs d, uint32_t color, uint32_t count, uint32_t first, uint32_t start) {
     __shared__ float slots[kStagedWords][kStagedSlots];
     __shared__ StagedBody info[kStagedGroups];
@@ -1653,10 +1820,8 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t color, uint32_t count,
     uint32_t cnt = 0, body = 0xFFFFFFFFu;
     StagedBody sb{};
     const bool mine = tid < kStagedGroups && head + tid < count;
-    float4 bodyShape = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (mine) {
         body = d.colorLaunch[s + head + tid];
-        bodyShape = d.shape[body];
         const uint4 seg = d.staticSeg[body];
         sb.preBase = seg.x; sb.nPre = seg.y; sb.postBase = seg.z; sb.nPost = seg.w;
         sb.nTet = d.postTets[body];
@@ -1667,7 +1832,6 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t color, uint32_t count,
             sb.dynBase = d.dynStart[body]; sb.nDyn = d.dynCount[body]; sb.nMan = d.dynSplit[body];
             cnt = sb.nPre + sb.nDyn + sb.nPost;
             sb.cnt = cnt;
-            if (GENERAL && bodyShape.w >= 0.0f) cnt = 0;           // rigid: stages nothing
         }
         uint32_t incl = cnt;
 #pragma unroll
@@ -1713,10 +1877,6 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t color, uint32_t count,
     const StagedBody b = info[g];
     const unsigned mask8 = 0xFFu << (tid & 24u);
     const float4 shp = d.shape[b.body];
-    if (GENERAL && shp.w >= 0.0f) {
-        primal_body(P, d, b.body, lane, mask8);
-        return;
-    }
     float4 pl = make_float4(0, 0, 0, 0), inert = make_float4(0, 0, 0, 0);
     if (lane == 0) { pl = d.posLin[b.body]; inert = d.inertLin[b.body]; }
     ParticleAccum acc{m3_zero(), s3(0)};
@@ -1738,28 +1898,26 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t color, uint32_t count,
         } else {
             particle_entry_terms<CLOTH>(P, d, staged_view(d, b), b.body, k, u, e);
         }
-        fold_particle_term<GENERAL, CLOTH>(P, d, u, e, b.body, acc);
+        fold_particle_term<false, CLOTH>(P, d, u, e, b.body, acc);
     }
 #pragma unroll
     for (int o = 4; o >= 1; o >>= 1) {
-        add_shfl3(mask8, acc.lhs.r0, o);
-        add_shfl3(mask8, acc.lhs.r1, o);
-        add_shfl3(mask8, acc.lhs.r2, o);
+        add_shfl_lower(mask8, acc.lhs, o);
         add_shfl3(mask8, acc.rhs, o);
     }
     if (lane != 0) return;
     particle_commit(P, d, b.body, shp, pl, inert, acc);
 }
 
-template <bool GENERAL, bool CLOTH>
+template <bool CLOTH>
 static void launch_primal_staged(const Params& P, const DevPtrs& d, uint32_t color, uint32_t count,
                                  uint32_t first, uint32_t start, cudaStream_t st) {
     const uint32_t blocks = (count + kStagedGroups - 1) / kStagedGroups;
-    launch_pdl(k_primal_staged<GENERAL, CLOTH>, blocks, kStagedThreads, st, P, d, color, count, first, start);
+    launch_pdl(k_primal_staged<CLOTH>, blocks, kStagedThreads, st, P, d, color, count, first, start);
 }
 
 void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t color, uint32_t count,
-                         uint32_t lanes, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
+                         uint32_t lanes, bool last, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
     const int T = 128;
     const uint32_t upper = count != 0xFFFFFFFFu ? count : z.numDynamicBodies;
     if (upper == 0) return;
@@ -1770,7 +1928,7 @@ void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint
         // 1.007 -> 0.965 ms per frame; half a wave measured 1.22 ms)
         const uint32_t TT = z.dynThreads ? z.dynThreads : (uint32_t)T;
         const uint32_t need = (upper * 8 + TT - 1) / TT, wave = z.dynBlocks ? z.dynBlocks : 148u * 4u;
-        launch_pdl(k_primal, need < wave ? need : wave, TT, st, P, d, color, count);
+        launch_pdl(k_primal, need < wave ? need : wave, TT, st, P, d, color, last ? 1u : 0u);
     } else {
         // The grouped and staged kernels need the color's body count on the
         // host.  The color's lean particles (the head of its launch order)
@@ -1788,13 +1946,13 @@ void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint
         }
         if (lean) {
             if (lanes == AVBD_PRIMAL_STAGED) {
-                if (cloth) launch_primal_staged<false, true>(P, d, color, lean, 0, start, st);
-                else launch_primal_staged<false, false>(P, d, color, lean, 0, start, st);
+                if (cloth) launch_primal_staged<true>(P, d, color, lean, 0, start, st);
+                else launch_primal_staged<false>(P, d, color, lean, 0, start, st);
             } else {
                 const uint32_t lanes_ = lanes < 8 ? 8 : (lanes > 32 ? 32 : lanes);
                 const uint32_t w = lanes_ <= 8 ? 8 : (lanes_ <= 16 ? 16 : 32);
-                if (cloth) launch_primal_group<false, true>(P, d, color, lean, 0, start, w, st);
-                else launch_primal_group<false, false>(P, d, color, lean, 0, start, w, st);
+                if (cloth) launch_primal_group<true>(P, d, color, lean, 0, start, w, st);
+                else launch_primal_group<false>(P, d, color, lean, 0, start, w, st);
             }
         }
         // the rest: a block per body (rigid bodies with many contacts)
@@ -1911,11 +2069,13 @@ __device__ void dual_spring(const Params& P, const DevPtrs& d, uint32_t si) {
     if (C > 0.0f) sp.dual.y = mn(sp.dual.y + C * P.betaLin, mn(sp.rA.w, PENALTY_MAX));
 }
 
-__device__ void dual_manifold(const Params& P, const DevPtrs& d, uint32_t gid) {
+// Points i0, i0 + step, ... of a manifold (a point's update reads and writes
+// that point only).
+__device__ void dual_manifold(const Params& P, const DevPtrs& d, uint32_t gid, uint32_t i0, uint32_t step) {
     ManifoldGPU& m = d.manifolds[gid];
     const u4 h = m.header;
     const uint32_t n = h.z;
-    if (n == 0) return;
+    if (i0 >= n) return;
     const uint32_t a = h.x, b = h.y;
     const bool sphA = (h.w & 2u) != 0, sphB = (h.w & 4u) != 0;
     const float4 pa4 = d.posLin[a], pb4 = d.posLin[b], qa = d.posAng[a], qb = d.posAng[b];
@@ -1927,7 +2087,7 @@ __device__ void dual_manifold(const Params& P, const DevPtrs& d, uint32_t gid) {
     const float lamCap = mn(P.lambdaMax, mx(10.0f, 1.0e5f * minMass));
     const float3 nrm = xyz(m.basisN), t1 = xyz(m.basisT1), t2 = cross(nrm, t1);
     const float dynF = m.basisN.w, statF = m.basisT1.w;
-    for (uint32_t i = 0; i < n; i++) {
+    for (uint32_t i = i0; i < n; i += step) {
         ContactGPU& c = m.contacts[i];
         const float3 rAW = sphA ? xyz(c.rA) : q_rotate(qa, xyz(c.rA));
         const float3 rBW = sphB ? xyz(c.rB) : q_rotate(qb, xyz(c.rB));
@@ -1974,40 +2134,68 @@ __device__ void dual_soft(const Params& P, const DevPtrs& d, uint32_t i) {
     sc.penalty = tof4(pen, sc.penalty.w);
 }
 
+// Item g of the dual: active joints, hard springs, `ways` threads for each
+// manifold with contacts (points w, w + ways, ...), element contacts.
 __device__ __forceinline__ void dual_item(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t g,
-                                          uint32_t numPairs) {
+                                          uint32_t numActive, uint32_t ways) {
     if (g < z.numActiveJoints) { dual_joint(P, d, d.activeJoints[g]); return; }
     g -= z.numActiveJoints;
     if (g < z.numHardSprings) { dual_spring(P, d, d.hardSprings[g]); return; }
     g -= z.numHardSprings;
-    if (g < numPairs) { dual_manifold(P, d, g); return; }
-    dual_soft(P, d, g - numPairs);
+    if (g < numActive * ways) { dual_manifold(P, d, d.activeManifolds[g / ways], g % ways, ways); return; }
+    dual_soft(P, d, g - numActive * ways);
 }
 
+// What bounds it: dependent loads of a few records per thread.  The manifolds
+// with contacts are listed once a frame (k_adj_dyn): of the mixed scene's
+// 117,600 candidate pairs the dual used to read every header in every
+// iteration.  Scenes of rigid bodies give a manifold four threads (a resting
+// box has four points); particles meet things in one point, and one thread.
+template <uint32_t WAYS>
 __global__ void k_dual(const Params P, const DevPtrs d, const Sizes z) {
     pdl_prologue();
-    const uint32_t numPairs = d.counters->numPairs;
+    const uint32_t numActive = d.counters->activeManifolds;
     const uint32_t numSoft = (P.cloth || P.ogc) ? d.counters->numSoft : 0u;
-    const uint32_t total = z.numActiveJoints + z.numHardSprings + numPairs + numSoft;
+    const uint32_t total = z.numActiveJoints + z.numHardSprings + numActive * WAYS + numSoft;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
-        dual_item(P, d, z, g, numPairs);
+        dual_item(P, d, z, g, numActive, WAYS);
 }
 
 void launch_dual(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    const uint32_t upper = z.numActiveJoints + z.numHardSprings + z.maxPairs + ((P.cloth || P.ogc) ? z.maxSoft : 0u);
-    launch_pdl(k_dual, stride_blocks(upper, 128), 128, st, P, d, z);
+    const bool rigid = z.numDynamicRigid == z.numDynamicBodies;
+    const uint32_t upper = z.numActiveJoints + z.numHardSprings + (rigid ? 4u : 1u) * z.maxPairs +
+                           ((P.cloth || P.ogc) ? z.maxSoft : 0u);
+    if (rigid) launch_pdl(k_dual<4>, stride_blocks(upper, 128), 128, st, P, d, z);
+    else launch_pdl(k_dual<1>, stride_blocks(upper, 128), 128, st, P, d, z);
 }
 
 // ---------------------------------------------------------------------------
-// Small scenes: the whole iteration loop in one thread block.  Colors and the
-// dual are separated by __syncthreads(), which orders the same way as the
-// per-color launches.
+// Small scenes: the whole iteration loop in one launch of a cluster of up to
+// eight CTAs, a color or the dual at a time between barriers, in the order of
+// the per-color launches.  The cluster grows with the scene so that the
+// largest color still has an 8-lane group per body: one CTA (its barrier is a
+// block barrier) up to 64 bodies, eight from 257 on.  One CTA of 256 threads
+// for every size took 1,810 us of the 2,060 us frame of 512 piled bodies.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_solve_small(const Params P, const DevPtrs d, const Sizes z,
-                                                     uint32_t colorBound) {
-    const uint32_t groups = blockDim.x >> 3;
-    const uint32_t group = threadIdx.x >> 3, lane = threadIdx.x & 7u;
+constexpr int kSmallThreads = 512;
+constexpr uint32_t kSmallSlots = kIncWords * kSmallThreads;      // floats of dynamic shared memory
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kSmallThreads, 1) k_solve_small(const Params P, const DevPtrs d, const Sizes z,
+                                                                  uint32_t colorBound) {
+    extern __shared__ float slots[];
+    const uint32_t ctas = gridDim.x, rank = blockIdx.x;          // the grid is one cluster
+    const uint32_t groups = (blockDim.x >> 3) * ctas;
+    // neighbouring bodies of a color go to different CTAs
+    const uint32_t group = (threadIdx.x >> 3) * ctas + rank, lane = threadIdx.x & 7u;
     const unsigned mask = 0xFFu << (threadIdx.x & 24u);
+    auto barrier = [&]() {
+        if (CLUSTER) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+    };
     // the color offsets do not change during the solve: one copy in shared
     // memory instead of a dependent global load per color per iteration
     __shared__ uint32_t cs[MAX_COLORS + 1];
@@ -2015,46 +2203,40 @@ __global__ void __launch_bounds__(256) k_solve_small(const Params P, const DevPt
     __syncthreads();
     uint32_t last = 0;                           // one past the last non-empty color
     for (uint32_t c = 0; c < colorBound; c++) if (cs[c + 1] != cs[c]) last = c + 1;
+    const uint32_t numActive = d.counters->activeManifolds;
+    const uint32_t total = z.numActiveJoints + z.numHardSprings + numActive * MAX_CONTACTS;
     for (uint32_t it = 0; it < P.iterations; it++) {
         for (uint32_t c = 0; c < last; c++) {
             const uint32_t s = cs[c], e = cs[c + 1];
-            if (s == e) continue;                // block-uniform
+            if (s == e) continue;                // the same in every CTA
             for (uint32_t slot = group; s + slot < e; slot += groups)
-                primal_body(P, d, d.colorList[s + slot], lane, mask);
-            __syncthreads();
+                primal_body(P, d, d.colorList[s + slot], lane, mask, slots + (threadIdx.x & ~7u), kSmallThreads);
+            barrier();
         }
-        const uint32_t numPairs = d.counters->numPairs;
-        const uint32_t total = z.numActiveJoints + z.numHardSprings + numPairs;
-        for (uint32_t g = threadIdx.x; g < total; g += blockDim.x) dual_item(P, d, z, g, numPairs);
-        __syncthreads();
+        for (uint32_t g = rank * blockDim.x + threadIdx.x; g < total; g += ctas * blockDim.x)
+            dual_item(P, d, z, g, numActive, MAX_CONTACTS);
+        barrier();
     }
+}
+
+// dynamic shared memory above 48 KiB (set once per device)
+static void small_attributes() {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load() & bit) return;
+    cudaFuncSetAttribute(k_solve_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmallSlots * 4));
+    cudaFuncSetAttribute(k_solve_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmallSlots * 4));
+    done.fetch_or(bit);
 }
 
 void launch_solve_small(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t colorBound, cudaStream_t st) {
-    k_solve_small<<<1, 256, 0, st>>>(P, d, z, colorBound);
-}
-
-// Dynamic coloring: the frame graph launches colors [0, first) one by one
-// and this single block handles any colors from `first` up (rare: a frame
-// that needs more colors than the graph was built for), color after color
-// with a block barrier between them — the same per-body solve in the same
-// color order.
-__global__ void __launch_bounds__(256) k_primal_tail(const Params P, const DevPtrs d, uint32_t first) {
-    pdl_prologue();
-    const uint32_t groups = blockDim.x >> 3;
-    const uint32_t group = threadIdx.x >> 3, lane = threadIdx.x & 7u;
-    const unsigned mask = 0xFFu << (threadIdx.x & 24u);
-    for (uint32_t c = first; c < (uint32_t)MAX_COLORS; c++) {
-        const uint32_t s = d.colorStart[c], e = d.colorStart[c + 1];
-        if (s == e) continue;                    // block-uniform
-        for (uint32_t slot = group; s + slot < e; slot += groups)
-            primal_body(P, d, d.colorList[s + slot], lane, mask);
-        __syncthreads();
-    }
-}
-
-void launch_primal_tail(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t first, cudaStream_t st) {
-    if (first < (uint32_t)MAX_COLORS) launch_pdl(k_primal_tail, 1, 256, st, P, d, first);
+    small_attributes();
+    const uint32_t n = z.numDynamicBodies;
+    const uint32_t ctas = n <= 64 ? 1u : (n <= 128 ? 2u : (n <= 256 ? 4u : 8u));
+    if (ctas == 1) launch_cluster(k_solve_small<false>, 1, kSmallThreads, kSmallSlots * 4, st, P, d, z, colorBound);
+    else launch_cluster(k_solve_small<true>, ctas, kSmallThreads, kSmallSlots * 4, st, P, d, z, colorBound);
 }
 
 // ---------------------------------------------------------------------------
