@@ -12,12 +12,13 @@
 #include "../../include/avbd.h"
 #include "dmath.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace avbd {
 
 // ---------------------------------------------------------------------------
-// Exclusive scan: 1024 words per block (256 threads x 4), a single-block scan
-// of the block sums, then a uniform add.
+// Exclusive scan: 1024 words per block (256 threads x 4), then an add of the
+// sums of the blocks before.
 // ---------------------------------------------------------------------------
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_GRAIN = 4;
@@ -50,8 +51,8 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* w
     return warpBase + x - v;
 }
 
-__global__ void k_scan_blocks(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                              uint32_t* __restrict__ blockSums, uint32_t n) {
+__global__ void k_scan_blocks(const uint32_t* in, uint32_t* out, uint32_t* blockSums, uint32_t n) {
+    pdl_prologue();
     __shared__ uint32_t warpSums[32];
     const uint32_t base = blockIdx.x * SCAN_BLOCK + threadIdx.x * SCAN_GRAIN;
     uint32_t v[SCAN_GRAIN];
@@ -71,29 +72,26 @@ __global__ void k_scan_blocks(const uint32_t* __restrict__ in, uint32_t* __restr
     if (threadIdx.x == 0) blockSums[blockIdx.x] = total;
 }
 
-__global__ void k_scan_block_sums(uint32_t* __restrict__ blockSums, uint32_t nblocks) {
-    __shared__ uint32_t warpSums[32];
-    // nblocks <= SCAN_BLOCK: each thread owns up to 4 consecutive sums
-    const uint32_t base = threadIdx.x * SCAN_GRAIN;
-    uint32_t v[SCAN_GRAIN];
-    uint32_t sum = 0;
+// Adds to every block of 1024 words the sum of the blocks before it.
+// SCANNED: `blockSums` already holds those prefixes; otherwise each block adds
+// up the sums before its own (nblocks <= 1024: four words a thread), which
+// costs less than the launch of a kernel that would scan them.
+template <bool SCANNED>
+__global__ void k_scan_add(uint32_t* out, const uint32_t* blockSums, uint32_t n) {
+    pdl_prologue();
+    uint32_t add = 0;
+    if (SCANNED) {
+        add = blockSums[blockIdx.x];
+    } else {
+        __shared__ uint32_t warpSums[32];
+        uint32_t sum = 0;
 #pragma unroll
-    for (int i = 0; i < SCAN_GRAIN; i++) {
-        v[i] = base + i < nblocks ? blockSums[base + i] : 0u;
-        sum += v[i];
+        for (int i = 0; i < SCAN_GRAIN; i++) {
+            const uint32_t k = threadIdx.x + i * SCAN_THREADS;
+            sum += k < blockIdx.x ? blockSums[k] : 0u;
+        }
+        block_exclusive_scan(sum, warpSums, add);
     }
-    uint32_t total;
-    uint32_t run = block_exclusive_scan(sum, warpSums, total);
-#pragma unroll
-    for (int i = 0; i < SCAN_GRAIN; i++) {
-        if (base + i < nblocks) blockSums[base + i] = run;
-        run += v[i];
-    }
-}
-
-__global__ void k_scan_add(uint32_t* __restrict__ out, const uint32_t* __restrict__ blockSums,
-                           uint32_t n) {
-    const uint32_t add = blockSums[blockIdx.x];
     const uint32_t base = blockIdx.x * SCAN_BLOCK + threadIdx.x * SCAN_GRAIN;
 #pragma unroll
     for (int i = 0; i < SCAN_GRAIN; i++)
@@ -104,24 +102,21 @@ void launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32
                            cudaStream_t st) {
     if (n == 0) return;
     const uint32_t nblocks = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
-    k_scan_blocks<<<nblocks, SCAN_THREADS, 0, st>>>(in, out, scratch, n);
-    if (nblocks > 1) {
-        k_scan_block_sums<<<1, SCAN_THREADS, 0, st>>>(scratch, nblocks);
-        k_scan_add<<<nblocks, SCAN_THREADS, 0, st>>>(out, scratch, n);
-    }
+    launch_pdl(k_scan_blocks, nblocks, SCAN_THREADS, st, in, out, scratch, n);
+    if (nblocks > 1) launch_pdl(k_scan_add<false>, nblocks, SCAN_THREADS, st, out, scratch, n);
 }
 
 // Any n < 2^30: scan blocks of 1024, scan the block sums recursively in
-// place (each thread reads its words before writing them), add back.
+// place (each thread reads its words before writing them) when a block of
+// the second pass cannot add them up itself, add back.
 void launch_exclusive_scan_large(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* scratch,
                                  cudaStream_t st) {
     if (n == 0) return;
     const uint32_t nblocks = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
-    k_scan_blocks<<<nblocks, SCAN_THREADS, 0, st>>>(in, out, scratch, n);
-    if (nblocks > 1) {
-        launch_exclusive_scan_large(scratch, scratch, nblocks, scratch + nblocks, st);
-        k_scan_add<<<nblocks, SCAN_THREADS, 0, st>>>(out, scratch, n);
-    }
+    if (nblocks <= (uint32_t)SCAN_BLOCK) { launch_exclusive_scan(in, out, n, scratch, st); return; }
+    launch_pdl(k_scan_blocks, nblocks, SCAN_THREADS, st, in, out, scratch, n);
+    launch_exclusive_scan_large(scratch, scratch, nblocks, scratch + nblocks, st);
+    launch_pdl(k_scan_add<true>, nblocks, SCAN_THREADS, st, out, scratch, n);
 }
 
 size_t scan_large_scratch_words(uint32_t n) {
@@ -146,6 +141,7 @@ __device__ __forceinline__ float3 collider_center(const DevPtrs& d, uint32_t c) 
 // on (P.fineBP), particle colliders are also binned into fine cells of twice
 // the largest particle radius (hash without group).
 __global__ void k_bp_count(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.numHashed) return;
     const uint32_t c = d.hashedIdx[i];
@@ -166,6 +162,7 @@ __global__ void k_bp_count(const Params P, const DevPtrs d) {
 }
 
 __global__ void k_bp_scatter(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.numHashed) return;
     const uint2 cs = d.bodyCellSlot[i];
@@ -189,6 +186,7 @@ static uint32_t stride_blocks_bp(uint32_t threads, int T) {
 // per lane instead of a serial insertion sort.
 __global__ void k_bp_sort_cells(const uint32_t* count, const uint32_t* start, const uint32_t* tmp, uint32_t* out,
                                 uint32_t buckets) {
+    pdl_prologue();
     rank_sort_buckets(count, start, tmp, out, buckets);
 }
 
@@ -196,6 +194,7 @@ __global__ void k_bp_sort_cells(const uint32_t* count, const uint32_t* start, co
 // reads a group of buckets' rigid counts at once (bucket_group) and
 // compacts each bucket that has any, one after another.
 __global__ void k_bp_rigid_compact(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     // a group of buckets' rigid counts per coalesced load, then one bucket
@@ -248,6 +247,7 @@ __device__ __forceinline__ bool domains_compatible(uint32_t ga, uint32_t gb, uin
 // Per-frame collider record: world center and |radius|, plus the metadata
 // the pair filters need, so a candidate test is two 16-byte loads.
 __global__ void k_bp_prep(const Params P, const DevPtrs d, uint32_t numColliders) {
+    pdl_prologue();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= numColliders) return;
     const uint32_t owner = d.colOwner[c];
@@ -263,6 +263,7 @@ __global__ void k_bp_prep(const Params P, const DevPtrs d, uint32_t numColliders
 // that a query ball misses cannot hold a candidate, so the global scans skip
 // it; the candidates they keep, and their order, are unchanged.
 __global__ void k_global_chunks(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t chunk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t g = chunk * 32u + lane;
@@ -324,6 +325,7 @@ __global__ void k_global_chunks(const Params P, const DevPtrs d) {
 // bucket, then by collider index.
 template <bool EMIT>
 __global__ void __launch_bounds__(128) k_bp_pairs(const Params P, const DevPtrs d, uint32_t producers) {
+    pdl_prologue();
     __shared__ uint32_t visitH[4][27];
     const uint32_t producer = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31u;
@@ -504,6 +506,7 @@ __global__ void __launch_bounds__(128) k_bp_pairs(const Params P, const DevPtrs 
 // whole warp: entries in chunks of 32, emitted in order by ballot rank.
 template <bool EMIT>
 __global__ void __launch_bounds__(128) k_bp_heavy(const Params P, const DevPtrs d, const uint32_t* list, uint32_t n) {
+    pdl_prologue();
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31u;
     if (w >= n * 28u) return;                               // warp-uniform
@@ -597,6 +600,7 @@ __global__ void __launch_bounds__(128) k_bp_heavy(const Params P, const DevPtrs 
 }
 
 __global__ void k_bp_finalize(const Params P, const DevPtrs d, uint32_t producers) {
+    pdl_prologue();
     const uint32_t n = producers == 0 ? 0u : d.pairStart[producers - 1] + d.pairCount[producers - 1];
     d.counters->pairCandidates = n;
     d.counters->numPairs = n < P.maxPairs ? n : P.maxPairs;
@@ -608,37 +612,37 @@ void launch_broadphase(const Params& P, const DevPtrs& d, const Sizes& z, cudaSt
     if (P.fineBP) cudaMemsetAsync(d.fineCount, 0, sizeof(uint32_t) * P.fineHashSize, st);
     const int T = 128;
     if (P.numHashed > 0) {
-        k_bp_count<<<(P.numHashed + T - 1) / T, T, 0, st>>>(P, d);
+        launch_pdl(k_bp_count, (P.numHashed + T - 1) / T, T, st, P, d);
         launch_exclusive_scan(d.cellCount, d.cellStart, P.gridHashSize, d.scanScratch, st);
         if (P.fineBP) launch_exclusive_scan(d.fineCount, d.fineStart, P.fineHashSize, d.scanScratch, st);
-        k_bp_scatter<<<(P.numHashed + T - 1) / T, T, 0, st>>>(P, d);
-        k_bp_sort_cells<<<stride_blocks_bp(P.gridHashSize * 32u, T), T, 0, st>>>(d.cellCount, d.cellStart, d.cellTmp,
+        launch_pdl(k_bp_scatter, (P.numHashed + T - 1) / T, T, st, P, d);
+        launch_pdl(k_bp_sort_cells, stride_blocks_bp(P.gridHashSize * 32u, T), T, st, d.cellCount, d.cellStart, d.cellTmp,
                                                                                    d.cellBodies, P.gridHashSize);
         if (P.numHashedRigid > 0) {
             launch_exclusive_scan(d.cellRigid, d.rigidStart, P.gridHashSize, d.scanScratch, st);
-            k_bp_rigid_compact<<<stride_blocks_bp(P.gridHashSize * 32u, T), T, 0, st>>>(P, d);
+            launch_pdl(k_bp_rigid_compact, stride_blocks_bp(P.gridHashSize * 32u, T), T, st, P, d);
         }
         if (P.fineBP)
-            k_bp_sort_cells<<<stride_blocks_bp(P.fineHashSize * 32u, T), T, 0, st>>>(d.fineCount, d.fineStart, d.fineTmp,
+            launch_pdl(k_bp_sort_cells, stride_blocks_bp(P.fineHashSize * 32u, T), T, st, d.fineCount, d.fineStart, d.fineTmp,
                                                                                        d.fineCells, P.fineHashSize);
     }
     if (z.producers > 0) {
-        k_bp_prep<<<(z.numColliders + T - 1) / T, T, 0, st>>>(P, d, z.numColliders);
+        launch_pdl(k_bp_prep, (z.numColliders + T - 1) / T, T, st, P, d, z.numColliders);
         if (P.numGlobals > 32) {
             const uint32_t chunks = (P.numGlobals + 31) / 32;
-            k_global_chunks<<<(chunks + 3) / 4, 128, 0, st>>>(P, d);
+            launch_pdl(k_global_chunks, (chunks + 3) / 4, 128, st, P, d);
         }
         const uint32_t warpsPerBlock = T / 32;
         const uint32_t blocks = (z.producers + warpsPerBlock - 1) / warpsPerBlock;
         const uint32_t nh = z.numHeavyProducers;
         const uint32_t hblocks = (nh * 28u + warpsPerBlock - 1) / warpsPerBlock;
-        if (nh) k_bp_heavy<false><<<hblocks, T, 0, st>>>(P, d, d.heavyProducers, nh);
-        k_bp_pairs<false><<<blocks, T, 0, st>>>(P, d, z.producers);
+        if (nh) launch_pdl(k_bp_heavy<false>, hblocks, T, st, P, d, d.heavyProducers, nh);
+        launch_pdl(k_bp_pairs<false>, blocks, T, st, P, d, z.producers);
         launch_exclusive_scan(d.pairCount, d.pairStart, z.producers, d.scanScratch, st);
-        if (nh) k_bp_heavy<true><<<hblocks, T, 0, st>>>(P, d, d.heavyProducers, nh);
-        k_bp_pairs<true><<<blocks, T, 0, st>>>(P, d, z.producers);
+        if (nh) launch_pdl(k_bp_heavy<true>, hblocks, T, st, P, d, d.heavyProducers, nh);
+        launch_pdl(k_bp_pairs<true>, blocks, T, st, P, d, z.producers);
     }
-    k_bp_finalize<<<1, 1, 0, st>>>(P, d, z.producers);
+    launch_pdl(k_bp_finalize, 1, 1, st, P, d, z.producers);
 }
 
 // ---------------------------------------------------------------------------
@@ -761,16 +765,12 @@ extern "C" int avbd_exclusive_scan_noalloc(const uint32_t* d_in, uint32_t* d_out
             if (ctx && g_noalloc_entries < kMaxContexts) g_noalloc_scratch[g_noalloc_entries++] = {ctx, scratch};
         }
     }
-    // The first pass writes block sum b before the block-sum scan and the
-    // uniform add read it, so the shared scratch needs no clearing between calls.
+    // The first pass writes block sum b before the second pass reads it, so the shared scratch needs no clearing between calls.
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     if (inPlace) {
         const uint32_t nblocks = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
         k_scan_blocks_inplace<<<nblocks, SCAN_THREADS, 0, st>>>(d_out, scratch, n);
-        if (nblocks > 1) {
-            k_scan_block_sums<<<1, SCAN_THREADS, 0, st>>>(scratch, nblocks);
-            k_scan_add<<<nblocks, SCAN_THREADS, 0, st>>>(d_out, scratch, n);
-        }
+        if (nblocks > 1) launch_pdl(k_scan_add<false>, nblocks, SCAN_THREADS, st, d_out, (const uint32_t*)scratch, n);
     } else {
         launch_exclusive_scan(d_in, d_out, n, scratch, st);
     }

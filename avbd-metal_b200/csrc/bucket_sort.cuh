@@ -20,9 +20,9 @@ __device__ __forceinline__ uint32_t bucket_group(uint32_t buckets, uint32_t warp
 // smaller ids) — one dependent count load per group instead of one per
 // bucket, which dominated the sparse grids (millions of buckets, a few
 // thousand in use).  Dense buckets cost n^2/32 compares per lane.
-__device__ __forceinline__ void rank_sort_buckets(const uint32_t* __restrict__ count,
-                                                  const uint32_t* __restrict__ start,
-                                                  const uint32_t* __restrict__ tmp, uint32_t* __restrict__ out,
+__device__ __forceinline__ void rank_sort_buckets(const uint32_t* count,
+                                                  const uint32_t* start,
+                                                  const uint32_t* tmp, uint32_t* out,
                                                   uint32_t buckets) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;

@@ -67,6 +67,7 @@ __device__ __forceinline__ float prefilter_reach(const Params& P) { return P.que
 // ---------------------------------------------------------------------------
 template <bool SCATTER>
 __global__ void k_elem_bin(const Params P, const DevPtrs d, uint32_t total) {
+    pdl_prologue();
     for (uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x; gid < total; gid += gridDim.x * blockDim.x) {
         float3 lo, hi;
         if (!SCATTER) {
@@ -224,6 +225,7 @@ constexpr uint32_t kDatCache = 16;
 // pairs are sorted by `other` after the emitting pass.
 template <bool EMIT>
 __global__ void __launch_bounds__(128, 8) k_dat_pairs(const Params P, const DevPtrs d, uint32_t owners) {
+    pdl_prologue();
     __shared__ uint32_t survivors[4][64];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -377,6 +379,7 @@ __global__ void __launch_bounds__(128, 8) k_dat_pairs(const Params P, const DevP
 
 // Totals of the pair stream (dat_finalize_pairs, 27_planar_dat.metal:208-228).
 __global__ void k_dat_pair_totals(const Params P, const DevPtrs d, uint32_t owners) {
+    pdl_prologue();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     Counters* c = d.counters;
     const uint32_t total = owners ? d.datOwnerStart[owners - 1] + d.datOwnerCount[owners - 1] : 0u;
@@ -404,6 +407,7 @@ __global__ void k_dat_pair_totals(const Params P, const DevPtrs d, uint32_t owne
 // rtCand; k_rt_write writes the records at the scanned offsets.
 template <bool WARP>
 __global__ void __launch_bounds__(128, 6) k_rt_emit(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t lane = WARP ? (threadIdx.x & 31u) : 0u;
     const uint32_t step = WARP ? (gridDim.x * blockDim.x) >> 5 : gridDim.x * blockDim.x;
     const uint32_t first = WARP ? (blockIdx.x * blockDim.x + threadIdx.x) >> 5 : blockIdx.x * blockDim.x + threadIdx.x;
@@ -599,6 +603,7 @@ __device__ __forceinline__ void rt_feature(float4 sh, float3 po, float4 qo, uint
 // One thread per triangle writes the records k_rt_emit found, in its order,
 // from the triangle's scanned offset (25_cloth.metal:1080-1142 is the record).
 __global__ void __launch_bounds__(128) k_rt_write(const Params P, const DevPtrs d) {
+    pdl_prologue();
     for (uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x; gid < P.numTris; gid += gridDim.x * blockDim.x) {
         const uint32_t count = d.rtCount[gid];
         if (count == 0) continue;
@@ -651,6 +656,7 @@ __global__ void __launch_bounds__(128) k_rt_write(const Params P, const DevPtrs 
 }
 
 __global__ void k_rt_totals(const Params P, const DevPtrs d) {
+    pdl_prologue();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const uint32_t n = P.numTris;
     d.counters->numSoftRT = n ? d.rtStart[n - 1] + d.rtCount[n - 1] : 0u;
@@ -803,6 +809,7 @@ __device__ bool dat_contact(const Params& P, const DevPtrs& d, uint4 pair, uint3
 
 template <bool EMIT>
 __global__ void __launch_bounds__(128) k_dat_contacts(const Params P, const DevPtrs d, uint32_t owners) {
+    pdl_prologue();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t below = (1u << lane) - 1u;
@@ -827,6 +834,7 @@ __global__ void __launch_bounds__(128) k_dat_contacts(const Params P, const DevP
 
 // soft_finalize (25_cloth.metal:1144-1165): raw demand and the stored count.
 __global__ void k_soft_totals(const Params P, const DevPtrs d, uint32_t owners) {
+    pdl_prologue();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     Counters* c = d.counters;
     const uint32_t dat = owners ? d.datEmitStart[owners - 1] + d.datEmit[owners - 1] : 0u;
@@ -838,6 +846,7 @@ __global__ void k_soft_totals(const Params P, const DevPtrs d, uint32_t owners) 
 // the three records before it (the same triangle's rigid features) is not
 // inserted, so the first record of a key is the one found.
 __global__ void k_softmap_insert(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t n = d.counters->numSoft;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t keyA = __float_as_uint(d.soft[i].lambda.w), keyB = __float_as_uint(d.soft[i].penalty.w);
@@ -858,6 +867,7 @@ __global__ void k_softmap_insert(const Params P, const DevPtrs d) {
 }
 
 __global__ void k_reanchor(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= P.numParticles) return;
     const uint32_t v = d.particleIdx[gid];
@@ -1071,6 +1081,7 @@ __device__ __forceinline__ bool dat_apply_one(const Params& P, const DevPtrs& d,
 }
 
 __global__ void k_dat_apply_particles(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= P.numParticles) return;
     const uint32_t v = d.particleIdx[gid];
@@ -1102,6 +1113,7 @@ __global__ void k_dat_apply_color(const Params P, const DevPtrs d, uint32_t colo
 
 // dat_restore_failed_surface (27_planar_dat.metal:1287-1310)
 __global__ void k_dat_restore(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= P.numBodies || d.shape[gid].w >= 0.0f) return;
     const Counters* c = d.counters;
@@ -1112,6 +1124,7 @@ __global__ void k_dat_restore(const Params P, const DevPtrs d) {
 
 // smooth_particle_velocities (40_solver.metal:2154-2180); velRead is a copy.
 __global__ void k_smooth(const Params P, const DevPtrs d, const float4* velRead) {
+    pdl_prologue();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= P.numParticles) return;
     const uint32_t v = d.particleIdx[gid];
@@ -1133,17 +1146,17 @@ void build_pairs(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t
     const uint32_t total = z.numTris + z.numEdges;
     const uint32_t buckets = 2 * z.elemHashSize;
     cudaMemsetAsync(d.elemCellCount, 0, sizeof(uint32_t) * buckets, st);
-    k_elem_bin<false><<<blocks_for(total, 128), 128, 0, st>>>(P, d, total);
+    launch_pdl(k_elem_bin<false>, blocks_for(total, 128), 128, st, P, d, total);
     launch_exclusive_scan_large(d.elemCellCount, d.elemCellStart, buckets, d.bigScanScratch, st);
     cudaMemcpyAsync(d.elemCursor, d.elemCellStart, sizeof(uint32_t) * buckets, cudaMemcpyDeviceToDevice, st);
-    k_elem_bin<true><<<blocks_for(total, 128), 128, 0, st>>>(P, d, total);
+    launch_pdl(k_elem_bin<true>, blocks_for(total, 128), 128, st, P, d, total);
     const uint32_t owners = z.numParticles + z.numEdges;
     if (owners == 0) return;
     const uint32_t wblocks = blocks_for(owners * 32u, 128);
-    k_dat_pairs<false><<<wblocks, 128, 0, st>>>(P, d, owners);
+    launch_pdl(k_dat_pairs<false>, wblocks, 128, st, P, d, owners);
     launch_exclusive_scan_large(d.datOwnerCount, d.datOwnerStart, owners, d.bigScanScratch, st);
-    k_dat_pairs<true><<<wblocks, 128, 0, st>>>(P, d, owners);
-    k_dat_pair_totals<<<1, 32, 0, st>>>(P, d, owners);
+    launch_pdl(k_dat_pairs<true>, wblocks, 128, st, P, d, owners);
+    launch_pdl(k_dat_pair_totals, 1, 32, st, P, d, owners);
 }
 
 }  // namespace
@@ -1151,17 +1164,17 @@ void build_pairs(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t
 void launch_rt_emit(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
     if (z.numTris == 0) return;
     const bool warp = P.numGlobals > 32;
-    if (warp) k_rt_emit<true><<<blocks_for(z.numTris * 32u, 128), 128, 0, st>>>(P, d);
-    else k_rt_emit<false><<<blocks_for(z.numTris, 128), 128, 0, st>>>(P, d);
+    if (warp) launch_pdl(k_rt_emit<true>, blocks_for(z.numTris * 32u, 128), 128, st, P, d);
+    else launch_pdl(k_rt_emit<false>, blocks_for(z.numTris, 128), 128, st, P, d);
     launch_exclusive_scan_large(d.rtCount, d.rtStart, z.numTris, d.bigScanScratch, st);
-    k_rt_write<<<blocks_for(z.numTris, 128), 128, 0, st>>>(P, d);
-    k_rt_totals<<<1, 32, 0, st>>>(P, d);
+    launch_pdl(k_rt_write, blocks_for(z.numTris, 128), 128, st, P, d);
+    launch_pdl(k_rt_totals, 1, 32, st, P, d);
 }
 
 void launch_soft_map(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t owners, cudaStream_t st) {
-    k_soft_totals<<<1, 32, 0, st>>>(P, d, owners);
+    launch_pdl(k_soft_totals, 1, 32, st, P, d, owners);
     cudaMemsetAsync(d.softKeyA, 0, sizeof(uint32_t) * P.softMapCapacity, st);
-    k_softmap_insert<<<blocks_for(z.maxSoft, 128), 128, 0, st>>>(P, d);
+    launch_pdl(k_softmap_insert, blocks_for(z.maxSoft, 128), 128, st, P, d);
 }
 
 void launch_cloth_detect(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
@@ -1172,19 +1185,19 @@ void launch_cloth_detect(const Params& P, const DevPtrs& d, const Sizes& z, cuda
 void launch_cloth_accept(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
     const uint32_t cap = 148u * 16u;
     // predictor pass over the step-start stream
-    k_dat_reduce<<<blocks_for(z.maxDatPairs, 128, cap), 128, 0, st>>>(P, d, FULL_PASS);
-    if (z.numParticles) k_dat_apply_particles<<<(z.numParticles + 127) / 128, 128, 0, st>>>(P, d);
+    launch_pdl(k_dat_reduce, blocks_for(z.maxDatPairs, 128, cap), 128, st, P, d, FULL_PASS);
+    if (z.numParticles) launch_pdl(k_dat_apply_particles, (z.numParticles + 127) / 128, 128, st, P, d);
     // accepted-pose stream, element contacts, soft map
     build_pairs(P, d, z, st);
     const uint32_t owners = z.numParticles + z.numEdges;
     if (owners) {
         const uint32_t wblocks = blocks_for(owners * 32u, 128);
-        k_dat_contacts<false><<<wblocks, 128, 0, st>>>(P, d, owners);
+        launch_pdl(k_dat_contacts<false>, wblocks, 128, st, P, d, owners);
         launch_exclusive_scan_large(d.datEmit, d.datEmitStart, owners, d.bigScanScratch, st);
-        k_dat_contacts<true><<<wblocks, 128, 0, st>>>(P, d, owners);
+        launch_pdl(k_dat_contacts<true>, wblocks, 128, st, P, d, owners);
     }
     launch_soft_map(P, d, z, owners, st);
-    if (z.numParticles) k_reanchor<<<(z.numParticles + 127) / 128, 128, 0, st>>>(P, d);
+    if (z.numParticles) launch_pdl(k_reanchor, (z.numParticles + 127) / 128, 128, st, P, d);
 }
 
 void launch_dat_color(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t color, uint32_t count,
@@ -1197,14 +1210,14 @@ void launch_dat_color(const Params& P, const DevPtrs& d, const Sizes& z, uint32_
 }
 
 void launch_cloth_restore(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    k_dat_restore<<<(z.numBodies + 127) / 128, 128, 0, st>>>(P, d);
+    launch_pdl(k_dat_restore, (z.numBodies + 127) / 128, 128, st, P, d);
 }
 
 void launch_cloth_smoothing(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
     if (!(P.clothViscosity > 0.0f) || z.numParticles == 0) return;
     // inertLin is dead after the solve and rewritten by the next warm start
     cudaMemcpyAsync(d.inertLin, d.velLin, sizeof(float4) * z.numBodies, cudaMemcpyDeviceToDevice, st);
-    k_smooth<<<(z.numParticles + 127) / 128, 128, 0, st>>>(P, d, d.inertLin);
+    launch_pdl(k_smooth, (z.numParticles + 127) / 128, 128, st, P, d, d.inertLin);
 }
 
 }  // namespace avbd

@@ -873,8 +873,8 @@ struct AdamArgs { float *prm, *m, *v; uint32_t step; float lr, b1, b2, eps; };
 // outputs and, after an exchange in shared memory, written along the inputs
 // (whole 32-byte sectors both ways).
 template <bool ADAM>
-__global__ void __launch_bounds__(256) k_train_reduce(const float* __restrict__ part, uint32_t parts, uint32_t n,
-                                                      float* __restrict__ grad, AdamArgs a, float* loss) {
+__global__ void __launch_bounds__(256) k_train_reduce(const float* part, uint32_t parts, uint32_t n, float* grad,
+                                                      AdamArgs a, float* loss) {
     using namespace mlp;
     __shared__ float ex[8][33];
     constexpr uint32_t B3 = 64, B2 = B3 + 64, B1 = B2 + 16, B4 = B1 + 8;   // blocks of dW3, dW2, dW1, dW4
@@ -1025,6 +1025,7 @@ __device__ __forceinline__ void learn_pose(const Params& P, const DevPtrs& d, ui
 // Contact state of every learned vertex: count of contact points, closest
 // gap and summed oriented normal of its manifolds and element contacts.
 __global__ void k_learn_contacts(const Params P, const DevPtrs d, uint32_t n) {
+    pdl_prologue();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t v = d.learnIdx[i];
@@ -1061,6 +1062,7 @@ __global__ void k_learn_contacts(const Params P, const DevPtrs d, uint32_t n) {
 // are precomputed at upload; the ring's contact state sums the neighbours'
 // contact counts (times their multiplicity) and takes their closest gap.
 __global__ void k_learn_features(const Params P, const DevPtrs d, uint32_t n) {
+    pdl_prologue();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t v = d.learnIdx[i];
@@ -1139,6 +1141,7 @@ __global__ void k_learn_features(const Params P, const DevPtrs d, uint32_t n) {
 
 // x0 = x_plain + s * prediction for every learned row
 __global__ void k_learn_apply(const Params P, const DevPtrs d, uint32_t n) {
+    pdl_prologue();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t v = d.learnIdx[i];
@@ -1147,6 +1150,7 @@ __global__ void k_learn_apply(const Params P, const DevPtrs d, uint32_t n) {
 
 // keep the prediction when its residual after the trial sweeps is no worse
 __global__ void k_learn_select(const Params P, const DevPtrs d, uint32_t n) {
+    pdl_prologue();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool accept = d.learnResid[1] <= d.learnResid[0];
     if (i == 0 && accept) atomicAdd(d.learnAccepted, 1u);
@@ -1158,6 +1162,7 @@ __global__ void k_learn_select(const Params P, const DevPtrs d, uint32_t n) {
 // Pose buffers of the predicted branch: the solver's pose with every
 // learned row (the first n slots) moved by its prediction.
 __global__ void k_learn_branch(const Params P, const DevPtrs d, uint32_t nb, uint32_t n) {
+    pdl_prologue();
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     const uint32_t slot = d.learnSlot[b];
@@ -1172,6 +1177,7 @@ __global__ void k_learn_branch(const Params P, const DevPtrs d, uint32_t nb, uin
 // After both trial sweeps: adopt the predicted branch's swept pose when its
 // residual is no worse; otherwise the plain branch's pose stays.
 __global__ void k_learn_adopt(const Params P, const DevPtrs d, uint32_t nb) {
+    pdl_prologue();
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     const bool accept = d.learnResid[1] <= d.learnResid[0];
     if (b == 0 && accept) atomicAdd(d.learnAccepted, 1u);
@@ -1186,6 +1192,7 @@ __global__ void k_learn_adopt(const Params P, const DevPtrs d, uint32_t nb) {
 // training target: the solve's correction of the plain warm start (the
 // rotation part zero for particles)
 __global__ void k_learn_target(const Params P, const DevPtrs d, uint32_t n) {
+    pdl_prologue();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t v = d.learnIdx[i];
@@ -1199,6 +1206,7 @@ __global__ void k_learn_target(const Params P, const DevPtrs d, uint32_t n) {
 }
 
 __global__ void k_copy_double(const double* src, double* dst) {
+    pdl_prologue();
     if (threadIdx.x == 0 && blockIdx.x == 0) *dst = *src;
 }
 
@@ -1206,25 +1214,25 @@ __global__ void k_copy_double(const double* src, double* dst) {
 
 void launch_learn_features(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
     if (!z.numLearn) return;
-    k_learn_contacts<<<(z.numLearn + 127) / 128, 128, 0, st>>>(P, d, z.numLearn);
-    k_learn_features<<<(z.numLearn + 127) / 128, 128, 0, st>>>(P, d, z.numLearn);
+    launch_pdl(k_learn_contacts, (z.numLearn + 127) / 128, 128, st, P, d, z.numLearn);
+    launch_pdl(k_learn_features, (z.numLearn + 127) / 128, 128, st, P, d, z.numLearn);
 }
 void launch_learn_apply(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    if (z.numLearn) k_learn_apply<<<(z.numLearn + 127) / 128, 128, 0, st>>>(P, d, z.numLearn);
+    if (z.numLearn) launch_pdl(k_learn_apply, (z.numLearn + 127) / 128, 128, st, P, d, z.numLearn);
 }
 void launch_learn_select(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    k_learn_select<<<(z.numLearn + 128) / 128, 128, 0, st>>>(P, d, z.numLearn);
+    launch_pdl(k_learn_select, (z.numLearn + 128) / 128, 128, st, P, d, z.numLearn);
 }
 void launch_learn_branch(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    k_learn_branch<<<(z.numBodies + 127) / 128, 128, 0, st>>>(P, d, z.numBodies, z.numLearn);
+    launch_pdl(k_learn_branch, (z.numBodies + 127) / 128, 128, st, P, d, z.numBodies, z.numLearn);
 }
 void launch_learn_adopt(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    k_learn_adopt<<<(z.numBodies + 127) / 128, 128, 0, st>>>(P, d, z.numBodies);
+    launch_pdl(k_learn_adopt, (z.numBodies + 127) / 128, 128, st, P, d, z.numBodies);
 }
 void launch_learn_target(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    if (z.numLearn) k_learn_target<<<(z.numLearn + 127) / 128, 128, 0, st>>>(P, d, z.numLearn);
+    if (z.numLearn) launch_pdl(k_learn_target, (z.numLearn + 127) / 128, 128, st, P, d, z.numLearn);
 }
-void launch_copy_double(const double* src, double* dst, cudaStream_t st) { k_copy_double<<<1, 32, 0, st>>>(src, dst); }
+void launch_copy_double(const double* src, double* dst, cudaStream_t st) { launch_pdl(k_copy_double, 1, 32, st, src, dst); }
 
 // weights, two input tiles, biases and normalisation: 98 KiB of shared memory
 // (set once per device)

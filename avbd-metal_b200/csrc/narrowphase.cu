@@ -8,6 +8,7 @@
 // the same collider pair (map lookup + feature key or proximity match).
 #include "dmath.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace avbd {
 
@@ -865,6 +866,7 @@ __device__ void narrow_one(const Params& P, const DevPtrs& d, uint32_t gid) {
 
 template <bool ROUND>
 __global__ void k_narrowphase(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t n = d.counters->numPairs;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x)
         narrow_one<ROUND>(P, d, g);
@@ -872,6 +874,7 @@ __global__ void k_narrowphase(const Params P, const DevPtrs d) {
 
 // Insert this frame's active manifolds (queried by next frame's narrowphase).
 __global__ void k_map_insert(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t n = d.counters->numPairs;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x) {
         const ManifoldGPU& m = d.manifolds[g];
@@ -896,13 +899,13 @@ static uint32_t stride_blocks(uint32_t upper, int threads) {
 }
 
 void launch_narrowphase(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    k_narrowphase<false><<<stride_blocks(z.maxPairs, 128), 128, 0, st>>>(P, d);
-    if (P.roundShapes) k_narrowphase<true><<<stride_blocks(z.maxPairs, 128), 128, 0, st>>>(P, d);
+    launch_pdl(k_narrowphase<false>, stride_blocks(z.maxPairs, 128), 128, st, P, d);
+    if (P.roundShapes) launch_pdl(k_narrowphase<true>, stride_blocks(z.maxPairs, 128), 128, st, P, d);
 }
 
 void launch_map_rebuild(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
     cudaMemsetAsync(d.mapKeyA, 0, sizeof(uint32_t) * P.mapCapacity, st);
-    k_map_insert<<<stride_blocks(z.maxPairs, 128), 128, 0, st>>>(P, d);
+    launch_pdl(k_map_insert, stride_blocks(z.maxPairs, 128), 128, st, P, d);
 }
 
 }  // namespace avbd

@@ -81,6 +81,7 @@ __device__ bool iso_bounds(const Params& P, const DevPtrs& d, uint32_t gid, floa
 
 template <bool SCATTER>
 __global__ void k_ogc_bin(const Params P, const DevPtrs d, uint32_t total) {
+    pdl_prologue();
     for (uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x; gid < total; gid += gridDim.x * blockDim.x) {
         float3 lo, hi;
         if (!iso_bounds(P, d, gid, lo, hi)) continue;
@@ -108,6 +109,7 @@ __global__ void k_ogc_bin(const Params P, const DevPtrs d, uint32_t total) {
 // Every bucket in element order (entries of a bucket are distinct element
 // indices): the ballot bucket sort of bucket_sort.cuh.
 __global__ void k_ogc_sort_cells(const DevPtrs d, uint32_t buckets) {
+    pdl_prologue();
     rank_sort_buckets(d.elemCellCount, d.elemCellStart, d.elemCellsTmp, d.elemCells, buckets);
 }
 
@@ -419,6 +421,7 @@ __device__ __forceinline__ void load_partial(const DevPtrs& d, uint32_t o, Best4
 // grid scans run without idle lanes.  Each owner's result is independent of
 // the queue order.
 __global__ void k_ogc_track(const Params P, const DevPtrs d, uint32_t owners) {
+    pdl_prologue();
     const uint32_t frame = d.frameCounter[0];
     for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < owners; o += gridDim.x * blockDim.x) {
         Best4 best;
@@ -567,6 +570,7 @@ __device__ void ee_consider_kept(const Params& P, const DevPtrs& d, const EeQuer
 }
 
 __global__ void __launch_bounds__(128) k_ogc_reseed(const Params P, const DevPtrs d) {
+    pdl_prologue();
     // per warp: the queue of candidates kept by the topological tests
     // (element, arrival), drained 32 at a time onto the lanes
     __shared__ uint32_t keptId[4][64], keptArr[4][64];
@@ -664,6 +668,7 @@ __global__ void __launch_bounds__(128) k_ogc_reseed(const Params P, const DevPtr
 }
 
 __global__ void k_ogc_emit(const Params P, const DevPtrs d, uint32_t owners) {
+    pdl_prologue();
     const uint32_t head = d.counters->numSoftRT;
     for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < owners; o += gridDim.x * blockDim.x) {
         uint32_t slot = head + d.datEmitStart[o];
@@ -689,6 +694,7 @@ __global__ void k_ogc_emit(const Params P, const DevPtrs d, uint32_t owners) {
 }
 
 __global__ void k_ogc_totals(const Params P, const DevPtrs d, uint32_t owners) {
+    pdl_prologue();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const uint32_t vt = P.numParticles < owners ? d.datEmitStart[P.numParticles]
                                                 : (owners ? d.datEmitStart[owners - 1] + d.datEmit[owners - 1] : 0u);
@@ -772,21 +778,21 @@ void launch_ogc_detect(const Params& P, const DevPtrs& d, const Sizes& z, cudaSt
     const uint32_t total = z.numTris + P.numEdges;
     const uint32_t buckets = 2 * z.elemHashSize;
     cudaMemsetAsync(d.elemCellCount, 0, sizeof(uint32_t) * buckets, st);
-    k_ogc_bin<false><<<grid_for(total, 128), 128, 0, st>>>(P, d, total);
+    launch_pdl(k_ogc_bin<false>, grid_for(total, 128), 128, st, P, d, total);
     launch_exclusive_scan_large(d.elemCellCount, d.elemCellStart, buckets, d.bigScanScratch, st);
     cudaMemcpyAsync(d.elemCursor, d.elemCellStart, sizeof(uint32_t) * buckets, cudaMemcpyDeviceToDevice, st);
-    k_ogc_bin<true><<<grid_for(total, 128), 128, 0, st>>>(P, d, total);
-    k_ogc_sort_cells<<<grid_for(buckets * 32u, 128), 128, 0, st>>>(d, buckets);
+    launch_pdl(k_ogc_bin<true>, grid_for(total, 128), 128, st, P, d, total);
+    launch_pdl(k_ogc_sort_cells, grid_for(buckets * 32u, 128), 128, st, d, buckets);
     const uint32_t owners = z.numParticles + P.numEdges;
     if (owners) {
-        k_ogc_track<<<grid_for(owners, 128), 128, 0, st>>>(P, d, owners);
-        k_ogc_reseed<<<grid_for(owners * 32u, 128), 128, 0, st>>>(P, d);
+        launch_pdl(k_ogc_track, grid_for(owners, 128), 128, st, P, d, owners);
+        launch_pdl(k_ogc_reseed, grid_for(owners * 32u, 128), 128, st, P, d);
     }
     launch_rt_emit(P, d, z, st);
     if (owners) {
         launch_exclusive_scan_large(d.datEmit, d.datEmitStart, owners, d.bigScanScratch, st);
-        k_ogc_emit<<<grid_for(owners, 128), 128, 0, st>>>(P, d, owners);
-        k_ogc_totals<<<1, 32, 0, st>>>(P, d, owners);
+        launch_pdl(k_ogc_emit, grid_for(owners, 128), 128, st, P, d, owners);
+        launch_pdl(k_ogc_totals, 1, 32, st, P, d, owners);
     }
     launch_soft_map(P, d, z, owners, st);
 }

@@ -1,4 +1,4 @@
-// pdl.cuh — programmatic dependent launch for the iteration loop, a chain
+// pdl.cuh — programmatic dependent launch for a frame, a chain
 // of ~100-300 dependent kernels per frame.  Each kernel lets the next one be
 // scheduled as soon as all of its own blocks are running, and waits for the
 // previous grid to complete (and its writes to be visible) before touching

@@ -42,6 +42,7 @@ static uint32_t stride_blocks(uint32_t upper, int threads) {
 // Warm start (40_solver.metal:546-722)
 // ---------------------------------------------------------------------------
 __global__ void k_warmstart_constraints(const Params P, const DevPtrs d, uint32_t nJ, uint32_t nS) {
+    pdl_prologue();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nJ + nS) return;
     if (t >= nJ) {
@@ -118,6 +119,7 @@ __global__ void k_warmstart_constraints(const Params P, const DevPtrs d, uint32_
 }
 
 __global__ void k_warmstart_bodies(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= P.numBodies) return;
     const float4 pl = d.posLin[gid], pa = d.posAng[gid];
@@ -158,8 +160,8 @@ __global__ void k_warmstart_bodies(const Params P, const DevPtrs d) {
 
 void launch_warmstart(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
     const uint32_t n = z.numActiveJoints + z.numHardSprings;
-    if (n) k_warmstart_constraints<<<(n + 127) / 128, 128, 0, st>>>(P, d, z.numActiveJoints, z.numHardSprings);
-    k_warmstart_bodies<<<(P.numBodies + 127) / 128, 128, 0, st>>>(P, d);
+    if (n) launch_pdl(k_warmstart_constraints, (n + 127) / 128, 128, st, P, d, z.numActiveJoints, z.numHardSprings);
+    launch_pdl(k_warmstart_bodies, (P.numBodies + 127) / 128, 128, st, P, d);
 }
 
 // ---------------------------------------------------------------------------
@@ -168,6 +170,7 @@ void launch_warmstart(const Params& P, const DevPtrs& d, const Sizes& z, cudaStr
 // Items: this frame's manifolds, then (cloth scenes) its element contacts.
 template <bool SCATTER>
 __global__ void k_adj_dyn(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t nm = d.counters->numPairs;
     const uint32_t ns = (P.cloth || P.ogc) ? d.counters->numSoft : 0u;
     auto put = [&](uint32_t b, uint32_t e) {
@@ -199,6 +202,7 @@ __global__ void k_adj_dyn(const Params P, const DevPtrs d) {
 constexpr uint32_t kLongSegment = 2048;   // entries a block sorts in shared memory
 
 __global__ void k_adj_dyn_sort(const DevPtrs d, uint32_t nb) {
+    pdl_prologue();
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     uint32_t* l = d.dynList + d.dynStart[b];
@@ -243,6 +247,7 @@ __global__ void k_adj_dyn_sort(const DevPtrs d, uint32_t nb) {
 // it back and marks the manifold run.  Entries are distinct, so the result
 // equals the serial sort.
 __global__ void __launch_bounds__(256) k_adj_long_sort(const DevPtrs d) {
+    pdl_prologue();
     __shared__ uint32_t buf[kLongSegment];
     const uint32_t count = d.counters->adjLong;
     for (uint32_t q = blockIdx.x; q < count; q += gridDim.x) {
@@ -286,12 +291,12 @@ __global__ void __launch_bounds__(256) k_adj_long_sort(const DevPtrs d) {
 void launch_adjacency(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
     cudaMemsetAsync(d.dynCount, 0, sizeof(uint32_t) * P.numBodies, st);
     const uint32_t items = z.maxPairs + ((P.cloth || P.ogc) ? z.maxSoft : 0u);
-    k_adj_dyn<false><<<stride_blocks(items, 128), 128, 0, st>>>(P, d);
+    launch_pdl(k_adj_dyn<false>, stride_blocks(items, 128), 128, st, P, d);
     launch_exclusive_scan(d.dynCount, d.dynStart, P.numBodies, d.scanScratch, st);
     cudaMemcpyAsync(d.dynCursor, d.dynStart, sizeof(uint32_t) * P.numBodies, cudaMemcpyDeviceToDevice, st);
-    k_adj_dyn<true><<<stride_blocks(items, 128), 128, 0, st>>>(P, d);
-    k_adj_dyn_sort<<<(P.numBodies + 127) / 128, 128, 0, st>>>(d, P.numBodies);
-    k_adj_long_sort<<<148, 256, 0, st>>>(d);
+    launch_pdl(k_adj_dyn<true>, stride_blocks(items, 128), 128, st, P, d);
+    launch_pdl(k_adj_dyn_sort, (P.numBodies + 127) / 128, 128, st, d, P.numBodies);
+    launch_pdl(k_adj_long_sort, 148, 256, st, d);
 }
 
 // The five runs in ascending (kind << 28 | index) order: static pre
@@ -448,6 +453,7 @@ constexpr int kColorPasses = 20;
 // Above 65,536 bodies the passes use the whole device, a launch each.
 template <bool CLUSTER>
 __global__ void __launch_bounds__(1024) k_color(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
     const volatile uint32_t* changed = d.counters->changed;
     auto barrier = [&]() {
@@ -506,13 +512,15 @@ static void launch_cluster(void (*kernel)(KArgs...), uint32_t ctas, uint32_t thr
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
@@ -1285,6 +1293,7 @@ __device__ void rigid_residual(const Params& P, const DevPtrs& d, uint32_t body,
 // a warp shuffle tree and a second tree over the warps combine the threads,
 // always in the same order.
 __global__ void __launch_bounds__(1024) k_sum_fixed(const float* v, uint32_t n, double* out) {
+    pdl_prologue();
     __shared__ double part[32];
     const uint32_t t = threadIdx.x, n4 = n / 4u;
     const float4* v4 = reinterpret_cast<const float4*>(v);
@@ -1977,13 +1986,13 @@ void launch_residual(const Params& P, const DevPtrs& d, const Sizes& z, float* p
             const uint32_t w = lanes <= 8 ? 8u : (lanes <= 16 ? 16u : 32u);
             const uint32_t blocks = (count * w + 127) / 128;
             if (z.particleFastPath) {
-                if (w == 8) k_primal_group<8, false, false, true><<<blocks, 128, 0, st>>>(P, g, color, count, 0u, NO_HOST_START);
-                else if (w == 16) k_primal_group<16, false, false, true><<<blocks, 128, 0, st>>>(P, g, color, count, 0u, NO_HOST_START);
-                else k_primal_group<32, false, false, true><<<blocks, 128, 0, st>>>(P, g, color, count, 0u, NO_HOST_START);
+                if (w == 8) launch_pdl(k_primal_group<8, false, false, true>, blocks, 128, st, P, g, color, count, 0u, NO_HOST_START);
+                else if (w == 16) launch_pdl(k_primal_group<16, false, false, true>, blocks, 128, st, P, g, color, count, 0u, NO_HOST_START);
+                else launch_pdl(k_primal_group<32, false, false, true>, blocks, 128, st, P, g, color, count, 0u, NO_HOST_START);
             } else if (P.cloth || P.ogc) {
-                k_primal_group<32, true, true, true><<<(count * 32 + 127) / 128, 128, 0, st>>>(P, g, color, count, 0u, NO_HOST_START);
+                launch_pdl(k_primal_group<32, true, true, true>, (count * 32 + 127) / 128, 128, st, P, g, color, count, 0u, NO_HOST_START);
             } else {
-                k_primal_group<32, true, false, true><<<(count * 32 + 127) / 128, 128, 0, st>>>(P, g, color, count, 0u, NO_HOST_START);
+                launch_pdl(k_primal_group<32, true, false, true>, (count * 32 + 127) / 128, 128, st, P, g, color, count, 0u, NO_HOST_START);
             }
         };
         // every body at once: 8 lanes per body keep the most bodies in
@@ -1995,10 +2004,10 @@ void launch_residual(const Params& P, const DevPtrs& d, const Sizes& z, float* p
         DevPtrs g = d;
         g.learnResidBodies = perBody;
         const uint32_t blocks = (n * 8 + 127) / 128;
-        if (P.cloth || P.ogc) k_primal_group<8, true, true, true><<<blocks, 128, 0, st>>>(P, g, 0u, n, 0u, NO_HOST_START);
-        else k_primal_group<8, true, false, true><<<blocks, 128, 0, st>>>(P, g, 0u, n, 0u, NO_HOST_START);
+        if (P.cloth || P.ogc) launch_pdl(k_primal_group<8, true, true, true>, blocks, 128, st, P, g, 0u, n, 0u, NO_HOST_START);
+        else launch_pdl(k_primal_group<8, true, false, true>, blocks, 128, st, P, g, 0u, n, 0u, NO_HOST_START);
     }
-    k_sum_fixed<<<1, 1024, 0, st>>>(perBody, n, total);
+    launch_pdl(k_sum_fixed, 1, 1024, st, perBody, n, total);
 }
 
 // ---------------------------------------------------------------------------
@@ -2182,6 +2191,7 @@ constexpr uint32_t kSmallSlots = kIncWords * kSmallThreads;      // floats of dy
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_solve_small(const Params P, const DevPtrs d, const Sizes z,
                                                                   uint32_t colorBound) {
+    pdl_prologue();
     extern __shared__ float slots[];
     const uint32_t ctas = gridDim.x, rank = blockIdx.x;          // the grid is one cluster
     const uint32_t groups = (blockDim.x >> 3) * ctas;
@@ -2243,6 +2253,7 @@ void launch_solve_small(const Params& P, const DevPtrs& d, const Sizes& z, uint3
 // BDF1 velocity finalize (40_solver.metal:2108-2147)
 // ---------------------------------------------------------------------------
 __global__ void k_finalize(const Params P, const DevPtrs d) {
+    pdl_prologue();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= P.numBodies) return;
     const float4 vold = d.velLin[gid];
@@ -2266,7 +2277,7 @@ __global__ void k_finalize(const Params P, const DevPtrs d) {
 }
 
 void launch_finalize(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    k_finalize<<<(P.numBodies + 127) / 128, 128, 0, st>>>(P, d);
+    launch_pdl(k_finalize, (P.numBodies + 127) / 128, 128, st, P, d);
 }
 
 // ---------------------------------------------------------------------------
@@ -2358,6 +2369,7 @@ void launch_reset_bodies(const Params& P, const DevPtrs& d, const Sizes& z, cuda
 // (the checks of `retire`, GPUSolver.swift:2885-2918).
 // ---------------------------------------------------------------------------
 __global__ void k_frame_end(const Params P, const DevPtrs d, const Sizes z, float dt) {
+    pdl_prologue();
     const uint32_t t = threadIdx.x;
     for (uint32_t i = t; i < d.numRateMotors; i += blockDim.x) {
         JointGPU& j = d.joints[d.rateJoint[i]];
@@ -2399,7 +2411,7 @@ __global__ void k_frame_end(const Params P, const DevPtrs d, const Sizes z, floa
 }
 
 void launch_frame_end(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    k_frame_end<<<1, 64, 0, st>>>(P, d, z, P.dt);
+    launch_pdl(k_frame_end, 1, 64, st, P, d, z, P.dt);
 }
 
 }  // namespace avbd
