@@ -90,6 +90,37 @@ constexpr uint32_t ELEM_EDGE_BIT = 0x80000000u;
 constexpr uint32_t RT_MAX_PER_TRI = 4;
 constexpr uint32_t FULL_PASS = 0xFFFFFFFFu;
 
+// Launch tables of the staged primal, built at upload: a block's bodies, the
+// static parts of their springs, membranes and bends (two 16-byte words each,
+// the first words of a body's records of one kind side by side, then the
+// second ones), their tets by index, and the bodies all of these refer to,
+// each listed once per body (the body itself first).
+struct alignas(16) StagedBody {
+    uint32_t body;
+    float radius;                 // shape.w
+    uint32_t rec, tet, pos;       // first record word, tet and position, within the block
+    uint32_t nPre, nTet, nRest;   // springs, tets, membranes and bends
+};
+struct alignas(16) StagedBlock {
+    uint32_t first, count;        // bodies
+    uint32_t rec, recLen;         // record words
+    uint32_t tet, tetLen;         // tets (even)
+    uint32_t ids, idLen;          // referenced bodies
+};
+struct StagedTet {
+    uint32_t index;               // tet, and this body's position in it << 28
+    uint32_t refs;                // the four vertices among the body's references, a byte each
+};
+struct alignas(16) TetConst { f4 r0, r1, r2, diag; };   // DmInv rows; w: alpha, muV, lamV; muV |w|^2 per vertex
+constexpr uint32_t STAGED_BODIES = 16;             // most bodies of a block (8 lanes each)
+constexpr uint32_t STAGED_MAX_WORDS = 2600;        // most 16-byte words of shared memory of a block
+constexpr uint32_t STAGED_MAX_REFS = 255;          // most bodies one body's records refer to
+// last word of a spring, membrane or bend record: this body's position in the
+// element (bits 0-1), then flags
+constexpr uint32_t STAGED_BEND = 4u;               // a bend, else a membrane
+constexpr uint32_t STAGED_HARD = 4u;               // spring: hard
+constexpr uint32_t STAGED_GENERIC = 8u;            // spring with levers or a rigid end: evaluated from its own record
+
 // Per-frame parameters (SimParams, 00_common.metal:233-288), passed by value.
 struct Params {
     float dt, gravity, alpha, betaLin, betaAng, gamma;

@@ -68,6 +68,13 @@ struct DevPtrs {
     uint32_t* tailTicket;                 // blocks done with the last launched color (zero between launches)
     uint32_t* postTets;                   // tet entries at the head of each static post segment
     const TetGPU* tetInc;                 // tet records in postList order (null without tets)
+    // staged primal (static palette): launch tables
+    const StagedBody* stagedBodies;
+    const StagedBlock* stagedBlocks;
+    const uint4* stagedRec;
+    const StagedTet* stagedTets;
+    const uint4* tetConst;                // TetConst records, four words each
+    const uint32_t* stagedIds;
     // coloring
     uint32_t *colorsA, *colorsB, *colorList, *bodySlot;
     uint32_t* colorLaunch;                // static palette: primal launch order per color
@@ -159,6 +166,9 @@ struct Sizes {
     const uint32_t* colorLanes;
     const uint32_t* colorLean;            // lean particles at the head of each color's launch order
     const uint32_t* colorStartHost;       // static palette: each color's start in the list
+    // staged primal: bodies of each color's launch order in blocks, the
+    // colors' first blocks, shared-memory words of a block
+    const uint32_t *colorStaged, *stagedStart, *stagedWords;
     // dynamic coloring: block shape of the rigid primal's grid-stride launch
     // (blocks, threads per block), chosen by the runtime's autotuner
     uint32_t dynBlocks, dynThreads;
@@ -177,8 +187,8 @@ void launch_dynamic_coloring(const Params& P, const DevPtrs& d, const Sizes& z, 
 // one color of the block-descent primal; `count` is the color's body count
 // when known on the host (static palette), else 0xFFFFFFFF (read on device);
 // `lanes` is 8, 16 or 32 lanes per body (grouped kernel) or
-// AVBD_PRIMAL_STAGED (staged kernel: block-wide term evaluation, then an
-// 8-lane fold per body), every choice computing the same floats
+// AVBD_PRIMAL_STAGED (staged kernel: a block's records and positions in shared
+// memory, 8 lanes per body), every choice computing the same floats
 // With a side stream and two events, the color's non-lean bodies (a block
 // each) run on the side stream beside the lean particles (a fork and a join
 // on `st`; in a captured frame, two parallel graph branches).

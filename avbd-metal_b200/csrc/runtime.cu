@@ -513,6 +513,9 @@ struct avbd_solver {
         z.colorCounts = H.dynamicColoring ? nullptr : H.colorCounts.data();
         z.colorLanes = H.colorLanes.data();
         z.colorLean = H.colorLean.data();
+        z.colorStaged = H.colorStaged.data();
+        z.stagedStart = H.stagedStart.data();
+        z.stagedWords = H.stagedWords.data();
         z.colorStartHost = H.dynamicColoring ? nullptr : H.colorStart.data();
         z.numDynamicRigid = 0;
         for (uint32_t b = 0; b < nb; b++) z.numDynamicRigid += (H.posLin[b].w > 0.0f && H.shape[b].w >= 0.0f) ? 1u : 0u;
@@ -597,6 +600,23 @@ struct avbd_solver {
             d.tetInc = ti;
         }
 #endif
+        if (!H.stagedBlocks.empty()) {
+            StagedBody* sb = nullptr;
+            StagedBlock* sk = nullptr;
+            u4* sr = nullptr;
+            StagedTet* stt = nullptr;
+            TetConst* tcn = nullptr;
+            uint32_t* si = nullptr;
+            ok = ok && upload(sb, H.stagedBodies, "stagedBodies") && upload(sk, H.stagedBlocks, "stagedBlocks") &&
+                 upload(sr, H.stagedRec, "stagedRecords") && upload(stt, H.stagedTets, "stagedTets") &&
+                 upload(tcn, H.tetConst, "tetConstants") && upload(si, H.stagedIds, "stagedReferences");
+            d.stagedBodies = sb;
+            d.stagedBlocks = sk;
+            d.stagedRec = reinterpret_cast<const uint4*>(sr);
+            d.stagedTets = stt;
+            d.tetConst = reinterpret_cast<const uint4*>(tcn);
+            d.stagedIds = si;
+        }
         ok = ok && alloc(d.adjLongQueue, nb, "adjLongQueue") && alloc(d.activeManifolds, H.maxPairs, "activeManifolds");
         ok = ok && alloc(d.dynList, 2 * (size_t)H.maxPairs + ((P.cloth || P.ogc) ? 4 * (size_t)P.maxSoft : 0), "dynList");
         // coloring

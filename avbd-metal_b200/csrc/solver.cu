@@ -998,11 +998,12 @@ __device__ __forceinline__ void add_shfl_lower(unsigned mask, M3& m, int o) {
 // 40_solver.metal:1361-1382): the displacement since the bound's anchor stays
 // within max(0.45 * bound distance, 0.2 * radius); every clamped step is
 // counted for the mid-solve refresh.
-__device__ __forceinline__ float3 ogc_truncate(const DevPtrs& d, uint32_t body, float3 dxLin, float3 cur, float partR) {
-    const float d2 = __uint_as_float(d.ogcBounds[body]);
+// d2: the body's squared bound distance; anchor: where the bound was taken.
+__device__ __forceinline__ float3 ogc_truncate(const DevPtrs& d, float d2, float4 anchor, float3 dxLin, float3 cur,
+                                               float partR) {
     if (d2 >= 1e37f) return dxLin;
     const float bv = mx(0.45f * sqrtf(d2), 0.2f * partR);
-    const float3 x0 = xyz(d.ogcPrev[body]);
+    const float3 x0 = xyz(anchor);
     float3 tot = (cur + dxLin) - x0;
     const float t2 = dot(tot, tot);
     if (t2 > bv * bv) {
@@ -1062,7 +1063,8 @@ __device__ __forceinline__ void body_commit(const Params& P, const DevPtrs& d, u
     const float maxLin = 0.35f * fabsf(shp.w);
     const float lin2 = dot(dxLin, dxLin);
     if (lin2 > maxLin * maxLin) dxLin *= maxLin * rsq(lin2);
-    if (!rigid && P.ogc) dxLin = ogc_truncate(d, body, dxLin, xyz(pl), -shp.w);
+    if (!rigid && P.ogc)
+        dxLin = ogc_truncate(d, __uint_as_float(d.ogcBounds[body]), d.ogcPrev[body], dxLin, xyz(pl), -shp.w);
     if (P.colorJacobi) {
         d.posNext[body] = mk4(xyz(pl) + dxLin, mass);
         if (rigid) d.angNext[body] = q_addw(d.posAng[body], dxAng);
@@ -1342,14 +1344,13 @@ struct ParticleTerms {
     uint32_t kind;       // TERM_*
 };
 
-// Stable Neo-Hookean tet terms of vertex `self` (stampTet, 40_solver.metal:972-1024)
-__device__ __forceinline__ void tet_terms(const DevPtrs& d, const TetGPU& tt, uint32_t self, ParticleTerms& t) {
-    const float3 x0 = xyz(d.posLin[tt.ids.x]), x1 = xyz(d.posLin[tt.ids.y]);
-    const float3 x2 = xyz(d.posLin[tt.ids.z]), x3 = xyz(d.posLin[tt.ids.w]);
-    const float muV = tt.r1.w, lamV = tt.r2.w;
-    const float alphaT = 1.0f + muV / mx(lamV, 1e-9f);
+// Stable Neo-Hookean tet terms of one vertex (stampTet, 40_solver.metal:
+// 972-1024): w is the vertex's row of DmInv (minus the sum of the rows for the
+// first vertex), alphaT and diag = muV |w|^2 depend on the tet alone.
+__device__ __forceinline__ void tet_core(float3 x0, float3 x1, float3 x2, float3 x3, float3 m0, float3 m1, float3 m2,
+                                         float muV, float lamV, float alphaT, float3 w, float diag,
+                                         ParticleTerms& t) {
     const float3 d0 = x1 - x0, d1 = x2 - x0, d2 = x3 - x0;
-    const float3 m0 = xyz(tt.r0), m1 = xyz(tt.r1), m2 = xyz(tt.r2);
     const float3 f0 = d0 * m0.x + d1 * m1.x + d2 * m2.x;
     const float3 f1 = d0 * m0.y + d1 * m1.y + d2 * m2.y;
     const float3 f2 = d0 * m0.z + d1 * m1.z + d2 * m2.z;
@@ -1359,18 +1360,85 @@ __device__ __forceinline__ void tet_terms(const DevPtrs& d, const TetGPU& tt, ui
     const float3 p0 = muV * f0 + s2 * j0;
     const float3 p1 = muV * f1 + s2 * j1;
     const float3 p2 = muV * f2 + s2 * j2;
-    float3 w;
-    if (self == tt.ids.y) w = m0;
-    else if (self == tt.ids.z) w = m1;
-    else if (self == tt.ids.w) w = m2;
-    else w = -mk3(m0.x + m1.x + m2.x, m0.y + m1.y + m2.y, m0.z + m1.z + m2.z);
     t.rhs = p0 * w.x + p1 * w.y + p2 * w.z;
     const float3 g = j0 * w.x + j1 * w.y + j2 * w.z;
     // lamV * outer(g, g) is exactly symmetric: g_i g_j == g_j g_i
     t.a = mk3((g.x * g.x) * lamV, (g.y * g.y) * lamV, (g.z * g.z) * lamV);
     t.b = mk3((g.y * g.x) * lamV, (g.z * g.x) * lamV, (g.z * g.y) * lamV);
-    t.c = mk3(muV * dot(w, w), 0.0f, 0.0f);
-    t.kind = 1;
+    t.c = mk3(diag, 0.0f, 0.0f);
+    t.kind = TERM_TET;
+}
+__device__ __forceinline__ void tet_terms(const DevPtrs& d, const TetGPU& tt, uint32_t self, ParticleTerms& t) {
+    const float muV = tt.r1.w, lamV = tt.r2.w;
+    const float3 m0 = xyz(tt.r0), m1 = xyz(tt.r1), m2 = xyz(tt.r2);
+    float3 w;
+    if (self == tt.ids.y) w = m0;
+    else if (self == tt.ids.z) w = m1;
+    else if (self == tt.ids.w) w = m2;
+    else w = -mk3(m0.x + m1.x + m2.x, m0.y + m1.y + m2.y, m0.z + m1.z + m2.z);
+    tet_core(xyz(d.posLin[tt.ids.x]), xyz(d.posLin[tt.ids.y]), xyz(d.posLin[tt.ids.z]), xyz(d.posLin[tt.ids.w]), m0,
+             m1, m2, muV, lamV, 1.0f + muV / mx(lamV, 1e-9f), w, muV * dot(w, w), t);
+}
+
+// Spring, membrane and bend terms from the ends' positions, shared by the
+// grouped and the staged kernels.
+__device__ __forceinline__ void spring_core(const Params& P, float3 pA, float3 pB, bool isA, float stiffness, float rest,
+                                            bool hard, float4 dual, ParticleTerms& t) {
+    // stamp_spring's linear block: outer(+-n, +-n) equals outer(n, n) bit for bit
+    const float3 dd = pA - pB;
+    const float dLen = len3(dd);
+    t.kind = TERM_NONE;
+    if (dLen <= 1.0e-6f) return;
+    const float3 n = dd / dLen;
+    float f;
+    if (hard) {
+        const float C = dLen - rest - dual.z * P.alpha;
+        stiffness = dual.y;
+        f = stiffness * C + dual.x;
+        if (f <= 0.0f) return;
+    } else {
+        f = stiffness * (dLen - rest);
+    }
+    const float3 jLin = isA ? n : -n;
+    t.rhs = jLin * f;
+    t.a = n;
+    t.s = mk3(stiffness, mx(f, 0.0f) / dLen, 0.0f);
+    t.kind = TERM_SPRING;
+}
+__device__ __forceinline__ void membrane_core(float3 x0, float3 x1, float3 x2, float4 dmv, float muA, float lamA,
+                                              uint32_t self, ParticleTerms& t) {
+    const float3 d0 = x1 - x0, d1 = x2 - x0;
+    const float a = dmv.x, b = dmv.y, c = dmv.z, dm = dmv.w;
+    const float3 f1 = d0 * a + d1 * b;
+    const float3 f2 = d0 * c + d1 * dm;
+    const float E11 = 0.5f * (dot(f1, f1) - 1.0f);
+    const float E22 = 0.5f * (dot(f2, f2) - 1.0f);
+    const float E12 = 0.5f * dot(f1, f2);
+    const float trE = E11 + E22;
+    const float S11 = 2.0f * muA * E11 + lamA * trE;
+    const float S22 = 2.0f * muA * E22 + lamA * trE;
+    const float S12 = 2.0f * muA * E12;
+    const float3 p1 = f1 * S11 + f2 * S12;
+    const float3 p2 = f1 * S12 + f2 * S22;
+    float wx, wy;
+    if (self == 1u) { wx = a; wy = c; }
+    else if (self == 2u) { wx = b; wy = dm; }
+    else { wx = -a - b; wy = -c - dm; }
+    t.rhs = p1 * wx + p2 * wy;
+    t.a = f1 * wx;
+    t.b = f2 * wy;
+    t.c = (f2 * wx + f1 * wy) * 0.5f;
+    t.e = t.a + t.b;
+    t.s = mk3(2.0f * muA, 4.0f * muA, lamA);
+    t.kind = TERM_MEMBRANE;
+}
+__device__ __forceinline__ void bend_core(float3 x0, float3 x1, float3 x2, float3 x3, float4 K, float sc, uint32_t self,
+                                          ParticleTerms& t) {
+    const float3 m = x0 * K.x + x1 * K.y + x2 * K.z + x3 * K.w;
+    const float k = self == 0u ? K.x : (self == 1u ? K.y : (self == 2u ? K.z : K.w));
+    t.rhs = m * (sc * k);
+    t.s = mk3(sc * k * k, 0.0f, 0.0f);
+    t.kind = TERM_BEND;
 }
 
 template <bool CLOTH>
@@ -1413,72 +1481,19 @@ __device__ __forceinline__ void particle_terms(const Params& P, const DevPtrs& d
     } else if (!CLOTH) {
         return;
     } else if (kind == FK_SPRING) {
-        // stamp_spring's linear block: outer(+-n, +-n) equals outer(n, n) bit for bit
         const SpringGPU sp = d.springs[idx];
         const uint32_t a = sp.header.x, b = sp.header.y;
-        float stiffness = sp.rA.w;
-        const float3 pA = xform(xyz(d.posLin[a]), d.posAng[a], xyz(sp.rA));
-        const float3 pB = xform(xyz(d.posLin[b]), d.posAng[b], xyz(sp.rB));
-        const float3 dd = pA - pB;
-        const float dLen = len3(dd);
-        t.kind = TERM_NONE;
-        if (dLen <= 1.0e-6f) return;
-        const float3 n = dd / dLen;
-        float f;
-        if (sp.header.z != 0) {
-            const float C = dLen - sp.rB.w - sp.dual.z * P.alpha;
-            stiffness = sp.dual.y;
-            f = stiffness * C + sp.dual.x;
-            if (f <= 0.0f) return;
-        } else {
-            f = stiffness * (dLen - sp.rB.w);
-        }
-        const float3 jLin = self == a ? n : -n;
-        t.rhs = jLin * f;
-        t.a = n;
-        t.s = mk3(stiffness, mx(f, 0.0f) / dLen, 0.0f);
-        t.kind = TERM_SPRING;
+        spring_core(P, xform(xyz(d.posLin[a]), d.posAng[a], xyz(sp.rA)), xform(xyz(d.posLin[b]), d.posAng[b], xyz(sp.rB)),
+                    self == a, sp.rA.w, sp.rB.w, sp.header.z != 0, tof(sp.dual), t);
     } else if (kind == FK_MEMBRANE) {
         const MembraneGPU mb = d.membranes[idx];
-        const float3 x0 = xyz(d.posLin[mb.ids.x]), x1 = xyz(d.posLin[mb.ids.y]), x2 = xyz(d.posLin[mb.ids.z]);
-        const float muA = mb.mat.x, lamA = mb.mat.y;
-        const float3 d0 = x1 - x0, d1 = x2 - x0;
-        const float a = mb.dm.x, b = mb.dm.y, c = mb.dm.z, dm = mb.dm.w;
-        const float3 f1 = d0 * a + d1 * b;
-        const float3 f2 = d0 * c + d1 * dm;
-        const float E11 = 0.5f * (dot(f1, f1) - 1.0f);
-        const float E22 = 0.5f * (dot(f2, f2) - 1.0f);
-        const float E12 = 0.5f * dot(f1, f2);
-        const float trE = E11 + E22;
-        const float S11 = 2.0f * muA * E11 + lamA * trE;
-        const float S22 = 2.0f * muA * E22 + lamA * trE;
-        const float S12 = 2.0f * muA * E12;
-        const float3 p1 = f1 * S11 + f2 * S12;
-        const float3 p2 = f1 * S12 + f2 * S22;
-        float wx, wy;
-        if (self == mb.ids.y) { wx = a; wy = c; }
-        else if (self == mb.ids.z) { wx = b; wy = dm; }
-        else { wx = -a - b; wy = -c - dm; }
-        t.rhs = p1 * wx + p2 * wy;
-        t.a = f1 * wx;
-        t.b = f2 * wy;
-        t.c = (f2 * wx + f1 * wy) * 0.5f;
-        t.e = t.a + t.b;
-        t.s = mk3(2.0f * muA, 4.0f * muA, lamA);
-        t.kind = TERM_MEMBRANE;
+        membrane_core(xyz(d.posLin[mb.ids.x]), xyz(d.posLin[mb.ids.y]), xyz(d.posLin[mb.ids.z]), tof(mb.dm), mb.mat.x,
+                      mb.mat.y, self == mb.ids.y ? 1u : (self == mb.ids.z ? 2u : 0u), t);
     } else if (kind == FK_BEND) {
         const BendGPU bd = d.bends[idx];
-        const float sc = bd.mat.x;
-        const float3 m = xyz(d.posLin[bd.ids.x]) * bd.K.x + xyz(d.posLin[bd.ids.y]) * bd.K.y +
-                         xyz(d.posLin[bd.ids.z]) * bd.K.z + xyz(d.posLin[bd.ids.w]) * bd.K.w;
-        float k;
-        if (self == bd.ids.x) k = bd.K.x;
-        else if (self == bd.ids.y) k = bd.K.y;
-        else if (self == bd.ids.z) k = bd.K.z;
-        else k = bd.K.w;
-        t.rhs = m * (sc * k);
-        t.s = mk3(sc * k * k, 0.0f, 0.0f);
-        t.kind = TERM_BEND;
+        bend_core(xyz(d.posLin[bd.ids.x]), xyz(d.posLin[bd.ids.y]), xyz(d.posLin[bd.ids.z]), xyz(d.posLin[bd.ids.w]),
+                  tof(bd.K), bd.mat.x,
+                  self == bd.ids.x ? 0u : (self == bd.ids.y ? 1u : (self == bd.ids.z ? 2u : 3u)), t);
     } else if (kind == FK_SOFT) {
         const SoftContactGPU& sc = d.soft[idx];
         float3 n, t1, t2, rAW;
@@ -1631,18 +1646,21 @@ __device__ __forceinline__ float3 solve3x3_particle(const M3& a, float3 b) {
 
 // Inertia, solve, trust region, OGC bound and commit of a particle whose
 // stamped system is (acc.lhs, acc.rhs); lane 0 of its group calls this.
-__device__ __forceinline__ void particle_commit(const Params& P, const DevPtrs& d, uint32_t body, float4 shp,
-                                                float4 pl, float4 inert, ParticleAccum acc) {
+// (bound, anchor): the body's OGC bound and its anchor, read before the solve
+// so that they are there when the step is known.
+__device__ __forceinline__ void particle_commit(const Params& P, const DevPtrs& d, uint32_t body, float radius,
+                                                float4 pl, float4 inert, float bound, float4 anchor,
+                                                ParticleAccum acc) {
     const float mass = pl.w;
     const float dt2 = P.dt * P.dt;
     acc.lhs = m3_add(acc.lhs, m3_diag(s3(mass / dt2)));
     acc.rhs += (xyz(pl) - xyz(inert)) * (mass / dt2);
     float3 dxLin = solve3x3_particle(acc.lhs, -acc.rhs);
     if (!finite3(dxLin)) { keep_body(P, d, body, pl, false); return; }
-    const float maxLin = 0.35f * fabsf(shp.w);
+    const float maxLin = 0.35f * fabsf(radius);
     const float lin2 = dot(dxLin, dxLin);
     if (lin2 > maxLin * maxLin) dxLin *= maxLin * rsq(lin2);
-    if (P.ogc) dxLin = ogc_truncate(d, body, dxLin, xyz(pl), -shp.w);
+    if (P.ogc) dxLin = ogc_truncate(d, bound, anchor, dxLin, xyz(pl), -radius);
     if (P.colorJacobi) { d.posNext[body] = mk4(xyz(pl) + dxLin, mass); return; }
     d.posLin[body] = mk4(xyz(pl) + dxLin, mass);
 }
@@ -1713,7 +1731,13 @@ __global__ void __launch_bounds__(128, GENERAL ? 4 : (CLOTH ? AVBD_LEAN_CLOTH_MI
     }
     // lane 0 needs these after the reduction; issue the loads now
     float4 pl = make_float4(0, 0, 0, 0), inert = make_float4(0, 0, 0, 0);
-    if (lane == 0) { pl = d.posLin[body]; inert = d.inertLin[body]; }
+    float bound = 0.0f;
+    float4 anchor = make_float4(0, 0, 0, 0);
+    if (lane == 0) {
+        pl = d.posLin[body];
+        inert = d.inertLin[body];
+        if (!RESID && P.ogc) { bound = __uint_as_float(d.ogcBounds[body]); anchor = d.ogcPrev[body]; }
+    }
     ParticleAccum acc{m3_zero(), s3(0)};
     const AdjView v = adj_view_from(d, body, seg, nTet);
     const uint32_t cnt = v.count();
@@ -1766,7 +1790,7 @@ __global__ void __launch_bounds__(128, GENERAL ? 4 : (CLOTH ? AVBD_LEAN_CLOTH_MI
         d.learnResidBodies[s + slot] = dot(r, r);
         return;
     }
-    particle_commit(P, d, body, shp, pl, inert, acc);
+    particle_commit(P, d, body, shp.w, pl, inert, bound, anchor, acc);
 }
 
 template <bool CLOTH>
@@ -1781,148 +1805,131 @@ static void launch_primal_group(const Params& P, const DevPtrs& d, uint32_t colo
 }
 
 // ---------------------------------------------------------------------------
-// Staged primal.  A block takes 16 bodies of the color (one 8-lane group
-// each, the reference's SIMD layout) and evaluates the terms of all their
-// adjacency entries as one flat list — every thread of the block on
-// consecutive entries, whatever each body's entry count — into shared
-// memory; each group then folds its body's entries in the fixed order
-// (logical lane l: entries l, l + 8, ...; xor butterfly 4, 2, 1) and lane 0
-// solves.  The grouped kernel above idles the lanes past a body's last
-// entry and moves every term through warp shuffles; here the evaluation
-// runs dense and the fold reads shared memory.  Entries past the block's
-// staging capacity are evaluated inline by the fold, in the same order.
+// Staged primal: 16 lean particles per block, 8 lanes each (the reference's
+// SIMD layout).  A color's chain used to be body -> adjacency -> element record
+// -> vertex positions, each a dependent trip to L2, after the previous color
+// had finished.  What no kernel writes (the launch tables built at upload: the
+// springs', membranes' and bends' constants, the tets' by index, the lists of
+// referenced bodies) is now copied to shared memory before the wait for the
+// previous grid, so that its latency is spent in the previous color's tail.
+// After the wait the block gathers each referenced body's position once (a
+// vertex of a soft body has some 24 tets but 15 distinct neighbours: 16 reads
+// in place of 96), and the lanes evaluate and fold their entries l, l + 8, ...
+// straight from shared memory; only contacts, and springs with levers, are read
+// through the adjacency.  Every expression and order is the grouped kernel's.
+// MEASURED_STAGED
 // ---------------------------------------------------------------------------
-constexpr int kStagedThreads = 128;
-constexpr int kStagedGroups = kStagedThreads / 8;
-constexpr int kStagedSlots = 512;       // staged entries per block
-constexpr int kStagedWords = 16;        // kind, rhs, a, b, c, s (e = a + b is recomputed)
+constexpr int kStagedThreads = 8 * (int)STAGED_BODIES;
 
-struct StagedBody {
-    uint32_t body, cnt, staged, off;
-    uint32_t preBase, nPre, dynBase, nMan, nDyn, postBase, nTet, nPost;
-};
-
-__device__ __forceinline__ AdjView staged_view(const DevPtrs& d, const StagedBody& b) {
-    AdjView v;
-    v.pre = d.preList + b.preBase; v.nPre = b.nPre;
-    v.dyn = d.dynList + b.dynBase; v.nDyn = b.nDyn; v.nMan = b.nMan;
-    v.post = d.postList + b.postBase; v.nPost = b.nPost; v.nTet = b.nTet; v.postBase = b.postBase;
-    return v;
+__device__ __forceinline__ void copy16(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
 }
 
 template <bool CLOTH>
 __global__ void __launch_bounds__(kStagedThreads, 5)
-k_primal_staged(const Params P, const DevPtrs d, uint32_t color, uint32_t count, uint32_t first, uint32_t start) {
-    __shared__ float slots[kStagedWords][kStagedSlots];
-    __shared__ StagedBody info[kStagedGroups];
-    __shared__ uint32_t offs[kStagedGroups + 1];
+k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock) {
+    extern __shared__ uint4 words[];
     pdl_trigger();
-    const uint32_t tid = threadIdx.x;
-    const uint32_t head = blockIdx.x * kStagedGroups;
-    const bool early = start != NO_HOST_START;
-    // bodies of the block, their adjacency views and an exclusive scan of
-    // their entry counts (warp 0, one lane per group); with the start known
-    // on the host the static part (launch order, shape, static segment) is
-    // read before waiting for the previous grid
-    if (!early) pdl_wait();
-    const uint32_t s = (early ? start : d.colorStart[color]) + first;
-    uint32_t cnt = 0, body = 0xFFFFFFFFu;
-    StagedBody sb{};
-    const bool mine = tid < kStagedGroups && head + tid < count;
-    if (mine) {
-        body = d.colorLaunch[s + head + tid];
-        const uint4 seg = d.staticSeg[body];
-        sb.preBase = seg.x; sb.nPre = seg.y; sb.postBase = seg.z; sb.nPost = seg.w;
-        sb.nTet = d.postTets[body];
+    const uint32_t tid = threadIdx.x, g = tid >> 3, lane = tid & 7u;
+    const StagedBlock B = d.stagedBlocks[firstBlock + blockIdx.x];
+    // records | tet constants (four words each) | tet references | positions
+    uint4* rec = words;
+    uint4* tets = rec + B.recLen;
+    StagedTet* refs = reinterpret_cast<StagedTet*>(tets + 4 * (size_t)B.tetLen);
+    float4* pos = reinterpret_cast<float4*>(tets + 4 * (size_t)B.tetLen + B.tetLen / 2);
+    for (uint32_t i = tid; i < 4 * B.tetLen; i += kStagedThreads) {
+        const uint32_t e = i >> 2, j = i & 3u;
+        copy16(tets + j * B.tetLen + e, d.tetConst + 4 * (size_t)(d.stagedTets[B.tet + e].index & ADJ_INDEX_MASK) + j);
     }
-    if (early) pdl_wait();                                   // every thread, before any per-frame read
-    if (tid < 32) {
-        if (mine) {
-            sb.dynBase = d.dynStart[body]; sb.nDyn = d.dynCount[body]; sb.nMan = d.dynSplit[body];
-            cnt = sb.nPre + sb.nDyn + sb.nPost;
-            sb.cnt = cnt;
-        }
-        uint32_t incl = cnt;
+    for (uint32_t i = tid; i < B.tetLen / 2; i += kStagedThreads) copy16(refs + 2 * i, d.stagedTets + B.tet + 2 * i);
+    for (uint32_t i = tid; i < B.recLen; i += kStagedThreads) copy16(rec + i, d.stagedRec + B.rec + i);
+    uint32_t id[4];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if ((int)tid >= o) incl += y;
-        }
-        const uint32_t off = incl - cnt;
-        if (tid < kStagedGroups) {
-            sb.body = body;
-            sb.off = off;
-            sb.staged = off >= (uint32_t)kStagedSlots ? 0u : min(cnt, (uint32_t)kStagedSlots - off);
-            info[tid] = sb;
-            offs[tid] = off;
-        }
-        if (tid == kStagedGroups - 1) offs[kStagedGroups] = min(incl, (uint32_t)kStagedSlots);
-    }
-    __syncthreads();
-    // every staged entry of the block, dense over the threads
-    const uint32_t total = offs[kStagedGroups];
-    for (uint32_t i = tid; i < total; i += kStagedThreads) {
-        uint32_t g = 0;
+    for (uint32_t j = 0; j < 4; j++) id[j] = tid + j * kStagedThreads < B.idLen ? d.stagedIds[B.ids + tid + j * kStagedThreads] : 0u;
+    const bool active = g < B.count;
+    const StagedBody b = d.stagedBodies[B.first + (active ? g : 0u)];
+    // the lane's first spring, whose multiplier is read right after the wait
+    const uint32_t spring = CLOTH && lane < b.nPre ? d.stagedRec[B.rec + b.rec + lane].w : 0u;
+    pdl_wait();
 #pragma unroll
-        for (uint32_t step = kStagedGroups / 2; step >= 1; step >>= 1)
-            if (offs[g + step] <= i) g += step;
-        const StagedBody& b = info[g];
-        const AdjView v = staged_view(d, b);
-        ParticleTerms t;
-        uint32_t entry = 0;
-        particle_entry_terms<CLOTH>(P, d, v, b.body, i - b.off, t, entry);
-        slots[0][i] = __uint_as_float(t.kind);
-        slots[1][i] = t.kind == TERM_SERIAL ? __uint_as_float(entry) : t.rhs.x;
-        slots[2][i] = t.rhs.y;  slots[3][i] = t.rhs.z;
-        slots[4][i] = t.a.x;    slots[5][i] = t.a.y;    slots[6][i] = t.a.z;
-        slots[7][i] = t.b.x;    slots[8][i] = t.b.y;    slots[9][i] = t.b.z;
-        slots[10][i] = t.c.x;   slots[11][i] = t.c.y;   slots[12][i] = t.c.z;
-        if (CLOTH) { slots[13][i] = t.s.x; slots[14][i] = t.s.y; slots[15][i] = t.s.z; }
+    for (uint32_t j = 0; j < 4; j++)
+        if (tid + j * kStagedThreads < B.idLen) copy16(pos + tid + j * kStagedThreads, d.posLin + id[j]);
+    for (uint32_t i = tid + 4 * kStagedThreads; i < B.idLen; i += kStagedThreads)
+        copy16(pos + i, d.posLin + d.stagedIds[B.ids + i]);
+    const uint32_t* dyn = d.dynList + d.dynStart[b.body];
+    const uint32_t nDyn = d.dynCount[b.body], nMan = d.dynSplit[b.body];
+    float4 dual = make_float4(0, 0, 0, 0), inert = dual, anchor = dual;
+    float bound = 0.0f;
+    if (CLOTH && lane < b.nPre) dual = tof(d.springs[spring].dual);
+    if (lane == 0) {
+        inert = d.inertLin[b.body];
+        if (P.ogc) { bound = __uint_as_float(d.ogcBounds[b.body]); anchor = d.ogcPrev[b.body]; }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // the fold: group g, logical lane l
-    const uint32_t g = tid >> 3, lane = tid & 7u;
-    if (head + g >= count) return;
-    const StagedBody b = info[g];
-    const unsigned mask8 = 0xFFu << (tid & 24u);
-    const float4 shp = d.shape[b.body];
-    float4 pl = make_float4(0, 0, 0, 0), inert = make_float4(0, 0, 0, 0);
-    if (lane == 0) { pl = d.posLin[b.body]; inert = d.inertLin[b.body]; }
+    if (!active) return;
+    const unsigned mask = 0xFFu << (tid & 24u);
+    rec += b.rec;
+    pos += b.pos;
+    auto at = [&](uint32_t r, uint32_t k) { return xyz(pos[(r >> (8 * k)) & 0xFFu]); };
     ParticleAccum acc{m3_zero(), s3(0)};
-    for (uint32_t k = lane; k < b.cnt; k += 8) {
-        ParticleTerms u;
-        uint32_t e = 0;
-        if (k < b.staged) {
-            const uint32_t i = b.off + k;
-            u.kind = __float_as_uint(slots[0][i]);
-            e = __float_as_uint(slots[1][i]);
-            u.rhs = mk3(slots[1][i], slots[2][i], slots[3][i]);
-            u.a = mk3(slots[4][i], slots[5][i], slots[6][i]);
-            u.b = mk3(slots[7][i], slots[8][i], slots[9][i]);
-            u.c = mk3(slots[10][i], slots[11][i], slots[12][i]);
-            if (CLOTH) {
-                u.s = mk3(slots[13][i], slots[14][i], slots[15][i]);
-                u.e = u.a + u.b;                             // as the membrane terms form it
+    const uint32_t endMan = b.nPre + nMan, endTet = endMan + b.nTet, endSoft = endTet + nDyn - nMan,
+                   cnt = endSoft + b.nRest;
+    for (uint32_t k = lane; k < cnt; k += 8) {
+        ParticleTerms t;
+        if (CLOTH && k < b.nPre) {
+            const uint4 q = rec[k];
+            const uint32_t flags = rec[b.nPre + k].x;
+            if (flags & STAGED_GENERIC) {
+                particle_terms<true>(P, d, (FK_SPRING << ADJ_KIND_SHIFT) | q.w, b.body, t);
+            } else {
+                if (k != lane) dual = tof(d.springs[q.w].dual);
+                spring_core(P, at(q.z, 0), at(q.z, 1), (flags & 1u) == 0u, __uint_as_float(q.x), __uint_as_float(q.y),
+                            (flags & STAGED_HARD) != 0u, dual, t);
+            }
+            fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
+        } else if (k >= endMan && k < endTet) {
+            const uint32_t e = b.tet + (k - endMan);
+            const StagedTet r = refs[e];
+            const uint4 q0 = tets[e], q1 = tets[B.tetLen + e], q2 = tets[2 * B.tetLen + e], q3 = tets[3 * B.tetLen + e];
+            const float3 m0 = mk3(__uint_as_float(q0.x), __uint_as_float(q0.y), __uint_as_float(q0.z));
+            const float3 m1 = mk3(__uint_as_float(q1.x), __uint_as_float(q1.y), __uint_as_float(q1.z));
+            const float3 m2 = mk3(__uint_as_float(q2.x), __uint_as_float(q2.y), __uint_as_float(q2.z));
+            const uint32_t self = r.index >> ADJ_KIND_SHIFT;
+            const float3 w = self == 1u ? m0 : (self == 2u ? m1 : (self == 3u ? m2
+                             : -mk3(m0.x + m1.x + m2.x, m0.y + m1.y + m2.y, m0.z + m1.z + m2.z)));
+            const float diag = __uint_as_float(self == 0u ? q3.x : (self == 1u ? q3.y : (self == 2u ? q3.z : q3.w)));
+            tet_core(at(r.refs, 0), at(r.refs, 1), at(r.refs, 2), at(r.refs, 3), m0, m1, m2, __uint_as_float(q1.w),
+                     __uint_as_float(q2.w), __uint_as_float(q0.w), w, diag, t);
+            fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
+        } else if (CLOTH && k >= endSoft) {
+            const uint32_t e = 2 * b.nPre + (k - endSoft);
+            const uint4 q = rec[e], r = rec[b.nRest + e];
+            const float4 v = make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z),
+                                         __uint_as_float(q.w));
+            if (r.w & STAGED_BEND) {
+                bend_core(at(r.z, 0), at(r.z, 1), at(r.z, 2), at(r.z, 3), v, __uint_as_float(r.x), r.w & 3u, t);
+                fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
+            } else {
+                membrane_core(at(r.z, 0), at(r.z, 1), at(r.z, 2), v, __uint_as_float(r.x), __uint_as_float(r.y),
+                              r.w & 3u, t);
+                fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
             }
         } else {
-            particle_entry_terms<CLOTH>(P, d, staged_view(d, b), b.body, k, u, e);
+            // a contact: manifolds, then element contacts
+            const uint32_t e = dyn[k < endMan ? k - b.nPre : nMan + (k - endTet)];
+            particle_terms<CLOTH>(P, d, e, b.body, t);
+            fold_particle_term<false, CLOTH>(P, d, t, e, b.body, acc);
         }
-        fold_particle_term<false, CLOTH>(P, d, u, e, b.body, acc);
     }
 #pragma unroll
     for (int o = 4; o >= 1; o >>= 1) {
-        add_shfl_lower(mask8, acc.lhs, o);
-        add_shfl3(mask8, acc.rhs, o);
+        add_shfl_lower(mask, acc.lhs, o);
+        add_shfl3(mask, acc.rhs, o);
     }
     if (lane != 0) return;
-    particle_commit(P, d, b.body, shp, pl, inert, acc);
-}
-
-template <bool CLOTH>
-static void launch_primal_staged(const Params& P, const DevPtrs& d, uint32_t color, uint32_t count,
-                                 uint32_t first, uint32_t start, cudaStream_t st) {
-    const uint32_t blocks = (count + kStagedGroups - 1) / kStagedGroups;
-    launch_pdl(k_primal_staged<CLOTH>, blocks, kStagedThreads, st, P, d, color, count, first, start);
+    particle_commit(P, d, b.body, b.radius, pos[0], inert, bound, anchor, acc);
 }
 
 void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t color, uint32_t count,
@@ -1953,16 +1960,19 @@ void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint
             cudaStreamWaitEvent(side, fork, 0);
             launch_primal_wide(P, d, color, rest, lean, start, side);
         }
-        if (lean) {
-            if (lanes == AVBD_PRIMAL_STAGED) {
-                if (cloth) launch_primal_staged<true>(P, d, color, lean, 0, start, st);
-                else launch_primal_staged<false>(P, d, color, lean, 0, start, st);
-            } else {
-                const uint32_t lanes_ = lanes < 8 ? 8 : (lanes > 32 ? 32 : lanes);
-                const uint32_t w = lanes_ <= 8 ? 8 : (lanes_ <= 16 ? 16 : 32);
-                if (cloth) launch_primal_group<true>(P, d, color, lean, 0, start, w, st);
-                else launch_primal_group<false>(P, d, color, lean, 0, start, w, st);
-            }
+        uint32_t staged = 0;
+        if (lanes == AVBD_PRIMAL_STAGED && z.colorStaged) {
+            staged = min(z.colorStaged[color], lean);
+            const uint32_t b0 = z.stagedStart[color], blocks = z.stagedStart[color + 1] - b0;
+            const size_t smem = 16 * (size_t)z.stagedWords[color];
+            if (staged && cloth) launch_pdl_smem(k_primal_staged<true>, blocks, kStagedThreads, smem, st, P, d, b0);
+            else if (staged) launch_pdl_smem(k_primal_staged<false>, blocks, kStagedThreads, smem, st, P, d, b0);
+        }
+        if (lean > staged) {
+            // pinned widths, and particles with more elements than a staged block holds
+            const uint32_t w = lanes <= 8 ? 8 : (lanes <= 16 ? 16 : 32);
+            if (cloth) launch_primal_group<true>(P, d, color, lean - staged, staged, start, w, st);
+            else launch_primal_group<false>(P, d, color, lean - staged, staged, start, w, st);
         }
         // the rest: a block per body (rigid bodies with many contacts)
         if (split) {

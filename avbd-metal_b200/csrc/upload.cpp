@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <array>
 #include <cmath>
+#include <cstring>
 #include <map>
 #include <set>
 #include <unordered_set>
@@ -357,6 +358,157 @@ void upload_cloth(const avbd_scene_desc* s, const std::vector<std::array<int, 3>
     const uint64_t iso = std::max<uint64_t>(1, 4ull * surf + 4ull * H.numTris + 4ull * H.numSurfaceEdges);
     H.maxSoftIso = (uint32_t)std::min<uint64_t>(iso, 0x7FFFFFFFull);
     H.softMapCapacityIso = next_pow2(std::max<uint32_t>(64u, 2u * H.maxSoftIso));
+}
+
+}  // namespace
+
+namespace {
+
+uint32_t float_bits(float x) {
+    uint32_t u;
+    std::memcpy(&u, &x, 4);
+    return u;
+}
+
+// 16-byte words of shared memory: records, tets (their constants and
+// references; an even number) and positions.
+size_t staged_words(size_t rec, size_t tets, size_t ids) { return rec + 9 * ((tets + 1) / 2) + ids; }
+
+// A tet's constants by the kernels' own expressions, so that a product formed
+// here has the bits it would have there.
+TetConst tet_const(const TetGPU& t) {
+    const float mu = t.r1.w, lam = t.r2.w;
+    TetConst o{t.r0, t.r1, t.r2, f4{}};
+    o.r0.w = 1.0f + mu / (lam > 1e-9f ? lam : 1e-9f);
+    const float w[3] = {-(t.r0.x + t.r1.x + t.r2.x), -(t.r0.y + t.r1.y + t.r2.y), -(t.r0.z + t.r1.z + t.r2.z)};
+    o.diag.x = mu * (w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+    o.diag.y = mu * (t.r0.x * t.r0.x + t.r0.y * t.r0.y + t.r0.z * t.r0.z);
+    o.diag.z = mu * (t.r1.x * t.r1.x + t.r1.y * t.r1.y + t.r1.z * t.r1.z);
+    o.diag.w = mu * (t.r2.x * t.r2.x + t.r2.y * t.r2.y + t.r2.z * t.r2.z);
+    return o;
+}
+
+// One body's part of the staged tables; false when its elements refer to too
+// many bodies or hold too many words for a block.
+bool stage_body(const HostScene& H, uint32_t b, StagedBody& o, std::vector<u4>& rec, std::vector<StagedTet>& tets,
+                std::vector<uint32_t>& ids, std::vector<u4>& seen) {
+    const u4 sg = H.staticSeg[b];
+    o = StagedBody{};
+    o.body = b;
+    o.radius = H.shape[b].w;
+    o.nPre = sg.y;
+    o.nTet = H.postTets[b];
+    o.nRest = sg.w - o.nTet;
+    rec.assign(2 * (size_t)o.nPre + 2 * (size_t)o.nRest, u4{0, 0, 0, 0});
+    tets.assign(o.nTet, StagedTet{0, 0});
+    ids.assign(1, b);
+    bool fits = (size_t)o.nPre + o.nTet + o.nRest < STAGED_MAX_WORDS;
+    seen[b] = u4{b, 0, 0, 0};                        // (body that referred last, its index for it)
+    auto local = [&](uint32_t v) {
+        if (seen[v].x == b) return seen[v].y;
+        seen[v] = u4{b, (uint32_t)ids.size(), 0, 0};
+        ids.push_back(v);
+        if (ids.size() > STAGED_MAX_REFS) fits = false;
+        return (uint32_t)ids.size() - 1u;
+    };
+    for (uint32_t k = 0; k < o.nPre && fits; k++) {
+        const uint32_t si = H.preList[sg.x + k] & ADJ_INDEX_MASK;
+        const SpringGPU& sp = H.springs[si];
+        const bool plain = H.shape[sp.header.x].w < 0.0f && H.shape[sp.header.y].w < 0.0f && sp.rA.x == 0.0f &&
+                           sp.rA.y == 0.0f && sp.rA.z == 0.0f && sp.rB.x == 0.0f && sp.rB.y == 0.0f && sp.rB.z == 0.0f;
+        const uint32_t flags = (b == sp.header.x ? 0u : 1u) | (sp.header.z != 0 ? STAGED_HARD : 0u) |
+                               (plain ? 0u : STAGED_GENERIC);
+        const uint32_t refs = plain ? local(sp.header.x) | (local(sp.header.y) << 8) : 0u;
+        rec[k] = u4{float_bits(sp.rA.w), float_bits(sp.rB.w), refs, si};
+        rec[o.nPre + k] = u4{flags, 0, 0, 0};
+    }
+    for (uint32_t k = 0; k < o.nTet && fits; k++) {
+        const uint32_t ti = H.postList[sg.z + k] & ADJ_INDEX_MASK;
+        const u4 v = H.tets[ti].ids;
+        const uint32_t self = b == v.y ? 1u : (b == v.z ? 2u : (b == v.w ? 3u : 0u));
+        tets[k] = StagedTet{ti | (self << ADJ_KIND_SHIFT),
+                            local(v.x) | (local(v.y) << 8) | (local(v.z) << 16) | (local(v.w) << 24)};
+    }
+    u4* rest = rec.data() + 2 * o.nPre;
+    for (uint32_t k = 0; k < o.nRest && fits; k++) {
+        const uint32_t e = H.postList[sg.z + o.nTet + k], idx = e & ADJ_INDEX_MASK;
+        if ((e >> ADJ_KIND_SHIFT) == FK_MEMBRANE) {
+            const MembraneGPU& m = H.membranes[idx];
+            const uint32_t self = b == m.ids.y ? 1u : (b == m.ids.z ? 2u : 0u);
+            const uint32_t refs = local(m.ids.x) | (local(m.ids.y) << 8) | (local(m.ids.z) << 16);
+            rest[k] = u4{float_bits(m.dm.x), float_bits(m.dm.y), float_bits(m.dm.z), float_bits(m.dm.w)};
+            rest[o.nRest + k] = u4{float_bits(m.mat.x), float_bits(m.mat.y), refs, self};
+        } else {
+            const BendGPU& m = H.bends[idx];
+            const uint32_t self = b == m.ids.x ? 0u : (b == m.ids.y ? 1u : (b == m.ids.z ? 2u : 3u));
+            const uint32_t refs = local(m.ids.x) | (local(m.ids.y) << 8) | (local(m.ids.z) << 16) | (local(m.ids.w) << 24);
+            rest[k] = u4{float_bits(m.K.x), float_bits(m.K.y), float_bits(m.K.z), float_bits(m.K.w)};
+            rest[o.nRest + k] = u4{float_bits(m.mat.x), 0, refs, self | STAGED_BEND};
+        }
+    }
+    return fits && staged_words(rec.size(), o.nTet, ids.size()) <= STAGED_MAX_WORDS;
+}
+
+// Blocks of the staged primal over each color's lean particles; those that
+// fit no block move to the end of the color's lean run.
+void build_staged(HostScene& H) {
+    H.colorStaged.assign(MAX_COLORS, 0);
+    H.stagedStart.assign(MAX_COLORS + 1, 0);
+    H.stagedWords.assign(MAX_COLORS, 0);
+    if (H.dynamicColoring) return;
+    H.tetConst.reserve(H.tets.size());
+    for (const TetGPU& t : H.tets) H.tetConst.push_back(tet_const(t));
+    StagedBody o;
+    std::vector<u4> rec;
+    std::vector<StagedTet> tets;
+    std::vector<uint32_t> ids, large;
+    std::vector<u4> seen(H.numBodies, u4{0xFFFFFFFFu, 0, 0, 0});
+    for (int c = 0; c < MAX_COLORS; c++) {
+        H.stagedStart[c] = (uint32_t)H.stagedBlocks.size();
+        const uint32_t s0 = H.colorStart[c], lean = H.particleFastPath ? H.colorStart[c + 1] - s0 : H.colorLean[c];
+        large.clear();
+        uint32_t kept = 0;
+        StagedBlock blk{};
+        auto close = [&]() {
+            if (blk.count == 0) return;
+            if (blk.tetLen & 1u) {
+                H.stagedTets.push_back(StagedTet{0, 0});
+                blk.tetLen++;
+            }
+            H.stagedWords[c] = std::max(H.stagedWords[c], (uint32_t)staged_words(blk.recLen, blk.tetLen, blk.idLen));
+            H.stagedBlocks.push_back(blk);
+            blk = StagedBlock{};
+        };
+        for (uint32_t i = 0; i < lean; i++) {
+            const uint32_t b = H.colorLaunch[s0 + i];
+            if (!stage_body(H, b, o, rec, tets, ids, seen)) { large.push_back(b); continue; }
+            if (blk.count == STAGED_BODIES ||
+                staged_words(blk.recLen + rec.size(), blk.tetLen + tets.size(), blk.idLen + ids.size()) > STAGED_MAX_WORDS)
+                close();
+            if (blk.count == 0) {
+                blk.first = (uint32_t)H.stagedBodies.size();
+                blk.rec = (uint32_t)H.stagedRec.size();
+                blk.tet = (uint32_t)H.stagedTets.size();
+                blk.ids = (uint32_t)H.stagedIds.size();
+            }
+            o.rec = blk.recLen;
+            o.tet = blk.tetLen;
+            o.pos = blk.idLen;
+            blk.count++;
+            blk.recLen += (uint32_t)rec.size();
+            blk.tetLen += (uint32_t)tets.size();
+            blk.idLen += (uint32_t)ids.size();
+            H.stagedBodies.push_back(o);
+            H.stagedRec.insert(H.stagedRec.end(), rec.begin(), rec.end());
+            H.stagedTets.insert(H.stagedTets.end(), tets.begin(), tets.end());
+            H.stagedIds.insert(H.stagedIds.end(), ids.begin(), ids.end());
+            H.colorLaunch[s0 + kept++] = b;
+        }
+        close();
+        H.colorStaged[c] = kept;
+        std::copy(large.begin(), large.end(), H.colorLaunch.begin() + s0 + kept);
+    }
+    H.stagedStart[MAX_COLORS] = (uint32_t)H.stagedBlocks.size();
 }
 
 }  // namespace
@@ -870,6 +1022,7 @@ int upload_scene(const avbd_scene_desc* s, HostScene& H, std::string& err) {
         P.maxSoft = H.maxSoftIso;
         P.softMapCapacity = H.softMapCapacityIso;
     }
+    build_staged(H);
     return AVBD_OK;
 }
 

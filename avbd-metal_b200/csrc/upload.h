@@ -55,6 +55,16 @@ struct HostScene {
     // particles with joints).  colorLean[c] counts the lean ones.
     std::vector<uint32_t> colorLaunch, colorLean;
 
+    // Staged primal: the first colorStaged[c] bodies of a color's launch
+    // order, in blocks stagedStart[c] .. stagedStart[c + 1]; stagedWords[c] is
+    // the most 16-byte words of shared memory a block takes.
+    std::vector<StagedBody> stagedBodies;
+    std::vector<StagedBlock> stagedBlocks;
+    std::vector<u4> stagedRec;
+    std::vector<StagedTet> stagedTets;
+    std::vector<TetConst> tetConst;
+    std::vector<uint32_t> stagedIds, colorStaged, stagedStart, stagedWords;
+
     // Static per-body adjacency, split around the per-frame contact entries:
     // pre = joints + springs (kinds 0, 1), post = tets (kind 3), each sorted.
     // The solver walks pre, then this frame's manifolds (kind 2), then post,
