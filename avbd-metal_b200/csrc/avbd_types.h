@@ -100,6 +100,7 @@ struct alignas(16) StagedBody {
     float radius;                 // shape.w
     uint32_t rec, tet, pos;       // first record word, tet and position, within the block
     uint32_t nPre, nTet, nRest;   // springs, tets, membranes and bends
+    uint32_t nMem, pad[3];        // the membranes, which come first
 };
 struct alignas(16) StagedBlock {
     uint32_t first, count;        // bodies
@@ -115,11 +116,9 @@ struct alignas(16) TetConst { f4 r0, r1, r2, diag; };   // DmInv rows; w: alpha,
 constexpr uint32_t STAGED_BODIES = 16;             // most bodies of a block (8 lanes each)
 constexpr uint32_t STAGED_MAX_WORDS = 2600;        // most 16-byte words of shared memory of a block
 constexpr uint32_t STAGED_MAX_REFS = 255;          // most bodies one body's records refer to
-// last word of a spring, membrane or bend record: this body's position in the
-// element (bits 0-1), then flags
-constexpr uint32_t STAGED_BEND = 4u;               // a bend, else a membrane
-constexpr uint32_t STAGED_HARD = 4u;               // spring: hard
-constexpr uint32_t STAGED_GENERIC = 8u;            // spring with levers or a rigid end: evaluated from its own record
+// flags of a spring's record, beside this body's position in it (bit 0)
+constexpr uint32_t STAGED_HARD = 4u;
+constexpr uint32_t STAGED_GENERIC = 8u;            // levers or a rigid end: evaluated from its own record
 
 // Per-frame parameters (SimParams, 00_common.metal:233-288), passed by value.
 struct Params {

@@ -189,14 +189,17 @@ void launch_dynamic_coloring(const Params& P, const DevPtrs& d, const Sizes& z, 
 // `lanes` is 8, 16 or 32 lanes per body (grouped kernel) or
 // AVBD_PRIMAL_STAGED (staged kernel: a block's records and positions in shared
 // memory, 8 lanes per body), every choice computing the same floats
+// `chained`: a grid of this stream's chain has started after the frame's
+// contact lists were complete (false at the head of a chain: the frame's
+// solve, or a trial sweep); `last`: the last color of a sweep.
 // With a side stream and two events, the color's non-lean bodies (a block
 // each) run on the side stream beside the lean particles (a fork and a join
 // on `st`; in a captured frame, two parallel graph branches).
 constexpr uint32_t NO_HOST_START = 0xFFFFFFFFu;   // a color start the kernel reads on the device
 constexpr uint32_t AVBD_PRIMAL_STAGED = 1;
 void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t color,
-                         uint32_t count, uint32_t lanes, bool last, cudaStream_t st, cudaStream_t side = nullptr,
-                         cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
+                         uint32_t count, uint32_t lanes, bool& chained, bool last, cudaStream_t st,
+                         cudaStream_t side = nullptr, cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
 // squared AL-gradient norm of every dynamic body (perBody[numDynamicBodies])
 // and their fixed-order sum (total)
 void launch_residual(const Params& P, const DevPtrs& d, const Sizes& z, float* perBody, double* total,

@@ -18,9 +18,10 @@ __device__ __forceinline__ void pdl_prologue() {
 }
 
 
+// `overlap`: the grid may start while the one before it still runs
 template <typename... KArgs, typename... Args>
-static void launch_pdl_smem(void (*kernel)(KArgs...), uint32_t blocks, uint32_t threads, size_t smem, cudaStream_t st,
-                            Args&&... args) {
+static void launch_chain(void (*kernel)(KArgs...), bool overlap, uint32_t blocks, uint32_t threads, size_t smem,
+                         cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(threads);
@@ -28,10 +29,16 @@ static void launch_pdl_smem(void (*kernel)(KArgs...), uint32_t blocks, uint32_t 
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+static void launch_pdl_smem(void (*kernel)(KArgs...), uint32_t blocks, uint32_t threads, size_t smem, cudaStream_t st,
+                            Args&&... args) {
+    launch_chain(kernel, true, blocks, threads, smem, st, std::forward<Args>(args)...);
 }
 
 template <typename... KArgs, typename... Args>

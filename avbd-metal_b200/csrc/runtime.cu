@@ -12,6 +12,7 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -165,6 +166,9 @@ struct avbd_solver {
     void* stage = nullptr;
     size_t stageBytes = 0;
     uint32_t* hostLatch = nullptr;     // pinned copy of the failure latch
+    uint8_t* hostRead = nullptr;       // pinned staging of small readbacks (grows to kReadStage)
+    size_t hostReadBytes = 0;
+    std::vector<uint8_t> motorMode;    // MOTOR_MODE_MASK bits of every joint, packed for the setters' checks
     // render surface (built on the first smooth-normals call): surface
     // vertices, their incident triangles, face normals
     bool renderSurfaceReady = false;
@@ -194,6 +198,7 @@ struct avbd_solver {
         if (pushtDev) cudaFree(pushtDev);
         if (pushtShapes) cudaFree(pushtShapes);
         if (hostLatch) cudaFreeHost(hostLatch);
+        if (hostRead) cudaFreeHost(hostRead);
         if (forkEvent) cudaEventDestroy(forkEvent);
         if (joinEvent) cudaEventDestroy(joinEvent);
         if (wideFork) cudaEventDestroy(wideFork);
@@ -277,6 +282,7 @@ struct avbd_solver {
         f.tailTicket = tickets;
         usedEvents = 0;
         uint32_t primalLaunch = 0;
+        bool chained = false;
         auto mark = [&](int stage) {
             if (!profiling || primalEvents) return;
             cudaEventRecordWithFlags(events[usedEvents], st, cudaEventRecordExternal);
@@ -313,10 +319,11 @@ struct avbd_solver {
         // One primal sweep over every color of pose buffers `g` (trial sweeps of
         // the learned warm start; the iteration loop inlines the same sequence).
         auto sweep = [&](const DevPtrs& g, cudaStream_t sst) {
+            bool chained = false;
             for (uint32_t c = 0; c < colorBound; c++) {
                 const uint32_t count = z.dynamicColoring ? 0xFFFFFFFFu : H.colorCounts[c];
                 if (count == 0) continue;
-                launch_primal_color(P, g, z, c, count, H.colorLanes[c], c + 1 == colorBound, sst);
+                launch_primal_color(P, g, z, c, count, H.colorLanes[c], chained, c + 1 == colorBound, sst);
                 if (P.ogc)
                     launch_publish_color(P, g, c, count, z.dynamicColoring ? NO_HOST_START : H.colorStart[c], sst);
             }
@@ -397,8 +404,8 @@ struct avbd_solver {
                     if (count == 0) continue;
                     mark(AVBD_STAGE_PRIMAL);
                     if (primalEvents) cudaEventRecord(primalEvents[2 * primalLaunch], st);
-                    launch_primal_color(P, g, z, c, count, lanes ? lanes[c] : H.colorLanes[c], c + 1 == colorBound, st,
-                                        branchStream, wideFork, wideJoin);
+                    launch_primal_color(P, g, z, c, count, lanes ? lanes[c] : H.colorLanes[c], chained,
+                                        c + 1 == colorBound, st, branchStream, wideFork, wideJoin);
                     if (primalEvents) cudaEventRecord(primalEvents[2 * primalLaunch + 1], st);
                     primalLaunch++;
                     if (P.cloth) {
@@ -490,6 +497,8 @@ struct avbd_solver {
         P = H.P;
         sync_params();
         const uint32_t nb = H.numBodies, nc = H.numColliders;
+        motorMode.reserve(H.joints.size());
+        for (const JointGPU& j : H.joints) motorMode.push_back((uint8_t)(j.header.w & MOTOR_MODE_MASK));
         z.numBodies = nb;
         z.numColliders = nc;
         z.numActiveJoints = (uint32_t)H.activeJoints.size();
@@ -779,12 +788,54 @@ struct avbd_solver {
         return AVBD_OK;
     }
 
+    // Readbacks up to this size go through pinned memory behind the frame and
+    // share its one wait; a stack of 20 boxes spent 37 us of a 231 us pass in
+    // the four waits of separate copies.  Larger ones are copied straight into
+    // the caller's memory, which costs no second pass over it.
+    static constexpr size_t kReadStage = 1u << 20;
+    struct Readback { void* dst; const void* src; size_t bytes; };
+
     // Wait for the stream, then surface an execution error or a latched
-    // capacity/coloring failure.
-    int retire() {
-        if (!check(cudaStreamSynchronize(launch), "frame execution")) return AVBD_ERR_RUNTIME_FAILURE;
-        if (!check(cudaMemcpy(hostLatch, d.failureLatch, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost), "latch readback"))
+    // capacity/coloring failure; `reads` (host destination, device source)
+    // are complete on AVBD_OK.
+    int retire(std::initializer_list<Readback> reads = {}) {
+        size_t small = 0;
+        for (const Readback& r : reads) if (r.dst && r.bytes <= kReadStage) small += (r.bytes + 255) & ~(size_t)255;
+        if (small > hostReadBytes) {
+            if (hostRead) cudaFreeHost(hostRead);
+            hostRead = nullptr;
+            hostReadBytes = 0;
+            if (cudaMallocHost(&hostRead, small) == cudaSuccess) hostReadBytes = small;
+            else { hostRead = nullptr; cudaGetLastError(); }
+        }
+        const bool staged = small > 0 && hostRead;
+        size_t at = 0;
+        if (staged)
+            for (const Readback& r : reads)
+                if (r.dst && r.bytes <= kReadStage) {
+                    cudaMemcpyAsync(hostRead + at, r.src, r.bytes, cudaMemcpyDeviceToHost, launch);
+                    at += (r.bytes + 255) & ~(size_t)255;
+                }
+        cudaMemcpyAsync(hostLatch, d.failureLatch, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, launch);
+        if (!check(cudaStreamSynchronize(launch), "frame execution") || !check(cudaGetLastError(), "readback"))
             return AVBD_ERR_RUNTIME_FAILURE;
+        const int rc = latch();
+        if (rc != AVBD_OK) return rc;
+        at = 0;
+        for (const Readback& r : reads) {
+            if (!r.dst) continue;
+            if (staged && r.bytes <= kReadStage) {
+                std::memcpy(r.dst, hostRead + at, r.bytes);
+                at += (r.bytes + 255) & ~(size_t)255;
+            } else if (!check(cudaMemcpy(r.dst, r.src, r.bytes, cudaMemcpyDeviceToHost), "readback")) {
+                return AVBD_ERR_RUNTIME_FAILURE;
+            }
+        }
+        return AVBD_OK;
+    }
+
+    // What the copied latch says: the color bound it asks for, the first failure.
+    int latch() {
         if (z.dynamicColoring && hostLatch[3] > 0) {
             // first retirement: fit the bound to the palette seen so far;
             // later frames only grow it (a frame that needs more colors
@@ -1183,11 +1234,7 @@ int avbd_sync(avbd_solver* s) {
 
 int avbd_get_positions(avbd_solver* s, uint32_t n, float* pos, float* rot) {
     if (!s || n > s->z.numBodies) return AVBD_ERR_INVALID_ARGUMENT;
-    int rc = s->retire();
-    if (rc != AVBD_OK) return rc;
-    if (pos && !s->check(cudaMemcpy(pos, s->d.posLin, (size_t)n * 16, cudaMemcpyDeviceToHost), "position readback")) return AVBD_ERR_RUNTIME_FAILURE;
-    if (rot && !s->check(cudaMemcpy(rot, s->d.posAng, (size_t)n * 16, cudaMemcpyDeviceToHost), "rotation readback")) return AVBD_ERR_RUNTIME_FAILURE;
-    return AVBD_OK;
+    return s->retire({{pos, s->d.posLin, (size_t)n * 16}, {rot, s->d.posAng, (size_t)n * 16}});
 }
 
 int avbd_get_body_states(avbd_solver* s, const uint32_t* ids, uint32_t n, avbd_body_state* out) {
@@ -1195,14 +1242,11 @@ int avbd_get_body_states(avbd_solver* s, const uint32_t* ids, uint32_t n, avbd_b
     const uint32_t nb = s->z.numBodies;
     if (!ids && n > nb) return AVBD_ERR_INVALID_ARGUMENT;
     for (uint32_t i = 0; ids && i < n; i++) if (ids[i] >= nb) return AVBD_ERR_INVALID_ARGUMENT;
-    int rc = s->retire();
-    if (rc != AVBD_OK) return rc;
     std::vector<float4> pl(nb), pa(nb), vl(nb), va(nb);
-    if (!s->check(cudaMemcpy(pl.data(), s->d.posLin, nb * 16, cudaMemcpyDeviceToHost), "state readback") ||
-        !s->check(cudaMemcpy(pa.data(), s->d.posAng, nb * 16, cudaMemcpyDeviceToHost), "state readback") ||
-        !s->check(cudaMemcpy(vl.data(), s->d.velLin, nb * 16, cudaMemcpyDeviceToHost), "state readback") ||
-        !s->check(cudaMemcpy(va.data(), s->d.velAng, nb * 16, cudaMemcpyDeviceToHost), "state readback"))
-        return AVBD_ERR_RUNTIME_FAILURE;
+    const size_t bytes = (size_t)nb * 16;
+    const int rc = s->retire({{pl.data(), s->d.posLin, bytes}, {pa.data(), s->d.posAng, bytes},
+                              {vl.data(), s->d.velLin, bytes}, {va.data(), s->d.velAng, bytes}});
+    if (rc != AVBD_OK) return rc;
     for (uint32_t i = 0; i < n; i++) {
         const uint32_t b = ids ? ids[i] : i;
         avbd_body_state& o = out[i];
@@ -1248,8 +1292,7 @@ int avbd_set_motor_targets(avbd_solver* s, const uint32_t* joints, uint32_t n, c
     if (!s || (n && (!joints || !targets))) return AVBD_ERR_INVALID_ARGUMENT;
     for (uint32_t i = 0; i < n; i++) {
         if (joints[i] >= s->H.joints.size() || !std::isfinite(targets[i])) return AVBD_ERR_INVALID_ARGUMENT;
-        uint32_t mode = s->H.joints[joints[i]].header.w & MOTOR_MODE_MASK;
-        if (mode == MOTOR_VELOCITY) return AVBD_ERR_INVALID_ARGUMENT;  // requires a position-PD motor
+        if (s->motorMode[joints[i]] == MOTOR_VELOCITY) return AVBD_ERR_INVALID_ARGUMENT;  // requires a position-PD motor
     }
     if (n == 0) return AVBD_OK;
     if (s->failure != AVBD_FAIL_NONE) return AVBD_ERR_RUNTIME_FAILURE;
@@ -1319,8 +1362,7 @@ int avbd_get_motor_states(avbd_solver* s, const uint32_t* joints, uint32_t n, fl
     for (uint32_t i = 0; i < n; i++)
         if (joints[i] >= s->H.joints.size()) return AVBD_ERR_INVALID_ARGUMENT;
     if (n == 0) return AVBD_OK;
-    int rc = s->retire();
-    if (rc != AVBD_OK) return rc;
+    if (s->failure != AVBD_FAIL_NONE) return AVBD_ERR_RUNTIME_FAILURE;
     const size_t idBytes = ((4 * (size_t)n) + 15) & ~(size_t)15;
     uint8_t* st = static_cast<uint8_t*>(s->staging(idBytes + 8 * (size_t)n + 16));
     if (!st) return AVBD_ERR_ALLOC_FAILED;
@@ -1329,10 +1371,9 @@ int avbd_get_motor_states(avbd_solver* s, const uint32_t* joints, uint32_t n, fl
     k_motor_states<<<(n + 127) / 128, 128, 0, s->launch>>>(s->d.joints, s->d.posAng, s->d.velAng,
                                                            reinterpret_cast<uint32_t*>(st), n, dOut);
     std::vector<float> out(2 * (size_t)n);
-    if (!s->check(cudaGetLastError(), "motor states") ||
-        !s->check(cudaMemcpyAsync(out.data(), dOut, 8 * (size_t)n, cudaMemcpyDeviceToHost, s->launch), "motor states readback") ||
-        !s->check(cudaStreamSynchronize(s->launch), "motor states"))
-        return AVBD_ERR_RUNTIME_FAILURE;
+    if (!s->check(cudaGetLastError(), "motor states")) return AVBD_ERR_RUNTIME_FAILURE;
+    const int rc = s->retire({{out.data(), dOut, 8 * (size_t)n}});
+    if (rc != AVBD_OK) return rc;
     for (uint32_t i = 0; i < n; i++) { angles[i] = out[2 * i]; velocities[i] = out[2 * i + 1]; }
     return AVBD_OK;
 }

@@ -1380,6 +1380,34 @@ __device__ __forceinline__ void tet_terms(const DevPtrs& d, const TetGPU& tt, ui
              m1, m2, muV, lamV, 1.0f + muV / mx(lamV, 1e-9f), w, muV * dot(w, w), t);
 }
 
+// Terms of a one-point manifold from its record and its bodies' poses.
+__device__ __forceinline__ void manifold_core(const Params& P, bool isA, uint32_t flags, float4 basisN, float4 basisT1,
+                                              const ContactGPU& c, float4 pa, float4 qa, float4 ia, float4 ja, float4 pb,
+                                              float4 qb, float4 ib, float4 jb, ParticleTerms& t) {
+    const bool sphA = (flags & 2u) != 0, sphB = (flags & 4u) != 0;
+    const float3 dqALin = xyz(pa) - xyz(ia);
+    const float3 dqAAng = q_sub(qa, ja);
+    const float3 dqBLin = xyz(pb) - xyz(ib);
+    const float3 dqBAng = q_sub(qb, jb);
+    const float3 nrm = xyz(basisN), t1 = xyz(basisT1), t2 = cross(nrm, t1);
+    const float3 rAW = sphA ? xyz(c.rA) : q_rotate(qa, xyz(c.rA));
+    const float3 rBW = sphB ? xyz(c.rB) : q_rotate(qb, xyz(c.rB));
+    float3 C;
+    float fs, bnd;
+    const float3 F = contact_force(c, nrm, t1, t2, basisN.w, basisT1.w, P.alpha, dqALin, dqAAng, dqBLin, dqBAng, rAW,
+                                   rBW, C, fs, bnd);
+    const float sg = isA ? 1.0f : -1.0f;
+    const M3 jLin = M3{nrm * sg, t1 * sg, t2 * sg};
+    const M3 K = m3_diag(xyz(c.penalty));
+    const M3 jLinT = m3_transpose(jLin);
+    const M3 M = m3_mulm(m3_mulm(jLinT, K), jLin);
+    t.a = M.r0;
+    t.b = M.r1;
+    t.c = M.r2;
+    t.rhs = m3_mul(jLinT, F);
+    t.kind = TERM_MANIFOLD;
+}
+
 // Spring, membrane and bend terms from the ends' positions, shared by the
 // grouped and the staged kernels.
 __device__ __forceinline__ void spring_core(const Params& P, float3 pA, float3 pB, bool isA, float stiffness, float rest,
@@ -1453,31 +1481,8 @@ __device__ __forceinline__ void particle_terms(const Params& P, const DevPtrs& d
         const u4 h = m.header;
         if (h.z != 1u) return;
         const uint32_t a = h.x, b = h.y;
-        const bool isA = self == a;
-        const bool sphA = (h.w & 2u) != 0, sphB = (h.w & 4u) != 0;
-        const float4 qa = d.posAng[a], qb = d.posAng[b];
-        const float3 dqALin = xyz(d.posLin[a]) - xyz(d.initLin[a]);
-        const float3 dqAAng = q_sub(qa, d.initAng[a]);
-        const float3 dqBLin = xyz(d.posLin[b]) - xyz(d.initLin[b]);
-        const float3 dqBAng = q_sub(qb, d.initAng[b]);
-        const float3 nrm = xyz(m.basisN), t1 = xyz(m.basisT1), t2 = cross(nrm, t1);
-        const ContactGPU c = m.contacts[0];
-        const float3 rAW = sphA ? xyz(c.rA) : q_rotate(qa, xyz(c.rA));
-        const float3 rBW = sphB ? xyz(c.rB) : q_rotate(qb, xyz(c.rB));
-        float3 C;
-        float fs, bnd;
-        const float3 F = contact_force(c, nrm, t1, t2, m.basisN.w, m.basisT1.w, P.alpha, dqALin, dqAAng, dqBLin,
-                                       dqBAng, rAW, rBW, C, fs, bnd);
-        const float sg = isA ? 1.0f : -1.0f;
-        const M3 jLin = M3{nrm * sg, t1 * sg, t2 * sg};
-        const M3 K = m3_diag(xyz(c.penalty));
-        const M3 jLinT = m3_transpose(jLin);
-        const M3 M = m3_mulm(m3_mulm(jLinT, K), jLin);
-        t.a = M.r0;
-        t.b = M.r1;
-        t.c = M.r2;
-        t.rhs = m3_mul(jLinT, F);
-        t.kind = 2;
+        manifold_core(P, self == a, h.w, tof(m.basisN), tof(m.basisT1), m.contacts[0], d.posLin[a], d.posAng[a],
+                      d.initLin[a], d.initAng[a], d.posLin[b], d.posAng[b], d.initLin[b], d.initAng[b], t);
     } else if (!CLOTH) {
         return;
     } else if (kind == FK_SPRING) {
@@ -1820,120 +1825,237 @@ static void launch_primal_group(const Params& P, const DevPtrs& d, uint32_t colo
 // MEASURED_STAGED
 // ---------------------------------------------------------------------------
 constexpr int kStagedThreads = 8 * (int)STAGED_BODIES;
+constexpr uint32_t kStagedContacts = 24;        // one-point manifolds of a block held in shared memory
+constexpr uint32_t kStagedContactWords = 16;    // header, basis, contact, the two bodies' start poses and poses
 
 __device__ __forceinline__ void copy16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
                  : "memory");
 }
 
-template <bool CLOTH>
+// AHEAD: the block's first manifolds are copied to shared memory as well, their
+// constant parts before the wait, the bodies' poses and the multipliers with
+// the positions: a contact adds its arithmetic to the color instead of four
+// dependent trips (2.3 us of the 4.3 us a small color took).
+template <bool CLOTH, bool AHEAD>
 __global__ void __launch_bounds__(kStagedThreads, 5)
-k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock) {
+k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock, bool early) {
     extern __shared__ uint4 words[];
+    __shared__ uint4 con[AHEAD ? kStagedContacts * kStagedContactWords : 1];
+    __shared__ uint32_t contacts;
     pdl_trigger();
     const uint32_t tid = threadIdx.x, g = tid >> 3, lane = tid & 7u;
+    if (AHEAD) {
+        if (tid == 0) contacts = 0u;
+        __syncthreads();
+    }
     const StagedBlock B = d.stagedBlocks[firstBlock + blockIdx.x];
     // records | tet constants (four words each) | tet references | positions
     uint4* rec = words;
     uint4* tets = rec + B.recLen;
     StagedTet* refs = reinterpret_cast<StagedTet*>(tets + 4 * (size_t)B.tetLen);
     float4* pos = reinterpret_cast<float4*>(tets + 4 * (size_t)B.tetLen + B.tetLen / 2);
-    for (uint32_t i = tid; i < 4 * B.tetLen; i += kStagedThreads) {
-        const uint32_t e = i >> 2, j = i & 3u;
-        copy16(tets + j * B.tetLen + e, d.tetConst + 4 * (size_t)(d.stagedTets[B.tet + e].index & ADJ_INDEX_MASK) + j);
-    }
-    for (uint32_t i = tid; i < B.tetLen / 2; i += kStagedThreads) copy16(refs + 2 * i, d.stagedTets + B.tet + 2 * i);
-    for (uint32_t i = tid; i < B.recLen; i += kStagedThreads) copy16(rec + i, d.stagedRec + B.rec + i);
-    uint32_t id[4];
+    // every index first: the copies between them would each wait for theirs
+    uint32_t ti[4], id[4];
 #pragma unroll
-    for (uint32_t j = 0; j < 4; j++) id[j] = tid + j * kStagedThreads < B.idLen ? d.stagedIds[B.ids + tid + j * kStagedThreads] : 0u;
+    for (uint32_t j = 0; j < 4; j++) {
+        const uint32_t e = tid + j * kStagedThreads;
+        ti[j] = e < B.tetLen ? d.stagedTets[B.tet + e].index & ADJ_INDEX_MASK : 0u;
+        id[j] = e < B.idLen ? d.stagedIds[B.ids + e] : 0u;
+    }
     const bool active = g < B.count;
     const StagedBody b = d.stagedBodies[B.first + (active ? g : 0u)];
+    // thread t solves body t at the end
+    const bool solver = tid < B.count;
+    const StagedBody mine = d.stagedBodies[B.first + (solver ? tid : 0u)];
+    auto copy_tet = [&](uint32_t e, uint32_t t) {
+#pragma unroll
+        for (uint32_t w = 0; w < 4; w++) copy16(tets + w * B.tetLen + e, d.tetConst + 4 * (size_t)t + w);
+    };
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++)
+        if (tid + j * kStagedThreads < B.tetLen) copy_tet(tid + j * kStagedThreads, ti[j]);
+    for (uint32_t e = tid + 4 * kStagedThreads; e < B.tetLen; e += kStagedThreads)
+        copy_tet(e, d.stagedTets[B.tet + e].index & ADJ_INDEX_MASK);
+    for (uint32_t i = tid; i < B.tetLen / 2; i += kStagedThreads) copy16(refs + 2 * i, d.stagedTets + B.tet + 2 * i);
+    for (uint32_t i = tid; i < B.recLen; i += kStagedThreads) copy16(rec + i, d.stagedRec + B.rec + i);
     // the lane's first spring, whose multiplier is read right after the wait
     const uint32_t spring = CLOTH && lane < b.nPre ? d.stagedRec[B.rec + b.rec + lane].w : 0u;
-    pdl_wait();
+    if (!early) pdl_wait();
+    // this frame's contacts (with `early`, see launch_primal_color: written
+    // before every grid that may still be running): the lane's first manifold,
+    // the first entry lane, lane + 8, ... past the springs
+    const uint32_t* dyn = d.dynList + __ldcg(d.dynStart + b.body);
+    const uint32_t nDyn = active ? __ldcg(d.dynCount + b.body) : 0u, nMan = active ? __ldcg(d.dynSplit + b.body) : 0u;
+    const uint32_t endMan = b.nPre + nMan;
+    const uint32_t kMan = lane >= b.nPre ? lane : lane + ((b.nPre - lane + 7u) & ~7u);
+    uint32_t slot = kStagedContacts, manifold = 0, bodyA = 0, bodyB = 0;
+    if (AHEAD && kMan < endMan) {
+        const uint32_t m = __ldcg(dyn + (kMan - b.nPre)) & ADJ_INDEX_MASK;
+        const uint4* mw = reinterpret_cast<const uint4*>(d.manifolds + m);
+        const uint4 h = __ldcg(mw);
+        bodyA = h.x;
+        bodyB = h.y;
+        if (h.z == 1u) slot = atomicAdd(&contacts, 1u);
+        if (slot < kStagedContacts) {
+            uint4* q = con + kStagedContactWords * slot;
+            q[0] = h;
+            copy16(q + 1, mw + 2);                   // normal
+            copy16(q + 2, mw + 3);                   // tangent
+            copy16(q + 3, mw + 4);                   // rA
+            copy16(q + 4, mw + 5);                   // rB
+            copy16(q + 5, mw + 6);                   // C0
+            copy16(q + 8, d.initLin + bodyA);
+            copy16(q + 9, d.initAng + bodyA);
+            copy16(q + 10, d.initLin + bodyB);
+            copy16(q + 11, d.initAng + bodyB);
+            manifold = m;
+        }
+    }
+    if (early) pdl_wait();
+    if (AHEAD && slot < kStagedContacts) {
+        uint4* q = con + kStagedContactWords * slot;
+        const uint4* mw = reinterpret_cast<const uint4*>(d.manifolds + manifold);
+        copy16(q + 6, mw + 7);                       // lambda
+        copy16(q + 7, mw + 8);                       // penalty
+        copy16(q + 12, d.posLin + bodyA);
+        copy16(q + 13, d.posAng + bodyA);
+        copy16(q + 14, d.posLin + bodyB);
+        copy16(q + 15, d.posAng + bodyB);
+    }
 #pragma unroll
     for (uint32_t j = 0; j < 4; j++)
         if (tid + j * kStagedThreads < B.idLen) copy16(pos + tid + j * kStagedThreads, d.posLin + id[j]);
     for (uint32_t i = tid + 4 * kStagedThreads; i < B.idLen; i += kStagedThreads)
         copy16(pos + i, d.posLin + d.stagedIds[B.ids + i]);
-    const uint32_t* dyn = d.dynList + d.dynStart[b.body];
-    const uint32_t nDyn = d.dynCount[b.body], nMan = d.dynSplit[b.body];
     float4 dual = make_float4(0, 0, 0, 0), inert = dual, anchor = dual;
     float bound = 0.0f;
     if (CLOTH && lane < b.nPre) dual = tof(d.springs[spring].dual);
-    if (lane == 0) {
-        inert = d.inertLin[b.body];
-        if (P.ogc) { bound = __uint_as_float(d.ogcBounds[b.body]); anchor = d.ogcPrev[b.body]; }
+    if (solver) {
+        inert = d.inertLin[mine.body];
+        if (P.ogc) { bound = __uint_as_float(d.ogcBounds[mine.body]); anchor = d.ogcPrev[mine.body]; }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (!active) return;
-    const unsigned mask = 0xFFu << (tid & 24u);
-    rec += b.rec;
-    pos += b.pos;
-    auto at = [&](uint32_t r, uint32_t k) { return xyz(pos[(r >> (8 * k)) & 0xFFu]); };
-    ParticleAccum acc{m3_zero(), s3(0)};
-    const uint32_t endMan = b.nPre + nMan, endTet = endMan + b.nTet, endSoft = endTet + nDyn - nMan,
-                   cnt = endSoft + b.nRest;
-    for (uint32_t k = lane; k < cnt; k += 8) {
-        ParticleTerms t;
-        if (CLOTH && k < b.nPre) {
-            const uint4 q = rec[k];
-            const uint32_t flags = rec[b.nPre + k].x;
-            if (flags & STAGED_GENERIC) {
-                particle_terms<true>(P, d, (FK_SPRING << ADJ_KIND_SHIFT) | q.w, b.body, t);
-            } else {
-                if (k != lane) dual = tof(d.springs[q.w].dual);
-                spring_core(P, at(q.z, 0), at(q.z, 1), (flags & 1u) == 0u, __uint_as_float(q.x), __uint_as_float(q.y),
-                            (flags & STAGED_HARD) != 0u, dual, t);
+    __shared__ float sums[9][STAGED_BODIES];
+    if (active) {
+        const unsigned mask = 0xFFu << (tid & 24u);
+        const uint4* br = rec + b.rec;
+        const float4* bp = pos + b.pos;
+        auto at = [&](uint32_t r, uint32_t k) { return xyz(bp[(r >> (8 * k)) & 0xFFu]); };
+        ParticleAccum acc{m3_zero(), s3(0)};
+        const uint32_t endTet = endMan + b.nTet, endSoft = endTet + nDyn - nMan, cnt = endSoft + b.nRest;
+        // a loop per kind: lanes whose entries of a kind fall into different
+        // rounds of eight still evaluate them together
+        uint32_t k = lane;
+        if (CLOTH) {
+            for (; k < b.nPre; k += 8) {
+                ParticleTerms t;
+                const uint4 q = br[k];
+                const uint32_t flags = br[b.nPre + k].x;
+                if (flags & STAGED_GENERIC) {
+                    particle_terms<true>(P, d, (FK_SPRING << ADJ_KIND_SHIFT) | q.w, b.body, t);
+                } else {
+                    if (k != lane) dual = tof(d.springs[q.w].dual);
+                    spring_core(P, at(q.z, 0), at(q.z, 1), (flags & 1u) == 0u, __uint_as_float(q.x),
+                                __uint_as_float(q.y), (flags & STAGED_HARD) != 0u, dual, t);
+                }
+                fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
             }
-            fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
-        } else if (k >= endMan && k < endTet) {
+        }
+        if (AHEAD && k < endMan && slot < kStagedContacts) {
+            ParticleTerms t;
+            const uint4* q = con + kStagedContactWords * slot;
+            const float4* f = reinterpret_cast<const float4*>(q);
+            ContactGPU c;
+            c.rA = tof4(f[3]); c.rB = tof4(f[4]); c.C0 = tof4(f[5]); c.lambda = tof4(f[6]); c.penalty = tof4(f[7]);
+            manifold_core(P, b.body == q[0].x, q[0].w, f[1], f[2], c, f[12], f[13], f[8], f[9], f[14], f[15], f[10],
+                          f[11], t);
+            fold_particle_term<false, false>(P, d, t, 0u, b.body, acc);
+            k += 8;
+        }
+        for (; k < endMan; k += 8) {
+            ParticleTerms t;
+            const uint32_t e = dyn[k - b.nPre];
+            particle_terms<false>(P, d, e, b.body, t);
+            fold_particle_term<false, false>(P, d, t, e, b.body, acc);
+        }
+        __syncwarp(mask);
+#pragma unroll 1
+        for (; k < endTet; k += 8) {
+            ParticleTerms t;
             const uint32_t e = b.tet + (k - endMan);
             const StagedTet r = refs[e];
-            const uint4 q0 = tets[e], q1 = tets[B.tetLen + e], q2 = tets[2 * B.tetLen + e], q3 = tets[3 * B.tetLen + e];
+            const uint4 q0 = tets[e], q1 = tets[B.tetLen + e], q2 = tets[2 * B.tetLen + e];
             const float3 m0 = mk3(__uint_as_float(q0.x), __uint_as_float(q0.y), __uint_as_float(q0.z));
             const float3 m1 = mk3(__uint_as_float(q1.x), __uint_as_float(q1.y), __uint_as_float(q1.z));
             const float3 m2 = mk3(__uint_as_float(q2.x), __uint_as_float(q2.y), __uint_as_float(q2.z));
             const uint32_t self = r.index >> ADJ_KIND_SHIFT;
             const float3 w = self == 1u ? m0 : (self == 2u ? m1 : (self == 3u ? m2
                              : -mk3(m0.x + m1.x + m2.x, m0.y + m1.y + m2.y, m0.z + m1.z + m2.z)));
-            const float diag = __uint_as_float(self == 0u ? q3.x : (self == 1u ? q3.y : (self == 2u ? q3.z : q3.w)));
+            const float diag = reinterpret_cast<const float*>(tets + 3 * B.tetLen + e)[self];
             tet_core(at(r.refs, 0), at(r.refs, 1), at(r.refs, 2), at(r.refs, 3), m0, m1, m2, __uint_as_float(q1.w),
                      __uint_as_float(q2.w), __uint_as_float(q0.w), w, diag, t);
             fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
-        } else if (CLOTH && k >= endSoft) {
-            const uint32_t e = 2 * b.nPre + (k - endSoft);
-            const uint4 q = rec[e], r = rec[b.nRest + e];
-            const float4 v = make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z),
-                                         __uint_as_float(q.w));
-            if (r.w & STAGED_BEND) {
-                bend_core(at(r.z, 0), at(r.z, 1), at(r.z, 2), at(r.z, 3), v, __uint_as_float(r.x), r.w & 3u, t);
-                fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
-            } else {
-                membrane_core(at(r.z, 0), at(r.z, 1), at(r.z, 2), v, __uint_as_float(r.x), __uint_as_float(r.y),
-                              r.w & 3u, t);
+        }
+        if (CLOTH) {
+            for (; k < endSoft; k += 8) {
+                ParticleTerms t;
+                const uint32_t e = dyn[nMan + (k - endTet)];
+                particle_terms<true>(P, d, e, b.body, t);
+                fold_particle_term<false, true>(P, d, t, e, b.body, acc);
+            }
+            __syncwarp(mask);
+            const uint32_t endMem = endSoft + b.nMem;
+            for (; k < endMem; k += 8) {
+                ParticleTerms t;
+                const uint32_t e = 2 * b.nPre + (k - endSoft);
+                const uint4 q = br[e], r = br[b.nRest + e];
+                membrane_core(at(r.z, 0), at(r.z, 1), at(r.z, 2),
+                              make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z),
+                                          __uint_as_float(q.w)),
+                              __uint_as_float(r.x), __uint_as_float(r.y), r.w, t);
                 fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
             }
-        } else {
-            // a contact: manifolds, then element contacts
-            const uint32_t e = dyn[k < endMan ? k - b.nPre : nMan + (k - endTet)];
-            particle_terms<CLOTH>(P, d, e, b.body, t);
-            fold_particle_term<false, CLOTH>(P, d, t, e, b.body, acc);
+            __syncwarp(mask);
+            for (; k < cnt; k += 8) {
+                ParticleTerms t;
+                const uint32_t e = 2 * b.nPre + (k - endSoft);
+                const uint4 q = br[e], r = br[b.nRest + e];
+                bend_core(at(r.z, 0), at(r.z, 1), at(r.z, 2), at(r.z, 3),
+                          make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z),
+                                      __uint_as_float(q.w)),
+                          __uint_as_float(r.x), r.w, t);
+                fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
+            }
+        }
+        __syncwarp(mask);
+#pragma unroll
+        for (int o = 4; o >= 1; o >>= 1) {
+            add_shfl_lower(mask, acc.lhs, o);
+            add_shfl3(mask, acc.rhs, o);
+        }
+        if (lane == 0) {
+            const float v[9] = {acc.lhs.r0.x, acc.lhs.r1.x, acc.lhs.r1.y, acc.lhs.r2.x, acc.lhs.r2.y,
+                                acc.lhs.r2.z, acc.rhs.x, acc.rhs.y, acc.rhs.z};
+#pragma unroll
+            for (int c = 0; c < 9; c++) sums[c][g] = v[c];
         }
     }
-#pragma unroll
-    for (int o = 4; o >= 1; o >>= 1) {
-        add_shfl_lower(mask, acc.lhs, o);
-        add_shfl3(mask, acc.rhs, o);
-    }
-    if (lane != 0) return;
-    particle_commit(P, d, b.body, b.radius, pos[0], inert, bound, anchor, acc);
+    __syncthreads();
+    // one warp solves the block's bodies side by side (a sixteenth of the
+    // issue slots that a lane per group would take)
+    if (!solver) return;
+    ParticleAccum acc{m3_zero(), mk3(sums[6][tid], sums[7][tid], sums[8][tid])};
+    acc.lhs.r0.x = sums[0][tid];
+    acc.lhs.r1.x = sums[1][tid]; acc.lhs.r1.y = sums[2][tid];
+    acc.lhs.r2.x = sums[3][tid]; acc.lhs.r2.y = sums[4][tid]; acc.lhs.r2.z = sums[5][tid];
+    particle_commit(P, d, mine.body, mine.radius, pos[mine.pos], inert, bound, anchor, acc);
 }
 
 void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t color, uint32_t count,
-                         uint32_t lanes, bool last, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
+                         uint32_t lanes, bool& chained, bool last, cudaStream_t st, cudaStream_t side, cudaEvent_t fork,
+                         cudaEvent_t join) {
     const int T = 128;
     const uint32_t upper = count != 0xFFFFFFFFu ? count : z.numDynamicBodies;
     if (upper == 0) return;
@@ -1965,8 +2087,23 @@ void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint
             staged = min(z.colorStaged[color], lean);
             const uint32_t b0 = z.stagedStart[color], blocks = z.stagedStart[color + 1] - b0;
             const size_t smem = 16 * (size_t)z.stagedWords[color];
-            if (staged && cloth) launch_pdl_smem(k_primal_staged<true>, blocks, kStagedThreads, smem, st, P, d, b0);
-            else if (staged) launch_pdl_smem(k_primal_staged<false>, blocks, kStagedThreads, smem, st, P, d, b0);
+            // The kernel reads this frame's contact lists before its wait.  That is
+            // safe behind one full dependency: the chain's first staged launch
+            // waits first and does not overlap what precedes it, and no later
+            // grid starts before it has started.
+            // Colors whose blocks all fit on the device at once are chains of
+            // latency and take their contacts ahead (12^3 soft cube 0.621 ->
+            // 0.547 ms a frame); for larger ones the registers and shared memory
+            // cost more (mixed scene 3.41 -> 3.62 ms, cloth 3.14 -> 3.30).
+            auto go = [&](auto kernel) {
+                launch_chain(kernel, chained, blocks, kStagedThreads, smem, st, P, d, b0, chained);
+            };
+            const bool ahead = blocks <= 3u * 148u;
+            if (staged && cloth && ahead) go(k_primal_staged<true, true>);
+            else if (staged && cloth) go(k_primal_staged<true, false>);
+            else if (staged && ahead) go(k_primal_staged<false, true>);
+            else if (staged) go(k_primal_staged<false, false>);
+            if (staged) chained = true;
         }
         if (lean > staged) {
             // pinned widths, and particles with more elements than a staged block holds
@@ -2182,8 +2319,12 @@ __global__ void k_dual(const Params P, const DevPtrs d, const Sizes z) {
 
 void launch_dual(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
     const bool rigid = z.numDynamicRigid == z.numDynamicBodies;
-    const uint32_t upper = z.numActiveJoints + z.numHardSprings + (rigid ? 4u : 1u) * z.maxPairs +
-                           ((P.cloth || P.ogc) ? z.maxSoft : 0u);
+    // The grid is sized for the items a frame usually has (a contact for every
+    // second particle), not for the capacities, and strides over more: idle
+    // blocks would keep the next color's from staging ahead (soft cube: its
+    // first color started 0.9 us after the dual had ended).
+    const uint32_t upper = z.numActiveJoints + z.numHardSprings +
+                           (rigid ? 4u * min(z.maxPairs, 2u * z.numDynamicBodies) : min(z.maxPairs, z.numDynamicBodies / 2u + 1u));
     if (rigid) launch_pdl(k_dual<4>, stride_blocks(upper, 128), 128, st, P, d, z);
     else launch_pdl(k_dual<1>, stride_blocks(upper, 128), 128, st, P, d, z);
 }

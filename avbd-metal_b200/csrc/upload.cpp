@@ -433,6 +433,7 @@ bool stage_body(const HostScene& H, uint32_t b, StagedBody& o, std::vector<u4>& 
     for (uint32_t k = 0; k < o.nRest && fits; k++) {
         const uint32_t e = H.postList[sg.z + o.nTet + k], idx = e & ADJ_INDEX_MASK;
         if ((e >> ADJ_KIND_SHIFT) == FK_MEMBRANE) {
+            o.nMem++;
             const MembraneGPU& m = H.membranes[idx];
             const uint32_t self = b == m.ids.y ? 1u : (b == m.ids.z ? 2u : 0u);
             const uint32_t refs = local(m.ids.x) | (local(m.ids.y) << 8) | (local(m.ids.z) << 16);
@@ -443,7 +444,7 @@ bool stage_body(const HostScene& H, uint32_t b, StagedBody& o, std::vector<u4>& 
             const uint32_t self = b == m.ids.x ? 0u : (b == m.ids.y ? 1u : (b == m.ids.z ? 2u : 3u));
             const uint32_t refs = local(m.ids.x) | (local(m.ids.y) << 8) | (local(m.ids.z) << 16) | (local(m.ids.w) << 24);
             rest[k] = u4{float_bits(m.K.x), float_bits(m.K.y), float_bits(m.K.z), float_bits(m.K.w)};
-            rest[o.nRest + k] = u4{float_bits(m.mat.x), 0, refs, self | STAGED_BEND};
+            rest[o.nRest + k] = u4{float_bits(m.mat.x), 0, refs, self};
         }
     }
     return fits && staged_words(rec.size(), o.nTet, ids.size()) <= STAGED_MAX_WORDS;
