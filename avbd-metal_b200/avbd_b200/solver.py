@@ -373,8 +373,8 @@ class GPUSolver:
 
     def set_primal_variant(self, variant: int):
         """Pin every static color's primal to one variant: 8, 16 or 32 lanes
-        per body, abi.PRIMAL_VARIANT_STAGED, or abi.PRIMAL_VARIANT_AUTO to
-        re-run the autotuner.  All variants compute the same floats."""
+        per body, abi.PRIMAL_VARIANT_STAGED, or abi.PRIMAL_VARIANT_AUTO for
+        the default (staged).  All variants compute the same floats."""
         self._check(load_library().avbd_set_primal_variant(self._h, int(variant)))
 
     def set_profiling(self, enabled: bool):

@@ -114,6 +114,7 @@ struct StagedTet {
 };
 struct alignas(16) TetConst { f4 r0, r1, r2, diag; };   // DmInv rows; w: alpha, muV, lamV; muV |w|^2 per vertex
 constexpr uint32_t STAGED_BODIES = 16;             // most bodies of a block (8 lanes each)
+constexpr uint32_t STAGED_WIDE = 2368;             // bodies of a tet color up to which a warp takes one body, four a block
 constexpr uint32_t STAGED_MAX_WORDS = 2600;        // most 16-byte words of shared memory of a block
 constexpr uint32_t STAGED_MAX_REFS = 255;          // most bodies one body's records refer to
 // flags of a spring's record, beside this body's position in it (bit 0)

@@ -148,6 +148,8 @@ struct DevPtrs {
     uint32_t* learnAccepted;                    // frames whose prediction was kept (running)
 };
 
+constexpr uint32_t SMALL_SCENE = 128;     // dynamic bodies up to which launch_solve_small runs the iterations
+
 struct Sizes {
     uint32_t numBodies, numColliders, numActiveJoints, numHardSprings, numTets;
     uint32_t maxPairs, producers, numDynamicBodies;
@@ -167,8 +169,8 @@ struct Sizes {
     const uint32_t* colorLean;            // lean particles at the head of each color's launch order
     const uint32_t* colorStartHost;       // static palette: each color's start in the list
     // staged primal: bodies of each color's launch order in blocks, the
-    // colors' first blocks, shared-memory words of a block
-    const uint32_t *colorStaged, *stagedStart, *stagedWords;
+    // colors' first blocks, shared-memory words of a block, lanes per body
+    const uint32_t *colorStaged, *stagedStart, *stagedWords, *stagedLanes;
     // dynamic coloring: block shape of the rigid primal's grid-stride launch
     // (blocks, threads per block), chosen by the runtime's autotuner
     uint32_t dynBlocks, dynThreads;

@@ -151,9 +151,8 @@ struct avbd_solver {
     // per-color launches are needed by the learned warm start's trial sweeps
     // and by the per-iteration residual trace
     void update_small_solve() {
-        smallSolve = z.numDynamicBodies <= 512 && !P.cloth && !P.ogc && learnMode == AVBD_WARM_START_PLAIN && !learnCapture &&
+        smallSolve = z.numDynamicBodies <= SMALL_SCENE && !P.cloth && !P.ogc && learnMode == AVBD_WARM_START_PLAIN && !learnCapture &&
                      !residualTrace;
-        if (smallSolve) tuneStage = -1;
     }
     uint64_t frame = 0;
     int failure = AVBD_FAIL_NONE;
@@ -261,12 +260,11 @@ struct avbd_solver {
     // One frame, in the reference's stage order.  `parity` selects which
     // manifold buffer is "current" (the buffers swap after every frame).
     // With profiling on, an event is recorded at every stage boundary.
-    void encode_frame(int parity) { encode_frame_on(parity, stream, nullptr, nullptr); }
+    void encode_frame(int parity) { encode_frame_on(parity, stream, nullptr); }
 
-    // One frame on stream `st`.  `lanes` overrides the per-color lane width
-    // and `primalEvents` (2 per primal launch, in launch order) brackets every
-    // primal launch; both are used by the autotuner's eager frames.
-    void encode_frame_on(int parity, cudaStream_t st, const uint32_t* lanes, cudaEvent_t* primalEvents) {
+    // One frame on stream `st`.  `primalEvents` (2 per primal launch, in launch
+    // order) brackets every primal launch of the autotuner's eager frames.
+    void encode_frame_on(int parity, cudaStream_t st, cudaEvent_t* primalEvents) {
         DevPtrs f = d;
         if (parity) {
             std::swap(f.manifolds, f.prevManifolds);
@@ -404,8 +402,8 @@ struct avbd_solver {
                     if (count == 0) continue;
                     mark(AVBD_STAGE_PRIMAL);
                     if (primalEvents) cudaEventRecord(primalEvents[2 * primalLaunch], st);
-                    launch_primal_color(P, g, z, c, count, lanes ? lanes[c] : H.colorLanes[c], chained,
-                                        c + 1 == colorBound, st, branchStream, wideFork, wideJoin);
+                    launch_primal_color(P, g, z, c, count, H.colorLanes[c], chained, c + 1 == colorBound, st,
+                                        branchStream, wideFork, wideJoin);
                     if (primalEvents) cudaEventRecord(primalEvents[2 * primalLaunch + 1], st);
                     primalLaunch++;
                     if (P.cloth) {
@@ -525,6 +523,7 @@ struct avbd_solver {
         z.colorStaged = H.colorStaged.data();
         z.stagedStart = H.stagedStart.data();
         z.stagedWords = H.stagedWords.data();
+        z.stagedLanes = H.stagedLanes.data();
         z.colorStartHost = H.dynamicColoring ? nullptr : H.colorStart.data();
         z.numDynamicRigid = 0;
         for (uint32_t b = 0; b < nb; b++) z.numDynamicRigid += (H.posLin[b].w > 0.0f && H.shape[b].w >= 0.0f) ? 1u : 0u;
@@ -782,7 +781,6 @@ struct avbd_solver {
         std::memset(hostLatch, 0, 4 * sizeof(uint32_t));
         // Small scenes run their whole iteration loop in one thread block.
         update_small_solve();
-        tuneStage = tuning_applies() ? 0 : -1;
         dyn_tune_setup();
         if (cudaDeviceSynchronize() != cudaSuccess) { error = "device error during upload"; return AVBD_ERR_NO_DEVICE; }
         return AVBD_OK;
@@ -876,56 +874,7 @@ struct avbd_solver {
         return failure == AVBD_FAIL_NONE ? AVBD_OK : AVBD_ERR_RUNTIME_FAILURE;
     }
 
-    // Primal variant autotuner.  Each static color's primal can run the
-    // grouped kernel with 8, 16 or 32 lanes per body or the staged kernel;
-    // the fold order is fixed, so every variant computes the same floats and
-    // only speed differs (it depends on the color's body count and adjacency
-    // sizes).  The first four frames run eagerly, one variant each, with
-    // events around every primal launch; each color then keeps its fastest
-    // variant and the frame graphs are captured with it.
-    static constexpr int kTuneVariants = 4;
-    static constexpr uint32_t kTuneWidths[kTuneVariants] = {8, 16, 32, AVBD_PRIMAL_STAGED};
-    int tuneStage = -1;                       // -1 off / done, else the next variant
-    double tuneMs[kTuneVariants][MAX_COLORS] = {};
     std::vector<cudaEvent_t> tuneEvents;
-
-    bool tuning_applies() const { return !z.dynamicColoring && !smallSolve && H.staticUsedColors > 0; }
-
-    int tune_frame() {
-        const uint32_t colorBound = H.staticUsedColors;
-        const size_t need = 2 * (size_t)P.iterations * colorBound;
-        while (tuneEvents.size() < need) {
-            cudaEvent_t e;
-            if (!check(cudaEventCreate(&e), "event create")) return AVBD_ERR_RUNTIME_FAILURE;
-            tuneEvents.push_back(e);
-        }
-        uint32_t lanes[MAX_COLORS];
-        for (int c = 0; c < MAX_COLORS; c++) lanes[c] = kTuneWidths[tuneStage];
-        encode_frame_on((int)(frame & 1), launch, lanes, tuneEvents.data());
-        if (!check(cudaGetLastError(), "tuning frame")) return AVBD_ERR_RUNTIME_FAILURE;
-        frame++;
-        if (!check(cudaStreamSynchronize(launch), "tuning frame")) return AVBD_ERR_RUNTIME_FAILURE;
-        uint32_t k = 0;
-        for (uint32_t it = 0; it < P.iterations; it++)
-            for (uint32_t c = 0; c < colorBound; c++) {
-                if (H.colorCounts[c] == 0) continue;
-                float ms = 0.0f;
-                if (!check(cudaEventElapsedTime(&ms, tuneEvents[2 * k], tuneEvents[2 * k + 1]), "tuning timing"))
-                    return AVBD_ERR_RUNTIME_FAILURE;
-                tuneMs[tuneStage][c] += ms;
-                k++;
-            }
-        if (++tuneStage == kTuneVariants) {
-            for (uint32_t c = 0; c < colorBound; c++) {
-                int best = 0;
-                for (int w = 1; w < kTuneVariants; w++) if (tuneMs[w][c] < tuneMs[best][c]) best = w;
-                H.colorLanes[c] = kTuneWidths[best];
-            }
-            tuneStage = -1;
-            graphsValid = false;
-        }
-        return AVBD_OK;
-    }
 
     // Block-shape autotuner of the dynamic-coloring primal (rigid scenes,
     // batched worlds).  Its grid-stride launch gives every body to one 8-lane
@@ -972,7 +921,7 @@ struct avbd_solver {
             tuneEvents.push_back(e);
         }
         const uint32_t launches = P.iterations * colorLaunchBound;
-        encode_frame_on((int)(frame & 1), launch, nullptr, tuneEvents.data());
+        encode_frame_on((int)(frame & 1), launch, tuneEvents.data());
         if (!check(cudaGetLastError(), "tuning frame")) return AVBD_ERR_RUNTIME_FAILURE;
         frame++;
         if (!check(cudaStreamSynchronize(launch), "tuning frame")) return AVBD_ERR_RUNTIME_FAILURE;
@@ -1003,11 +952,6 @@ struct avbd_solver {
     int step(uint32_t frames) {
         if (failure != AVBD_FAIL_NONE) return AVBD_ERR_RUNTIME_FAILURE;
         uint32_t f = 0;
-        while (tuneStage >= 0 && f < frames) {
-            int rc = tune_frame();
-            if (rc != AVBD_OK) return rc;
-            f++;
-        }
         while (dynTuneStage >= 0 && f < frames) {
             int rc = dyn_tune_frame();
             if (rc != AVBD_OK) return rc;
@@ -1814,13 +1758,7 @@ int avbd_set_primal_variant(avbd_solver* s, uint32_t variant) {
         return AVBD_ERR_INVALID_ARGUMENT;
     int rc = s->retire();
     if (rc != AVBD_OK) return rc;
-    if (variant == 0) {
-        s->tuneStage = s->tuning_applies() ? 0 : -1;
-        std::memset(s->tuneMs, 0, sizeof(s->tuneMs));
-    } else {
-        s->tuneStage = -1;
-        for (auto& l : s->H.colorLanes) l = variant;
-    }
+    for (auto& l : s->H.colorLanes) l = variant ? variant : (uint32_t)AVBD_PRIMAL_STAGED;
     s->graphsValid = false;
     return AVBD_OK;
 }

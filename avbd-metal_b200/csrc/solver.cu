@@ -1822,7 +1822,9 @@ static void launch_primal_group(const Params& P, const DevPtrs& d, uint32_t colo
 // in place of 96), and the lanes evaluate and fold their entries l, l + 8, ...
 // straight from shared memory; only contacts, and springs with levers, are read
 // through the adjacency.  Every expression and order is the grouped kernel's.
-// MEASURED_STAGED
+// What bounds it: for small colors the chain (0.6 us gather, 1.4 us for three
+// tets a lane, 0.6 us solve, 1 us between grids); for large ones issue slots
+// (0.6 of them used on the 256^2 cloth, 18-22 us a color of 32,767).
 // ---------------------------------------------------------------------------
 constexpr int kStagedThreads = 8 * (int)STAGED_BODIES;
 constexpr uint32_t kStagedContacts = 24;        // one-point manifolds of a block held in shared memory
@@ -1837,14 +1839,19 @@ __device__ __forceinline__ void copy16(void* smem, const void* gmem) {
 // constant parts before the wait, the bodies' poses and the multipliers with
 // the positions: a contact adds its arithmetic to the color instead of four
 // dependent trips (2.3 us of the 4.3 us a small color took).
-template <bool CLOTH, bool AHEAD>
-__global__ void __launch_bounds__(kStagedThreads, 5)
+//
+// LANES = 32 (tet colors of at most STAGED_WIDE bodies): four bodies a block,
+// a warp each.  Its lanes evaluate 32 entries at once and pass the terms to the
+// eight folding lanes by shuffles: the color's chain is one tet long instead of
+// three, which pays while the device has room for a warp per body.
+template <bool CLOTH, bool AHEAD, int LANES>
+__global__ void __launch_bounds__(kStagedThreads, LANES == 32 ? 4 : 5)
 k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock, bool early) {
     extern __shared__ uint4 words[];
     __shared__ uint4 con[AHEAD ? kStagedContacts * kStagedContactWords : 1];
     __shared__ uint32_t contacts;
     pdl_trigger();
-    const uint32_t tid = threadIdx.x, g = tid >> 3, lane = tid & 7u;
+    const uint32_t tid = threadIdx.x, g = tid / LANES, lane = tid & (LANES - 1u);
     if (AHEAD) {
         if (tid == 0) contacts = 0u;
         __syncthreads();
@@ -1888,7 +1895,7 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock, bool early
     const uint32_t* dyn = d.dynList + __ldcg(d.dynStart + b.body);
     const uint32_t nDyn = active ? __ldcg(d.dynCount + b.body) : 0u, nMan = active ? __ldcg(d.dynSplit + b.body) : 0u;
     const uint32_t endMan = b.nPre + nMan;
-    const uint32_t kMan = lane >= b.nPre ? lane : lane + ((b.nPre - lane + 7u) & ~7u);
+    const uint32_t kMan = lane >= b.nPre ? lane : lane + ((b.nPre - lane + LANES - 1u) & ~(LANES - 1u));
     uint32_t slot = kStagedContacts, manifold = 0, bodyA = 0, bodyB = 0;
     if (AHEAD && kMan < endMan) {
         const uint32_t m = __ldcg(dyn + (kMan - b.nPre)) & ADJ_INDEX_MASK;
@@ -1939,12 +1946,67 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock, bool early
     __syncthreads();
     __shared__ float sums[9][STAGED_BODIES];
     if (active) {
-        const unsigned mask = 0xFFu << (tid & 24u);
+        const unsigned mask = LANES == 32 ? 0xFFu : 0xFFu << (tid & 24u);
         const uint4* br = rec + b.rec;
         const float4* bp = pos + b.pos;
         auto at = [&](uint32_t r, uint32_t k) { return xyz(bp[(r >> (8 * k)) & 0xFFu]); };
         ParticleAccum acc{m3_zero(), s3(0)};
         const uint32_t endTet = endMan + b.nTet, endSoft = endTet + nDyn - nMan, cnt = endSoft + b.nRest;
+        auto staged_contact = [&](ParticleTerms& t) {
+            const uint4* q = con + kStagedContactWords * slot;
+            const float4* f = reinterpret_cast<const float4*>(q);
+            ContactGPU c;
+            c.rA = tof4(f[3]); c.rB = tof4(f[4]); c.C0 = tof4(f[5]); c.lambda = tof4(f[6]); c.penalty = tof4(f[7]);
+            manifold_core(P, b.body == q[0].x, q[0].w, f[1], f[2], c, f[12], f[13], f[8], f[9], f[14], f[15], f[10],
+                          f[11], t);
+        };
+        auto tet = [&](uint32_t e, ParticleTerms& t) {
+            const StagedTet r = refs[e];
+            const uint4 q0 = tets[e], q1 = tets[B.tetLen + e], q2 = tets[2 * B.tetLen + e];
+            const float3 m0 = mk3(__uint_as_float(q0.x), __uint_as_float(q0.y), __uint_as_float(q0.z));
+            const float3 m1 = mk3(__uint_as_float(q1.x), __uint_as_float(q1.y), __uint_as_float(q1.z));
+            const float3 m2 = mk3(__uint_as_float(q2.x), __uint_as_float(q2.y), __uint_as_float(q2.z));
+            const uint32_t self = r.index >> ADJ_KIND_SHIFT;
+            const float3 w = self == 1u ? m0 : (self == 2u ? m1 : (self == 3u ? m2
+                             : -mk3(m0.x + m1.x + m2.x, m0.y + m1.y + m2.y, m0.z + m1.z + m2.z)));
+            const float diag = reinterpret_cast<const float*>(tets + 3 * B.tetLen + e)[self];
+            tet_core(at(r.refs, 0), at(r.refs, 1), at(r.refs, 2), at(r.refs, 3), m0, m1, m2, __uint_as_float(q1.w),
+                     __uint_as_float(q2.w), __uint_as_float(q0.w), w, diag, t);
+        };
+        if (LANES == 32) {
+            // manifolds and tets only (tet colors)
+            for (uint32_t base = 0; base < cnt; base += 32) {
+                const uint32_t k = base + lane;
+                ParticleTerms t;
+                t.kind = TERM_NONE;
+                uint32_t e = 0;
+                if (k < endMan) {
+                    if (AHEAD && k == kMan && slot < kStagedContacts) {
+                        staged_contact(t);
+                    } else {
+                        e = dyn[k - b.nPre];
+                        particle_terms<false>(P, d, e, b.body, t);
+                    }
+                } else if (k < endTet) {
+                    tet(b.tet + (k - endMan), t);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int src = (int)(lane & 7u) + 8 * j;
+                    ParticleTerms u = t;
+                    if (j > 0) {
+                        if (base + 8u * j >= cnt) break;             // the same in the whole warp
+                        u.kind = __shfl_sync(0xffffffffu, t.kind, src);
+                        u.rhs = shfl_idx3(t.rhs, src);
+                        u.a = shfl_idx3(t.a, src);
+                        u.b = shfl_idx3(t.b, src);
+                        u.c = shfl_idx3(t.c, src);
+                    }
+                    if (lane < 8) fold_particle_term<false, false>(P, d, u, 0u, b.body, acc);
+                }
+            }
+        } else {
         // a loop per kind: lanes whose entries of a kind fall into different
         // rounds of eight still evaluate them together
         uint32_t k = lane;
@@ -1965,12 +2027,7 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock, bool early
         }
         if (AHEAD && k < endMan && slot < kStagedContacts) {
             ParticleTerms t;
-            const uint4* q = con + kStagedContactWords * slot;
-            const float4* f = reinterpret_cast<const float4*>(q);
-            ContactGPU c;
-            c.rA = tof4(f[3]); c.rB = tof4(f[4]); c.C0 = tof4(f[5]); c.lambda = tof4(f[6]); c.penalty = tof4(f[7]);
-            manifold_core(P, b.body == q[0].x, q[0].w, f[1], f[2], c, f[12], f[13], f[8], f[9], f[14], f[15], f[10],
-                          f[11], t);
+            staged_contact(t);
             fold_particle_term<false, false>(P, d, t, 0u, b.body, acc);
             k += 8;
         }
@@ -1984,18 +2041,7 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock, bool early
 #pragma unroll 1
         for (; k < endTet; k += 8) {
             ParticleTerms t;
-            const uint32_t e = b.tet + (k - endMan);
-            const StagedTet r = refs[e];
-            const uint4 q0 = tets[e], q1 = tets[B.tetLen + e], q2 = tets[2 * B.tetLen + e];
-            const float3 m0 = mk3(__uint_as_float(q0.x), __uint_as_float(q0.y), __uint_as_float(q0.z));
-            const float3 m1 = mk3(__uint_as_float(q1.x), __uint_as_float(q1.y), __uint_as_float(q1.z));
-            const float3 m2 = mk3(__uint_as_float(q2.x), __uint_as_float(q2.y), __uint_as_float(q2.z));
-            const uint32_t self = r.index >> ADJ_KIND_SHIFT;
-            const float3 w = self == 1u ? m0 : (self == 2u ? m1 : (self == 3u ? m2
-                             : -mk3(m0.x + m1.x + m2.x, m0.y + m1.y + m2.y, m0.z + m1.z + m2.z)));
-            const float diag = reinterpret_cast<const float*>(tets + 3 * B.tetLen + e)[self];
-            tet_core(at(r.refs, 0), at(r.refs, 1), at(r.refs, 2), at(r.refs, 3), m0, m1, m2, __uint_as_float(q1.w),
-                     __uint_as_float(q2.w), __uint_as_float(q0.w), w, diag, t);
+            tet(b.tet + (k - endMan), t);
             fold_particle_term<false, CLOTH>(P, d, t, 0u, b.body, acc);
         }
         if (CLOTH) {
@@ -2030,10 +2076,13 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock, bool early
             }
         }
         __syncwarp(mask);
+        }
+        if (lane < 8) {
 #pragma unroll
-        for (int o = 4; o >= 1; o >>= 1) {
-            add_shfl_lower(mask, acc.lhs, o);
-            add_shfl3(mask, acc.rhs, o);
+            for (int o = 4; o >= 1; o >>= 1) {
+                add_shfl_lower(mask, acc.lhs, o);
+                add_shfl3(mask, acc.rhs, o);
+            }
         }
         if (lane == 0) {
             const float v[9] = {acc.lhs.r0.x, acc.lhs.r1.x, acc.lhs.r1.y, acc.lhs.r2.x, acc.lhs.r2.y,
@@ -2099,10 +2148,12 @@ void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint
                 launch_chain(kernel, chained, blocks, kStagedThreads, smem, st, P, d, b0, chained);
             };
             const bool ahead = blocks <= 3u * 148u;
-            if (staged && cloth && ahead) go(k_primal_staged<true, true>);
-            else if (staged && cloth) go(k_primal_staged<true, false>);
-            else if (staged && ahead) go(k_primal_staged<false, true>);
-            else if (staged) go(k_primal_staged<false, false>);
+            const bool wide = z.stagedLanes[color] == 32u;
+            if (staged && cloth && ahead) go(k_primal_staged<true, true, 8>);
+            else if (staged && cloth) go(k_primal_staged<true, false, 8>);
+            else if (staged && wide) go(k_primal_staged<false, true, 32>);
+            else if (staged && ahead) go(k_primal_staged<false, true, 8>);
+            else if (staged) go(k_primal_staged<false, false, 8>);
             if (staged) chained = true;
         }
         if (lean > staged) {
@@ -2319,23 +2370,30 @@ __global__ void k_dual(const Params P, const DevPtrs d, const Sizes z) {
 
 void launch_dual(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
     const bool rigid = z.numDynamicRigid == z.numDynamicBodies;
-    // The grid is sized for the items a frame usually has (a contact for every
-    // second particle), not for the capacities, and strides over more: idle
-    // blocks would keep the next color's from staging ahead (soft cube: its
-    // first color started 0.9 us after the dual had ended).
-    const uint32_t upper = z.numActiveJoints + z.numHardSprings +
-                           (rigid ? 4u * min(z.maxPairs, 2u * z.numDynamicBodies) : min(z.maxPairs, z.numDynamicBodies / 2u + 1u));
+    // The grid is sized for the items a frame usually has (two contacts a rigid
+    // body, one for every second particle), not for the capacities, and strides
+    // over more: idle blocks would keep the next color's from staging ahead
+    // (soft cube: its first color started 0.9 us after the dual had ended).
+    // Scenes with element contacts fill the device either way (mixed 3.48 ms a
+    // frame with the capacities, 3.50 without).
+    const bool elements = P.cloth || P.ogc;
+    const uint32_t contacts = elements ? z.maxPairs + z.maxSoft
+                              : min(z.maxPairs, rigid ? 2u * z.numDynamicBodies : z.numDynamicBodies / 2u + 1u);
+    const uint32_t upper = z.numActiveJoints + z.numHardSprings + (rigid ? 4u : 1u) * contacts;
     if (rigid) launch_pdl(k_dual<4>, stride_blocks(upper, 128), 128, st, P, d, z);
     else launch_pdl(k_dual<1>, stride_blocks(upper, 128), 128, st, P, d, z);
 }
 
 // ---------------------------------------------------------------------------
-// Small scenes: the whole iteration loop in one launch of a cluster of up to
-// eight CTAs, a color or the dual at a time between barriers, in the order of
-// the per-color launches.  The cluster grows with the scene so that the
-// largest color still has an 8-lane group per body: one CTA (its barrier is a
-// block barrier) up to 64 bodies, eight from 257 on.  One CTA of 256 threads
-// for every size took 1,810 us of the 2,060 us frame of 512 piled bodies.
+// Small scenes (SMALL_SCENE bodies): the whole iteration loop in one launch of
+// a cluster of up to eight CTAs, a color or the dual at a time between
+// barriers, in the order of the per-color launches.  A rigid body's solve is
+// some 4,000 instructions of a warp, so the CTAs are few enough to meet
+// quickly and many enough that an SM scheduler has a warp or two: one CTA (its
+// barrier is a block barrier) up to 32 bodies, four up to 64, eight above.
+// Larger scenes spread each color over the whole device instead: 512 piled
+// bodies took 1,810 us a frame in one CTA, 405 in eight, 370 with a launch per
+// color; 100 boxes 574 us in one CTA, 219 in eight.
 // ---------------------------------------------------------------------------
 constexpr int kSmallThreads = 512;
 constexpr uint32_t kSmallSlots = kIncWords * kSmallThreads;      // floats of dynamic shared memory
@@ -2395,7 +2453,7 @@ static void small_attributes() {
 void launch_solve_small(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t colorBound, cudaStream_t st) {
     small_attributes();
     const uint32_t n = z.numDynamicBodies;
-    const uint32_t ctas = n <= 64 ? 1u : (n <= 128 ? 2u : (n <= 256 ? 4u : 8u));
+    const uint32_t ctas = n <= 32 ? 1u : (n <= 64 ? 4u : 8u);
     if (ctas == 1) launch_cluster(k_solve_small<false>, 1, kSmallThreads, kSmallSlots * 4, st, P, d, z, colorBound);
     else launch_cluster(k_solve_small<true>, ctas, kSmallThreads, kSmallSlots * 4, st, P, d, z, colorBound);
 }

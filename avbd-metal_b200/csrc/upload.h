@@ -57,13 +57,14 @@ struct HostScene {
 
     // Staged primal: the first colorStaged[c] bodies of a color's launch
     // order, in blocks stagedStart[c] .. stagedStart[c + 1]; stagedWords[c] is
-    // the most 16-byte words of shared memory a block takes.
+    // the most 16-byte words of shared memory a block takes,
+    // stagedLanes[c] the lanes per body that the blocks are made for.
     std::vector<StagedBody> stagedBodies;
     std::vector<StagedBlock> stagedBlocks;
     std::vector<u4> stagedRec;
     std::vector<StagedTet> stagedTets;
     std::vector<TetConst> tetConst;
-    std::vector<uint32_t> stagedIds, colorStaged, stagedStart, stagedWords;
+    std::vector<uint32_t> stagedIds, colorStaged, stagedStart, stagedWords, stagedLanes;
 
     // Static per-body adjacency, split around the per-frame contact entries:
     // pre = joints + springs (kinds 0, 1), post = tets (kind 3), each sorted.

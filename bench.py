@@ -101,7 +101,7 @@ def parse():
                     help="with --frames-only: the warm start of the frames")
     ap.add_argument("--iterations", type=int, default=0, help="with --frames-only: override the iterations")
     ap.add_argument("--primal-variant", choices=["auto", "staged", "8", "16", "32"], default="auto",
-                    help="with --frames-only: pin the static-palette primal variant (default: autotuned)")
+                    help="with --frames-only: pin the static-palette primal variant (default: staged)")
     ap.add_argument("--pusht-obs", action="store_true",
                     help="time the Push-T pixel-observation kernel instead (--obs-envs x --obs-res^2 x 3 "
                          "bytes per launch) and print its own JSON line")
@@ -662,7 +662,7 @@ def run_ours(args, world, rank, local):
             "data": "synthetic (seeded SplitMix64 scene)",
             "config": cfg,
             "timing": "CUDA events on the solver stream per step, max over ranks",
-            # per static color: the primal variant the autotuner kept for its
+            # per static color: the primal variant of its
             # lean particles (8 / 16 / 32 lanes per body, 1 = staged kernel)
             "primal_launch": {"colors": int(counters.used_colors),
                               "lanes_per_body": prof["color_lanes"][:int(counters.used_colors)]},

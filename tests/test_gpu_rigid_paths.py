@@ -1,0 +1,109 @@
+"""The paths that a rigid or mixed frame takes by its size, bit for bit against
+the oracle: one CTA, four, eight or a launch per color for the iterations; one
+block or a cluster for the coloring; a frame that needs more colors than its
+graph was built for; manifolds of one to eight points shared out to the lanes;
+and, for particles, elements that do not fit the staged tables."""
+import math
+
+import numpy as np
+import pytest
+
+from avbd_b200 import demos
+from avbd_b200.scene import PhysicsScene, SceneSpring, SceneTet
+from avbd_b200.solver import GPUSolver
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(g, o, what):
+    for a, b in zip(g.positions(), o.positions()):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), what
+
+
+def _run(scene, oracle_lib, frames, every=1):
+    g, o = GPUSolver(scene), oracle_lib.OracleSolver(scene, threads=8)
+    for f in range(0, frames, every):
+        g.step(every)
+        assert o.step(every) == 0
+        _same(g, o, f"frame {f + every}")
+    return g
+
+
+def pile(count, layers=4):
+    """Boxes in columns, a little apart: colors appear as they land."""
+    s = PhysicsScene("pile")
+    demos.add_ground(s, friction=0.6)
+    side = max(1, int(math.ceil(math.sqrt(count / layers))))
+    for k in range(count):
+        col, layer = k % (side * side), k // (side * side)
+        s.add_body((0.3, 0.3, 0.3), 500.0, 0.6, ((col % side) * 0.32, (col // side) * 0.32, 0.18 + 0.34 * layer))
+    s.settings.iterations = 6
+    return s
+
+
+@pytest.mark.parametrize("count", [1, 32, 33, 64, 65, 128, 129, 513])
+def test_iteration_paths(cuda_lib, oracle_lib, count):
+    _run(pile(count), oracle_lib, 24, every=4)
+
+
+@pytest.mark.parametrize("count", [1022, 1023, 1024, 4096])
+def test_coloring_sizes(cuda_lib, oracle_lib, count):
+    # with the ground, 1,023 boxes are the last scene of the one-block coloring
+    # and 4,095 the last of the four-CTA cluster
+    _run(pile(count), oracle_lib, 12, every=6)
+
+
+def test_more_colors_than_launched(cuda_lib, oracle_lib):
+    """The color bound is fitted while the boxes are apart (one color); the
+    frames in which they land are submitted without a retirement between."""
+    s = pile(160, layers=8)
+    g, o = GPUSolver(s), oracle_lib.OracleSolver(s, threads=8)
+    for frames in (8, 1, 40):
+        g.step(frames)
+        assert o.step(frames) == 0
+        _same(g, o, f"after {frames} more")
+    assert g.counters().used_colors > 1
+
+
+def test_shapes_between_the_paths(cuda_lib, oracle_lib):
+    for count in (60, 140):
+        _run(demos.shapes_scene(seed=3, count=count), oracle_lib, 60, every=10)
+
+
+def rods(levers):
+    """Hard and soft springs of particles under a cloth scene's kinds; with
+    `levers`, anchors off the particles' centres."""
+    s = demos.drape_scene(res=10)
+    first = len(s.bodies)
+    for k in range(12):
+        s.add_particle(0.02, 0.05, position=(5.0 + 0.2 * k, 0.0, 1.0))
+    for k in range(11):
+        a = (0.01, 0.0, 0.0) if levers else (0, 0, 0)
+        s.add_spring(SceneSpring(first + k, first + k + 1, a, (0, 0, 0), 200.0 if k % 2 else 1e5, hard=k % 2 == 0))
+    return s
+
+
+@pytest.mark.parametrize("levers", [False, True])
+def test_staged_springs(cuda_lib, oracle_lib, levers):
+    _run(rods(levers), oracle_lib, 20, every=5)
+
+
+@pytest.mark.parametrize("tets", [80, 84, 90, 300])
+def test_staged_reference_limit(cuda_lib, oracle_lib, tets):
+    """A hub of `tets` tets refers to 3 tets + 1 bodies: 253 fit a byte with
+    one to spare, 271 do not and take the grouped kernel, in one color with
+    particles that are staged."""
+    s = PhysicsScene("hub")
+    s.settings.iterations = 8
+    demos.add_ground(s, friction=0.5)
+    hub = s.add_particle(0.02, 0.05, position=(0.0, 0.0, 2.0))
+    for k in range(tets):
+        z = 1.0 - 2.0 * (k + 0.5) / tets
+        r, phi = math.sqrt(max(0.0, 1.0 - z * z)), k * 2.399963229728653
+        d = np.array([r * math.cos(phi), r * math.sin(phi), z])
+        u = np.cross(d, [0.0, 0.0, 1.0] if abs(z) < 0.9 else [1.0, 0.0, 0.0])
+        u /= np.linalg.norm(u)
+        c = np.array([0.0, 0.0, 2.0]) + 0.5 * d
+        ids = [s.add_particle(0.01, 0.02, position=tuple(c + 0.04 * w)) for w in (u, np.cross(d, u), d)]
+        s.add_tet(SceneTet((hub, *ids), 500.0, 2000.0))
+    _run(s, oracle_lib, 10, every=2)
