@@ -1105,7 +1105,7 @@ __global__ void k_dat_apply_color(const Params P, const DevPtrs d, uint32_t colo
     const float3 next = xyz(d.posNext[v]);
     if (unclothed) {
         d.posLin[v] = mk4(next, mass);
-        d.posAng[v] = d.angNext[v];
+        if (d.shape[v].w >= 0.0f) d.posAng[v] = d.angNext[v];   // a particle's solve leaves no pending rotation
         return;
     }
     if (!dat_apply_one(P, d, v, next, mass)) d.posLin[v] = mk4(next, mass);
