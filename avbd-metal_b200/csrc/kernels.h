@@ -148,7 +148,9 @@ struct DevPtrs {
     uint32_t* learnAccepted;                    // frames whose prediction was kept (running)
 };
 
-constexpr uint32_t SMALL_SCENE = 128;     // dynamic bodies up to which launch_solve_small runs the iterations
+// dynamic bodies up to which launch_solve_small runs the iterations: dynamic
+// coloring, and a static palette
+constexpr uint32_t SMALL_SCENE = 512, SMALL_PARTICLES = 32;
 
 struct Sizes {
     uint32_t numBodies, numColliders, numActiveJoints, numHardSprings, numTets;

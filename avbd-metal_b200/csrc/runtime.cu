@@ -151,7 +151,7 @@ struct avbd_solver {
     // per-color launches are needed by the learned warm start's trial sweeps
     // and by the per-iteration residual trace
     void update_small_solve() {
-        smallSolve = z.numDynamicBodies <= SMALL_SCENE && !P.cloth && !P.ogc && learnMode == AVBD_WARM_START_PLAIN && !learnCapture &&
+        smallSolve = z.numDynamicBodies <= (z.dynamicColoring ? SMALL_SCENE : SMALL_PARTICLES) && !P.cloth && !P.ogc && learnMode == AVBD_WARM_START_PLAIN && !learnCapture &&
                      !residualTrace;
     }
     uint64_t frame = 0;

@@ -2385,15 +2385,17 @@ void launch_dual(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t
 }
 
 // ---------------------------------------------------------------------------
-// Small scenes (SMALL_SCENE bodies): the whole iteration loop in one launch of
-// a cluster of up to eight CTAs, a color or the dual at a time between
-// barriers, in the order of the per-color launches.  A rigid body's solve is
-// some 4,000 instructions of a warp, so the CTAs are few enough to meet
-// quickly and many enough that an SM scheduler has a warp or two: one CTA (its
-// barrier is a block barrier) up to 32 bodies, four up to 64, eight above.
-// Larger scenes spread each color over the whole device instead: 512 piled
-// bodies took 1,810 us a frame in one CTA, 405 in eight, 370 with a launch per
-// color; 100 boxes 574 us in one CTA, 219 in eight.
+// Small scenes: the whole iteration loop in one launch of a cluster, a color or
+// the dual at a time between barriers, in the order of the per-color launches.
+// A rigid body's solve is some 4,000 instructions of a warp, so the CTAs are
+// few enough to meet quickly and many enough that an SM scheduler has a warp or
+// two: one CTA (its barrier is a block barrier) up to 32 bodies, four up to 64,
+// eight up to 128, sixteen up to SMALL_SCENE.  Against a launch per color (one
+// CTA of 256 threads in parentheses), a frame: 512 piled shapes 0.530 ms /
+// 0.563 (2.06), 130 shapes 0.446 / 0.512, 400 boxes 0.226 / 0.243, 100 boxes
+// 0.219 in eight CTAs (0.574); above 512 bodies an SM holds too many.  Particles
+// of a static palette leave at SMALL_PARTICLES, where the staged launches win
+// (512 of them 0.277 ms / 0.491 here).
 // ---------------------------------------------------------------------------
 constexpr int kSmallThreads = 512;
 constexpr uint32_t kSmallSlots = kIncWords * kSmallThreads;      // floats of dynamic shared memory
@@ -2438,24 +2440,44 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_solve_small(const Params P
     }
 }
 
-// dynamic shared memory above 48 KiB (set once per device)
-static void small_attributes() {
-    static std::atomic<uint64_t> done{0};
+// Dynamic shared memory above 48 KiB and clusters above eight CTAs (asked once
+// per device); the largest cluster that the device can place.
+static uint32_t small_attributes() {
+    static std::atomic<uint64_t> done{0}, sixteen{0};
     int dev = 0;
     cudaGetDevice(&dev);
     const uint64_t bit = 1ull << (dev & 63);
-    if (done.load() & bit) return;
-    cudaFuncSetAttribute(k_solve_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmallSlots * 4));
-    cudaFuncSetAttribute(k_solve_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmallSlots * 4));
-    done.fetch_or(bit);
+    if (!(done.load() & bit)) {
+        cudaFuncSetAttribute(k_solve_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmallSlots * 4));
+        cudaFuncSetAttribute(k_solve_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmallSlots * 4));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = kSmallSlots * 4;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 16;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaFuncSetAttribute(k_solve_small<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, k_solve_small<true>, &cfg) == cudaSuccess && clusters > 0)
+            sixteen.fetch_or(bit);
+        else
+            cudaGetLastError();
+        done.fetch_or(bit);
+    }
+    return sixteen.load() & bit ? 16u : 8u;
 }
 
 void launch_solve_small(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t colorBound, cudaStream_t st) {
-    small_attributes();
+    const uint32_t most = small_attributes();
     const uint32_t n = z.numDynamicBodies;
-    const uint32_t ctas = n <= 32 ? 1u : (n <= 64 ? 4u : 8u);
-    if (ctas == 1) launch_cluster(k_solve_small<false>, 1, kSmallThreads, kSmallSlots * 4, st, P, d, z, colorBound);
-    else launch_cluster(k_solve_small<true>, ctas, kSmallThreads, kSmallSlots * 4, st, P, d, z, colorBound);
+    const uint32_t ctas = n <= 32 ? 1u : (n <= 64 ? 4u : (n <= 128 ? 8u : most)), threads = ctas == 16 ? 256u : kSmallThreads;
+    if (ctas == 1) launch_cluster(k_solve_small<false>, 1, threads, kSmallSlots * 4, st, P, d, z, colorBound);
+    else launch_cluster(k_solve_small<true>, ctas, threads, kSmallSlots * 4, st, P, d, z, colorBound);
 }
 
 // ---------------------------------------------------------------------------
