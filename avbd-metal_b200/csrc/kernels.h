@@ -228,9 +228,8 @@ static_assert(sizeof(PushTDev) == 48, "PushTDev layout");
 // out: 24 floats per instance (avbd_render_instance)
 void launch_build_instances(const DevPtrs& d, const uint32_t* ids, const float4* colors, uint32_t n,
                             uint32_t colorMode, float* out, cudaStream_t st);
-void launch_soft_normals(const DevPtrs& d, uint32_t numTris, const uint32_t* surfVerts, const uint32_t* vtStart,
-                         const uint32_t* vtCount, const uint32_t* vtList, uint32_t numSurf, float4* faceN,
-                         float clothScale, float4* out, cudaStream_t st);
+void launch_soft_normals(const DevPtrs& d, const uint32_t* surfVerts, const uint32_t* vtStart, const uint32_t* vtCount,
+                         const uint32_t* vtList, uint32_t numSurf, float clothScale, float4* out, cudaStream_t st);
 void launch_skin_deform(const float4* posLin, const SkinBinding* b, uint32_t n, float4* out, cudaStream_t st);
 // shapes: 6 float4 of scratch per environment
 constexpr uint32_t PUSHT_RECORD = 11;   // float4 of an environment's shapes: 24 floats, five pixel ranges

@@ -79,36 +79,29 @@ __global__ void k_build_instances(const DevPtrs d, const uint32_t* ids, const fl
     store4(o + 20, sh.x, sh.y, sh.w, pl.w > 0.0f ? 1.0f : 0.0f);
 }
 
-// Raw face normals (twice the area along the normal), 50_render.metal:104-117.
-__global__ void k_face_normals(const DevPtrs d, uint32_t numTris, float4* faceN) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= numTris) return;
-    const uint4 tr = d.tris[t];
-    const float3 a = xyz(d.posLin[tr.x]), b = xyz(d.posLin[tr.y]), c = xyz(d.posLin[tr.z]);
-    faceN[t] = mk4(cross(b - a, c - a), 0.0f);
-}
-
 // Angle x area weighted vertex normals with the curvature-thinned render
-// thickness (50_render.metal:119-180).
+// thickness (50_render.metal:104-180).  The raw face normals (twice the area
+// along the normal, (b - a) x (c - a) in the triangle's own order) are formed
+// here, from positions that the angles need anyway, instead of by a kernel and
+// a buffer of their own: the call is bounded by its launches (24^3 soft cube,
+// normals and skin, 11.6 us a pass with three launches, 9.5 with two).
 __global__ void k_vertex_normals(const DevPtrs d, const uint32_t* surfVerts, const uint32_t* vtStart,
                                  const uint32_t* vtCount, const uint32_t* vtList, uint32_t numSurf,
-                                 const float4* faceN, float clothScale, float4* out) {
+                                 float clothScale, float4* out) {
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= numSurf) return;
     const uint32_t v = surfVerts[gid];
     const float3 p = xyz(d.posLin[v]);
-    float3 acc = s3(0.0f);
+    float3 acc = s3(0.0f), firstFace = s3(0.0f);
     float wsum = 0.0f;
     const uint32_t s = vtStart[gid], e = s + vtCount[gid];
     for (uint32_t k = s; k < e; k++) {
-        const uint32_t t = vtList[k];
-        const uint4 tr = d.tris[t];
-        const float3 fn = xyz(faceN[t]);
+        const uint4 tr = d.tris[vtList[k]];
+        const float3 a = xyz(d.posLin[tr.x]), b = xyz(d.posLin[tr.y]), c = xyz(d.posLin[tr.z]);
+        const float3 fn = cross(b - a, c - a);
+        if (k == s) firstFace = fn;
         const float area = 0.5f * len3(fn);
-        float3 ea, eb;
-        if (tr.x == v) { ea = xyz(d.posLin[tr.y]) - p; eb = xyz(d.posLin[tr.z]) - p; }
-        else if (tr.y == v) { ea = xyz(d.posLin[tr.x]) - p; eb = xyz(d.posLin[tr.z]) - p; }
-        else { ea = xyz(d.posLin[tr.x]) - p; eb = xyz(d.posLin[tr.y]) - p; }
+        const float3 ea = (tr.x == v ? b : a) - p, eb = (tr.x == v || tr.y == v ? c : b) - p;
         const float ang = acosf(clampf(dot(safe_normalize(ea), safe_normalize(eb)), -1.0f, 1.0f));
         const float w = area * ang;
         acc += safe_normalize(fn) * w;
@@ -116,7 +109,7 @@ __global__ void k_vertex_normals(const DevPtrs d, const uint32_t* surfVerts, con
     }
     // a fold-over can cancel the weighted sum: fall back to the first face
     const float coherence = wsum > 1e-9f ? len3(acc) / wsum : 0.0f;
-    if (len3(acc) < 1e-6f && e > s) acc = xyz(faceN[vtList[s]]);
+    if (len3(acc) < 1e-6f && e > s) acc = firstFace;
     const float sc = d.clothVert[v] != 0u ? clothScale : 1.0f;
     const float c2 = clampf(coherence * coherence, 0.0f, 1.0f);
     const float thick = fabsf(d.shape[v].w) * sc * (0.25f + (1.0f - 0.25f) * c2);
@@ -337,13 +330,11 @@ void launch_build_instances(const DevPtrs& d, const uint32_t* ids, const float4*
     if (n) k_build_instances<<<blocks_for(n, 128), 128, 0, st>>>(d, ids, colors, n, colorMode, out);
 }
 
-void launch_soft_normals(const DevPtrs& d, uint32_t numTris, const uint32_t* surfVerts, const uint32_t* vtStart,
-                         const uint32_t* vtCount, const uint32_t* vtList, uint32_t numSurf, float4* faceN,
-                         float clothScale, float4* out, cudaStream_t st) {
-    if (!numTris || !numSurf) return;
-    k_face_normals<<<blocks_for(numTris, 256), 256, 0, st>>>(d, numTris, faceN);
-    k_vertex_normals<<<blocks_for(numSurf, 128), 128, 0, st>>>(d, surfVerts, vtStart, vtCount, vtList, numSurf,
-                                                               faceN, clothScale, out);
+void launch_soft_normals(const DevPtrs& d, const uint32_t* surfVerts, const uint32_t* vtStart, const uint32_t* vtCount,
+                         const uint32_t* vtList, uint32_t numSurf, float clothScale, float4* out, cudaStream_t st) {
+    if (!numSurf) return;
+    k_vertex_normals<<<blocks_for(numSurf, 64), 64, 0, st>>>(d, surfVerts, vtStart, vtCount, vtList, numSurf, clothScale,
+                                                             out);
 }
 
 void launch_skin_deform(const float4* posLin, const SkinBinding* b, uint32_t n, float4* out, cudaStream_t st) {

@@ -169,12 +169,11 @@ struct avbd_solver {
     size_t hostReadBytes = 0;
     std::vector<uint8_t> motorMode;    // MOTOR_MODE_MASK bits of every joint, packed for the setters' checks
     // render surface (built on the first smooth-normals call): surface
-    // vertices, their incident triangles, face normals
+    // vertices, their incident triangles
     bool renderSurfaceReady = false;
     uint32_t numSurfVerts = 0;
     uint32_t *surfVerts = nullptr, *surfVtStart = nullptr, *surfVtCount = nullptr, *surfVtList = nullptr;
     uint32_t* surfClothVert = nullptr;
-    float4* faceNormals = nullptr;
     // skin bindings (replaced by each upload)
     SkinBinding* skin = nullptr;
     uint32_t numSkin = 0;
@@ -1434,8 +1433,7 @@ int avbd_soft_normals(avbd_solver* s, float cloth_scale, float* out, int out_on_
         cloth.resize(nb, 0);
         bool ok = s->upload(s->surfVerts, verts, "surfaceVertices") && s->upload(s->surfVtStart, start, "surfaceVtStart") &&
                   s->upload(s->surfVtCount, count, "surfaceVtCount") && s->upload(s->surfVtList, list, "surfaceVtList") &&
-                  s->upload(s->surfClothVert, cloth, "surfaceClothVert") &&
-                  s->alloc(s->faceNormals, nt, "faceNormals");
+                  s->upload(s->surfClothVert, cloth, "surfaceClothVert");
         if (!ok) return AVBD_ERR_ALLOC_FAILED;
         s->numSurfVerts = (uint32_t)verts.size();
         s->renderSurfaceReady = true;
@@ -1448,8 +1446,8 @@ int avbd_soft_normals(avbd_solver* s, float cloth_scale, float* out, int out_on_
     if (!out_on_device) cudaMemcpyAsync(dOut, out, outBytes, cudaMemcpyHostToDevice, s->launch);  // untouched entries
     DevPtrs d = s->d;
     d.clothVert = s->surfClothVert;
-    launch_soft_normals(d, nt, s->surfVerts, s->surfVtStart, s->surfVtCount, s->surfVtList, s->numSurfVerts,
-                        s->faceNormals, cloth_scale, dOut, s->launch);
+    launch_soft_normals(d, s->surfVerts, s->surfVtStart, s->surfVtCount, s->surfVtList, s->numSurfVerts, cloth_scale, dOut,
+                        s->launch);
     return render_finish(s, out_on_device ? nullptr : out, dOut, outBytes, "soft normals");
 }
 
