@@ -1268,12 +1268,33 @@ void launch_primal_wide(const Params& P, const DevPtrs& d, uint32_t color, uint3
 // Squared AL gradient of one rigid body (linear and angular parts) by an
 // 8-lane group: lanes stamp entries lane, lane + 8, ..., an xor butterfly
 // folds them and lane 0 writes *out.
-__device__ void rigid_residual(const Params& P, const DevPtrs& d, uint32_t body, uint32_t lane, unsigned mask,
-                               float* out) {
+__device__ __forceinline__ void rigid_residual(const Params& P, const DevPtrs& d, uint32_t body, uint32_t lane,
+                                               unsigned mask, float* out) {
+    // only the right-hand sides are kept, so a contact point's blocks are not formed
     Accum acc{m3_zero(), m3_zero(), m3_zero(), s3(0), s3(0)};
+    float3 rhsLin = s3(0), rhsAng = s3(0);
     const AdjView v = adj_view(d, body);
     const uint32_t cnt = v.count();
-    for (uint32_t k = lane; k < cnt; k += 8) stamp_entry(P, d, v.at(k), body, acc);
+    for (uint32_t k = lane; k < cnt; k += 8) {
+        const uint32_t entry = v.at(k);
+        if ((entry >> ADJ_KIND_SHIFT) == FK_MANIFOLD) {
+            const ManifoldGPU& m = d.manifolds[entry & ADJ_INDEX_MASK];
+            const uint32_t n = m.header.z;
+            const ManifoldCtx x = manifold_ctx(d, m, body);
+            for (uint32_t i = 0; i < n; i++) {
+                const PointInc inc = manifold_point_inc(P, x, m.contacts[i]);
+                rhsLin += inc.rhsLin;
+                rhsAng += inc.rhsAng;
+            }
+        } else {
+            Accum one{m3_zero(), m3_zero(), m3_zero(), rhsLin, rhsAng};
+            stamp_entry<false>(P, d, entry, body, one);
+            rhsLin = one.rhsLin;
+            rhsAng = one.rhsAng;
+        }
+    }
+    acc.rhsLin = rhsLin;
+    acc.rhsAng = rhsAng;
 #pragma unroll
     for (int o = 4; o >= 1; o >>= 1) {
         add_shfl3(mask, acc.rhsLin, o);
