@@ -1931,7 +1931,6 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock, bool early
             copy16(q + 1, mw + 2);                   // normal
             copy16(q + 2, mw + 3);                   // tangent
             copy16(q + 3, mw + 4);                   // rA
-            copy16(q + 4, mw + 5);                   // rB
             copy16(q + 5, mw + 6);                   // C0
             copy16(q + 8, d.initLin + bodyA);
             copy16(q + 9, d.initAng + bodyA);
@@ -1944,6 +1943,7 @@ k_primal_staged(const Params P, const DevPtrs d, uint32_t firstBlock, bool early
     if (AHEAD && slot < kStagedContacts) {
         uint4* q = con + kStagedContactWords * slot;
         const uint4* mw = reinterpret_cast<const uint4*>(d.manifolds + manifold);
+        copy16(q + 4, mw + 5);                       // rB (the dual stores the stick flag in its w)
         copy16(q + 6, mw + 7);                       // lambda
         copy16(q + 7, mw + 8);                       // penalty
         copy16(q + 12, d.posLin + bodyA);
