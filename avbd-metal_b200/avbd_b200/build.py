@@ -35,6 +35,16 @@ def up_to_date() -> bool:
     return all(os.path.getmtime(f) <= t for f in sources() + headers())
 
 
+def compile_report(source: str) -> str:
+    """What ptxas said of a source's kernels (registers, stack frames, spills)
+    when it was last compiled."""
+    path = os.path.join(LIBDIR, "obj", source + ".ptxas")
+    if not os.path.exists(path) or not up_to_date():
+        build(force=True)
+    with open(path) as f:
+        return f.read()
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and up_to_date():
         return LIB
@@ -43,13 +53,18 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(objdir, exist_ok=True)
     objs = []
     common = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-prec-div=true", "-prec-sqrt=true",
-              "-Xcompiler", "-fPIC,-ffp-contract=off,-fno-fast-math", "-I", CSRC]
+              "-Xcompiler", "-fPIC,-ffp-contract=off,-fno-fast-math", "-Xptxas", "-v", "-I", CSRC]
     for src in sources():
         obj = os.path.join(objdir, os.path.basename(src) + ".o")
         cmd = [NVCC] + ARCH + common + ["-c", src, "-o", obj]
         if verbose:
             print(" ".join(cmd), file=sys.stderr)
-        subprocess.check_call(cmd)
+        done = subprocess.run(cmd, stderr=subprocess.PIPE, text=True)
+        sys.stderr.writelines(line + "\n" for line in done.stderr.splitlines()
+                              if done.returncode or "warning" in line)
+        done.check_returncode()
+        with open(os.path.join(objdir, os.path.basename(src) + ".ptxas"), "w") as f:
+            f.write(done.stderr)
         objs.append(obj)
     cmd = [NVCC] + ARCH + ["-shared", "-cudart", "static", "-o", LIB] + objs
     if verbose:

@@ -556,7 +556,11 @@ __device__ __forceinline__ M3 geom_stiff_ball_socket(int k, float3 v) {
     return m;
 }
 
-__device__ void stamp_joint(const Params& P, const DevPtrs& d, const JointGPU& j, uint32_t self, Accum& acc) {
+// inlined in every caller: as a called function it would take Params and
+// DevPtrs by address, and each thread of a caller would copy both (1.5 KB) to
+// local memory first
+__device__ __forceinline__ void stamp_joint(const Params& P, const DevPtrs& d, const JointGPU& j, uint32_t self,
+                                            Accum& acc) {
     const uint32_t a = j.header.x, b = j.header.y;
     const bool isA = self == a;
     const float torqueArm = j.C0Lin.w;

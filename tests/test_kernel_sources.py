@@ -1,7 +1,10 @@
-"""What the kernels' sources promise about the order of their reads, checked on
-the CPU (a read that races another grid cannot be shown by a run)."""
+"""Properties of the kernels that a run on the device does not show, checked on
+the CPU: the order of reads that could race another grid, and what the compiler
+made of the kernels."""
 import os
 import re
+
+from avbd_b200 import build
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "avbd-metal_b200", "csrc")
 
@@ -40,3 +43,16 @@ def test_staged_primal_reads_what_the_dual_writes_after_its_wait():
     copied = lambda part: {int(w) for w in re.findall(r"copy16\([^,]*,\s*mw\s*\+\s*(\d+)\)", part)}
     assert written <= copied(after)
     assert not written & copied(before), written & copied(before)
+
+
+def test_no_kernel_copies_its_arguments_to_local_memory():
+    """A device function that is called instead of inlined takes the launch
+    arguments by address: every thread of its callers then copies them (1.5 KB)
+    to local memory, which cost the residual kernels of the learned warm start
+    half their speed."""
+    report = build.compile_report("solver.cu")
+    functions = re.findall(r"Function properties for (\S+)\s+(\d+) bytes stack frame", report)
+    called = [f for f, _ in functions if re.search(r"RKNS_(6Params|7DevPtrs)E", f)]
+    assert not called, called
+    residual = {f: int(frame) for f, frame in functions if re.search(r"k_primal_groupILi\d+ELb1ELb[01]ELb1E", f)}
+    assert residual and not any(residual.values()), residual
