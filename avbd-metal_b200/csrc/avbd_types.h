@@ -183,7 +183,7 @@ struct Counters {
     uint32_t numSoftVT, numSoftEE;   // isotropic element contacts of this frame
     uint32_t ogcQueue;               // trackers that reseed from the grid this frame
     uint32_t adjLong;                // bodies whose contact segment is sorted by a block
-    uint32_t tailTickets[2];         // DevPtrs::tailTicket of the solve and of a predicted trial branch
+    uint32_t tails[2][3];            // DevPtrs::tail of the solve and of a predicted trial branch
     uint32_t activeManifolds;        // manifolds with contacts (DevPtrs::activeManifolds)
 };
 

@@ -65,7 +65,8 @@ struct DevPtrs {
     uint32_t* dynSplit;                   // manifold entries at the head of each sorted dyn segment
     uint32_t* adjLongQueue;               // bodies with long contact segments this frame
     uint32_t* activeManifolds;            // manifolds with contacts, in no order
-    uint32_t* tailTicket;                 // blocks done with the last launched color (zero between launches)
+    uint32_t* tail;                       // colors past the last launched one: next chunk, finished chunks, blocks
+                                          // that left (zero between launches)
     uint32_t* postTets;                   // tet entries at the head of each static post segment
     const TetGPU* tetInc;                 // tet records in postList order (null without tets)
     // staged primal (static palette): launch tables

@@ -132,8 +132,8 @@ struct avbd_solver {
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     bool graphsValid = false;
     // Dynamic coloring: the frame graph launches this many colors one by one;
-    // one block of the last launch takes the rest.  It grows (and the graphs
-    // are re-captured) when a retired frame used more colors.
+    // the last launch takes the rest.  It grows (and the graphs are
+    // re-captured) when a retired frame used more colors.
     uint32_t colorLaunchBound = 8;
     bool colorBoundFitted = false;
     // batched worlds (avbd_create_batched): ragged body ranges, the bodies'
@@ -275,8 +275,8 @@ struct avbd_solver {
                                                                       offsetof(Counters, ogcSlots))
                                         : nullptr;
         f.ogcExceed = ogcSlots;
-        uint32_t* tickets = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(d.counters) + offsetof(Counters, tailTickets));
-        f.tailTicket = tickets;
+        uint32_t* tails = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(d.counters) + offsetof(Counters, tails));
+        f.tail = tails;
         usedEvents = 0;
         uint32_t primalLaunch = 0;
         bool chained = false;
@@ -350,7 +350,7 @@ struct avbd_solver {
             DevPtrs fb = f, fp = f;
             fb.posLin = f.learnSweptLin;
             fb.posAng = f.learnSweptAng;
-            fb.tailTicket = tickets + 1;       // the two branches' sweeps run side by side
+            fb.tail = tails + 3;               // the two branches' sweeps run side by side
             // the trial sweeps count OGC bound exceeders in slots 2 (plain) and 3 (predicted)
             if (ogcSlots) { fp.ogcExceed = ogcSlots + 2; fb.ogcExceed = ogcSlots + 3; }
             launch_mlp_infer(f.learnHalf, f.learnPrm, f.learnNorm, f.learnFeat, z.numLearn, f.learnPred,
@@ -860,8 +860,7 @@ struct avbd_solver {
                 std::snprintf(buf, sizeof buf, "Planar-DAT element grid span exceeded at frame %u: %u elements",
                               hostLatch[1], hostLatch[2]);
             else if (failure == AVBD_FAIL_WAIT_TIMEOUT)
-                std::snprintf(buf, sizeof buf, "a bounded device wait (warm-start MLP inference) gave up during "
-                              "frame %u", hostLatch[1]);
+                std::snprintf(buf, sizeof buf, "a bounded device wait gave up during frame %u", hostLatch[1]);
             else if (failure == AVBD_FAIL_PLANAR_DAT_INVALID_ANCHOR)
                 std::snprintf(buf, sizeof buf, "Planar-DAT invalid anchor at frame %u: %u pairs", hostLatch[1],
                               hostLatch[2]);

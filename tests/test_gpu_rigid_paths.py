@@ -53,16 +53,54 @@ def test_coloring_sizes(cuda_lib, oracle_lib, count):
     _run(pile(count), oracle_lib, 12, every=6)
 
 
-def test_more_colors_than_launched(cuda_lib, oracle_lib):
-    """The color bound is fitted while the boxes are apart (one color); the
-    frames in which they land are submitted without a retirement between."""
-    s = pile(160, layers=8)
+def falling(count):
+    """Four layers of boxes, each shifted against the one below: one color in
+    the air (up to frame 16), four once they have landed (from frame 32)."""
+    s = PhysicsScene("falling")
+    demos.add_ground(s, friction=0.6)
+    side = int(math.ceil(math.sqrt(count / 4)))
+    for k in range(count):
+        col, layer = k % (side * side), k // (side * side)
+        s.add_body((0.3, 0.3, 0.3), 500.0, 0.6, ((col % side) * 0.34 + 0.15 * (layer % 2),
+                                                 (col // side) * 0.34 + 0.15 * (layer // 2 % 2), 0.5 + 0.4 * layer))
+    s.settings.iterations = 6
+    return s
+
+
+@pytest.mark.parametrize("count", [640, 2600])
+def test_more_colors_than_launched(cuda_lib, oracle_lib, count):
+    """The color bound is fitted while the boxes are apart; the frames in which
+    they land are submitted without a retirement between, so that the launch of
+    the only color solves all of them.  (Above 512 bodies: a launch per color.)"""
+    import time
+    import torch
+    s = falling(count)
     g, o = GPUSolver(s), oracle_lib.OracleSolver(s, threads=8)
-    for frames in (8, 1, 40):
-        g.step(frames)
-        assert o.step(frames) == 0
-        _same(g, o, f"after {frames} more")
-    assert g.counters().used_colors > 1
+    g.step(9)                                    # seven of them time the block shapes
+    assert o.step(9) == 0
+    _same(g, o, "in the air")                    # retired: the bound is one color
+    assert g.counters().used_colors == 1
+    g.step(1)
+    one = g.profile()["kernels_per_frame"]
+
+    def burst():
+        torch.cuda.synchronize()                 # waits without retiring
+        t = time.perf_counter()
+        g.step(20)
+        torch.cuda.synchronize()
+        return time.perf_counter() - t
+
+    g.step(30)
+    unfitted = burst()
+    assert o.step(51) == 0
+    _same(g, o, "landed")
+    used = g.counters().used_colors
+    assert used >= 3
+    g.step(4)                                    # captures the graphs of the fitted bound
+    assert g.profile()["kernels_per_frame"] >= one + s.settings.iterations * (used - 1)
+    fitted = min(burst() for _ in range(3))
+    # one block for the other colors takes 5 to 60 times a launch per color
+    assert unfitted < 2.5 * fitted, (unfitted, fitted)
 
 
 def test_shapes_between_the_paths(cuda_lib, oracle_lib):
