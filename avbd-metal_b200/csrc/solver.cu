@@ -445,15 +445,24 @@ __device__ __forceinline__ void color_place(const DevPtrs& d, uint32_t gid, cons
 }
 
 constexpr int kColorPasses = 20;
+constexpr int kColorLaunched = 8;                 // passes launched over the whole device
+constexpr uint32_t kColorCluster = 10240;         // bodies up to which a cluster does everything
 
 // The whole coloring in one launch of a cluster (one CTA for small scenes):
 // passes between barriers until one changes nothing, usually the first or
 // second because a frame starts from the last frame's colors, then count, scan
 // and place.  As 24 launches, most of which found nothing to do, it took 28 us
-// of a 250 us frame of 20 bodies and 54 us at 28,673 bodies (4,096 worlds).
-// Above 65,536 bodies the passes use the whole device, a launch each.
+// of a 250 us frame of 20 bodies.  Where the contacts change in every frame it
+// is four to ten passes, and a cluster's pass grows with the bodies: above
+// kColorCluster the first kColorLaunched passes and the rest use the whole
+// device, a launch each, and the cluster only goes on with later passes and the
+// repair (`from` > 0, `all` = false).  Coloring stage, median of 60 frames,
+// cluster / launches (24 launches): tumbling shapes 5,000 39 / 47 us (66), 8,000
+// 45 / 51 (68), 12,000 64 / 53 (74), 28,000 111 / 61 (72), 60,000 217 / 82 (98);
+// settled worlds of 8,398 bodies 25 / 27 (47), 16,739 35 / 31 (51), 28,626
+// 45 / 35 (55).
 template <bool CLUSTER>
-__global__ void __launch_bounds__(1024) k_color(const Params P, const DevPtrs d) {
+__global__ void __launch_bounds__(1024) k_color(const Params P, const DevPtrs d, int from, bool all) {
     pdl_prologue();
     const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
     const volatile uint32_t* changed = d.counters->changed;
@@ -465,7 +474,7 @@ __global__ void __launch_bounds__(1024) k_color(const Params P, const DevPtrs d)
             __syncthreads();
         }
     };
-    for (int pass = 0; pass < kColorPasses; pass++) {
+    for (int pass = from; pass < kColorPasses; pass++) {
         if (pass > 0 && changed[pass - 1] == 0u) break;          // the same in every thread
         const uint32_t* src = (pass & 1) ? d.colorsB : d.colorsA;
         uint32_t* dst = (pass & 1) ? d.colorsA : d.colorsB;
@@ -476,6 +485,7 @@ __global__ void __launch_bounds__(1024) k_color(const Params P, const DevPtrs d)
         if (first == 0) color_repair(P, d, d.colorsA);
         barrier();
     }
+    if (!all) return;
     for (uint32_t gid = first; gid < P.numBodies; gid += step) color_count(d, gid, d.colorsA);
     barrier();
     if (first == 0) color_scan(d);
@@ -484,22 +494,23 @@ __global__ void __launch_bounds__(1024) k_color(const Params P, const DevPtrs d)
 }
 
 __global__ void k_color_iterate(const Params P, const DevPtrs d, const uint32_t* src, uint32_t* dst, uint32_t pass) {
+    pdl_prologue();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= P.numBodies) return;
     if (pass > 0 && d.counters->changed[pass - 1] == 0u) return;
     color_step(d, gid, src, dst, pass);
 }
-__global__ void k_color_repair(const Params P, const DevPtrs d, uint32_t* colors, uint32_t finalPass) {
-    if (threadIdx.x == 0 && d.counters->changed[finalPass] != 0u) color_repair(P, d, colors);
-}
 __global__ void k_color_validate_count(const Params P, const DevPtrs d, const uint32_t* colors) {
+    pdl_prologue();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid < P.numBodies) color_count(d, gid, colors);
 }
 __global__ void k_color_scan(const DevPtrs d) {
+    pdl_prologue();
     if (threadIdx.x == 0) color_scan(d);
 }
 __global__ void k_color_scatter(const Params P, const DevPtrs d, const uint32_t* colors) {
+    pdl_prologue();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid < P.numBodies) color_place(d, gid, colors);
 }
@@ -526,22 +537,21 @@ static void launch_cluster(void (*kernel)(KArgs...), uint32_t ctas, uint32_t thr
 }
 
 void launch_dynamic_coloring(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st) {
-    if (P.numBodies <= 1024u) { launch_cluster(k_color<false>, 1, 1024, 0, st, P, d); return; }
-    if (P.numBodies <= 65536u) {
-        launch_cluster(k_color<true>, P.numBodies <= 4096u ? 4 : 8, 1024, 0, st, P, d);
+    if (P.numBodies <= 1024u) { launch_cluster(k_color<false>, 1, 1024, 0, st, P, d, 0, true); return; }
+    if (P.numBodies <= kColorCluster) {
+        launch_cluster(k_color<true>, P.numBodies <= 4096u ? 4 : 8, 1024, 0, st, P, d, 0, true);
         return;
     }
-    const int T = 128;
-    const uint32_t blocks = (P.numBodies + T - 1) / T;
-    for (int pass = 0; pass < kColorPasses; pass++) {
+    const uint32_t T = 128, blocks = (P.numBodies + T - 1) / T;
+    for (int pass = 0; pass < kColorLaunched; pass++) {
         const uint32_t* src = (pass & 1) ? d.colorsB : d.colorsA;
         uint32_t* dst = (pass & 1) ? d.colorsA : d.colorsB;
-        k_color_iterate<<<blocks, T, 0, st>>>(P, d, src, dst, (uint32_t)pass);
+        launch_pdl(k_color_iterate, blocks, T, st, P, d, src, dst, (uint32_t)pass);
     }
-    k_color_repair<<<1, 32, 0, st>>>(P, d, d.colorsA, kColorPasses - 1);
-    k_color_validate_count<<<blocks, T, 0, st>>>(P, d, d.colorsA);
-    k_color_scan<<<1, 32, 0, st>>>(d);
-    k_color_scatter<<<blocks, T, 0, st>>>(P, d, d.colorsA);
+    launch_cluster(k_color<true>, 8, 1024, 0, st, P, d, kColorLaunched, false);
+    launch_pdl(k_color_validate_count, blocks, T, st, P, d, (const uint32_t*)d.colorsA);
+    launch_pdl(k_color_scan, 1, 32, st, d);
+    launch_pdl(k_color_scatter, blocks, T, st, P, d, (const uint32_t*)d.colorsA);
 }
 
 // ---------------------------------------------------------------------------

@@ -53,6 +53,20 @@ def test_coloring_sizes(cuda_lib, oracle_lib, count):
     _run(pile(count), oracle_lib, 12, every=6)
 
 
+@pytest.mark.parametrize("count,length", [(10239, 12), (10240, 12), (10240, 40)])
+def test_coloring_passes(cuda_lib, oracle_lib, count, length):
+    """Rows of touching boxes, all of one color at first: a pass settles one box
+    of each row.  With the ground, 10,239 boxes are the last scene of the eight-CTA
+    cluster; above it the passes are launched, rows of 12 settle in the passes that
+    follow the launched eight, and rows of 40 only in the repair."""
+    s = PhysicsScene("rows")
+    demos.add_ground(s, friction=0.6)
+    for k in range(count):
+        s.add_body((0.3, 0.3, 0.3), 500.0, 0.6, ((k % length) * 0.298, (k // length) * 0.5, 0.15))
+    s.settings.iterations = 3
+    _run(s, oracle_lib, 3)
+
+
 def falling(count):
     """Four layers of boxes, each shifted against the one below: one color in
     the air (up to frame 16), four once they have landed (from frame 32)."""
