@@ -8,7 +8,7 @@ GPU: the failures are counters read back on the host."""
 import pytest
 
 from avbd_b200 import abi, demos
-from avbd_b200.solver import RuntimeFailure
+from avbd_b200.solver import GPUSolver, RuntimeFailure
 
 from test_gpu_parity import compare_state, pair
 
@@ -63,3 +63,18 @@ def test_planar_dat_pair_capacity(cuda_lib, oracle_lib):
     assert o.runtime_failure() == abi.FAIL_PLANAR_DAT_PAIR_CAPACITY
     assert g.counters().dat_pairs > 4
     assert_sticky(g, abi.FAIL_PLANAR_DAT_PAIR_CAPACITY)
+
+
+def test_another_calls_error_is_not_a_frames(cuda_lib):
+    """A solver whose creation ran out of device memory leaves an error behind on
+    the host thread; frames and readbacks of a sound solver do not report it."""
+    scene = demos.rigid_stack_scene(count=10)
+    g = GPUSolver(scene)
+    g.step(1)
+    before = g.positions()[0]
+    with pytest.raises(RuntimeError):
+        GPUSolver(scene, max_pairs_per_body=50_000_000)      # 0.4 TB of manifolds
+    g.step(1)
+    g.synchronize()
+    assert not (g.positions()[0] == before).all()
+    assert g.runtime_failure() == abi.FAIL_NONE
