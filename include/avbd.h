@@ -376,7 +376,8 @@ typedef struct avbd_profile {
     uint32_t color_lanes[64];     /* primal variant of each static color's
                                    * lean particles: 8, 16 or 32 lanes per
                                    * body or AVBD_PRIMAL_VARIANT_STAGED (the
-                                   * default)                              */
+                                   * default; particles whose elements fit no
+                                   * staged block then take 32 lanes)      */
     /* dynamic coloring: block shape of the rigid primal's grid-stride
      * launch, chosen per body-count bucket (floor(log2(dynamic bodies)))
      * by timing candidate shapes on the first frames of the first solver
@@ -389,9 +390,9 @@ typedef struct avbd_profile {
 /* Pin the per-color primal variant of a static-palette scene: 8, 16 or 32
  * lanes per body (grouped kernel), AVBD_PRIMAL_VARIANT_STAGED (a block's
  * element records and positions staged in shared memory), or 0 for the
- * default, the staged kernel wherever a body's elements fit a block.  Every
- * variant computes the same floats.  No counterpart in the reference, whose
- * primal has one launch shape (primal_particles_split,
+ * default, the staged kernel wherever a body's elements fit a block (32 lanes
+ * elsewhere).  Every variant computes the same floats.  No counterpart in the
+ * reference, whose primal has one launch shape (primal_particles_split,
  * 40_solver.metal:1544-1686).                                              */
 enum { AVBD_PRIMAL_VARIANT_AUTO = 0, AVBD_PRIMAL_VARIANT_STAGED = 1 };
 int avbd_set_primal_variant(avbd_solver* solver, uint32_t variant);

@@ -87,3 +87,22 @@ def test_primal_variant_rejects_unknown(cuda_lib):
     g.set_primal_variant(abi.PRIMAL_VARIANT_AUTO)
     g.step(6)                                   # four tuning frames, then graphs
     assert all(v in (1, 8, 16, 32) for v in g.profile()["color_lanes"][:4])
+
+
+def test_oversize_particle_takes_a_warp(cuda_lib):
+    """A hub of more tets than a staged block holds is not left to 8 lanes."""
+    import time
+
+    def frame(variant):
+        g = GPUSolver(tet_fan_scene(600))
+        g.set_primal_variant(variant)
+        best = math.inf
+        for _ in range(4):
+            g.synchronize()
+            t = time.perf_counter()
+            g.step(10)
+            g.synchronize()
+            best = min(best, time.perf_counter() - t)
+        return best
+
+    assert frame(abi.PRIMAL_VARIANT_AUTO) < 0.8 * frame(8)
