@@ -2256,22 +2256,15 @@ void launch_residual(const Params& P, const DevPtrs& d, const Sizes& z, float* p
         // once, writing the per-body values to perBody
         DevPtrs g = d;
         g.learnResidBodies = perBody;
-        auto run = [&](uint32_t color, uint32_t count, uint32_t lanes) {
-            const uint32_t w = lanes <= 8 ? 8u : (lanes <= 16 ? 16u : 32u);
-            const uint32_t blocks = (count * w + 127) / 128;
-            if (z.particleFastPath) {
-                if (w == 8) launch_pdl(k_primal_group<8, false, false, true>, blocks, 128, st, P, g, color, count, 0u, NO_HOST_START);
-                else if (w == 16) launch_pdl(k_primal_group<16, false, false, true>, blocks, 128, st, P, g, color, count, 0u, NO_HOST_START);
-                else launch_pdl(k_primal_group<32, false, false, true>, blocks, 128, st, P, g, color, count, 0u, NO_HOST_START);
-            } else if (P.cloth || P.ogc) {
-                launch_pdl(k_primal_group<32, true, true, true>, (count * 32 + 127) / 128, 128, st, P, g, color, count, 0u, NO_HOST_START);
-            } else {
-                launch_pdl(k_primal_group<32, true, false, true>, (count * 32 + 127) / 128, 128, st, P, g, color, count, 0u, NO_HOST_START);
-            }
-        };
         // every body at once: 8 lanes per body keep the most bodies in
         // flight (measured faster than 16 or 32 for the 13,824-body soft cube)
-        run(0u, n, 8u);
+        const uint32_t blocks = (n * 32 + 127) / 128;
+        if (z.particleFastPath)
+            launch_pdl(k_primal_group<8, false, false, true>, (n * 8 + 127) / 128, 128, st, P, g, 0u, n, 0u, NO_HOST_START);
+        else if (P.cloth || P.ogc)
+            launch_pdl(k_primal_group<32, true, true, true>, blocks, 128, st, P, g, 0u, n, 0u, NO_HOST_START);
+        else
+            launch_pdl(k_primal_group<32, true, false, true>, blocks, 128, st, P, g, 0u, n, 0u, NO_HOST_START);
     } else if (n) {
         // rigid bodies present: particles through the primal's particle
         // terms, rigid bodies through the generic stamps, 8 lanes per body
