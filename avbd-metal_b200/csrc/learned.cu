@@ -555,9 +555,10 @@ static_assert(SMEM <= 227 * 1024, "shared memory of a training CTA");
 // TMEM columns: D (layer outputs, input gradients) | dW3 | dW2 | dW1 | dW4^T
 constexpr uint32_t TD = 0, TW3 = 128, TW2 = 256, TW1 = 384, TW4 = 416, TMEM_COLS = 512;
 // a CTA's partial gradient (floats): dW3, dW2, dW1 as [in][out], dW4 as
-// [out][in], the biases, the loss; the lane of every TMEM row is contiguous
+// [out][in], the biases, the loss, 1 where all of this is valid; the lane of every
+// TMEM row is contiguous
 constexpr uint32_t P3 = 0, P2 = P3 + 128 * 128, P1 = P2 + 128 * 128, P4 = P1 + 32 * 128, PB1 = P4 + 16 * 128,
-                   PB2 = PB1 + 128, PB3 = PB2 + 128, PB4 = PB3 + 128, PL = PB4 + 16, PART = PL + 16;
+                   PB2 = PB1 + 128, PB3 = PB2 + 128, PB4 = PB3 + 128, PL = PB4 + 16, PV = PL + 1, PART = PL + 16;
 
 // K-major descriptor (second 8-column K chunk 128 B on) and MN-major one of
 // the same image: 8-column groups 128 B apart, 8-row (K) groups `sbo` apart
@@ -584,7 +585,7 @@ __device__ __forceinline__ float column_sums(float (&v)[32], uint32_t lane) {
 
 __global__ void __launch_bounds__(tt::THREADS, 1)
 k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, const float* __restrict__ Xg,
-             const float* __restrict__ Tg, uint32_t n, float* __restrict__ part, uint32_t* status) {
+             const float* __restrict__ Tg, uint32_t n, float* __restrict__ part, uint32_t* status, bool issue) {
     using namespace mlp;
     extern __shared__ __align__(128) unsigned char sm[];
     const uint32_t t = threadIdx.x, warp = tc::uniform(t >> 5), lane = t & 31u;
@@ -688,8 +689,8 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
             *reinterpret_cast<uint4*>(sm + tt::X + tc::off(row, c, tt::SBO32)) = pack8(v);
         }
         publish();
-        // forward
-        if (warp == 0 && tc::elect_one()) {
+        // forward (issue = false only in the timeout test)
+        if (warp == 0 && issue && tc::elect_one()) {
             for (uint32_t s = 0; s < DIN / 16; s++)
                 tc::mma(tmem + tt::TD, tt::kmajor(sbase + tt::X + 256u * s, tt::SBO32),
                         tt::kmajor(sbase + tc::W1 + 256u * s, tc::SBO_K32), tc::idesc(128, 128), s > 0);
@@ -848,14 +849,19 @@ k_train_tile(const float* __restrict__ prm, const float* __restrict__ norm, cons
             if (t < USED_OUT) s = ((red[t] + red[8 + t]) + red[16 + t]) + red[24 + t];
             out[tt::PB4 + t] = s;
         }
-        if (t == 32) out[tt::PL] = ((red[USED_OUT] + red[8 + USED_OUT]) + red[16 + USED_OUT]) + red[24 + USED_OUT];
+        if (t == 32) {
+            out[tt::PL] = ((red[USED_OUT] + red[8 + USED_OUT]) + red[16 + USED_OUT]) + red[24 + USED_OUT];
+            out[tt::PV] = 1.0f;
+        }
     } else {
-        // products still in flight, the weight gradients' included (bounded waits)
         if (t == 0) {
             atomicCAS(status, 0u, (uint32_t)AVBD_FAIL_WAIT_TIMEOUT);
-            tc::commit(bar);
+            out[tt::PV] = 0.0f;
         }
-        if (tc::wait(bar, phase ^ 1u)) tc::wait(bar, phase);
+        if (issue) {                    // products still in flight, the weight gradients' included (bounded waits)
+            if (t == 0) tc::commit(bar);
+            if (tc::wait(bar, phase ^ 1u)) tc::wait(bar, phase);
+        }
     }
     tc::fence_before();
     __syncthreads();
@@ -881,6 +887,7 @@ __global__ void __launch_bounds__(256) k_train_reduce(const float* part, uint32_
     const uint32_t t = threadIdx.x, b = blockIdx.x;
     uint32_t src, dst = 0xFFFFFFFFu;
     const bool turn = b < B1;
+    bool idle = false;
     if (turn) {
         const uint32_t q = b < B3 ? b : (b < B2 ? b - B3 : b - B2);
         const uint32_t cols = b < B2 ? 128u : 32u, i0 = (q >> 2) * 8u, o0 = (q & 3u) * 32u;
@@ -896,9 +903,11 @@ __global__ void __launch_bounds__(256) k_train_reduce(const float* part, uint32_
         else if (i < 256) dst = OB2 + i - 128u;
         else if (i < 384) dst = OB3 + i - 256u;
         else if (i < 400) dst = OB4 + i - 384u;
-        else if (i > 400) return;                             // i == 400: the loss
+        else idle = i > 400;                                  // i == 400: the loss
     }
     pdl_wait();
+    // a CTA that gave up a wait left no partial: nothing is stored
+    if (__syncthreads_or(t < parts && part[(size_t)t * tt::PART + tt::PV] != 1.0f) || idle) return;
     float s = 0.0f;
     uint32_t z = 0;
     for (; z + 8 <= parts; z += 8) {
@@ -986,10 +995,10 @@ void train_attributes() {
 // Forward, loss and partial gradients; then their sum into `grad` (a == null)
 // or Adam on the parameters.
 void forward_backward(const float* prm, const float* norm, const float* X, const float* T, uint32_t B, const Work& w,
-                      float* grad, const AdamArgs* a, float* loss, cudaStream_t st) {
+                      float* grad, const AdamArgs* a, float* loss, bool issue, cudaStream_t st) {
     train_attributes();
     const uint32_t ctas = train_ctas(B);
-    k_train_tile<<<ctas, tt::THREADS, tt::SMEM, st>>>(prm, norm, X, T, B, w.part, w.status);
+    k_train_tile<<<ctas, tt::THREADS, tt::SMEM, st>>>(prm, norm, X, T, B, w.part, w.status, issue);
     if (a) launch_pdl(k_train_reduce<true>, kTrainReduceBlocks, 256, st, (const float*)w.part, ctas, B, (float*)nullptr, *a, loss);
     else if (grad || loss)
         launch_pdl(k_train_reduce<false>, kTrainReduceBlocks, 256, st, (const float*)w.part, ctas, B, grad, AdamArgs{}, loss);
@@ -1293,12 +1302,12 @@ static int workspace_status(const Work& w, cudaStream_t st) {
 
 static int gradients(const float* params, const float* norm, const float* features, const float* targets,
                      uint32_t batch, void* workspace, float* grad_out, const AdamArgs* adam, float* loss_out,
-                     cudaStream_t st) {
+                     bool issue, cudaStream_t st) {
     if (!params || !norm || !features || !targets || !workspace || batch == 0) return AVBD_ERR_INVALID_ARGUMENT;
     Work w{};
     work_layout(batch, static_cast<char*>(workspace), &w);
     if (!adam) cudaMemsetAsync(w.status, 0, sizeof(uint32_t), st);
-    forward_backward(params, norm, features, targets, batch, w, grad_out, adam, loss_out, st);
+    forward_backward(params, norm, features, targets, batch, w, grad_out, adam, loss_out, issue, st);
     if (cudaGetLastError() != cudaSuccess) return AVBD_ERR_RUNTIME_FAILURE;
     // a tensor-core wait that gave up fails the call (the kernel latches it
     // in the workspace's status word); the training step stays asynchronous
@@ -1307,7 +1316,7 @@ static int gradients(const float* params, const float* norm, const float* featur
 
 int avbd_mlp_gradients(const float* params, const float* norm, const float* features, const float* targets,
                        uint32_t batch, void* workspace, float* grad_out, float* loss_out, void* stream) {
-    return gradients(params, norm, features, targets, batch, workspace, grad_out, nullptr, loss_out,
+    return gradients(params, norm, features, targets, batch, workspace, grad_out, nullptr, loss_out, true,
                      static_cast<cudaStream_t>(stream));
 }
 
@@ -1318,9 +1327,9 @@ int avbd_mlp_workspace_status(const void* workspace, uint32_t batch, void* strea
     return workspace_status(w, static_cast<cudaStream_t>(stream));
 }
 
-int avbd_mlp_train_step(float* params, const float* norm, const float* features, const float* targets,
-                        uint32_t batch, float* adam_m, float* adam_v, uint32_t step, float lr, void* workspace,
-                        float* loss_out, void* stream) {
+static int train_step(float* params, const float* norm, const float* features, const float* targets, uint32_t batch,
+                      float* adam_m, float* adam_v, uint32_t step, float lr, void* workspace, float* loss_out,
+                      void* stream, bool issue) {
     if (!params || !adam_m || !adam_v || step == 0) return AVBD_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (workspace && batch && step == 1) {
@@ -1329,7 +1338,22 @@ int avbd_mlp_train_step(float* params, const float* norm, const float* features,
         cudaMemsetAsync(w.status, 0, sizeof(uint32_t), st);   // sticky from here on
     }
     const AdamArgs adam{params, adam_m, adam_v, step, lr, 0.9f, 0.999f, 1e-8f};
-    return gradients(params, norm, features, targets, batch, workspace, nullptr, &adam, loss_out, st);
+    return gradients(params, norm, features, targets, batch, workspace, nullptr, &adam, loss_out, issue, st);
+}
+
+int avbd_mlp_train_step(float* params, const float* norm, const float* features, const float* targets,
+                        uint32_t batch, float* adam_m, float* adam_v, uint32_t step, float lr, void* workspace,
+                        float* loss_out, void* stream) {
+    return train_step(params, norm, features, targets, batch, adam_m, adam_v, step, lr, workspace, loss_out, stream,
+                      true);
+}
+
+int avbd_mlp_train_step_wait_timeout_for_testing(float* params, const float* norm, const float* features,
+                                                 const float* targets, uint32_t batch, float* adam_m, float* adam_v,
+                                                 uint32_t step, float lr, void* workspace, float* loss_out,
+                                                 void* stream) {
+    return train_step(params, norm, features, targets, batch, adam_m, adam_v, step, lr, workspace, loss_out, stream,
+                      false);
 }
 
 static int mlp_infer(const float* params, const float* norm, const float* features, uint32_t n, float* out,

@@ -448,7 +448,8 @@ int avbd_get_residual_trace(avbd_solver* solver, double* out, uint32_t n);
  * status word in the workspace.  avbd_mlp_gradients synchronises `stream`
  * and fails on it; avbd_mlp_train_step stays asynchronous (the word is
  * cleared at step 1 and sticky afterwards) and avbd_mlp_workspace_status
- * synchronises and reports it.                                             */
+ * synchronises and reports it.  A call whose wait gave up stores neither
+ * gradient nor loss and leaves parameters and moments as they were.        */
 uint32_t avbd_mlp_param_count(void);
 size_t avbd_mlp_workspace_bytes(uint32_t batch);
 int avbd_mlp_gradients(const float* params, const float* norm, const float* features,
@@ -458,6 +459,13 @@ int avbd_mlp_train_step(float* params, const float* norm, const float* features,
                         const float* targets, uint32_t batch, float* adam_m, float* adam_v,
                         uint32_t step, float lr, void* workspace, float* loss_out, void* stream);
 int avbd_mlp_workspace_status(const void* workspace, uint32_t batch, void* stream);
+/* Test of the training kernel's bounded wait: a step with no tensor-core work
+ * issued, whose wait runs out after about one second.  No counterpart in the
+ * reference.                                                               */
+int avbd_mlp_train_step_wait_timeout_for_testing(float* params, const float* norm, const float* features,
+                                                 const float* targets, uint32_t batch, float* adam_m,
+                                                 float* adam_v, uint32_t step, float lr, void* workspace,
+                                                 float* loss_out, void* stream);
 /* Inference over n feature rows into out[n][6] on the tensor cores
  * (tcgen05.mma, accumulators in tensor memory); synchronises `stream` and
  * returns AVBD_ERR_RUNTIME_FAILURE if the kernel's bounded wait for its MMA

@@ -6,7 +6,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from avbd_b200 import learned
+from avbd_b200 import abi, learned
 from avbd_b200.solver import load_library
 
 pytestmark = pytest.mark.gpu
@@ -60,3 +60,37 @@ def test_gradients_of_unaligned_inputs(cuda_lib):
     assert rc == 0
     assert float(loss.item()) == want_loss
     assert np.array_equal(grad.cpu().numpy(), want)
+
+
+def _device_step(B):
+    """(tensors, arguments of a training step up to the step number) of a fresh network."""
+    import torch
+    p, norm, X, T = _case(B)
+    t = {"prm": p, "norm": norm, "x": X, "t": T, "m": np.zeros_like(p), "v": np.zeros_like(p)}
+    t = {k: torch.from_numpy(np.ascontiguousarray(v, np.float32)).cuda() for k, v in t.items()}
+    # a workspace with another step's partial gradients in it
+    t["ws"] = torch.ones(load_library().avbd_mlp_workspace_bytes(B) // 4, dtype=torch.float32, device="cuda")
+    t["loss"] = torch.full((1,), 7.0, device="cuda")
+    return t, [t[k].data_ptr() for k in ("prm", "norm", "x", "t")] + [B] + [t[k].data_ptr() for k in ("m", "v")]
+
+
+@pytest.mark.parametrize("B", [100, 1000])
+def test_step_whose_wait_gave_up_changes_nothing(cuda_lib, B):
+    import torch
+    lib = load_library()
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    t, args = _device_step(B)
+    before = t["prm"].clone()
+    tail = (C.c_float(1e-2), t["ws"].data_ptr(), t["loss"].data_ptr(), stream)
+    assert lib.avbd_mlp_train_step_wait_timeout_for_testing(*args, 1, *tail) == 0
+    assert lib.avbd_mlp_workspace_status(t["ws"].data_ptr(), B, stream) == abi.ERR_RUNTIME_FAILURE
+    assert torch.equal(t["prm"], before) and not t["m"].any() and not t["v"].any()
+    assert float(t["loss"]) == 7.0
+    # the device and the workspace are as good as new
+    assert lib.avbd_mlp_train_step(*args, 1, *tail) == 0
+    assert lib.avbd_mlp_workspace_status(t["ws"].data_ptr(), B, stream) == 0
+    fresh, fresh_args = _device_step(B)
+    assert lib.avbd_mlp_train_step(*fresh_args, 1, C.c_float(1e-2), fresh["ws"].data_ptr(), fresh["loss"].data_ptr(),
+                                   stream) == 0
+    assert all(torch.equal(t[k], fresh[k]) for k in ("prm", "m", "v", "loss"))
+    assert not torch.equal(t["prm"], before)
