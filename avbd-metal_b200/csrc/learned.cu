@@ -959,10 +959,12 @@ __global__ void k_mirror_umma(const float* prm, unsigned char* img) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Host side of training.  Workspace for a batch of B rows: the status word
-// (256 bytes), then one partial gradient per CTA of k_train_tile.
+// Host side of training.  Workspace for a batch of B rows: the status words
+// (256 bytes: training's at 0, an inference's at 128), then one partial
+// gradient per CTA of k_train_tile.
 // ---------------------------------------------------------------------------
 namespace {
+constexpr uint32_t kInferStatus = 32;   // words
 inline uint32_t blocks(size_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t); }
 
 // one 128-row tile per CTA while the batch has no more tiles than the device
@@ -1365,7 +1367,8 @@ static int mlp_infer(const float* params, const float* norm, const float* featur
          reinterpret_cast<uintptr_t>(params) | reinterpret_cast<uintptr_t>(norm)) & 15u)
         return AVBD_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    uint32_t* status = static_cast<uint32_t*>(workspace);
+    // not the training status word, which is sticky in a shared workspace
+    uint32_t* status = static_cast<uint32_t*>(workspace) + kInferStatus;
     cudaMemsetAsync(status, 0, sizeof(uint32_t), st);
     if (issue) {
         launch_mlp_infer(nullptr, params, norm, features, n, out, status, st);

@@ -94,3 +94,16 @@ def test_step_whose_wait_gave_up_changes_nothing(cuda_lib, B):
                                    stream) == 0
     assert all(torch.equal(t[k], fresh[k]) for k in ("prm", "m", "v", "loss"))
     assert not torch.equal(t["prm"], before)
+
+
+def test_inference_keeps_a_shared_workspaces_training_status(cuda_lib):
+    import torch
+    lib, B = load_library(), 1000
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    t, args = _device_step(B)
+    tail = (C.c_float(1e-2), t["ws"].data_ptr(), t["loss"].data_ptr(), stream)
+    assert lib.avbd_mlp_train_step_wait_timeout_for_testing(*args, 1, *tail) == 0
+    out = torch.zeros(B, learned.USED, device="cuda")
+    assert lib.avbd_mlp_infer(*(t[k].data_ptr() for k in ("prm", "norm", "x")), B, out.data_ptr(), t["ws"].data_ptr(),
+                              stream) == 0
+    assert lib.avbd_mlp_workspace_status(t["ws"].data_ptr(), B, stream) == abi.ERR_RUNTIME_FAILURE
