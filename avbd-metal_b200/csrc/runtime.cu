@@ -108,6 +108,16 @@ struct avbd_snapshot {
     uint64_t frame;
 };
 
+// false when the device has no room; the failure is the return value alone and
+// does not stay behind as the host thread's last error, which later calls read
+template <typename T>
+static bool device_alloc(T** p, size_t bytes) {
+    if (cudaMalloc(reinterpret_cast<void**>(p), bytes) == cudaSuccess) return true;
+    *p = nullptr;
+    cudaGetLastError();
+    return false;
+}
+
 struct avbd_solver {
     HostScene H;
     DevPtrs d{};
@@ -218,7 +228,7 @@ struct avbd_solver {
     bool alloc(T*& ptr, size_t count, const char* label, bool snapshot = false) {
         size_t bytes = sizeof(T) * (count ? count : 1);
         void* p = nullptr;
-        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        if (!device_alloc(&p, bytes)) {
             error = std::string("allocation failed: ") + label;
             return false;
         }
@@ -990,7 +1000,7 @@ struct avbd_solver {
             if (stage) cudaFree(stage);
             stage = nullptr;
             stageBytes = 0;
-            if (cudaMalloc(&stage, bytes) != cudaSuccess) return nullptr;
+            if (!device_alloc(&stage, bytes)) return nullptr;
             stageBytes = bytes;
         }
         return stage;
@@ -1476,7 +1486,7 @@ int avbd_set_skin_bindings(avbd_solver* s, const avbd_skin_binding* b, uint32_t 
     if (s->skin) { cudaFree(s->skin); s->skin = nullptr; }
     s->numSkin = 0;
     if (n == 0) return AVBD_OK;
-    if (cudaMalloc(&s->skin, sizeof(SkinBinding) * (size_t)n) != cudaSuccess) return AVBD_ERR_ALLOC_FAILED;
+    if (!device_alloc(&s->skin, sizeof(SkinBinding) * (size_t)n)) return AVBD_ERR_ALLOC_FAILED;
     if (cudaMemcpy(s->skin, host.data(), sizeof(SkinBinding) * (size_t)n, cudaMemcpyHostToDevice) != cudaSuccess)
         return AVBD_ERR_ALLOC_FAILED;
     s->numSkin = n;
@@ -1526,8 +1536,8 @@ int avbd_render_pusht_obs(avbd_solver* s, const avbd_pusht_env* envs, uint32_t n
             s->pushtDev = nullptr;
             s->pushtShapes = nullptr;
             s->pushtCap = 0;
-            if (cudaMalloc(&s->pushtDev, sizeof(PushTDev) * (size_t)num_envs) != cudaSuccess ||
-                cudaMalloc(&s->pushtShapes, PUSHT_RECORD * sizeof(float4) * (size_t)num_envs) != cudaSuccess)
+            if (!device_alloc(&s->pushtDev, sizeof(PushTDev) * (size_t)num_envs) ||
+                !device_alloc(&s->pushtShapes, PUSHT_RECORD * sizeof(float4) * (size_t)num_envs))
                 return AVBD_ERR_ALLOC_FAILED;
             s->pushtCap = num_envs;
         }

@@ -66,14 +66,15 @@ def test_planar_dat_pair_capacity(cuda_lib, oracle_lib):
 
 
 def test_another_calls_error_is_not_a_frames(cuda_lib):
-    """A solver whose creation ran out of device memory leaves an error behind on
-    the host thread; frames and readbacks of a sound solver do not report it."""
+    """A solver whose creation ran out of device memory leaves no error behind on
+    the host thread: uploads, frames and readbacks of a sound solver go on."""
     scene = demos.rigid_stack_scene(count=10)
     g = GPUSolver(scene)
     g.step(1)
     before = g.positions()[0]
     with pytest.raises(RuntimeError):
         GPUSolver(scene, max_pairs_per_body=50_000_000)      # 0.4 TB of manifolds
+    g.set_positions(before[:, :3] + [0.0, 0.0, 0.5])
     g.step(1)
     g.synchronize()
     assert not (g.positions()[0] == before).all()
