@@ -1443,15 +1443,18 @@ __device__ __forceinline__ void tet_core(float3 x0, float3 x1, float3 x2, float3
     t.kind = TERM_TET;
 }
 __device__ __forceinline__ void tet_terms(const DevPtrs& d, const TetGPU& tt, uint32_t self, ParticleTerms& t) {
+    // the positions first: the division below must not stand before their loads
+    const float3 x0 = xyz(d.posLin[tt.ids.x]), x1 = xyz(d.posLin[tt.ids.y]);
+    const float3 x2 = xyz(d.posLin[tt.ids.z]), x3 = xyz(d.posLin[tt.ids.w]);
     const float muV = tt.r1.w, lamV = tt.r2.w;
+    const float alphaT = 1.0f + muV / mx(lamV, 1e-9f);
     const float3 m0 = xyz(tt.r0), m1 = xyz(tt.r1), m2 = xyz(tt.r2);
     float3 w;
     if (self == tt.ids.y) w = m0;
     else if (self == tt.ids.z) w = m1;
     else if (self == tt.ids.w) w = m2;
     else w = -mk3(m0.x + m1.x + m2.x, m0.y + m1.y + m2.y, m0.z + m1.z + m2.z);
-    tet_core(xyz(d.posLin[tt.ids.x]), xyz(d.posLin[tt.ids.y]), xyz(d.posLin[tt.ids.z]), xyz(d.posLin[tt.ids.w]), m0,
-             m1, m2, muV, lamV, 1.0f + muV / mx(lamV, 1e-9f), w, muV * dot(w, w), t);
+    tet_core(x0, x1, x2, x3, m0, m1, m2, muV, lamV, alphaT, w, muV * dot(w, w), t);
 }
 
 // Terms of a one-point manifold from its record and its bodies' poses.
