@@ -1,12 +1,11 @@
 """Every variant of the static-palette primal against the oracle, bit for bit.
 
-The autotuner picks per color between the grouped kernel (8, 16 or 32 lanes
-per body) and the staged kernel (the block's adjacency entries evaluated
-densely into shared memory, then folded per body by 8 lanes).  Each variant
-folds the entries of a body in the order of the reference's 8-lane SIMD
-group (primal_particles_split, 40_solver.metal:1544-1686), so each must
-reproduce the oracle's frames exactly; here every variant is pinned for
-the whole run instead of only for the tuner's timing frame.
+A color's lean particles run in the staged kernel (a block's element records
+and positions in shared memory, folded per body by 8 lanes) or, pinned, in the
+grouped kernel with 8, 16 or 32 lanes per body.  Each variant folds the entries
+of a body in the order of the reference's 8-lane SIMD group
+(primal_particles_split, 40_solver.metal:1544-1686), so each must reproduce the
+oracle's frames exactly; here every variant is pinned for the whole run.
 """
 import math
 
@@ -24,7 +23,7 @@ VARIANTS = [abi.PRIMAL_VARIANT_STAGED, 8, 16, 32]
 
 def tet_fan_scene(tets: int = 600, pinned: bool = False) -> PhysicsScene:
     """One hub particle shared by `tets` tets (600 adjacency entries: more
-    than a staged block holds, so the fold also evaluates entries inline)."""
+    than a staged block holds, so the grouped kernel takes the hub)."""
     s = PhysicsScene("tet-fan")
     s.settings.iterations = 10
     hub = s.add_particle(0.02, 0.05, position=(0.0, 0.0, 2.0))
@@ -85,8 +84,8 @@ def test_primal_variant_rejects_unknown(cuda_lib):
     with pytest.raises(Exception):
         g.set_primal_variant(12)
     g.set_primal_variant(abi.PRIMAL_VARIANT_AUTO)
-    g.step(6)                                   # four tuning frames, then graphs
-    assert all(v in (1, 8, 16, 32) for v in g.profile()["color_lanes"][:4])
+    g.step(6)
+    assert all(v == abi.PRIMAL_VARIANT_STAGED for v in g.profile()["color_lanes"][:4])
 
 
 def test_oversize_particle_takes_a_warp(cuda_lib):

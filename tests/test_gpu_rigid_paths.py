@@ -1,8 +1,9 @@
 """The paths that a rigid or mixed frame takes by its size, bit for bit against
-the oracle: one CTA, four, eight or a launch per color for the iterations; one
-block or a cluster for the coloring; a frame that needs more colors than its
-graph was built for; manifolds of one to eight points shared out to the lanes;
-and, for particles, elements that do not fit the staged tables."""
+the oracle: one CTA, four, eight or sixteen or a launch per color for the
+iterations; one block, a cluster or launched passes for the coloring; a frame
+that needs more colors than its graph was built for; manifolds of one to eight
+points shared out to the lanes; and, for particles, colors of more blocks than
+the device holds and elements that do not fit the staged tables."""
 import math
 
 import numpy as np
@@ -41,7 +42,7 @@ def pile(count, layers=4):
     return s
 
 
-@pytest.mark.parametrize("count", [1, 32, 33, 64, 65, 128, 129, 513])
+@pytest.mark.parametrize("count", [1, 32, 33, 64, 65, 128, 129, 300, 511, 512, 513])
 def test_iteration_paths(cuda_lib, oracle_lib, count):
     _run(pile(count), oracle_lib, 24, every=4)
 
@@ -120,6 +121,14 @@ def test_more_colors_than_launched(cuda_lib, oracle_lib, count):
 def test_shapes_between_the_paths(cuda_lib, oracle_lib):
     for count in (60, 140):
         _run(demos.shapes_scene(seed=3, count=count), oracle_lib, 60, every=10)
+
+
+def test_staged_large_color(cuda_lib, oracle_lib):
+    """Above 444 blocks of 16 bodies a color does not take its contacts ahead."""
+    s = demos.soft_cube_scene(n=26)
+    s.settings.iterations = 4
+    g = _run(s, oracle_lib, 9, every=3)
+    assert max(g.counters().color_counts) > 444 * 16
 
 
 def rods(levers):
