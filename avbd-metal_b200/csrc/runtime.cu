@@ -1774,7 +1774,8 @@ int avbd_set_primal_variant(avbd_solver* s, uint32_t variant) {
         return AVBD_ERR_INVALID_ARGUMENT;
     int rc = s->retire();
     if (rc != AVBD_OK) return rc;
-    for (auto& l : s->H.colorLanes) l = variant ? variant : (uint32_t)AVBD_PRIMAL_STAGED;
+    for (auto& l : s->H.colorLanes)
+        l = variant ? variant : (s->z.dynamicColoring ? 8u : (uint32_t)AVBD_PRIMAL_STAGED);
     s->graphsValid = false;
     return AVBD_OK;
 }

@@ -880,12 +880,14 @@ int upload_scene(const avbd_scene_desc* s, HostScene& H, std::string& err) {
         if (H.shape[b].w >= 0.0f || !pre[b].empty()) { H.particleFastPath = false; break; }
     }
     // The staged kernel solves every static color's lean particles.  Measured
-    // against the grouped kernel's best width, a frame each: soft cube 24^3
-    // 0.575 ms / 0.582, 12^3 0.527 / 0.616, 256^2 cloth 3.20 / 3.64, mixed scene
-    // 3.50 / 3.81.  (Timing the variants launch by launch picked the grouped
-    // one for soft cubes: apart from its neighbours a staged launch shows the
-    // copies that it otherwise makes while the previous color runs.)
-    H.colorLanes.assign(MAX_COLORS, 1);                  // AVBD_PRIMAL_STAGED
+    // against the grouped kernel at the scene's best width, a frame of many
+    // submitted back to back: soft cube 24^3 0.574 ms / 0.728, 12^3 0.528 / 0.609,
+    // 256^2 cloth 3.20 / 3.65, mixed scene 3.49 / 3.76.  (Timing the variants
+    // launch by launch picked the grouped one for soft cubes: apart from its
+    // neighbours a staged launch shows the copies that it otherwise makes while
+    // the previous color runs.)
+    // (A dynamic coloring's bodies take 8 lanes each.)
+    H.colorLanes.assign(MAX_COLORS, H.dynamicColoring ? 8 : AVBD_PRIMAL_VARIANT_STAGED);
     // launch order of each static color: lean particles, then the rest
     // (bodies are independent within a color, so the order only decides
     // which kernel instance takes a body)

@@ -88,6 +88,14 @@ def test_primal_variant_rejects_unknown(cuda_lib):
     assert all(v == abi.PRIMAL_VARIANT_STAGED for v in g.profile()["color_lanes"][:4])
 
 
+def test_profile_of_a_dynamic_coloring(cuda_lib):
+    """No staged kernel there: every color's bodies take 8 lanes."""
+    g = GPUSolver(demos.box_field_scene(count=600))
+    assert set(g.profile()["color_lanes"]) == {8}
+    g.set_primal_variant(abi.PRIMAL_VARIANT_AUTO)
+    assert set(g.profile()["color_lanes"]) == {8}
+
+
 def test_oversize_particle_takes_a_warp(cuda_lib):
     """A hub of more tets than a staged block holds is not left to 8 lanes."""
     import time
