@@ -193,7 +193,8 @@ void launch_dynamic_coloring(const Params& P, const DevPtrs& d, const Sizes& z, 
 // when known on the host (static palette), else 0xFFFFFFFF (read on device);
 // `lanes` is 8, 16 or 32 lanes per body (grouped kernel) or
 // AVBD_PRIMAL_STAGED (staged kernel: a block's records and positions in shared
-// memory, 8 lanes per body), every choice computing the same floats
+// memory; 32 lanes for the particles that fit no block), every choice computing
+// the same floats
 // `chained`: a grid of this stream's chain has started after the frame's
 // contact lists were complete (false at the head of a chain: the frame's
 // solve, or a trial sweep); `last`: the last color of a sweep.
@@ -209,8 +210,7 @@ void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint
 // and their fixed-order sum (total)
 void launch_residual(const Params& P, const DevPtrs& d, const Sizes& z, float* perBody, double* total,
                      cudaStream_t st);
-// dynamic coloring: colors [first, 64) in one block, after the per-color launches
-// every iteration of a small scene in one thread block
+// every iteration of a small scene in one launch of 1 to 16 CTAs
 void launch_solve_small(const Params& P, const DevPtrs& d, const Sizes& z, uint32_t colorBound,
                         cudaStream_t st);
 void launch_dual(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t st);
@@ -232,7 +232,7 @@ void launch_build_instances(const DevPtrs& d, const uint32_t* ids, const float4*
 void launch_soft_normals(const DevPtrs& d, const uint32_t* surfVerts, const uint32_t* vtStart, const uint32_t* vtCount,
                          const uint32_t* vtList, uint32_t numSurf, float clothScale, float4* out, cudaStream_t st);
 void launch_skin_deform(const float4* posLin, const SkinBinding* b, uint32_t n, float4* out, cudaStream_t st);
-// shapes: 6 float4 of scratch per environment
+// shapes: PUSHT_RECORD float4 of scratch per environment
 constexpr uint32_t PUSHT_RECORD = 11;   // float4 of an environment's shapes: 24 floats, five pixel ranges
 void launch_pusht_obs(const float4* posLin, const float4* posAng, const PushTDev* envs, uint32_t numEnvs,
                       uint32_t res, float4* shapes, uint8_t* out, cudaStream_t st);

@@ -788,7 +788,7 @@ struct avbd_solver {
             return AVBD_ERR_ALLOC_FAILED;
         }
         std::memset(hostLatch, 0, 4 * sizeof(uint32_t));
-        // Small scenes run their whole iteration loop in one thread block.
+        // Small scenes run their whole iteration loop in one launch.
         update_small_solve();
         dyn_tune_setup();
         if (cudaDeviceSynchronize() != cudaSuccess) { error = "device error during upload"; return AVBD_ERR_NO_DEVICE; }

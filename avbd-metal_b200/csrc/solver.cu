@@ -7,11 +7,14 @@
 // primal_particles_split :1544-1684, dual :1729-1906, finalize :2108-2147,
 // diag_error :2189-2229.
 //
-// The primal gives every body of the current color a group of 8 consecutive
-// lanes.  Lane l stamps adjacency entries l, l+8, l+16, ... of the body; the
-// lanes then sum their 6x6 systems with an xor butterfly (offsets 4, 2, 1)
-// and lane 0 solves.  The static part of the adjacency (joints, springs,
-// tets) is built once at upload; only contact entries are rebuilt per frame.
+// Every primal kernel adds a body's entries in the order of the reference's
+// group of 8 lanes: logical lane l takes adjacency entries l, l+8, l+16, ... of
+// the body, and an xor butterfly (offsets 4, 2, 1) sums the lanes.  Who
+// evaluates an entry differs: k_primal and k_solve_small (dynamic coloring,
+// small scenes) deal contact points out to the 8 lanes, k_primal_staged and
+// k_primal_group take particles, k_primal_wide a rigid body per block.  The
+// static part of the adjacency (joints, springs, tets) is built once at upload;
+// only contact entries are rebuilt per frame.
 #include <utility>
 
 #include <atomic>
@@ -1747,13 +1750,16 @@ __device__ __forceinline__ void particle_commit(const Params& P, const DevPtrs& 
     d.posLin[body] = mk4(xyz(pl) + dxLin, mass);
 }
 
-// Primal for one color with LANES consecutive lanes per body (8, 16 or 32,
-// chosen per color from its bodies' adjacency sizes).  Lane p of a group
-// evaluates entry base + p; logical lane l < 8 then folds entries
+// Grouped primal for one color, LANES consecutive lanes per body: the width
+// that a caller pinned, 32 for particles that fit no staged block.  Lane p of a
+// group evaluates entry base + p; logical lane l < 8 then folds entries
 // base + l, base + l + 8, ... in order.  Any LANES gives the same floats.
 // RESID: evaluate instead of solve — lane 0 stores the body's squared
 // right-hand side (the AL gradient) in d.learnResidBodies[slot] and leaves
-// the pose alone (particle-only scenes; called over all colors at once).
+// the pose alone (called over all colors at once).  What bounds it there are
+// dependent loads and, in GENERAL instances, registers: the mixed scene's
+// learned stage, two residuals included, takes 422 us (699 with a called
+// stamp_joint and its 1.5 KB of local memory per thread).
 // GENERAL instances keep four blocks per SM (at most 128 registers): the
 // rigid-body path would otherwise take ~160 registers for every thread and
 // cap large colors at three blocks (measured 7% slower mixed frames).
@@ -1912,9 +1918,9 @@ __device__ __forceinline__ void copy16(void* smem, const void* gmem) {
                  : "memory");
 }
 
-// AHEAD: the block's first manifolds are copied to shared memory as well, their
-// constant parts before the wait, the bodies' poses and the multipliers with
-// the positions: a contact adds its arithmetic to the color instead of four
+// AHEAD: the block's first manifolds are copied to shared memory as well, what
+// the solve does not write before the wait, the bodies' poses and the words that
+// the dual stores to with the positions: a contact adds its arithmetic to the color instead of four
 // dependent trips (2.3 us of the 4.3 us a small color took).
 //
 // LANES = 32 (tet colors of at most STAGED_WIDE bodies): four bodies a block,
@@ -2218,9 +2224,10 @@ void launch_primal_color(const Params& P, const DevPtrs& d, const Sizes& z, uint
             // waits first and does not overlap what precedes it, and no later
             // grid starts before it has started.
             // Colors whose blocks all fit on the device at once are chains of
-            // latency and take their contacts ahead (12^3 soft cube 0.621 ->
-            // 0.547 ms a frame); for larger ones the registers and shared memory
-            // cost more (mixed scene 3.41 -> 3.62 ms, cloth 3.14 -> 3.30).
+            // latency and take their contacts ahead (frames submitted back to
+            // back: 12^3 soft cube 0.621 -> 0.547 ms); for larger ones the
+            // registers and shared memory cost more (mixed scene 3.41 -> 3.62 ms,
+            // cloth 3.14 -> 3.30).
             auto go = [&](auto kernel) {
                 launch_chain(kernel, chained, blocks, kStagedThreads, smem, st, P, d, b0, chained);
             };
@@ -2466,8 +2473,10 @@ void launch_dual(const Params& P, const DevPtrs& d, const Sizes& z, cudaStream_t
 // CTA of 256 threads in parentheses), a frame: 512 piled shapes 0.530 ms /
 // 0.563 (2.06), 130 shapes 0.446 / 0.512, 400 boxes 0.226 / 0.243, 100 boxes
 // 0.219 in eight CTAs (0.574); above 512 bodies an SM holds too many.  Particles
-// of a static palette leave at SMALL_PARTICLES, where the staged launches win
-// (512 of them 0.277 ms / 0.491 here).
+// of a static palette leave at SMALL_PARTICLES, where the staged launches win or
+// tie: soft cubes of 64 / 216 / 512 particles 0.250 / 0.253 / 0.239 ms (one CTA
+// of 256 threads 0.337 / 0.488 / 0.939), ropes of 33 / 64 / 128 0.213 / 0.222 /
+// 0.219 (0.208 / 0.221 / 0.322); a cube of 27 takes 0.304 here.
 // ---------------------------------------------------------------------------
 constexpr int kSmallThreads = 512;
 constexpr uint32_t kSmallSlots = kIncWords * kSmallThreads;      // floats of dynamic shared memory

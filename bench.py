@@ -669,7 +669,7 @@ def run_ours(args, world, rank, local):
             "clocks": clock, "e2e": e2e,
             "gpu_launches": int(kernels_per_frame * K),
             "roofline": {"bound": "hbm",
-                         "kernel": "per-color block-descent primal (k_primal_group lean particles, k_primal_wide rigid and joint-carrying bodies beside them, k_primal_staged where tuned; k_primal / k_solve_small for dynamic coloring and small scenes)",
+                         "kernel": "per-color block-descent primal (k_primal_staged lean particles, k_primal_wide rigid and joint-carrying bodies beside them; k_primal / k_solve_small for dynamic coloring and small scenes)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": (f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)" if peak_kind == "measured"
                                          else "fallback 6.65 TB/s"),
