@@ -177,9 +177,9 @@ __device__ __forceinline__ void heading(float4 q, float& cs, float& sn) {
 // of the coordinates; a pixel outside it cannot pass the shape's test.  A
 // bound that is not finite (an empty window, a lost pose) covers everything.
 //
-// What bounds it: the 3 bytes a pixel of output and a call's two launches;
-// 4096 environments of 64 x 64 in 24.7 us a call (41.2 us when every quad of
-// pixels ran five bounding-circle tests).
+// What bounds it: issue slots (0.6 of them used) and the barriers between a
+// tile's fill, its shapes and its copy; 4096 environments of 64 x 64 in 24.7 us a
+// call (41.2 us when every quad of pixels ran five bounding-circle tests).
 constexpr uint32_t kObsThreads = 256;
 constexpr uint32_t kObsTile = 16384;             // bytes of whole rows a block draws at once
 constexpr uint32_t kObsRecord = PUSHT_RECORD;    // float4 per environment: 24 floats, five ranges
@@ -345,8 +345,8 @@ void launch_pusht_obs(const float4* posLin, const float4* posAng, const PushTDev
                       uint32_t res, float4* shapes, uint8_t* out, cudaStream_t st) {
     if (!numEnvs) return;
     k_pusht_shapes<<<blocks_for(numEnvs, 64), 64, 0, st>>>(posLin, posAng, envs, numEnvs, res, shapes);
-    // one resident wave of blocks walks the tiles (about 17 KB of shared
-    // memory and 256 threads each: eight blocks an SM)
+    // two waves of blocks walk the tiles (256 threads of 64 registers: four
+    // blocks an SM at a time)
     const uint32_t rows = obs_rows(res);
     const uint64_t tiles = (uint64_t)numEnvs * ((res + rows - 1u) / rows);
     const uint32_t grid = (uint32_t)(tiles < 148u * 8u ? tiles : 148u * 8u);
