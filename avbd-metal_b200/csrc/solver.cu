@@ -449,7 +449,8 @@ __device__ __forceinline__ void color_place(const DevPtrs& d, uint32_t gid, cons
 
 constexpr int kColorPasses = 20;
 constexpr int kColorLaunched = 8;                 // passes launched over the whole device
-constexpr uint32_t kColorCluster = 10240;         // bodies up to which a cluster does everything
+constexpr uint32_t kColorCluster = 10240;         // bodies up to which a cluster does everything,
+constexpr uint32_t kColorLater = 32768;           // and up to which it does the passes not launched
 
 // The whole coloring in one launch of a cluster (one CTA for small scenes):
 // passes between barriers until one changes nothing, usually the first or
@@ -459,7 +460,9 @@ constexpr uint32_t kColorCluster = 10240;         // bodies up to which a cluste
 // is four to ten passes, and a cluster's pass grows with the bodies: above
 // kColorCluster the first kColorLaunched passes and the rest use the whole
 // device, a launch each, and the cluster only goes on with later passes and the
-// repair (`from` > 0, `all` = false).  Coloring stage, median of 60 frames,
+// repair (`from` > 0, `all` = false).  Above kColorLater, where a pass of the
+// cluster would cost as much as a dozen idle launches, every pass is launched
+// (83 / 94 us at 40,000 / 60,000 shapes instead of 72 / 82).  Coloring stage, median of 60 frames,
 // cluster / launches (24 launches): tumbling shapes 5,000 39 / 47 us (66), 8,000
 // 45 / 51 (68), 12,000 64 / 53 (74), 28,000 111 / 61 (72), 60,000 217 / 82 (98);
 // settled worlds of 8,398 bodies 25 / 27 (47), 16,739 35 / 31 (51), 28,626
@@ -546,12 +549,13 @@ void launch_dynamic_coloring(const Params& P, const DevPtrs& d, const Sizes& z, 
         return;
     }
     const uint32_t T = 128, blocks = (P.numBodies + T - 1) / T;
-    for (int pass = 0; pass < kColorLaunched; pass++) {
+    const int launched = P.numBodies <= kColorLater ? kColorLaunched : kColorPasses;
+    for (int pass = 0; pass < launched; pass++) {
         const uint32_t* src = (pass & 1) ? d.colorsB : d.colorsA;
         uint32_t* dst = (pass & 1) ? d.colorsA : d.colorsB;
         launch_pdl(k_color_iterate, blocks, T, st, P, d, src, dst, (uint32_t)pass);
     }
-    launch_cluster(k_color<true>, 8, 1024, 0, st, P, d, kColorLaunched, false);
+    launch_cluster(k_color<true>, 8, 1024, 0, st, P, d, launched, false);
     launch_pdl(k_color_validate_count, blocks, T, st, P, d, (const uint32_t*)d.colorsA);
     launch_pdl(k_color_scan, 1, 32, st, d);
     launch_pdl(k_color_scatter, blocks, T, st, P, d, (const uint32_t*)d.colorsA);

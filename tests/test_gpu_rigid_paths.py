@@ -54,12 +54,13 @@ def test_coloring_sizes(cuda_lib, oracle_lib, count):
     _run(pile(count), oracle_lib, 12, every=6)
 
 
-@pytest.mark.parametrize("count,length", [(10239, 12), (10240, 12), (10240, 40)])
+@pytest.mark.parametrize("count,length", [(10239, 12), (10240, 12), (10240, 40), (32768, 40)])
 def test_coloring_passes(cuda_lib, oracle_lib, count, length):
     """Rows of touching boxes, all of one color at first: a pass settles one box
     of each row.  With the ground, 10,239 boxes are the last scene of the eight-CTA
     cluster; above it the passes are launched, rows of 12 settle in the passes that
-    follow the launched eight, and rows of 40 only in the repair."""
+    follow the launched eight, and rows of 40 only in the repair.  Above 32,767
+    boxes all twenty passes are launched."""
     s = PhysicsScene("rows")
     demos.add_ground(s, friction=0.6)
     for k in range(count):
