@@ -462,11 +462,11 @@ constexpr uint32_t kColorLater = 32768;           // and up to which it does the
 // device, a launch each, and the cluster only goes on with later passes and the
 // repair (`from` > 0, `all` = false).  Above kColorLater, where a pass of the
 // cluster would cost as much as a dozen idle launches, every pass is launched
-// (83 / 94 us at 40,000 / 60,000 shapes instead of 72 / 82).  Coloring stage, median of 60 frames,
-// cluster / launches (24 launches): tumbling shapes 5,000 39 / 47 us (66), 8,000
-// 45 / 51 (68), 12,000 64 / 53 (74), 28,000 111 / 61 (72), 60,000 217 / 82 (98);
-// settled worlds of 8,398 bodies 25 / 27 (47), 16,739 35 / 31 (51), 28,626
-// 45 / 35 (55).
+// (83 / 94 us at 40,000 / 60,000 shapes instead of 72 / 82).  Coloring stage,
+// median of 60 frames, cluster / eight launched passes (24 launches): tumbling
+// shapes 5,000 39 / 47 us (66), 8,000 45 / 51 (68), 12,000 64 / 53 (74), 28,000
+// 111 / 61 (72), 60,000 217 / 82 (98); settled worlds of 8,398 bodies 25 / 27
+// (47), 16,739 35 / 31 (51), 28,626 45 / 35 (55).
 template <bool CLUSTER>
 __global__ void __launch_bounds__(1024) k_color(const Params P, const DevPtrs d, int from, bool all) {
     pdl_prologue();
@@ -1157,7 +1157,9 @@ __device__ __forceinline__ void primal_body(const Params& P, const DevPtrs& d, u
 constexpr int kPrimalThreads = 128;         // most threads of a k_primal block
 constexpr uint64_t kTailWaitNs = 1000000000ull;   // a wait gives up after one second
 
-// true once `finished` has reached `target`; false (and the failure latched) when it does not
+// true once `finished` has reached `target`; false when it does not within the
+// limit (the failure is latched, unless another one already is) or a wait has
+// given up before
 __device__ __forceinline__ bool tail_wait(const DevPtrs& d, const volatile uint32_t* finished, uint32_t target) {
     const volatile uint32_t* failed = d.failureLatch;
     uint64_t t0 = 0;
@@ -1166,7 +1168,10 @@ __device__ __forceinline__ bool tail_wait(const DevPtrs& d, const volatile uint3
         uint64_t t;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
         if (t0 == 0) t0 = t;
-        if (t - t0 > kTailWaitNs) atomicCAS(d.failureLatch, 0u, AVBD_FAIL_WAIT_TIMEOUT_);
+        if (t - t0 > kTailWaitNs) {
+            atomicCAS(d.failureLatch, 0u, AVBD_FAIL_WAIT_TIMEOUT_);
+            return false;
+        }
         if (*failed == AVBD_FAIL_WAIT_TIMEOUT_) return false;
     }
     return true;
@@ -1186,6 +1191,7 @@ __global__ void __launch_bounds__(kPrimalThreads, 4) k_primal(const Params P, co
     // the group)
     uint32_t slot = d.colorStart[color] + (tid >> 3), end = d.colorStart[color + 1], step = groups * gridDim.x;
     uint32_t c = color, before = 0;              // chunks of the colors color .. c - 1
+    bool waits = true;                           // thread 0: no wait of this block has given up
     for (;;) {
         if (tail) {
             if (threadIdx.x == 0) ticket = atomicAdd(d.tail, 1u);
@@ -1197,7 +1203,7 @@ __global__ void __launch_bounds__(kPrimalThreads, 4) k_primal(const Params P, co
             }
             if (c == used) break;
             if (before && threadIdx.x == 0) {
-                tail_wait(d, d.tail + 1, before);
+                waits = waits && tail_wait(d, d.tail + 1, before);
                 __threadfence();
             }
             __syncthreads();
